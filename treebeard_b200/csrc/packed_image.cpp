@@ -118,6 +118,20 @@ void put_image(const PackedImage &im, Out &o) {
     o.vec(q.scale);
     o.pod(q.num_classes);
     o.vec(q.group_class);
+  } else if (im.kind == PackedImage::kRank) {
+    const RankForest &q = im.rf;
+    put_key_forest_head(o, q.num_features, q.transform, q.initial_value, q.num_trees, q.num_nodes, q.max_depth);
+    o.pod(q.num_classes);
+    o.pod(q.whole_compare);
+    o.vec(q.groups);
+    o.vec(q.node_plane);
+    o.vec(q.leaf_plane);
+    o.vec(q.orig_leaf);
+    o.vec(q.tree_index);
+    o.vec(q.class_begin);
+    o.vec(q.features);
+    o.vec(q.lut);
+    o.vec(q.thresholds);
   } else {
     const DeepForest &q = im.df;
     put_key_forest_head(o, q.num_features, q.transform, q.initial_value, q.num_trees, q.num_nodes, q.max_depth);
@@ -227,6 +241,34 @@ std::string deserialize_image(const uint8_t *data, uint64_t size, PackedImage *i
     for (const QuantGroup &g : q.groups)
       if (in.ok && (g.depth < 1 || g.depth > (uint32_t)kQuantMaxDepth || g.slots != (1u << g.depth) ||
                     g.elem_off + (uint64_t)g.slots * kQuantCols > n))
+        in.ok = false;
+  } else if (im->kind == PackedImage::kRank) {
+    RankForest &q = im->rf;
+    key_head(&q.num_features, &q.transform, &q.initial_value, &q.num_trees, &q.num_nodes, &q.max_depth);
+    q.num_classes = in.pod<int32_t>();
+    q.whole_compare = in.pod<int32_t>();
+    in.vec(&q.groups);
+    in.vec(&q.node_plane);
+    in.vec(&q.leaf_plane);
+    in.vec(&q.orig_leaf);
+    in.vec(&q.tree_index);
+    in.vec(&q.class_begin);
+    in.vec(&q.features);
+    in.vec(&q.lut);
+    in.vec(&q.thresholds);
+    const size_t n = q.node_plane.size(), columns = q.groups.size() * kRankCols;
+    if (in.ok && (q.leaf_plane.size() != n || q.orig_leaf.size() != n || q.tree_index.size() != columns ||
+                  q.features.size() != (size_t)q.num_features || q.num_features > kRankMaxFeatures || q.max_depth > kRankMaxDepth ||
+                  q.num_classes < 0 || q.class_begin.size() != (q.num_classes > 0 ? (size_t)q.num_classes + 1 : 0)))
+      in.ok = false;
+    for (size_t c = 0; in.ok && c < q.class_begin.size(); ++c)
+      if (q.class_begin[c] < (c ? q.class_begin[c - 1] : 0) || (size_t)q.class_begin[c] > columns) in.ok = false;
+    for (const RankFeature &rf : q.features)
+      if (in.ok && (rf.buckets < 1 || (uint64_t)rf.lut_off + rf.buckets + 1 > q.lut.size() || (uint64_t)rf.thr_off + rf.n > q.thresholds.size()))
+        in.ok = false;
+    for (const QuantGroup &g : q.groups)
+      if (in.ok && (g.depth < 1 || g.depth > (uint32_t)q.max_depth || g.slots != (1u << g.depth) ||
+                    g.elem_off + (uint64_t)g.slots * kRankCols > n))
         in.ok = false;
   } else if (im->kind == PackedImage::kDeep) {
     DeepForest &q = im->df;

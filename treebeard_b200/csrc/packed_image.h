@@ -1,6 +1,6 @@
 // A packed forest as it lies in host memory just before the upload: the layout that was
-// chosen for it (general tiles / 16-bit keys for wide rows / one tree per stage for deep
-// trees) and that layout's buffers.  It can be serialised, which is what a compiled-model
+// chosen for it (general tiles / rank keys for narrow rows / 16-bit keys for wide rows / one tree
+// per stage for deep trees) and that layout's buffers.  It can be serialised, which is what a compiled-model
 // file caches so that loading it skips the packer -- the counterpart of the buffers the
 // reference's serializer writes next to a compiled module and reloads
 // (src/utils/TreeTilingUtils.cpp:95-170, src/runtime/runtime.cpp:35-54).
@@ -9,6 +9,7 @@
 #include "deep_pack.h"
 #include "pack.h"
 #include "quant_pack.h"
+#include "rank_pack.h"
 
 #include <cstdint>
 #include <string>
@@ -17,7 +18,7 @@
 namespace tb {
 
 struct PackedImage {
-  enum Kind : int32_t { kGeneral = 0, kQuant = 1, kDeep = 2 };
+  enum Kind : int32_t { kGeneral = 0, kQuant = 1, kDeep = 2, kRank = 3 };
   int32_t kind = kGeneral;
   // what was asked for (the key under which a cached image may be reused) ...
   int32_t requested_representation = 0, requested_tile_size = 1, requested_feature_bits = 0;
@@ -28,9 +29,10 @@ struct PackedImage {
   PackedForest packed; // kGeneral
   QuantForest qf;      // kQuant
   DeepForest df;       // kDeep
+  RankForest rf;       // kRank
 };
 
-constexpr uint32_t kPackedImageVersion = 6; // changes whenever a packer's output does
+constexpr uint32_t kPackedImageVersion = 7; // changes whenever a packer's output does
 
 void serialize_image(const PackedImage &im, std::vector<uint8_t> *out);
 uint64_t serialized_image_size(const PackedImage &im); // without serialising

@@ -1,0 +1,226 @@
+#include "rank_pack.h"
+
+#include <algorithm>
+#include <atomic>
+#include <numeric>
+
+namespace tb {
+
+namespace {
+
+// Bucket of a value in [lo, hi]; the device computes the same two roundings.
+uint32_t bucket_of(const RankFeature &f, float x) {
+  const float d = x - f.lo;
+  const float y = d * f.scale;
+  return std::min((uint32_t)y, f.buckets - 1);
+}
+
+// The bucket table of one feature whose sorted distinct thresholds are t[0..n).
+void fill_table(RankFeature *f, const float *t, uint16_t *lut) {
+  for (uint32_t b = 0; b <= f->buckets; ++b) lut[b] = 0;
+  for (uint32_t i = 0; i < f->n; ++i) ++lut[bucket_of(*f, t[i]) + 1];
+  for (uint32_t b = 1; b <= f->buckets; ++b) lut[b] = (uint16_t)(lut[b] + lut[b - 1]);
+}
+
+} // namespace
+
+std::string pack_rank(const Forest &f, RankForest *out) {
+  const int64_t T = f.num_trees(), N = f.num_nodes();
+  const int F = f.num_features;
+  if (F > kRankMaxFeatures) return "more than " + std::to_string(kRankMaxFeatures) + " features";
+  RankForest &q = *out;
+  q = RankForest();
+  q.num_features = F;
+  q.transform = f.transform;
+  q.num_classes = f.num_classes;
+  q.initial_value = f.initial_value;
+  q.num_trees = T;
+  q.num_nodes = N;
+
+  // ---- distinct thresholds per feature, and every split's rank among them
+  std::vector<int64_t> first(F + 1, 0);
+  bool finite = true;
+  for (int64_t g = 0; g < N; ++g) {
+    finite &= std::isfinite(f.thr[g]);
+    if (!f.is_leaf(g)) ++first[f.feat[g] + 1];
+  }
+  if (!finite) return "non-finite threshold or leaf value";
+  for (int i = 0; i < F; ++i) first[i + 1] += first[i];
+  std::vector<std::pair<float, int32_t>> split(first[F]); // (threshold, node) by feature
+  if (N > INT32_MAX) return "more than 2^31 nodes";
+  {
+    std::vector<int64_t> at(first.begin(), first.end() - 1);
+    for (int64_t g = 0; g < N; ++g)
+      if (!f.is_leaf(g)) split[at[f.feat[g]]++] = {f.thr[g], (int32_t)g};
+  }
+  std::vector<uint16_t> rank(N, 0);
+  std::vector<std::vector<float>> distinct(F);
+  std::atomic<uint32_t> most{0};
+#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads())
+  for (int i = 0; i < F; ++i) {
+    std::sort(split.begin() + first[i], split.begin() + first[i + 1]);
+    auto &d = distinct[i];
+    for (int64_t k = first[i]; k < first[i + 1]; ++k) {
+      if (d.empty() || d.back() != split[k].first) d.push_back(split[k].first);
+      rank[split[k].second] = (uint16_t)std::min<size_t>(d.size(), kRankMax + 1);
+    }
+    uint32_t seen = most.load();
+    while (d.size() > seen && !most.compare_exchange_weak(seen, (uint32_t)d.size())) {}
+  }
+  if (most > kRankMax) return "a feature has more than " + std::to_string(kRankMax) + " distinct thresholds";
+  q.whole_compare = most > kRankHalfMax;
+
+  // ---- rank tables
+  q.features.resize(F);
+  uint32_t lut_size = 0, thr_size = 0;
+  for (int i = 0; i < F; ++i) {
+    const auto &d = distinct[i];
+    RankFeature &rf = q.features[i];
+    rf = RankFeature{0.f, -1.f, 0.f, 1, lut_size, thr_size, (uint32_t)d.size(), 0};
+    if (!d.empty()) {
+      rf.lo = d.front();
+      rf.hi = d.back();
+      bool whole = std::fabs(rf.lo) <= 0x1p22f && std::fabs(rf.hi) <= 0x1p22f && rf.hi - rf.lo <= std::max(4096.f, 4.f * (float)d.size());
+      for (size_t k = 0; k < d.size() && whole; ++k) whole = d[k] == std::floor(d[k]);
+      if (whole) {
+        rf.lattice = 1;
+        rf.buckets = (uint32_t)(rf.hi - rf.lo) + 1;
+        rf.scale = 1.f;
+      } else {
+        // half a bucket per threshold: the table stays small beside the thresholds, and two or
+        // three steps of the search finish a bucket
+        rf.buckets = std::max<uint32_t>(1, ((uint32_t)d.size() + 1) / 2);
+        const float range = rf.hi - rf.lo;
+        rf.scale = range > 0.f && std::isfinite(range) ? (float)rf.buckets / range : 0.f;
+        if (!std::isfinite(rf.scale) || rf.scale == 0.f) { // a range that fp32 cannot cut up: one bucket
+          rf.scale = 0.f;
+          rf.buckets = 1;
+        }
+      }
+    }
+    lut_size += (rf.buckets + 1 + 7) / 8 * 8; // (tables start on 16-byte boundaries)
+    thr_size += ((uint32_t)d.size() + 3) / 4 * 4;
+  }
+  q.lut.assign(lut_size, 0);
+  q.thresholds.assign(thr_size, 0.f);
+#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads())
+  for (int i = 0; i < F; ++i) {
+    RankFeature &rf = q.features[i];
+    std::copy(distinct[i].begin(), distinct[i].end(), q.thresholds.begin() + rf.thr_off);
+    fill_table(&rf, distinct[i].data(), q.lut.data() + rf.lut_off);
+  }
+
+  // ---- columns: trees by (class,) depth
+  std::vector<int32_t> depth(T);
+  int32_t deepest = 0;
+#pragma omp parallel for schedule(dynamic, 64) reduction(max : deepest) num_threads(pack_threads())
+  for (int64_t t = 0; t < T; ++t) {
+    depth[t] = tree_depth(f, t);
+    deepest = std::max(deepest, depth[t]);
+  }
+  q.max_depth = std::max(1, deepest);
+  if (deepest > kRankMaxDepth) return "trees deeper than " + std::to_string(kRankMaxDepth) + " levels";
+  std::vector<int64_t> order(T);
+  std::iota(order.begin(), order.end(), 0);
+  const bool multi = f.num_classes > 0;
+  std::stable_sort(order.begin(), order.end(), [&](int64_t a, int64_t b) {
+    if (multi && f.class_id[a] != f.class_id[b]) return f.class_id[a] < f.class_id[b];
+    return depth[a] < depth[b];
+  });
+  if (multi) {
+    q.class_begin.assign(f.num_classes + 1, 0);
+    for (int64_t t = 0; t < T; ++t) ++q.class_begin[f.class_id[t] + 1];
+    for (int32_t c = 0; c < f.num_classes; ++c) q.class_begin[c + 1] += q.class_begin[c];
+  }
+  const int64_t G = (T + kRankCols - 1) / kRankCols;
+  q.groups.resize(G);
+  q.tree_index.assign(G * kRankCols, -1);
+  uint64_t elems = 0;
+  for (int64_t g = 0; g < G; ++g) {
+    uint32_t d = 1;
+    for (int64_t k = g * kRankCols; k < std::min(T, (g + 1) * kRankCols); ++k) d = std::max<uint32_t>(d, depth[order[k]]);
+    q.groups[g] = QuantGroup{elems, d, 1u << d};
+    elems += (uint64_t)(1u << d) * kRankCols;
+  }
+  const uint32_t always_left = q.whole_compare ? 0xffffu : kRankHalfMax + 1;
+  q.node_plane.assign(elems, always_left);
+  q.leaf_plane.assign(elems, 0.f);
+  q.orig_leaf.assign(elems, -1);
+#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads())
+  for (int64_t g = 0; g < G; ++g) {
+    const QuantGroup &gm = q.groups[g];
+    struct Item { int32_t node; uint32_t path, level; };
+    std::vector<Item> stack;
+    for (int c = 0; c < kRankCols && g * kRankCols + c < T; ++c) {
+      const int64_t t = order[g * kRankCols + c], a = f.tree_off[t];
+      q.tree_index[g * kRankCols + c] = (int32_t)t;
+      stack.assign(1, Item{0, 0, 0});
+      while (!stack.empty()) {
+        const Item it = stack.back();
+        stack.pop_back();
+        const int64_t n = a + it.node;
+        if (f.left[n] < 0) { // all-left from here on
+          const uint64_t e = gm.elem_off + (uint64_t)it.path * kRankCols + c;
+          q.leaf_plane[e] = f.thr[n];
+          q.orig_leaf[e] = it.node;
+          continue;
+        }
+        const uint64_t e = gm.elem_off + (uint64_t)((1u << it.level) - 1 + it.path) * kRankCols + c;
+        q.node_plane[e] = ((uint32_t)f.feat[n] * 2u << 16) | rank[n];
+        stack.push_back({f.left[n], it.path, it.level + 1});
+        stack.push_back({f.right[n], it.path | (1u << it.level), it.level + 1});
+      }
+    }
+  }
+  return "";
+}
+
+uint32_t rank_of(const RankForest &q, int32_t feature, float x, bool *searched) {
+  const RankFeature &f = q.features[feature];
+  *searched = false;
+  if (f.n == 0 || x < f.lo) return 0;
+  if (!(x < f.hi)) return f.n;
+  const uint32_t b = bucket_of(f, x);
+  uint32_t s = q.lut[f.lut_off + b], e = q.lut[f.lut_off + b + 1];
+  if (f.lattice && x == std::floor(x)) return e;
+  *searched = s < e;
+  while (s < e) {
+    const uint32_t m = (s + e) >> 1;
+    if (x < q.thresholds[f.thr_off + m]) e = m;
+    else s = m + 1;
+  }
+  return s;
+}
+
+void walk_rank_on_host(const RankForest &q, const float *rows, int64_t n_rows, int64_t ld, int32_t *leaf_ids, float *sums,
+                       int64_t *searched) {
+  const int C = std::max(1, q.num_classes);
+  std::vector<uint32_t> key(q.num_features + 1, 0);
+  int64_t count = 0;
+  for (int64_t r = 0; r < n_rows; ++r) {
+    for (int i = 0; i < q.num_features; ++i) {
+      bool s;
+      key[i] = rank_of(q, i, rows[r * ld + i], &s);
+      count += s;
+    }
+    if (sums) std::fill(sums + r * C, sums + (r + 1) * C, 0.f);
+    int32_t cls = 0;
+    for (size_t k = 0; k < q.tree_index.size(); ++k) {
+      if (q.tree_index[k] < 0) continue;
+      const QuantGroup &gm = q.groups[k / kRankCols];
+      const uint64_t base = gm.elem_off + k % kRankCols;
+      uint32_t path = 0;
+      for (uint32_t d = 0; d < gm.depth; ++d) {
+        const uint32_t node = q.node_plane[base + (uint64_t)((1u << d) - 1 + path) * kRankCols];
+        if (key[(node >> 16) / 2] >= (node & 0xffffu)) path |= 1u << d;
+      }
+      const uint64_t e = base + (uint64_t)path * kRankCols;
+      while (q.num_classes > 0 && (int32_t)k >= q.class_begin[cls + 1]) ++cls;
+      if (sums) sums[r * C + cls] += q.leaf_plane[e];
+      if (leaf_ids) leaf_ids[r * q.num_trees + q.tree_index[k]] = q.orig_leaf[e];
+    }
+  }
+  if (searched) *searched = count;
+}
+
+} // namespace tb

@@ -1,0 +1,83 @@
+// "Rank keys": the packed layout for forests of at most 8 levels over rows that are narrow
+// enough for the rank kernels (walk_rank.cuh).
+//
+// A threshold is compared with one feature only, so all that a walk needs to know of a row value
+// x is its RANK among the feature's distinct thresholds t_0 < t_1 < ...:
+//     rank(x) = number of thresholds with !(x < t)          (NaN: all of them)
+//     x < t_j  <=>  rank(x) < j + 1
+// A row is ranked once per batch (tb_rank_rows); from then on a decision is ONE comparison of
+// 16-bit whole numbers that is never in doubt -- there are no ties to flag and to walk again, as
+// there are with the rounded keys of quant_pack.h.
+//
+// Ranking uses a table per feature: the range of its thresholds is cut into equal buckets,
+// lut[b] = thresholds in the buckets before b, and the thresholds of the value's own bucket are
+// searched.  Bucket numbers are computed with one subtraction and one multiplication, both
+// monotone, on the host and on the device alike, so a bucket separates values exactly.  A
+// LATTICE feature (whole-number thresholds close together) has one bucket per whole number; a
+// whole-number row value is ranked by the table alone.
+//
+// Planes, per group of 32 trees of (padded) depth D, 2^D slots x 32 columns each:
+//   node plane  u32  (key offset << 16) | (j + 1); the offset is the byte offset of the
+//                    feature's key in a row of keys
+//   leaf plane  f32  leaf values
+// Slots: node on level d reached by the decisions r_0 .. r_(d-1) (1 = right) is slot
+// 2^d - 1 + sum r_i 2^i, leaf sum r_i 2^i.  With the decision of level i worth 2^i slots on EVERY
+// level below, a walk keeps one offset that a right turn adds 2^i * 128 bytes to, and the start of
+// a level is an immediate of the load: a comparison and a predicated addition advance the walk.
+// A leaf above the bottom level fills the all-left path below it with nodes that always go left
+// (key offset 0, threshold rank kRankAlwaysLeft).
+//
+// Columns are trees ordered by depth; for a multiclass forest by (class, depth) WITHOUT padding
+// the classes to whole groups: class c owns the columns class_begin[c] .. class_begin[c+1] - 1.
+#pragma once
+#include "forest.h"
+#include "quant_pack.h"
+
+namespace tb {
+
+constexpr int kRankCols = 32, kRankMaxDepth = 8;
+// A forest all of whose ranks fit the positive half-precision numbers is compared by the half2
+// comparison, which needs no masking (one instruction per decision less than whole numbers).
+constexpr uint32_t kRankHalfMax = 31742, kRankMax = 65534;
+constexpr int kRankMaxFeatures = 64; // 16-bit keys of a row in 32 four-byte words: one bank each
+
+struct RankFeature { // 32 bytes, the same on the device
+  float lo, hi;      // smallest and largest threshold (lo > hi: the feature is not used)
+  float scale;       // buckets per unit
+  uint32_t buckets;
+  uint32_t lut_off;  // first of buckets + 1 entries
+  uint32_t thr_off;  // first of n thresholds
+  uint32_t n;
+  uint32_t lattice;
+};
+
+struct RankForest {
+  int32_t num_features = 0, transform = 0, num_classes = 0;
+  double initial_value = 0.0;
+  int64_t num_trees = 0, num_nodes = 0;
+  int32_t max_depth = 0;   // at least 1
+  int32_t whole_compare = 0; // some rank exceeds kRankHalfMax: compare as whole numbers
+  std::vector<QuantGroup> groups; // elem_off in elements of either plane
+  std::vector<uint32_t> node_plane;
+  std::vector<float> leaf_plane;
+  std::vector<int32_t> orig_leaf;   // original node id per leaf-plane element
+  std::vector<int32_t> tree_index;  // [groups*32] original tree index, -1 = filler
+  std::vector<int32_t> class_begin; // multiclass: [num_classes + 1] first column of every class
+  std::vector<RankFeature> features;
+  std::vector<uint16_t> lut;
+  std::vector<float> thresholds;
+};
+
+// Empty string on success; fails (so that the caller can take another layout) for trees deeper
+// than 8 levels, more than kRankMaxFeatures features, non-finite thresholds or leaves, or a
+// feature with more than kRankMax distinct thresholds.
+std::string pack_rank(const Forest &f, RankForest *out);
+
+// Rank of a row value; *searched: the value's bucket held thresholds it was compared with.
+uint32_t rank_of(const RankForest &q, int32_t feature, float x, bool *searched);
+
+// Host interpreter of the packed planes (layout verification only).
+void walk_rank_on_host(const RankForest &q, const float *rows, int64_t n_rows, int64_t ld, int32_t *leaf_ids, float *sums,
+                       int64_t *searched);
+
+} // namespace tb

@@ -3,18 +3,22 @@
 #include "../../include/tbk.h"
 #include "pack.h"
 #include "quant_pack.h"
+#include "rank_pack.h"
 #include "deep_pack.h"
 #include "schedule.h"
 #include "walk_kernels.cuh"
 #include "walk_quant.cuh"
 #include "walk_quant_batch.cuh"
 #include "walk_deep.cuh"
+#include "rank_rows.cuh"
+#include "walk_rank.cuh"
 #include "packed_image.h"
 
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <list>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -81,6 +85,28 @@ struct tbk_forest {
   int32_t *d_qset_groups = nullptr, *d_qgroup_class = nullptr; // multiclass key layout
   int32_t qset_count[2] = {0, 0};
   unsigned long long *d_ties = nullptr;
+  // rank keys (narrow rows)
+  bool rank = false;
+  tb::RankForest rf;
+  uint32_t *d_rnode = nullptr;
+  float *d_rleaf = nullptr, *d_rthr = nullptr;
+  int32_t *d_rorig = nullptr, *d_rtree_index = nullptr, *d_rclass_begin = nullptr;
+  tb::DevQuantGroup *d_rgroups = nullptr;
+  tb::DevRankFeature *d_rfeatures = nullptr;
+  uint16_t *d_rlut = nullptr;
+  int rank_width = 0, rank_pieces = 1, rank_smem = 0; // the ranking kernel's tables (plan_rank_tables)
+  struct Workspace {
+    unsigned char *mem = nullptr;
+    size_t bytes = 0;
+    cudaStream_t stream = nullptr;
+    bool used = false;
+    cudaEvent_t done = nullptr;
+  };
+  static constexpr int kWorkspaces = 4;
+  Workspace workspace[kWorkspaces];
+  int next_victim = 0;
+  std::list<Workspace> captured; // of calls that were captured into graphs
+  std::vector<const void *> smem_allowed;
   // one-tree-per-stage layout (deep trees); shares the device buffers of the key layout
   bool deep = false;
   tb::DeepForest df;
@@ -455,6 +481,299 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   return TBK_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Rank keys (rank_pack.h)
+
+// Device memory that a call needs from its first kernel to its last: the keys of the rows and
+// the partial sums of tree chunks.  Calls on one stream are ordered and share one workspace; a call
+// on a further stream gets one of its own, up to four, and after that waits on the device for the
+// previous user of the one that it takes over.
+int workspace_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_forest::Workspace **out) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) {
+    // a captured graph may be replayed at any time: its memory is its own for the forest's life
+    f->captured.emplace_back();
+    tbk_forest::Workspace *w = &f->captured.back();
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    cudaError_t e = cudaMalloc(&w->mem, bytes);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w->mem, 0, tb::kRankArrivalBytes, stream);
+    if (e != cudaSuccess) return fail(TBK_ERR_CUDA, "workspace of a captured call: %s", cudaGetErrorString(e));
+    w->bytes = bytes;
+    *out = w;
+    return TBK_OK;
+  }
+  tbk_forest::Workspace *w = nullptr;
+  for (auto &c : f->workspace)
+    if (c.used && c.stream == stream) w = &c;
+  if (!w)
+    for (auto &c : f->workspace)
+      if (!c.used && (!w || c.bytes > w->bytes)) w = &c;
+  if (!w) {
+    w = &f->workspace[f->next_victim++ % tbk_forest::kWorkspaces];
+    CUDA_TRY(cudaStreamWaitEvent(stream, w->done, 0));
+  }
+  w->stream = stream;
+  w->used = true;
+  if (w->bytes < bytes) {
+    if (w->mem) CUDA_TRY(cudaFree(w->mem)); // (waits for the work that uses it)
+    w->mem = nullptr;
+    w->bytes = 0;
+    CUDA_TRY(cudaMalloc(&w->mem, bytes));
+    w->bytes = bytes;
+    CUDA_TRY(cudaMemsetAsync(w->mem, 0, tb::kRankArrivalBytes, stream));
+  }
+  if (!w->done) CUDA_TRY(cudaEventCreateWithFlags(&w->done, cudaEventDisableTiming));
+  *out = w;
+  return TBK_OK;
+}
+
+// Dynamic shared memory beyond 48 KB has to be asked for once per kernel and device.
+int allow_smem(tbk_forest *f, const void *kernel) {
+  for (const void *k : f->smem_allowed)
+    if (k == kernel) return TBK_OK;
+  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f->max_smem_optin));
+  f->smem_allowed.push_back(kernel);
+  return TBK_OK;
+}
+
+int rank_stride(int num_features) { return num_features <= 32 ? 64 : 128; }
+
+using RankKernel = void (*)(const tb::RankWalkParams);
+template <int S, int R, bool WHOLE> RankKernel pick_rank(int mode) {
+  return mode == tb::kRankLeafIds ? tb::tb_walk_rank_kernel<S, R, WHOLE, tb::kRankLeafIds>
+         : mode == tb::kRankClasses ? tb::tb_walk_rank_kernel<S, R, WHOLE, tb::kRankClasses>
+                                    : tb::tb_walk_rank_kernel<S, R, WHOLE, tb::kRankSums>;
+}
+RankKernel pick_rank_kernel(int stride, int rows_per_warp, bool whole, int mode) {
+  if (stride == 64) {
+    if (rows_per_warp == 16) return whole ? pick_rank<64, 16, true>(mode) : pick_rank<64, 16, false>(mode);
+    return whole ? pick_rank<64, 4, true>(mode) : pick_rank<64, 4, false>(mode);
+  }
+  if (rows_per_warp == 16) return whole ? pick_rank<128, 16, true>(mode) : pick_rank<128, 16, false>(mode);
+  return whole ? pick_rank<128, 4, true>(mode) : pick_rank<128, 4, false>(mode);
+}
+
+struct RankPlan {
+  int rows_per_warp = 16, chunks = 1, per_chunk = 1; // per_chunk: groups, or classes of a multiclass forest
+  int stages = 2, smem = 0;
+  uint32_t stage_bytes = 0;
+  int64_t grid_x = 1;
+};
+
+// Launch shape of the walk over `n_rows` rows: rows per warp (16, or 4 for batches so small that
+// 16 would leave most warps idle) and tree chunks, by what the slowest block costs in clocks.  A
+// group takes a warp about 2 D - 1 shared-memory wavefronts per row, and the block at least what
+// its stage's copy takes (70 bytes a clock); a block starts up for about 4000 clocks, and
+// combining chunks adds about 1500.
+RankPlan plan_rank(const tbk_forest *f, int64_t n_rows, bool leaf_ids) {
+  const auto &q = f->rf;
+  const int G = (int)q.groups.size(), S = rank_stride(q.num_features);
+  const bool multi = q.num_classes > 0;
+  const int units = multi && !leaf_ids ? q.num_classes : G; // what chunks are made of
+  RankPlan best;
+  double best_cost = -1.0;
+  for (int R : {16, 4}) {
+    RankPlan p;
+    p.rows_per_warp = R;
+    p.stage_bytes = 256u << q.max_depth;
+    p.stages = std::min(tb::kRWMaxStages, (f->max_smem_optin - tb::rank_walk_smem_bytes(R, S, 0, 0)) / (int)p.stage_bytes);
+    p.smem = tb::rank_walk_smem_bytes(R, S, p.stages, p.stage_bytes);
+    const int64_t RB = tb::kRWWalkers * R, batches = (n_rows + RB - 1) / RB;
+    const double group = std::max(1.15 * RB * (2 * q.max_depth - 1), p.stage_bytes / 70.0);
+    const int most = f->user.tree_chunks > 0 ? f->user.tree_chunks : batches < f->num_sms ? 64 : 1;
+    for (int c = f->user.tree_chunks > 0 ? most : 1; c <= std::min(most, units) || c == 1; ++c) {
+      const int per = (units + c - 1) / c, chunks = (units + per - 1) / per;
+      const double groups = multi && !leaf_ids ? (double)G * per / units + (chunks > 1) : per;
+      const double waves = (double)((batches * chunks + f->num_sms - 1) / f->num_sms);
+      const double cost = waves * groups * group + (chunks > 1 ? waves * 4000.0 + 1500.0 : 4000.0);
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best = p;
+        best.chunks = chunks;
+        best.per_chunk = per;
+        best.grid_x = chunks > 1 ? batches : std::min<int64_t>(batches, f->num_sms);
+      }
+      if (f->user.tree_chunks > 0) break;
+    }
+  }
+  return best;
+}
+
+tb::LaunchPlan rank_launch_plan(const RankPlan &r) {
+  tb::LaunchPlan plan;
+  plan.row_warps = tb::kRWWalkers * r.rows_per_warp / 32;
+  plan.tree_threads = tb::kRWWalkers;
+  plan.rows_per_lane = 1;
+  plan.chunks = r.chunks;
+  plan.groups_per_chunk = r.per_chunk;
+  plan.staged = 1;
+  plan.cache_rows = 1;
+  plan.stage_bytes = r.stage_bytes;
+  plan.smem_bytes = r.smem;
+  plan.threads = tb::kRWThreads;
+  plan.grid_x = r.grid_x;
+  return plan;
+}
+
+// Rows per pass: the keys of a pass stay in L2 between the two kernels, and a pass of several
+// chunks has an arrival counter for every row batch.
+int64_t rank_rows_per_pass(const tbk_forest *f) {
+  const int64_t by_keys = ((int64_t)96 << 20) / rank_stride(f->rf.num_features);
+  const int64_t round = (int64_t)tb::kRWWalkers * 16 * f->num_sms;
+  return std::max(round, by_keys / round * round);
+}
+
+size_t rank_workspace_bytes(const tbk_forest *f, const RankPlan &plan, int64_t rows) {
+  size_t bytes = tb::kRankArrivalBytes + ((size_t)rows * rank_stride(f->rf.num_features) + 255) / 256 * 256;
+  if (plan.chunks > 1) bytes += (size_t)plan.chunks * rows * (f->rf.num_classes > 0 ? 8 : 4);
+  return bytes;
+}
+
+// The kernel that ranks `n` rows into `keys`.
+int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, uint16_t *keys, cudaStream_t stream) {
+  const auto &q = f->rf;
+  const int F = q.num_features;
+  tb::RankRowsParams p{};
+  p.rows = rows;
+  p.n_rows = n;
+  p.ld = ld;
+  p.features = f->d_rfeatures;
+  p.lut = f->d_rlut;
+  p.thr = f->d_rthr;
+  p.keys = keys;
+  p.num_features = F;
+  p.stride = rank_stride(F);
+  p.vec4_ok = F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
+  p.searched = f->d_ties;
+  // Tables in shared memory pay once every SM has a few thousand values to rank: loading them
+  // takes about as long as ranking 2000 values through L2 (a gather there costs a wavefront per lane).
+  if (f->rank_width > 0 && n * F > (int64_t)f->num_sms * 2048) {
+    const int w = f->rank_width, slabs = (F + w * f->rank_pieces - 1) / (w * f->rank_pieces);
+    p.pieces = f->rank_pieces;
+    const int64_t want = (n * p.pieces + 1023) / 1024;
+    const dim3 grid((unsigned)std::min<int64_t>(want, std::max(1, f->num_sms / slabs)), (unsigned)slabs);
+    using K = void (*)(const tb::RankRowsParams);
+    const K k = w == 8 ? tb::tb_rank_rows<8, true> : w == 4 ? tb::tb_rank_rows<4, true>
+                : w == 2 ? tb::tb_rank_rows<2, true> : tb::tb_rank_rows<1, true>;
+    const int rc = allow_smem(f, (const void *)k);
+    if (rc) return rc;
+    k<<<grid, 1024, f->rank_smem, stream>>>(p);
+  } else {
+    p.pieces = (F + 7) / 8;
+    const int64_t want = (n * p.pieces + 255) / 256;
+    tb::tb_rank_rows<8, false><<<(unsigned)std::min<int64_t>(want, 8ll * f->num_sms), 256, 0, stream>>>(p);
+  }
+  CUDA_TRY(cudaGetLastError());
+  ++f->launches;
+  return TBK_OK;
+}
+
+// How the ranking kernel's tables fit shared memory: the widest piece (features a thread ranks
+// together) and then the most pieces per block whose tables fit; rank_width 0: not even one feature's.
+void plan_rank_tables(tbk_forest *f) {
+  const auto &q = f->rf;
+  const int F = q.num_features, room = 200 * 1024;
+  auto bytes = [&](int first, int end) { // tables of the features [first, end)
+    size_t b = 0;
+    for (int i = first; i < end; ++i)
+      b += sizeof(tb::RankFeature) + (q.features[i].buckets + 1 + 7) / 8 * 16 + (q.features[i].n + 3) / 4 * 16;
+    return b;
+  };
+  f->rank_width = 0;
+  for (int w : {8, 4, 2, 1}) {
+    const int all = (F + w - 1) / w;
+    for (int pieces = w == 8 ? all : 1; pieces >= 1; --pieces) {
+      size_t most = 0;
+      for (int first = 0; first < F; first += w * pieces) most = std::max(most, bytes(first, std::min(F, first + w * pieces)));
+      if (most <= (size_t)room) {
+        f->rank_width = w;
+        f->rank_pieces = pieces;
+        f->rank_smem = (int)most;
+        return;
+      }
+    }
+  }
+}
+
+int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out, int32_t out_kind,
+             float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream) {
+  const auto &q = f->rf;
+  const int S = rank_stride(q.num_features), W = std::max(1, q.num_classes);
+  const int kmode = mode == kLeafIds ? tb::kRankLeafIds : q.num_classes > 0 ? tb::kRankClasses : tb::kRankSums;
+  int64_t pass = std::min(n_rows, rank_rows_per_pass(f));
+  RankPlan plan = plan_rank(f, pass, mode == kLeafIds);
+  if (plan.chunks > 1) {
+    pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * tb::kRWWalkers * plan.rows_per_warp);
+    plan = plan_rank(f, pass, mode == kLeafIds);
+  }
+  f->last_plan = rank_launch_plan(plan);
+  tbk_forest::Workspace *ws = nullptr;
+  int rc = workspace_acquire(f, stream, rank_workspace_bytes(f, plan, pass), &ws);
+  if (rc) return rc;
+  unsigned char *keys = ws->mem + tb::kRankArrivalBytes;
+  const RankKernel kernel = pick_rank_kernel(S, plan.rows_per_warp, q.whole_compare != 0, kmode);
+  rc = allow_smem(f, (const void *)kernel);
+  if (rc) return rc;
+  tb::RankWalkParams p{};
+  p.node_plane = f->d_rnode;
+  p.leaf_plane = reinterpret_cast<const uint32_t *>(f->d_rleaf);
+  if (mode == kLeafIds) p.leaf_plane = reinterpret_cast<const uint32_t *>(f->d_rorig);
+  p.groups = f->d_rgroups;
+  p.tree_index = f->d_rtree_index;
+  p.class_begin = f->d_rclass_begin;
+  p.keys = keys;
+  p.scratch = reinterpret_cast<float *>(keys + ((size_t)pass * S + 255) / 256 * 256);
+  p.arrivals = reinterpret_cast<unsigned int *>(ws->mem);
+  p.num_trees = q.num_trees;
+  p.num_groups = (int32_t)q.groups.size();
+  p.groups_per_chunk = kmode == tb::kRankClasses ? 0 : plan.per_chunk;
+  p.num_classes = q.num_classes;
+  p.classes_per_chunk = kmode == tb::kRankClasses ? plan.per_chunk : 0;
+  p.write_partial = mode == kPartial ? 1 : 0;
+  p.out_kind = out_kind == TBK_OUT_I8 ? 1 : 0;
+  p.transform = q.transform;
+  p.initial_value = (float)q.initial_value;
+  p.stages = plan.stages;
+  p.stage_bytes = plan.stage_bytes;
+  p.status = f->d_status;
+  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
+  for (int64_t done = 0; done < n_rows; done += pass) {
+    const int64_t n = std::min(pass, n_rows - done);
+    rc = launch_rank_rows(f, d_rows + done * ld, n, ld, reinterpret_cast<uint16_t *>(keys), stream);
+    if (rc) return rc;
+    p.n_rows = n;
+    p.partial = d_partial ? d_partial + done * W : nullptr;
+    p.out = d_out ? static_cast<unsigned char *>(d_out) + done * (out_kind == TBK_OUT_I8 ? 1 : 4) : nullptr;
+    p.leaf_ids = d_leaf_ids ? d_leaf_ids + done * q.num_trees : nullptr;
+    p.skip_first_copy = f->expire_next_wait ? 1 : 0;
+    p.wait_tries = f->expire_next_wait ? 2000u : 0u;
+    f->expire_next_wait = false;
+    const int64_t batches = (n + tb::kRWWalkers * plan.rows_per_warp - 1) / (tb::kRWWalkers * plan.rows_per_warp);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)std::min(batches, plan.grid_x), (unsigned)plan.chunks);
+    cfg.blockDim = dim3(tb::kRWThreads);
+    cfg.dynamicSmemBytes = (size_t)plan.smem;
+    cfg.stream = stream;
+    // the walk starts its tree copies while the rows are still being ranked
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
+    ++f->launches;
+  }
+  if (f->timing) {
+    CUDA_TRY(cudaEventRecord(f->ev1, stream));
+    f->ev_pending = true;
+  }
+  if (ws->done) CUDA_TRY(cudaEventRecord(ws->done, stream));
+  return TBK_OK;
+}
+
 // One prediction over device-resident rows.
 int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
         int32_t out_kind, float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot = 0) {
@@ -468,6 +787,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
     if (out_kind != TBK_OUT_F32 && out_kind != TBK_OUT_I8) return fail(TBK_ERR_INVALID, "unknown output kind %d", out_kind);
   }
   CUDA_TRY(cudaSetDevice(f->device));
+  if (f->rank) return run_rank(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
   if (f->quant) return run_quant(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream, slot);
   if (f->deep) return run_deep(f, mode, d_rows, n_rows, ld, d_out, d_partial, d_leaf_ids, stream, slot);
 
@@ -710,6 +1030,16 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
                     (bits == 0 && (rep == TBK_REP_AUTO || rep == TBK_REP_REORG) && ts == 1 && !fp32_tile_fits &&
                      host.num_classes == 0) ||
                     (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && batch_fits && max_depth <= tb::kQuantMaxDepth);
+  // rank keys: whatever the batch kernel would take, over at most 64 features
+  if (want_quant && batch_fits && host.num_features <= tb::kRankMaxFeatures) {
+    if (tb::pack_rank(host, &im.rf).empty()) {
+      im.kind = tb::PackedImage::kRank;
+      im.user.representation = TBK_REP_REORG;
+      *out = img.release();
+      return TBK_OK;
+    }
+    im.rf = tb::RankForest(); // (a feature with too many distinct thresholds, for one)
+  }
   if (want_quant) {
     // narrow rows (batch kernel): features with whole-number thresholds become lattice features
     std::string qerr = tb::pack_quant(host, &im.qf, batch_fits);
@@ -893,6 +1223,61 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     *out = f;
     return TBK_OK;
   }
+  if (im.kind == tb::PackedImage::kRank) {
+    const auto &q = im.rf;
+    f->rank = true;
+    f->packed.representation = tb::kReorg;
+    f->packed.tile_size = 1;
+    f->packed.num_features = q.num_features;
+    f->packed.num_classes = q.num_classes;
+    f->packed.transform = q.transform;
+    f->packed.initial_value = q.initial_value;
+    f->packed.num_trees = q.num_trees;
+    f->packed.num_nodes = q.num_nodes;
+    f->packed.max_depth = q.max_depth;
+    static_assert(sizeof(tb::RankFeature) == sizeof(tb::DevRankFeature) && sizeof(tb::RankFeature) == 32, "rank table layout");
+    auto upload = [](auto **dst, const auto &v) { // (an empty vector gets a few bytes)
+      const size_t bytes = v.size() * sizeof(v[0]);
+      cudaError_t e = cudaMalloc(dst, std::max<size_t>(16, bytes));
+      if (e == cudaSuccess && bytes) e = cudaMemcpy((void *)*dst, v.data(), bytes, cudaMemcpyHostToDevice);
+      return e;
+    };
+    CUDA_TRY_F(upload(&f->d_rnode, q.node_plane));
+    CUDA_TRY_F(upload(&f->d_rleaf, q.leaf_plane));
+    CUDA_TRY_F(upload(&f->d_rorig, q.orig_leaf));
+    CUDA_TRY_F(upload(&f->d_rgroups, q.groups));
+    CUDA_TRY_F(upload(&f->d_rtree_index, q.tree_index));
+    CUDA_TRY_F(upload(&f->d_rclass_begin, q.class_begin));
+    CUDA_TRY_F(upload(&f->d_rfeatures, q.features));
+    CUDA_TRY_F(upload(&f->d_rlut, q.lut));
+    CUDA_TRY_F(upload(&f->d_rthr, q.thresholds));
+    CUDA_TRY_F(cudaMalloc(&f->d_ties, 128));
+    CUDA_TRY_F(cudaMemset(f->d_ties, 0, 128));
+    // of the host copy only the sizes and the feature table stay
+    f->rf.num_features = q.num_features;
+    f->rf.num_classes = q.num_classes;
+    f->rf.transform = q.transform;
+    f->rf.initial_value = q.initial_value;
+    f->rf.num_trees = q.num_trees;
+    f->rf.num_nodes = q.num_nodes;
+    f->rf.max_depth = q.max_depth;
+    f->rf.whole_compare = q.whole_compare;
+    f->rf.groups = q.groups;
+    f->rf.features = q.features;
+    plan_rank_tables(f);
+    const int64_t rows = std::min(batch_hint > 0 ? batch_hint : 65536, rank_rows_per_pass(f));
+    const RankPlan plan = plan_rank(f, rows, false);
+    f->last_plan = rank_launch_plan(plan);
+    if (batch_hint > 0) { // the batches to come are known: their workspace is laid out now
+      tbk_forest::Workspace &w = f->workspace[0];
+      const size_t bytes = rank_workspace_bytes(f, plan, rows);
+      CUDA_TRY_F(cudaMalloc(&w.mem, bytes));
+      CUDA_TRY_F(cudaMemset(w.mem, 0, tb::kRankArrivalBytes));
+      w.bytes = bytes;
+    }
+    *out = f;
+    return TBK_OK;
+  }
   if (im.kind == tb::PackedImage::kQuant) {
     f->qf = im.qf;
     const auto &q = f->qf;
@@ -999,6 +1384,14 @@ int tbk_forest_free(tbk_forest *f) {
   cudaFree(f->d_qlo);
   cudaFree(f->d_qscale);
   cudaFree(f->d_ties);
+  for (void *d : {(void *)f->d_rnode, (void *)f->d_rleaf, (void *)f->d_rorig, (void *)f->d_rgroups, (void *)f->d_rtree_index,
+                  (void *)f->d_rclass_begin, (void *)f->d_rfeatures, (void *)f->d_rlut, (void *)f->d_rthr})
+    cudaFree(d);
+  for (auto &w : f->workspace) {
+    cudaFree(w.mem);
+    if (w.done) cudaEventDestroy(w.done);
+  }
+  for (auto &w : f->captured) cudaFree(w.mem);
   for (int i = 0; i < 2; ++i)
     if (f->scratch_done[i]) cudaEventDestroy(f->scratch_done[i]);
   if (f->ev0) cudaEventDestroy(f->ev0);
@@ -1013,8 +1406,9 @@ int tbk_forest_get_info(const tbk_forest *f, tbk_forest_info *info) {
   const auto &p = f->packed;
   info->num_trees = p.num_trees;
   info->num_nodes = p.num_nodes;
-  info->num_groups = f->quant ? (int64_t)f->qf.groups.size() : f->deep ? (int64_t)f->df.pairs.size() : (int64_t)p.groups.size();
-  info->packed_bytes = f->deep ? (int64_t)(f->df.pairs.empty() ? 0 : 8 * (f->df.pairs.back().elem_off + 2ull * f->df.pairs.back().slots)) :
+  info->num_groups = f->rank ? (int64_t)f->rf.groups.size() : f->quant ? (int64_t)f->qf.groups.size() : f->deep ? (int64_t)f->df.pairs.size() : (int64_t)p.groups.size();
+  info->packed_bytes = f->rank ? (int64_t)(8 * (f->rf.groups.back().elem_off + (uint64_t)f->rf.groups.back().slots * tb::kRankCols)) :
+                       f->deep ? (int64_t)(f->df.pairs.empty() ? 0 : 8 * (f->df.pairs.back().elem_off + 2ull * f->df.pairs.back().slots)) :
                        f->quant ? (int64_t)(f->qf.groups.empty() ? 0 : 8 * (f->qf.groups.back().elem_off + (uint64_t)f->qf.groups.back().slots * tb::kQuantCols)) :
                        p.groups.empty() ? 0 : (int64_t)(p.groups.back().byte_off +
       (((uint64_t)p.groups.back().slots * tb::kGroupTrees * p.tile_bytes + 15) & ~15ull));
@@ -1031,12 +1425,13 @@ int tbk_forest_get_info(const tbk_forest *f, tbk_forest_info *info) {
   info->schedule.tree_threads = pl.tree_threads;
   info->schedule.tree_chunks = pl.chunks;
   info->schedule.cache_trees = pl.staged ? 1 : 2;
-  info->schedule.feature_bits = (f->quant || f->deep) ? 16 : 32;
+  info->schedule.feature_bits = (f->rank || f->quant || f->deep) ? 16 : 32;
   info->staged = pl.staged;
   info->smem_bytes = pl.smem_bytes;
   info->threads_per_block = pl.threads;
-  if ((f->quant || f->deep) && f->d_ties) {
-    // key ties resolved on exact values so far (statistics; synchronises with the device)
+  if (f->d_ties) {
+    // key ties resolved on exact values so far -- with rank keys, row values that had to be compared
+    // with thresholds (statistics; synchronises with the device)
     unsigned long long ties = 0;
     if (cudaMemcpy(&ties, f->d_ties, 8, cudaMemcpyDeviceToHost) == cudaSuccess) {
       info->reserved[0] = (int32_t)(ties & 0x7fffffff);
@@ -1242,7 +1637,7 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   if (!f) return fail(TBK_ERR_INVALID, "null forest");
   std::lock_guard<std::mutex> lock(f->mu);
   const auto &pk = f->packed;
-  if (f->quant || f->deep) return fail(TBK_ERR_UNSUPPORTED, "tbk_predict_noalloc does not cover the 16-bit key layouts");
+  if (f->rank || f->quant || f->deep) return fail(TBK_ERR_UNSUPPORTED, "tbk_predict_noalloc does not cover the 16-bit key layouts");
   if (n_rows < 0 || ld < pk.num_features) return fail(TBK_ERR_INVALID, "ld (%lld) is smaller than the row size (%d)", (long long)ld, pk.num_features);
   if (n_rows == 0) return TBK_OK;
   if (!d_rows || !d_out) return fail(TBK_ERR_INVALID, "null pointer");
@@ -1347,7 +1742,17 @@ int tbk_host_layout_check(const tbk_forest_arrays *fa, const tbk_schedule *sched
       const bool narrow = (227 * 1024 - tb::kQBBarBytes - tb::kQBRingBytes) / tb::quant_batch_tile_bytes(host.num_features) >= 4;
       std::string qerr = tb::pack_quant(host, &q, narrow);
       if (!qerr.empty()) return fail(TBK_ERR_UNSUPPORTED, "%s", qerr.c_str());
-      if (rows && n_rows > 0) tb::walk_quant_on_host(q, rows, n_rows, ld, leaf_ids, sums, &ties);
+      if (rows && n_rows > 0) {
+        tb::walk_quant_on_host(q, rows, n_rows, ld, leaf_ids, sums, &ties);
+        // forests over narrow rows are uploaded as rank keys: those planes must select the same leaves
+        tb::RankForest r;
+        if (leaf_ids && tb::pack_rank(host, &r).empty()) {
+          std::vector<int32_t> again((size_t)n_rows * T);
+          int64_t searched = 0;
+          tb::walk_rank_on_host(r, rows, n_rows, ld, again.data(), nullptr, &searched);
+          if (std::memcmp(again.data(), leaf_ids, again.size() * 4) != 0) return fail(TBK_ERR_INVALID, "rank keys and quantised keys select different leaves");
+        }
+      }
       groups = (int64_t)q.groups.size();
       elems = (int64_t)q.node_plane.size();
     } else {

@@ -1,0 +1,421 @@
+// Walk kernel for rank keys (rank_pack.h): forests of at most 8 levels over rows of at most 64
+// features.
+//
+// LANE = TREE.  A warp owns R rows of the batch and walks them through the 32 trees of a group,
+// one tree per lane, four rows in lock-step.  What that buys over lane = row:
+//  * a lane's tree is the same for all R rows, so the nodes of its two topmost levels live in
+//    registers and cost no shared-memory load;
+//  * the keys of one row are read by all lanes at once: 16-bit keys of up to 64 features lie in
+//    32 words, so whatever features the 32 trees ask for, the load is one wavefront;
+//  * leaf values are added to R running sums per lane and meet across lanes once per batch, not
+//    once per tree: no table of leaf numbers, no second set of warps, and every sum has only
+//    trees / 32 terms;
+//  * a warp's work is R rows, not 32: small batches still spread over the GPU.
+// Node loads are conflict-free (32 columns = 32 banks).  A level costs a node load, a shift-add to
+// the key's address, a key load, a comparison and a predicated add (rank_pack.h on the slot
+// numbering); a tree of 8 levels 15 shared-memory wavefronts and about 40 instructions.  Bound:
+// the shared-memory pipe.
+//
+// A block = 20 walker warps, a warp that streams the tree groups (node plane and leaf plane of a
+// group = one stage, as many stages as fit) and a warp that fetches the keys of the next batch of
+// 20 R rows while the current one is walked.  All hand-offs are mbarriers with bounded waits; a
+// wait that gives up ends the launch with a status word.  Blocks are persistent over row batches
+// (blockIdx.x, + gridDim.x, ...); blockIdx.y is a chunk of the trees.  With several chunks a block
+// takes one row batch, leaves its partial sums in scratch memory, and the last block to finish
+// with a row batch adds them up in chunk order: one launch, and the same result every time.
+//
+// Multiclass: the running sums belong to one class at a time (a class owns consecutive columns);
+// when the class changes they are combined across the lanes -- afterwards a lane holds the class
+// sum of ONE row -- and the best class so far is updated with the reference's tie rule (ties go
+// to the higher class index, src/reduction/LowerReduceOps.cpp:148-189).  Tree chunks are then
+// ranges of whole classes.
+//
+// Reference counterparts: the scalar walk src/mlir/CodeGenStateMachine.cpp:149-243, the row and
+// tree caches src/gpu/GPURepresentations.cpp:279-399, :630-715, the cross-thread reduction
+// src/reduction/LowerReduceOps.cpp:921-1003.
+#pragma once
+#include "walk_quant.cuh"
+
+namespace tb {
+
+struct RankWalkParams {
+  const uint32_t *node_plane;
+  const uint32_t *leaf_plane; // leaf values, or original node ids where leaf ids are recorded
+  const DevQuantGroup *groups;
+  const int32_t *tree_index;
+  const int32_t *class_begin; // multiclass
+  const unsigned char *keys;  // [n_rows][S]
+  long long n_rows;
+  float *partial;             // where write_partial asks for raw sums
+  float *scratch;             // [chunks][n_rows] partial sums, or (best sum, class) pairs
+  void *out;
+  int32_t *leaf_ids;
+  unsigned int *arrivals;     // per row batch: chunks that are done (zero between launches)
+  long long num_trees;
+  int32_t num_groups, groups_per_chunk, num_classes, classes_per_chunk;
+  int32_t write_partial, out_kind, transform;
+  float initial_value;
+  int32_t stages;
+  uint32_t stage_bytes;
+  int32_t *status;
+  int32_t skip_first_copy; // failure drill
+  uint32_t wait_tries;
+};
+
+constexpr int kRWWalkers = 20, kRWThreads = 32 * (kRWWalkers + 2);
+constexpr int kRWBarBytes = 256; // full[8], empty[8], keys_full[2], keys_empty[2]; flag at 192
+constexpr int kRWMaxStages = 8;
+constexpr int kRankArrivals = 4096;                    // row batches of a launch with several tree chunks
+constexpr size_t kRankArrivalBytes = 4 * kRankArrivals;
+
+__host__ __device__ constexpr int rank_walk_smem_bytes(int rows_per_warp, int stride, int stages, uint32_t stage_bytes) {
+  return kRWBarBytes + 2 * kRWWalkers * rows_per_warp * stride + stages * (int)stage_bytes;
+}
+
+template <int IMM> __device__ __forceinline__ uint32_t lds_u32_imm(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(IMM));
+  return v;
+}
+template <int IMM> __device__ __forceinline__ uint32_t lds_u16_imm(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(IMM));
+  return v;
+}
+// One decision: where key >= threshold rank (the low half of the node word), `off` moves on by IMM.
+// WHOLE = false compares the low halves as half-precision numbers (ranks up to kRankHalfMax).
+template <bool WHOLE, uint32_t IMM> __device__ __forceinline__ void rank_step(uint32_t &off, uint32_t key, uint32_t node) {
+  if constexpr (WHOLE)
+    asm volatile("{\n .reg .pred p;\n .reg .b32 t;\n and.b32 t, %2, 0xffff;\n setp.ge.u32 p, %1, t;\n @p add.u32 %0, %0, %3;\n}"
+                 : "+r"(off) : "r"(key), "r"(node), "n"(IMM));
+  else
+    asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %1, %2;\n @p add.u32 %0, %0, %3;\n}"
+                 : "+r"(off) : "r"(key), "r"(node), "n"(IMM));
+}
+// The decision at the root: picks the node of level 1 and the offset together.
+template <bool WHOLE>
+__device__ __forceinline__ void rank_root(uint32_t &off, uint32_t &next, uint32_t key, uint32_t root, uint32_t off_left,
+                                          uint32_t off_right, uint32_t left, uint32_t right) {
+  if constexpr (WHOLE)
+    asm volatile("{\n .reg .pred p;\n .reg .b32 t;\n and.b32 t, %3, 0xffff;\n setp.ge.u32 p, %2, t;\n"
+                 " selp.b32 %0, %5, %4, p;\n selp.b32 %1, %7, %6, p;\n}"
+                 : "=&r"(off), "=&r"(next)
+                 : "r"(key), "r"(root), "r"(off_left), "r"(off_right), "r"(left), "r"(right));
+  else
+    asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %2, %3;\n"
+                 " selp.b32 %0, %5, %4, p;\n selp.b32 %1, %7, %6, p;\n}"
+                 : "=&r"(off), "=&r"(next)
+                 : "r"(key), "r"(root), "r"(off_left), "r"(off_right), "r"(left), "r"(right));
+}
+
+// Walks four rows (keys at kb + (ROW0 + q) * S) through this lane's tree of depth D, whose
+// column starts at `col` (node plane; leaf plane 2^D * 128 bytes on); v = leaf words.
+template <int D, int S, int ROW0, bool WHOLE>
+__device__ __forceinline__ void rank_walk4(uint32_t (&v)[4], uint32_t col, uint32_t kb, uint32_t root, uint32_t ka0,
+                                           uint32_t left, uint32_t right) {
+  uint32_t off[4], node[4], key[4];
+#define TBR_ROWS(stmt)                                                                                              \
+  { constexpr int q = 0; stmt; } { constexpr int q = 1; stmt; } { constexpr int q = 2; stmt; } { constexpr int q = 3; stmt; }
+  TBR_ROWS(key[q] = lds_u16_imm<(ROW0 + q) * S>(ka0))
+  TBR_ROWS((rank_root<WHOLE>(off[q], node[q], key[q], root, col, col + 128u, left, right)))
+#define TBR_DECIDE(level)                                                                                           \
+  if constexpr (D > level) {                                                                                        \
+    if constexpr (level > 1) TBR_ROWS(node[q] = lds_u32_imm<128 * ((1 << level) - 1)>(off[q]))                      \
+    TBR_ROWS(key[q] = lds_u16_imm<(ROW0 + q) * S>((node[q] >> 16) + kb))                                            \
+    TBR_ROWS((rank_step<WHOLE, (128u << level)>(off[q], key[q], node[q])))                                          \
+  }
+  TBR_DECIDE(1) TBR_DECIDE(2) TBR_DECIDE(3) TBR_DECIDE(4) TBR_DECIDE(5) TBR_DECIDE(6) TBR_DECIDE(7)
+  TBR_ROWS(v[q] = lds_u32_imm<(128 << D)>(off[q]))
+#undef TBR_DECIDE
+#undef TBR_ROWS
+}
+
+// Adds up v over the 32 lanes for every of R rows: afterwards lane l holds the sum of row
+// l * R / 32 (32 / R neighbouring lanes hold the same row).
+template <int R> __device__ __forceinline__ float rank_reduce_rows(float (&v)[R], int lane) {
+  int bit = 16;
+#pragma unroll
+  for (int half = R / 2; half >= 1; half /= 2, bit /= 2) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float keep = up ? v[i + half] : v[i], give = up ? v[i] : v[i + half];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+    }
+  }
+  float s = v[0];
+  for (; bit >= 1; bit /= 2) s += __shfl_xor_sync(0xffffffffu, s, bit);
+  return s;
+}
+// One group of depth D for all R rows of the warp; use(c, v) takes the leaf words of rows 4c .. 4c+3.
+template <int D, int S, int R, bool WHOLE, typename Use>
+__device__ __forceinline__ void rank_walk_rows(uint32_t col, uint32_t kb, Use use) {
+  const uint32_t root = lds_u32_imm<0>(col), ka0 = (root >> 16) + kb;
+  uint32_t left = 0, right = 0, v[4];
+  if constexpr (D > 1) {
+    left = lds_u32_imm<128>(col);
+    right = lds_u32_imm<256>(col);
+  }
+  rank_walk4<D, S, 0, WHOLE>(v, col, kb, root, ka0, left, right);
+  use(0, v);
+  if constexpr (R > 4) {
+    rank_walk4<D, S, 4, WHOLE>(v, col, kb, root, ka0, left, right);
+    use(1, v);
+  }
+  if constexpr (R > 8) {
+    rank_walk4<D, S, 8, WHOLE>(v, col, kb, root, ka0, left, right);
+    use(2, v);
+    rank_walk4<D, S, 12, WHOLE>(v, col, kb, root, ka0, left, right);
+    use(3, v);
+  }
+}
+template <int S, int R, bool WHOLE, typename Use>
+__device__ __forceinline__ void rank_walk_group(uint32_t depth, uint32_t col, uint32_t kb, Use use) {
+  switch (depth) {
+  case 1: return rank_walk_rows<1, S, R, WHOLE>(col, kb, use);
+  case 2: return rank_walk_rows<2, S, R, WHOLE>(col, kb, use);
+  case 3: return rank_walk_rows<3, S, R, WHOLE>(col, kb, use);
+  case 4: return rank_walk_rows<4, S, R, WHOLE>(col, kb, use);
+  case 5: return rank_walk_rows<5, S, R, WHOLE>(col, kb, use);
+  case 6: return rank_walk_rows<6, S, R, WHOLE>(col, kb, use);
+  case 7: return rank_walk_rows<7, S, R, WHOLE>(col, kb, use);
+  default: return rank_walk_rows<8, S, R, WHOLE>(col, kb, use);
+  }
+}
+
+enum RankMode { kRankSums, kRankClasses, kRankLeafIds };
+
+// S: bytes per row of keys; R: rows per warp.
+template <int S, int R, bool WHOLE, int MODE>
+__global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankWalkParams p) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); // uniform by construction
+  constexpr int RB = kRWWalkers * R;                      // rows per batch
+  const uint32_t bars_s = smem_u32(smem_raw);
+  const uint32_t full_s = bars_s, empty_s = bars_s + 64u, keys_full_s = bars_s + 128u, keys_empty_s = bars_s + 144u;
+  volatile uint32_t *last_flag = reinterpret_cast<volatile uint32_t *>(smem_raw + 192);
+  unsigned char *keys = smem_raw + kRWBarBytes;           // two batches of keys
+  unsigned char *ring = keys + 2 * RB * S;
+  const int num_batches = (int)((p.n_rows + RB - 1) / RB);
+  const int my_batches = (num_batches - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  // this chunk's groups; with classes: those that hold the columns of classes c0 .. c1 - 1
+  int g0 = (int)blockIdx.y * p.groups_per_chunk, g1 = min(p.num_groups, g0 + p.groups_per_chunk);
+  [[maybe_unused]] int c0 = 0, c1 = 0, col0 = 0;
+  if constexpr (MODE == kRankClasses) {
+    c0 = (int)blockIdx.y * p.classes_per_chunk;
+    c1 = min(p.num_classes, c0 + p.classes_per_chunk);
+    col0 = p.class_begin[c0];
+    const int col1 = p.class_begin[c1];
+    g0 = col0 / 32;
+    g1 = col1 > col0 ? (col1 + 31) / 32 : g0;
+  }
+  const int NG = g1 - g0;
+
+  if (tid == 0) {
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
+    for (int i = 0; i < kRWMaxStages; ++i) mbar_init(bars + i, 1);              // full: the copies' bytes
+    for (int i = 0; i < kRWMaxStages; ++i) mbar_init(bars + 8 + i, kRWWalkers); // empty: one arrival per walker warp
+    for (int i = 0; i < 2; ++i) mbar_init(bars + 16 + i, 1);                    // keys_full
+    for (int i = 0; i < 2; ++i) mbar_init(bars + 18 + i, kRWWalkers);           // keys_empty
+    fence_barrier_init();
+  }
+  __syncthreads();
+
+  bool ok = true;
+  [[maybe_unused]] uint32_t issued = 0; // copies (of a stage, of a batch's keys) this producer warp has started
+  const uint32_t tries = p.wait_tries ? p.wait_tries : kQWaitTries;
+  // (the warp agrees on the outcome: shuffles follow)
+  auto wait = [tries](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_all_lanes(bar, parity, tries)) != 0; };
+
+  if (warp == kRWWalkers) {
+    // ---- tree groups, batch after batch
+    const uint64_t keep = l2_policy_keep();
+    int slot = 0;
+    uint32_t round = 0;
+    for (int it = 0; it < my_batches && ok; ++it)
+      for (int k = 0; k < NG && ok; ++k) {
+        if (round > 0) ok = wait(empty_s + 8u * (uint32_t)slot, (round - 1u) & 1u);
+        issued += ok;
+        if (ok && lane == 0 && !(p.skip_first_copy && it == 0 && k == 0)) {
+          const DevQuantGroup gm = p.groups[g0 + k];
+          const uint32_t bytes = gm.slots * 128u;
+          unsigned char *dst = ring + (size_t)slot * p.stage_bytes;
+          uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw) + slot;
+          mbar_expect_tx(bar, 2u * bytes);
+          bulk_g2s_hint(dst, p.node_plane + gm.elem_off, bytes, bar, keep);
+          bulk_g2s_hint(dst + bytes, p.leaf_plane + gm.elem_off, bytes, bar, keep);
+        }
+        if (++slot == p.stages) {
+          slot = 0;
+          ++round;
+        }
+      }
+  } else if (warp == kRWWalkers + 1) {
+    // ---- the batches' keys, one batch ahead of the walk; the kernel that ranks the rows may
+    // still be running when this one starts
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint64_t stream = l2_policy_stream();
+    for (int it = 0; it < my_batches && ok; ++it) {
+      const uint32_t buf = (uint32_t)it & 1u;
+      if (it >= 2) ok = wait(keys_empty_s + 8u * buf, (uint32_t)((it >> 1) - 1) & 1u);
+      issued += ok;
+      if (ok && lane == 0) {
+        const long long row0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * RB;
+        const uint32_t bytes = (uint32_t)min((long long)RB, p.n_rows - row0) * (uint32_t)S;
+        uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw) + 16 + buf;
+        mbar_expect_tx(bar, bytes);
+        bulk_g2s_hint(keys + (size_t)buf * RB * S, p.keys + row0 * S, bytes, bar, stream);
+      }
+    }
+  } else {
+    // ---- the walkers
+    const bool elected = lane == 0;
+    const uint32_t ring_col = smem_u32(ring) + (uint32_t)lane * 4u;
+    const int my_row = warp * R + lane * R / 32;       // the row whose sum this lane ends up with
+    const bool writer = (lane & (32 / R - 1)) == 0;
+    int slot = 0;
+    uint32_t parity = 0;
+    for (int it = 0; it < my_batches && ok; ++it) {
+      const long long row0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * RB;
+      const long long row = row0 + my_row;
+      const bool live = writer && row < p.n_rows;
+      ok = wait(keys_full_s + 8u * ((uint32_t)it & 1u), (uint32_t)(it >> 1) & 1u);
+      if (!ok) break;
+      const uint32_t kb = smem_u32(keys) + ((uint32_t)it & 1u) * (uint32_t)(RB * S) + (uint32_t)(warp * R * S);
+      float acc[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) acc[i] = 0.f;
+      [[maybe_unused]] int cls = c0, lo = col0 & 31, best_class = c0;
+      [[maybe_unused]] float sum = 0.f, best = -INFINITY;
+      // class `cls` is complete, its sum for this lane's row in `sum`
+      [[maybe_unused]] auto finish = [&]() {
+        if (p.write_partial) {
+          if (live) p.partial[row * p.num_classes + cls] = sum;
+        }
+        if (sum >= best) {
+          best = sum;
+          best_class = cls;
+        }
+        sum = 0.f;
+        ++cls;
+      };
+      uint32_t next_depth = NG > 0 ? p.groups[g0].depth : 0u;
+      for (int k = 0; k < NG; ++k) {
+        const uint32_t depth = next_depth;
+        next_depth = p.groups[min(g0 + k + 1, g1 - 1)].depth;
+        ok = wait(full_s + 8u * (uint32_t)slot, parity);
+        if (!ok) break;
+        const uint32_t col = ring_col + (uint32_t)slot * p.stage_bytes;
+        if constexpr (MODE == kRankLeafIds) {
+          const int t = p.tree_index[(g0 + k) * 32 + lane];
+          int32_t *dst = p.leaf_ids + (row0 + warp * R) * p.num_trees + t;
+          const int rows = (int)min((long long)R, p.n_rows - (row0 + warp * R));
+          rank_walk_group<S, R, WHOLE>(depth, col, kb, [&](int c, const uint32_t(&v)[4]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (t >= 0 && 4 * c + q < rows) dst[(4 * c + q) * p.num_trees] = (int32_t)v[q];
+          });
+        } else {
+          auto add = [&](int c, const uint32_t(&v)[4]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[4 * c + q] += __uint_as_float(v[q]);
+          };
+          if constexpr (MODE == kRankClasses) {
+            int next = p.class_begin[cls + 1] - (g0 + k) * 32; // first column of the next class
+            const bool pure = lo == 0 && next >= 32;
+            if (!pure && lo == 0) { // the group starts in this class and ends in another
+              sum += rank_reduce_rows<R>(acc, lane);
+#pragma unroll
+              for (int i = 0; i < R; ++i) acc[i] = 0.f;
+            }
+            rank_walk_group<S, R, WHOLE>(depth, col, kb, add);
+            while (cls < c1 && next <= 32) { // classes that end in this group
+              float part[R];
+#pragma unroll
+              for (int i = 0; i < R; ++i) part[i] = lane >= lo && lane < next ? acc[i] : 0.f;
+              sum += rank_reduce_rows<R>(part, lane);
+              finish();
+              lo = next;
+              if (cls < c1) next = p.class_begin[cls + 1] - (g0 + k) * 32;
+            }
+            if (lo > 0)
+#pragma unroll
+              for (int i = 0; i < R; ++i) acc[i] = lane >= lo ? acc[i] : 0.f;
+            lo = 0;
+          } else {
+            rank_walk_group<S, R, WHOLE>(depth, col, kb, add);
+          }
+        }
+        __syncwarp();
+        if (elected) mbar_arrive(empty_s + 8u * (uint32_t)slot);
+        if (++slot == p.stages) {
+          slot = 0;
+          parity ^= 1u;
+        }
+      }
+      if (!ok) break;
+      if (elected) mbar_arrive(keys_empty_s + 8u * ((uint32_t)it & 1u));
+      // ---- the batch's results
+      if constexpr (MODE == kRankSums) {
+        const float s = rank_reduce_rows<R>(acc, lane);
+        if (live) {
+          if (gridDim.y > 1) p.scratch[(long long)blockIdx.y * p.n_rows + row] = s;
+          else if (p.write_partial) p.partial[row] = s;
+          else reinterpret_cast<float *>(p.out)[row] = apply_transform(p.initial_value + s, p.transform);
+        }
+      } else if constexpr (MODE == kRankClasses) {
+        while (cls < c1) finish(); // classes without trees
+        if (live && !p.write_partial) {
+          if (gridDim.y > 1)
+            reinterpret_cast<float2 *>(p.scratch)[(long long)blockIdx.y * p.n_rows + row] = make_float2(best, __int_as_float(best_class));
+          else if (p.out_kind == 1) reinterpret_cast<int8_t *>(p.out)[row] = (int8_t)best_class;
+          else reinterpret_cast<float *>(p.out)[row] = (float)best_class;
+        }
+      }
+    }
+  }
+  // every wait above is bounded: a wait that gave up ends the launch with a status word
+  const bool chunked = gridDim.y > 1 && MODE != kRankLeafIds && !(MODE == kRankClasses && p.write_partial);
+  if (chunked) __threadfence();
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0) atomicExch(p.status, 4);
+    if (warp >= kRWWalkers) { // no copy may land after the block is gone
+      const uint32_t bars = warp == kRWWalkers ? full_s : keys_full_s, n = warp == kRWWalkers ? (uint32_t)p.stages : 2u;
+      for (uint32_t s = 0; s < min(n, issued); ++s) wait(bars + 8u * s, ((issued - 1u - s) / n) & 1u);
+    }
+  }
+  if (!chunked) return;
+  // ---- tree chunks: the last block to finish with this row batch combines them
+  if (tid == 0) {
+    const bool last = atomicAdd(p.arrivals + blockIdx.x, 1u) + 1u == gridDim.y;
+    if (last) p.arrivals[blockIdx.x] = 0; // for the next launch
+    *last_flag = last;
+  }
+  __syncthreads();
+  if (!*last_flag) return;
+  __threadfence();
+  const long long row = (long long)blockIdx.x * RB + tid;
+  if (tid >= RB || row >= p.n_rows) return;
+  if constexpr (MODE == kRankClasses) {
+    float best = -INFINITY;
+    int best_class = 0;
+    for (int y = 0; y < (int)gridDim.y; ++y) { // (classes rise with the chunks: a later one wins ties)
+      const float2 b = __ldcg(reinterpret_cast<const float2 *>(p.scratch) + (long long)y * p.n_rows + row);
+      if (b.x >= best) {
+        best = b.x;
+        best_class = __float_as_int(b.y);
+      }
+    }
+    if (p.out_kind == 1) reinterpret_cast<int8_t *>(p.out)[row] = (int8_t)best_class;
+    else reinterpret_cast<float *>(p.out)[row] = (float)best_class;
+  } else {
+    float s = 0.f;
+#pragma unroll 4
+    for (int y = 0; y < (int)gridDim.y; ++y) s += __ldcg(p.scratch + (long long)y * p.n_rows + row);
+    if (p.write_partial) p.partial[row] = s;
+    else reinterpret_cast<float *>(p.out)[row] = apply_transform(p.initial_value + s, p.transform);
+  }
+}
+
+} // namespace tb
