@@ -1,0 +1,92 @@
+"""Rank keys (forests of at most 8 levels over at most 64 features) at the edges of their kernels:
+unit and batch sizes of the walk, rows in pairs and one by one, groups of mixed depth, classes that
+share a group of trees, more thresholds than the half-precision comparison holds, and the direct
+and the shared-memory ranking of rows."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from tests.helpers import assert_predictions_close
+from treebeard_b200 import kernels, synth
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _forest(trees, levels, features, classes=0, p=0.2, seed=5, whole=False):
+    marg = synth.Marginal("int16" if whole else "normal", features)
+    f = synth.generate_forest(seed, trees, levels, features, p, 0.1, marg, num_classes=classes)
+    if classes:   # uneven classes, one of them empty: several class boundaries fall into one group
+        rng = np.random.Generator(np.random.PCG64(seed))
+        f.class_id[:] = np.minimum(rng.integers(0, classes, trees), rng.integers(0, classes, trees))
+        f.class_id[f.class_id == 1] = 2
+    return f, marg
+
+
+def _rows(f, marg, n, seed=9):
+    rng = np.random.Generator(np.random.PCG64(seed))
+    X = marg.sample_rows(rng, n)
+    split = np.nonzero(f.left >= 0)[0]
+    for i in range(min(400, 4 * n)):   # values equal to thresholds, and their neighbours
+        g = split[(i * 37) % len(split)]
+        X[(i * 13) % n, f.feat[g]] = np.nextafter(f.thr[g], np.float32([-np.inf, np.inf, f.thr[g]][i % 3]))
+    if n > 6:
+        X[3, :], X[4, 0], X[5, f.num_features - 1] = np.nan, np.inf, -np.inf
+    return X
+
+
+@pytest.mark.parametrize("trees,levels,features,classes,rows", [
+    (1, 1, 1, 0, 1), (31, 2, 32, 0, 79), (33, 3, 33, 0, 81), (100, 6, 8, 0, 320), (97, 8, 64, 0, 321),
+    (300, 7, 20, 0, 148 * 80 * 4 + 77), (64, 8, 28, 3, 5), (45, 5, 16, 7, 12003), (400, 8, 40, 26, 2500),
+    (140, 8, 1, 0, 4000)])
+def test_rank_key_walk_is_exact(trees, levels, features, classes, rows):
+    f, marg = _forest(trees, levels, features, classes, p=0.0 if features == 1 and trees > 1 else 0.2)
+    X = _rows(f, marg, rows)
+    want, want_ids = oracle.predict(f, X, leaf_ids=True)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows)
+    assert df.info().schedule.feature_bits == 16
+    dX = torch.from_numpy(X).cuda()
+    ids = df.predict_leaf_ids(dX).cpu().numpy()
+    df.check_status()
+    assert np.array_equal(ids, want_ids)
+    got, part = df.predict(dX), df.predict_partial(dX)
+    df.check_status()
+    if classes:
+        _, sums = oracle.predict(f, X, class_sums=True)
+        sums[:, np.bincount(f.class_id, minlength=classes) == 0] = f.initial_value   # classes without trees
+        best = sums.max(axis=1)
+        cls = got.cpu().numpy().astype(int)
+        assert (sums[np.arange(rows), cls] >= best - 1e-5 * np.abs(best) - 1e-5).all()
+        assert np.allclose(part.cpu().numpy() + f.initial_value, sums, rtol=1e-5, atol=1e-5)
+        assert np.array_equal(df.predict(dX, int8=True).cpu().numpy(), cls.astype(np.int8))
+    else:
+        assert_predictions_close(got.cpu().numpy(), want)
+        assert_predictions_close(df.finalize(part).cpu().numpy(), want)
+
+
+def test_rank_keys_on_several_streams_and_in_a_graph():
+    """Every stream has its own key memory; a captured call keeps the memory it was captured with."""
+    f, marg = _forest(200, 8, 28)
+    batches = [torch.from_numpy(_rows(f, marg, 3000 + 500 * i, seed=i)).cuda() for i in range(6)]
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=3000)
+    want = [df.predict(b).clone() for b in batches]
+    streams = [torch.cuda.Stream() for _ in batches]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        got = []
+        for b, s in zip(batches, streams):
+            with torch.cuda.stream(s):
+                got.append(df.predict(b))
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, w) for g, w in zip(got, want))
+    out = torch.empty_like(want[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        df.predict(batches[0], out=out)
+    out.zero_()
+    graph.replay()
+    other = df.predict(batches[1])
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[0]) and torch.equal(other, want[1])
+    df.check_status()

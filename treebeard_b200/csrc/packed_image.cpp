@@ -122,6 +122,7 @@ void put_image(const PackedImage &im, Out &o) {
     const RankForest &q = im.rf;
     put_key_forest_head(o, q.num_features, q.transform, q.initial_value, q.num_trees, q.num_nodes, q.max_depth);
     o.pod(q.num_classes);
+    o.pod(q.lattice);
     o.pod(q.whole_compare);
     o.vec(q.groups);
     o.vec(q.node_plane);
@@ -246,6 +247,7 @@ std::string deserialize_image(const uint8_t *data, uint64_t size, PackedImage *i
     RankForest &q = im->rf;
     key_head(&q.num_features, &q.transform, &q.initial_value, &q.num_trees, &q.num_nodes, &q.max_depth);
     q.num_classes = in.pod<int32_t>();
+    q.lattice = in.pod<int32_t>();
     q.whole_compare = in.pod<int32_t>();
     in.vec(&q.groups);
     in.vec(&q.node_plane);

@@ -8,11 +8,11 @@ namespace tb {
 
 namespace {
 
-// Bucket of a value in [lo, hi]; the device computes the same two roundings.
+// Bucket of a value; the device computes the same two roundings.
 uint32_t bucket_of(const RankFeature &f, float x) {
   const float d = x - f.lo;
   const float y = d * f.scale;
-  return std::min((uint32_t)y, f.buckets - 1);
+  return (uint32_t)std::fmax(std::fmin(y, f.top), 0.f); // (NaN: the last bucket)
 }
 
 // The bucket table of one feature whose sorted distinct thresholds are t[0..n).
@@ -76,21 +76,22 @@ std::string pack_rank(const Forest &f, RankForest *out) {
   for (int i = 0; i < F; ++i) {
     const auto &d = distinct[i];
     RankFeature &rf = q.features[i];
-    rf = RankFeature{0.f, -1.f, 0.f, 1, lut_size, thr_size, (uint32_t)d.size(), 0};
+    rf = RankFeature{0.f, 0.f, 0.f, lut_size, thr_size, (uint32_t)d.size(), 1, 0};
     if (!d.empty()) {
       rf.lo = d.front();
-      rf.hi = d.back();
-      bool whole = std::fabs(rf.lo) <= 0x1p22f && std::fabs(rf.hi) <= 0x1p22f && rf.hi - rf.lo <= std::max(4096.f, 4.f * (float)d.size());
+      const float hi = d.back();
+      bool whole = std::fabs(rf.lo) <= 0x1p22f && std::fabs(hi) <= 0x1p22f && hi - rf.lo <= std::max(4096.f, 4.f * (float)d.size());
       for (size_t k = 0; k < d.size() && whole; ++k) whole = d[k] == std::floor(d[k]);
       if (whole) {
         rf.lattice = 1;
-        rf.buckets = (uint32_t)(rf.hi - rf.lo) + 1;
+        q.lattice = 1;
+        rf.buckets = (uint32_t)(hi - rf.lo) + 1;
         rf.scale = 1.f;
       } else {
-        // half a bucket per threshold: the table stays small beside the thresholds, and two or
-        // three steps of the search finish a bucket
-        rf.buckets = std::max<uint32_t>(1, ((uint32_t)d.size() + 1) / 2);
-        const float range = rf.hi - rf.lo;
+        // a bucket per threshold: the table takes half the thresholds' bytes, and three or four
+        // steps finish the search of the fullest bucket that a warp meets
+        rf.buckets = (uint32_t)d.size();
+        const float range = hi - rf.lo;
         rf.scale = range > 0.f && std::isfinite(range) ? (float)rf.buckets / range : 0.f;
         if (!std::isfinite(rf.scale) || rf.scale == 0.f) { // a range that fp32 cannot cut up: one bucket
           rf.scale = 0.f;
@@ -98,6 +99,7 @@ std::string pack_rank(const Forest &f, RankForest *out) {
         }
       }
     }
+    rf.top = (float)(rf.buckets - 1);
     lut_size += (rf.buckets + 1 + 7) / 8 * 8; // (tables start on 16-byte boundaries)
     thr_size += ((uint32_t)d.size() + 3) / 4 * 4;
   }
@@ -166,7 +168,7 @@ std::string pack_rank(const Forest &f, RankForest *out) {
           continue;
         }
         const uint64_t e = gm.elem_off + (uint64_t)((1u << it.level) - 1 + it.path) * kRankCols + c;
-        q.node_plane[e] = ((uint32_t)f.feat[n] * 2u << 16) | rank[n];
+        q.node_plane[e] = (rank_key_offset(F, (uint32_t)f.feat[n]) << 16) | rank[n];
         stack.push_back({f.left[n], it.path, it.level + 1});
         stack.push_back({f.right[n], it.path | (1u << it.level), it.level + 1});
       }
@@ -177,12 +179,9 @@ std::string pack_rank(const Forest &f, RankForest *out) {
 
 uint32_t rank_of(const RankForest &q, int32_t feature, float x, bool *searched) {
   const RankFeature &f = q.features[feature];
-  *searched = false;
-  if (f.n == 0 || x < f.lo) return 0;
-  if (!(x < f.hi)) return f.n;
   const uint32_t b = bucket_of(f, x);
   uint32_t s = q.lut[f.lut_off + b], e = q.lut[f.lut_off + b + 1];
-  if (f.lattice && x == std::floor(x)) return e;
+  if (f.lattice && x == std::floor(x)) s = e = x < f.lo ? 0 : e;
   *searched = s < e;
   while (s < e) {
     const uint32_t m = (s + e) >> 1;
@@ -212,7 +211,7 @@ void walk_rank_on_host(const RankForest &q, const float *rows, int64_t n_rows, i
       uint32_t path = 0;
       for (uint32_t d = 0; d < gm.depth; ++d) {
         const uint32_t node = q.node_plane[base + (uint64_t)((1u << d) - 1 + path) * kRankCols];
-        if (key[(node >> 16) / 2] >= (node & 0xffffu)) path |= 1u << d;
+        if (key[(node >> 16) / rank_key_offset(q.num_features, 1)] >= (node & 0xffffu)) path |= 1u << d;
       }
       const uint64_t e = base + (uint64_t)path * kRankCols;
       while (q.num_classes > 0 && (int32_t)k >= q.class_begin[cls + 1]) ++cls;

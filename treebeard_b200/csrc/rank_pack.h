@@ -17,8 +17,8 @@
 // whole-number row value is ranked by the table alone.
 //
 // Planes, per group of 32 trees of (padded) depth D, 2^D slots x 32 columns each:
-//   node plane  u32  (key offset << 16) | (j + 1); the offset is the byte offset of the
-//                    feature's key in a row of keys
+//   node plane  u32  (key offset << 16) | (j + 1); the offset is the byte offset of the feature's
+//                    key in a row of keys (2 f) or, for at most 32 features, in a pair of rows (4 f)
 //   leaf plane  f32  leaf values
 // Slots: node on level d reached by the decisions r_0 .. r_(d-1) (1 = right) is slot
 // 2^d - 1 + sum r_i 2^i, leaf sum r_i 2^i.  With the decision of level i worth 2^i slots on EVERY
@@ -39,15 +39,21 @@ constexpr int kRankCols = 32, kRankMaxDepth = 8;
 // A forest all of whose ranks fit the positive half-precision numbers is compared by the half2
 // comparison, which needs no masking (one instruction per decision less than whole numbers).
 constexpr uint32_t kRankHalfMax = 31742, kRankMax = 65534;
+constexpr int kRankPairFeatures = 32; // up to here the keys of two rows lie side by side
 constexpr int kRankMaxFeatures = 64; // 16-bit keys of a row in 32 four-byte words: one bank each
 
+inline uint32_t rank_key_offset(int32_t num_features, uint32_t feature) {
+  return num_features <= kRankPairFeatures ? 4 * feature : 2 * feature;
+}
+
 struct RankFeature { // 32 bytes, the same on the device
-  float lo, hi;      // smallest and largest threshold (lo > hi: the feature is not used)
+  float lo;          // smallest threshold
   float scale;       // buckets per unit
-  uint32_t buckets;
+  float top;         // buckets - 1
   uint32_t lut_off;  // first of buckets + 1 entries
   uint32_t thr_off;  // first of n thresholds
-  uint32_t n;
+  uint32_t n;        // distinct thresholds (0: the feature is not used)
+  uint32_t buckets;
   uint32_t lattice;
 };
 
@@ -56,6 +62,7 @@ struct RankForest {
   double initial_value = 0.0;
   int64_t num_trees = 0, num_nodes = 0;
   int32_t max_depth = 0;   // at least 1
+  int32_t lattice = 0;       // some feature is a lattice feature
   int32_t whole_compare = 0; // some rank exceeds kRankHalfMax: compare as whole numbers
   std::vector<QuantGroup> groups; // elem_off in elements of either plane
   std::vector<uint32_t> node_plane;

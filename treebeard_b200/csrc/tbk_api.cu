@@ -52,6 +52,14 @@ struct tbk_image {
   tb::PackedImage im;
 };
 
+struct RankPlan {
+  int units = tb::kRWBatchUnits; // units of rows in a block's (first) batch
+  int chunks = 1, per_chunk = 1; // per_chunk: groups, or classes of a multiclass forest
+  int stages = 2, smem = 0;
+  uint32_t stage_bytes = 0;
+  int64_t grid_x = 1;
+};
+
 struct tbk_forest {
   tb::PackedForest packed; // host copy (orig_node kept for lazy upload)
   int device = 0;
@@ -107,6 +115,9 @@ struct tbk_forest {
   int next_victim = 0;
   std::list<Workspace> captured; // of calls that were captured into graphs
   std::vector<const void *> smem_allowed;
+  RankPlan rank_plan;          // of the last batch size
+  int64_t rank_plan_rows = -1;
+  bool rank_plan_ids = false;
   // one-tree-per-stage layout (deep trees); shares the device buffers of the key layout
   bool deep = false;
   tb::DeepForest df;
@@ -539,72 +550,81 @@ int allow_smem(tbk_forest *f, const void *kernel) {
   return TBK_OK;
 }
 
-int rank_stride(int num_features) { return num_features <= 32 ? 64 : 128; }
+// bytes of keys per row
+int rank_stride(int num_features) { return num_features <= tb::kRankPairFeatures ? 64 : 128; }
 
 using RankKernel = void (*)(const tb::RankWalkParams);
-template <int S, int R, bool WHOLE> RankKernel pick_rank(int mode) {
-  return mode == tb::kRankLeafIds ? tb::tb_walk_rank_kernel<S, R, WHOLE, tb::kRankLeafIds>
-         : mode == tb::kRankClasses ? tb::tb_walk_rank_kernel<S, R, WHOLE, tb::kRankClasses>
-                                    : tb::tb_walk_rank_kernel<S, R, WHOLE, tb::kRankSums>;
+template <int S, bool WHOLE> RankKernel pick_rank(int mode) {
+  return mode == tb::kRankLeafIds ? tb::tb_walk_rank_kernel<S, WHOLE, tb::kRankLeafIds>
+         : mode == tb::kRankClasses ? tb::tb_walk_rank_kernel<S, WHOLE, tb::kRankClasses>
+                                    : tb::tb_walk_rank_kernel<S, WHOLE, tb::kRankSums>;
 }
-RankKernel pick_rank_kernel(int stride, int rows_per_warp, bool whole, int mode) {
-  if (stride == 64) {
-    if (rows_per_warp == 16) return whole ? pick_rank<64, 16, true>(mode) : pick_rank<64, 16, false>(mode);
-    return whole ? pick_rank<64, 4, true>(mode) : pick_rank<64, 4, false>(mode);
-  }
-  if (rows_per_warp == 16) return whole ? pick_rank<128, 16, true>(mode) : pick_rank<128, 16, false>(mode);
-  return whole ? pick_rank<128, 4, true>(mode) : pick_rank<128, 4, false>(mode);
+RankKernel pick_rank_kernel(int stride, bool whole, int mode) {
+  if (stride == 64) return whole ? pick_rank<64, true>(mode) : pick_rank<64, false>(mode);
+  return whole ? pick_rank<128, true>(mode) : pick_rank<128, false>(mode);
 }
 
-struct RankPlan {
-  int rows_per_warp = 16, chunks = 1, per_chunk = 1; // per_chunk: groups, or classes of a multiclass forest
-  int stages = 2, smem = 0;
-  uint32_t stage_bytes = 0;
-  int64_t grid_x = 1;
-};
-
-// Launch shape of the walk over `n_rows` rows: rows per warp (16, or 4 for batches so small that
-// 16 would leave most warps idle) and tree chunks, by what the slowest block costs in clocks.  A
-// group takes a warp about 2 D - 1 shared-memory wavefronts per row, and the block at least what
-// its stage's copy takes (70 bytes a clock); a block starts up for about 4000 clocks, and
-// combining chunks adds about 1500.
-RankPlan plan_rank(const tbk_forest *f, int64_t n_rows, bool leaf_ids) {
+// Launch shape of the walk over `n_rows` rows: blocks along the rows and tree chunks, by what the
+// slowest block costs in clocks.  A group takes a warp about 2 D - 1 shared-memory wavefronts per
+// row and 20 warps share the pipe; a few hundred clocks go into the hand-off and the chain of
+// dependent loads, and the stage's copy needs its time too (70 bytes a clock).  A block starts up
+// for about 4000 clocks, and combining chunks adds about 1500.
+RankPlan make_rank_plan(const tbk_forest *f, int64_t n_rows, bool leaf_ids) {
   const auto &q = f->rf;
   const int G = (int)q.groups.size(), S = rank_stride(q.num_features);
-  const bool multi = q.num_classes > 0;
-  const int units = multi && !leaf_ids ? q.num_classes : G; // what chunks are made of
-  RankPlan best;
-  double best_cost = -1.0;
-  for (int R : {16, 4}) {
-    RankPlan p;
-    p.rows_per_warp = R;
-    p.stage_bytes = 256u << q.max_depth;
-    p.stages = std::min(tb::kRWMaxStages, (f->max_smem_optin - tb::rank_walk_smem_bytes(R, S, 0, 0)) / (int)p.stage_bytes);
-    p.smem = tb::rank_walk_smem_bytes(R, S, p.stages, p.stage_bytes);
-    const int64_t RB = tb::kRWWalkers * R, batches = (n_rows + RB - 1) / RB;
-    const double group = std::max(1.15 * RB * (2 * q.max_depth - 1), p.stage_bytes / 70.0);
-    const int most = f->user.tree_chunks > 0 ? f->user.tree_chunks : batches < f->num_sms ? 64 : 1;
-    for (int c = f->user.tree_chunks > 0 ? most : 1; c <= std::min(most, units) || c == 1; ++c) {
-      const int per = (units + c - 1) / c, chunks = (units + per - 1) / per;
-      const double groups = multi && !leaf_ids ? (double)G * per / units + (chunks > 1) : per;
-      const double waves = (double)((batches * chunks + f->num_sms - 1) / f->num_sms);
-      const double cost = waves * groups * group + (chunks > 1 ? waves * 4000.0 + 1500.0 : 4000.0);
-      if (best_cost < 0 || cost < best_cost) {
-        best_cost = cost;
-        best = p;
-        best.chunks = chunks;
-        best.per_chunk = per;
-        best.grid_x = chunks > 1 ? batches : std::min<int64_t>(batches, f->num_sms);
+  const bool multi = q.num_classes > 0 && !leaf_ids;
+  const int parts = multi ? q.num_classes : G; // what chunks are made of
+  const int64_t units = (n_rows + tb::kRWUnitRows - 1) / tb::kRWUnitRows;
+  RankPlan p;
+  p.stage_bytes = 256u << q.max_depth;
+  p.stages = std::min(tb::kRWMaxStages, (f->max_smem_optin - tb::rank_walk_smem_bytes(S, 0, 0)) / (int)p.stage_bytes);
+  p.smem = tb::rank_walk_smem_bytes(S, p.stages, p.stage_bytes);
+  auto group_clocks = [&](int batch_units) {
+    return std::max(1.15 * tb::kRWUnitRows * batch_units * (2 * q.max_depth - 1) + 60.0 * q.max_depth + 200.0, p.stage_bytes / 70.0);
+  };
+  auto set = [&](int64_t grid_x, int chunks) {
+    p.grid_x = grid_x;
+    p.per_chunk = (parts + chunks - 1) / chunks;
+    p.chunks = (parts + p.per_chunk - 1) / p.per_chunk;
+    p.units = (int)std::min<int64_t>(tb::kRWBatchUnits, (units + grid_x - 1) / grid_x);
+  };
+  // one chunk, as many blocks as there are units or SMs
+  const int64_t whole_x = std::min<int64_t>(units, f->num_sms);
+  const int64_t whole_units = (units + whole_x - 1) / whole_x;
+  double best = 4000.0 + (double)G * ((double)(whole_units / 4) * group_clocks(4) + (whole_units % 4 ? group_clocks((int)(whole_units % 4)) : 0.0));
+  set(whole_x, 1);
+  if (f->user.tree_chunks > 0) {
+    if (f->user.tree_chunks > 1) set((units + tb::kRWBatchUnits - 1) / tb::kRWBatchUnits, std::min(parts, f->user.tree_chunks));
+    return p;
+  }
+  for (int u = 1; u <= tb::kRWBatchUnits; ++u) {
+    const int64_t x = (units + u - 1) / u;
+    for (int c = 2; c <= std::min(parts, 64) && x < f->num_sms; ++c) {
+      const int per = (parts + c - 1) / c, chunks = (parts + per - 1) / per;
+      const double groups = multi ? (double)G * per / parts + 1.0 : per;
+      const double waves = (double)((x * chunks + f->num_sms - 1) / f->num_sms);
+      const double cost = waves * (4000.0 + groups * group_clocks(u)) + 1500.0;
+      if (cost < best) {
+        best = cost;
+        set(x, c);
       }
-      if (f->user.tree_chunks > 0) break;
     }
   }
-  return best;
+  return p;
+}
+
+RankPlan plan_rank(tbk_forest *f, int64_t n_rows, bool leaf_ids) { // (a server's batches are mostly alike)
+  if (f->rank_plan_rows != n_rows || f->rank_plan_ids != leaf_ids) {
+    f->rank_plan = make_rank_plan(f, n_rows, leaf_ids);
+    f->rank_plan_rows = n_rows;
+    f->rank_plan_ids = leaf_ids;
+  }
+  return f->rank_plan;
 }
 
 tb::LaunchPlan rank_launch_plan(const RankPlan &r) {
   tb::LaunchPlan plan;
-  plan.row_warps = tb::kRWWalkers * r.rows_per_warp / 32;
+  plan.row_warps = std::max(1, tb::kRWUnitRows * r.units / 32);
   plan.tree_threads = tb::kRWWalkers;
   plan.rows_per_lane = 1;
   plan.chunks = r.chunks;
@@ -622,12 +642,15 @@ tb::LaunchPlan rank_launch_plan(const RankPlan &r) {
 // chunks has an arrival counter for every row batch.
 int64_t rank_rows_per_pass(const tbk_forest *f) {
   const int64_t by_keys = ((int64_t)96 << 20) / rank_stride(f->rf.num_features);
-  const int64_t round = (int64_t)tb::kRWWalkers * 16 * f->num_sms;
+  const int64_t round = (int64_t)tb::kRWBatchRows * f->num_sms;
   return std::max(round, by_keys / round * round);
 }
 
+size_t rank_key_bytes(const tbk_forest *f, int64_t rows) { // (the last pair of rows may be half empty)
+  return ((size_t)(rows + 1) * rank_stride(f->rf.num_features) + 255) / 256 * 256;
+}
 size_t rank_workspace_bytes(const tbk_forest *f, const RankPlan &plan, int64_t rows) {
-  size_t bytes = tb::kRankArrivalBytes + ((size_t)rows * rank_stride(f->rf.num_features) + 255) / 256 * 256;
+  size_t bytes = tb::kRankArrivalBytes + rank_key_bytes(f, rows);
   if (plan.chunks > 1) bytes += (size_t)plan.chunks * rows * (f->rf.num_classes > 0 ? 8 : 4);
   return bytes;
 }
@@ -647,24 +670,32 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
   p.num_features = F;
   p.stride = rank_stride(F);
   p.vec4_ok = F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
+  p.lattice = q.lattice;
   p.searched = f->d_ties;
+  const bool pair = F <= tb::kRankPairFeatures;
+  const int64_t lines = pair ? (n + 1) / 2 : n;
   // Tables in shared memory pay once every SM has a few thousand values to rank: loading them
   // takes about as long as ranking 2000 values through L2 (a gather there costs a wavefront per lane).
   if (f->rank_width > 0 && n * F > (int64_t)f->num_sms * 2048) {
     const int w = f->rank_width, slabs = (F + w * f->rank_pieces - 1) / (w * f->rank_pieces);
     p.pieces = f->rank_pieces;
-    const int64_t want = (n * p.pieces + 1023) / 1024;
+    const int64_t want = (lines * p.pieces + 1023) / 1024;
     const dim3 grid((unsigned)std::min<int64_t>(want, std::max(1, f->num_sms / slabs)), (unsigned)slabs);
     using K = void (*)(const tb::RankRowsParams);
-    const K k = w == 8 ? tb::tb_rank_rows<8, true> : w == 4 ? tb::tb_rank_rows<4, true>
-                : w == 2 ? tb::tb_rank_rows<2, true> : tb::tb_rank_rows<1, true>;
+    const K k = pair ? (w == 4 ? tb::tb_rank_rows<4, true, true> : w == 2 ? tb::tb_rank_rows<2, true, true> : tb::tb_rank_rows<1, true, true>)
+                     : (w == 8   ? tb::tb_rank_rows<8, false, true>
+                        : w == 4 ? tb::tb_rank_rows<4, false, true>
+                        : w == 2 ? tb::tb_rank_rows<2, false, true>
+                                 : tb::tb_rank_rows<1, false, true>);
     const int rc = allow_smem(f, (const void *)k);
     if (rc) return rc;
     k<<<grid, 1024, f->rank_smem, stream>>>(p);
   } else {
-    p.pieces = (F + 7) / 8;
-    const int64_t want = (n * p.pieces + 255) / 256;
-    tb::tb_rank_rows<8, false><<<(unsigned)std::min<int64_t>(want, 8ll * f->num_sms), 256, 0, stream>>>(p);
+    // (one feature per thread: a small batch is all latency)
+    p.pieces = F;
+    const unsigned grid = (unsigned)std::min<int64_t>((lines * p.pieces + 255) / 256, 8ll * f->num_sms);
+    if (pair) tb::tb_rank_rows<1, true, false><<<grid, 256, 0, stream>>>(p);
+    else tb::tb_rank_rows<1, false, false><<<grid, 256, 0, stream>>>(p);
   }
   CUDA_TRY(cudaGetLastError());
   ++f->launches;
@@ -683,9 +714,8 @@ void plan_rank_tables(tbk_forest *f) {
     return b;
   };
   f->rank_width = 0;
-  for (int w : {8, 4, 2, 1}) {
-    const int all = (F + w - 1) / w;
-    for (int pieces = w == 8 ? all : 1; pieces >= 1; --pieces) {
+  for (int w = F <= tb::kRankPairFeatures ? 4 : 8; w >= 1; w /= 2) {
+    for (int pieces = (F + w - 1) / w; pieces >= 1; --pieces) {
       size_t most = 0;
       for (int first = 0; first < F; first += w * pieces) most = std::max(most, bytes(first, std::min(F, first + w * pieces)));
       if (most <= (size_t)room) {
@@ -706,7 +736,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   int64_t pass = std::min(n_rows, rank_rows_per_pass(f));
   RankPlan plan = plan_rank(f, pass, mode == kLeafIds);
   if (plan.chunks > 1) {
-    pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * tb::kRWWalkers * plan.rows_per_warp);
+    pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * tb::kRWUnitRows);
     plan = plan_rank(f, pass, mode == kLeafIds);
   }
   f->last_plan = rank_launch_plan(plan);
@@ -714,7 +744,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   int rc = workspace_acquire(f, stream, rank_workspace_bytes(f, plan, pass), &ws);
   if (rc) return rc;
   unsigned char *keys = ws->mem + tb::kRankArrivalBytes;
-  const RankKernel kernel = pick_rank_kernel(S, plan.rows_per_warp, q.whole_compare != 0, kmode);
+  const RankKernel kernel = pick_rank_kernel(S, q.whole_compare != 0, kmode);
   rc = allow_smem(f, (const void *)kernel);
   if (rc) return rc;
   tb::RankWalkParams p{};
@@ -725,7 +755,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   p.tree_index = f->d_rtree_index;
   p.class_begin = f->d_rclass_begin;
   p.keys = keys;
-  p.scratch = reinterpret_cast<float *>(keys + ((size_t)pass * S + 255) / 256 * 256);
+  p.scratch = reinterpret_cast<float *>(keys + rank_key_bytes(f, pass));
   p.arrivals = reinterpret_cast<unsigned int *>(ws->mem);
   p.num_trees = q.num_trees;
   p.num_groups = (int32_t)q.groups.size();
@@ -751,9 +781,9 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     p.skip_first_copy = f->expire_next_wait ? 1 : 0;
     p.wait_tries = f->expire_next_wait ? 2000u : 0u;
     f->expire_next_wait = false;
-    const int64_t batches = (n + tb::kRWWalkers * plan.rows_per_warp - 1) / (tb::kRWWalkers * plan.rows_per_warp);
+    const int64_t units = (n + tb::kRWUnitRows - 1) / tb::kRWUnitRows; // (chunks: at most four units to a block)
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)std::min(batches, plan.grid_x), (unsigned)plan.chunks);
+    cfg.gridDim = dim3((unsigned)std::min(units, plan.grid_x), (unsigned)plan.chunks);
     cfg.blockDim = dim3(tb::kRWThreads);
     cfg.dynamicSmemBytes = (size_t)plan.smem;
     cfg.stream = stream;
@@ -1261,6 +1291,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     f->rf.num_trees = q.num_trees;
     f->rf.num_nodes = q.num_nodes;
     f->rf.max_depth = q.max_depth;
+    f->rf.lattice = q.lattice;
     f->rf.whole_compare = q.whole_compare;
     f->rf.groups = q.groups;
     f->rf.features = q.features;

@@ -1,16 +1,16 @@
 // Walk kernel for rank keys (rank_pack.h): forests of at most 8 levels over rows of at most 64
 // features.
 //
-// LANE = TREE.  A warp owns R rows of the batch and walks them through the 32 trees of a group,
-// one tree per lane, four rows in lock-step.  What that buys over lane = row:
-//  * a lane's tree is the same for all R rows, so the nodes of its two topmost levels live in
+// LANE = TREE.  A warp owns up to 16 rows of the batch and walks them through the 32 trees of a
+// group, one tree per lane, four rows in lock-step.  What that buys over lane = row:
+//  * a lane's tree is the same for all its rows, so the nodes of its two topmost levels live in
 //    registers and cost no shared-memory load;
 //  * the keys of one row are read by all lanes at once: 16-bit keys of up to 64 features lie in
 //    32 words, so whatever features the 32 trees ask for, the load is one wavefront;
-//  * leaf values are added to R running sums per lane and meet across lanes once per batch, not
+//  * leaf values are added to 16 running sums per lane and meet across lanes once per batch, not
 //    once per tree: no table of leaf numbers, no second set of warps, and every sum has only
 //    trees / 32 terms;
-//  * a warp's work is R rows, not 32: small batches still spread over the GPU.
+//  * a warp's work is 4 to 16 rows, not 32: small batches still spread over the GPU.
 // Node loads are conflict-free (32 columns = 32 banks).  A level costs a node load, a shift-add to
 // the key's address, a key load, a comparison and a predicated add (rank_pack.h on the slot
 // numbering); a tree of 8 levels 15 shared-memory wavefronts and about 40 instructions.  Bound:
@@ -18,11 +18,13 @@
 //
 // A block = 20 walker warps, a warp that streams the tree groups (node plane and leaf plane of a
 // group = one stage, as many stages as fit) and a warp that fetches the keys of the next batch of
-// 20 R rows while the current one is walked.  All hand-offs are mbarriers with bounded waits; a
-// wait that gives up ends the launch with a status word.  Blocks are persistent over row batches
-// (blockIdx.x, + gridDim.x, ...); blockIdx.y is a chunk of the trees.  With several chunks a block
-// takes one row batch, leaves its partial sums in scratch memory, and the last block to finish
-// with a row batch adds them up in chunk order: one launch, and the same result every time.
+// rows while the current one is walked.  All hand-offs are mbarriers with bounded waits; a
+// wait that gives up ends the launch with a status word.  The rows are dealt to the blocks of a
+// row (blockIdx.x) evenly in units of 80 (4 per warp), so that all end at the same time; a block
+// takes its share in batches of up to 4 units, 16 rows per warp.  blockIdx.y is a chunk of the
+// trees: with several chunks a block has one batch, leaves its partial sums in scratch memory, and
+// the last block to finish with a batch adds them up in chunk order -- one launch, and the same
+// result every time.
 //
 // Multiclass: the running sums belong to one class at a time (a class owns consecutive columns);
 // when the class changes they are combined across the lanes -- afterwards a lane holds the class
@@ -63,13 +65,14 @@ struct RankWalkParams {
 };
 
 constexpr int kRWWalkers = 20, kRWThreads = 32 * (kRWWalkers + 2);
+constexpr int kRWUnitRows = 4 * kRWWalkers, kRWBatchUnits = 4, kRWBatchRows = kRWUnitRows * kRWBatchUnits;
 constexpr int kRWBarBytes = 256; // full[8], empty[8], keys_full[2], keys_empty[2]; flag at 192
 constexpr int kRWMaxStages = 8;
 constexpr int kRankArrivals = 4096;                    // row batches of a launch with several tree chunks
 constexpr size_t kRankArrivalBytes = 4 * kRankArrivals;
 
-__host__ __device__ constexpr int rank_walk_smem_bytes(int rows_per_warp, int stride, int stages, uint32_t stage_bytes) {
-  return kRWBarBytes + 2 * kRWWalkers * rows_per_warp * stride + stages * (int)stage_bytes;
+__host__ __device__ constexpr int rank_walk_smem_bytes(int stride, int stages, uint32_t stage_bytes) {
+  return kRWBarBytes + 2 * kRWBatchRows * stride + stages * (int)stage_bytes;
 }
 
 template <int IMM> __device__ __forceinline__ uint32_t lds_u32_imm(uint32_t a) {
@@ -92,50 +95,95 @@ template <bool WHOLE, uint32_t IMM> __device__ __forceinline__ void rank_step(ui
     asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %1, %2;\n @p add.u32 %0, %0, %3;\n}"
                  : "+r"(off) : "r"(key), "r"(node), "n"(IMM));
 }
-// The decision at the root: picks the node of level 1 and the offset together.
-template <bool WHOLE>
-__device__ __forceinline__ void rank_root(uint32_t &off, uint32_t &next, uint32_t key, uint32_t root, uint32_t off_left,
-                                          uint32_t off_right, uint32_t left, uint32_t right) {
+// The nodes of a lane's tree that live in registers: levels 0 to 2.
+struct RankTop {
+  uint32_t root;   // the root's threshold rank, in both halves where two rows are decided together
+  uint32_t ka0;    // address of the root's key of row 0
+  uint32_t n1[2];  // level 1
+  uint32_t n2[4];  // level 2
+};
+// What the decision at the root leaves of them: the node of level 1, the two of level 2 that are
+// still possible, the offset.
+struct RankPath {
+  uint32_t off, node, lo2, hi2;
+};
+#define TBR_ROOT_SELECTS(p, off, node, lo2, hi2)                                                                    \
+  " selp.b32 " off ", %11, %10, " p ";\n selp.b32 " node ", %13, %12, " p ";\n"                                    \
+  " selp.b32 " lo2 ", %15, %14, " p ";\n selp.b32 " hi2 ", %17, %16, " p ";\n"
+#define TBR_ROOT_OPERANDS                                                                                           \
+  "r"(t.root), "r"(col), "r"(col + 128u), "r"(t.n1[0]), "r"(t.n1[1]), "r"(t.n2[0]), "r"(t.n2[1]), "r"(t.n2[2]), "r"(t.n2[3])
+// Two rows whose keys share a word: one comparison decides both.
+__device__ __forceinline__ void rank_root_pair(RankPath &a, RankPath &b, uint32_t keys, const RankTop &t, uint32_t col) {
+  asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %8, %9;\n"
+               TBR_ROOT_SELECTS("p", "%0", "%1", "%2", "%3") TBR_ROOT_SELECTS("q", "%4", "%5", "%6", "%7") "}"
+               : "=&r"(a.off), "=&r"(a.node), "=&r"(a.lo2), "=&r"(a.hi2), "=&r"(b.off), "=&r"(b.node), "=&r"(b.lo2), "=&r"(b.hi2)
+               : "r"(keys), TBR_ROOT_OPERANDS);
+}
+template <bool WHOLE> __device__ __forceinline__ void rank_root_one(RankPath &a, uint32_t key, const RankTop &t, uint32_t col) {
+  const bool right = WHOLE ? key >= (t.root & 0xffffu) : false;
+  if constexpr (WHOLE) {
+    a.off = right ? col + 128u : col;
+    a.node = right ? t.n1[1] : t.n1[0];
+    a.lo2 = right ? t.n2[1] : t.n2[0];
+    a.hi2 = right ? t.n2[3] : t.n2[2];
+  } else {
+    [[maybe_unused]] uint32_t x0, x1, x2, x3;
+    asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %8, %9;\n" TBR_ROOT_SELECTS("p", "%0", "%1", "%2", "%3")
+                 " mov.b32 %4, 0;\n mov.b32 %5, 0;\n mov.b32 %6, 0;\n mov.b32 %7, 0;\n}"
+                 : "=&r"(a.off), "=&r"(a.node), "=&r"(a.lo2), "=&r"(a.hi2), "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3)
+                 : "r"(key), TBR_ROOT_OPERANDS);
+  }
+}
+// The decision on level 1 also picks the node of level 2.
+template <bool WHOLE> __device__ __forceinline__ void rank_step1(RankPath &a, uint32_t key) {
   if constexpr (WHOLE)
-    asm volatile("{\n .reg .pred p;\n .reg .b32 t;\n and.b32 t, %3, 0xffff;\n setp.ge.u32 p, %2, t;\n"
-                 " selp.b32 %0, %5, %4, p;\n selp.b32 %1, %7, %6, p;\n}"
-                 : "=&r"(off), "=&r"(next)
-                 : "r"(key), "r"(root), "r"(off_left), "r"(off_right), "r"(left), "r"(right));
+    asm volatile("{\n .reg .pred p;\n .reg .b32 t;\n and.b32 t, %1, 0xffff;\n setp.ge.u32 p, %2, t;\n @p add.u32 %0, %0, 256;\n"
+                 " selp.b32 %1, %4, %3, p;\n}"
+                 : "+r"(a.off), "+r"(a.node) : "r"(key), "r"(a.lo2), "r"(a.hi2));
   else
-    asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %2, %3;\n"
-                 " selp.b32 %0, %5, %4, p;\n selp.b32 %1, %7, %6, p;\n}"
-                 : "=&r"(off), "=&r"(next)
-                 : "r"(key), "r"(root), "r"(off_left), "r"(off_right), "r"(left), "r"(right));
+    asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %2, %1;\n @p add.u32 %0, %0, 256;\n selp.b32 %1, %4, %3, p;\n}"
+                 : "+r"(a.off), "+r"(a.node) : "r"(key), "r"(a.lo2), "r"(a.hi2));
 }
 
-// Walks four rows (keys at kb + (ROW0 + q) * S) through this lane's tree of depth D, whose
+// Offset of row r's keys from row 0's: rows in pairs share the words of a 128-byte line.
+template <int S> __host__ __device__ constexpr int rank_row_offset(int r) { return S == 64 ? (r >> 1) * 128 + (r & 1) * 2 : r * S; }
+
+// Walks rows ROW0 .. ROW0 + 3 (row 0's keys at kb) through this lane's tree of depth D, whose
 // column starts at `col` (node plane; leaf plane 2^D * 128 bytes on); v = leaf words.
 template <int D, int S, int ROW0, bool WHOLE>
-__device__ __forceinline__ void rank_walk4(uint32_t (&v)[4], uint32_t col, uint32_t kb, uint32_t root, uint32_t ka0,
-                                           uint32_t left, uint32_t right) {
-  uint32_t off[4], node[4], key[4];
+__device__ __forceinline__ void rank_walk4(uint32_t (&v)[4], uint32_t col, uint32_t kb, const RankTop &t) {
+  RankPath a[4];
+  uint32_t key[4];
 #define TBR_ROWS(stmt)                                                                                              \
-  { constexpr int q = 0; stmt; } { constexpr int q = 1; stmt; } { constexpr int q = 2; stmt; } { constexpr int q = 3; stmt; }
-  TBR_ROWS(key[q] = lds_u16_imm<(ROW0 + q) * S>(ka0))
-  TBR_ROWS((rank_root<WHOLE>(off[q], node[q], key[q], root, col, col + 128u, left, right)))
+  { { constexpr int q = 0; stmt; } { constexpr int q = 1; stmt; } { constexpr int q = 2; stmt; } { constexpr int q = 3; stmt; } }
+  if constexpr (S == 64 && !WHOLE) {
+    key[0] = lds_u32_imm<rank_row_offset<S>(ROW0)>(t.ka0);
+    key[2] = lds_u32_imm<rank_row_offset<S>(ROW0 + 2)>(t.ka0);
+    rank_root_pair(a[0], a[1], key[0], t, col);
+    rank_root_pair(a[2], a[3], key[2], t, col);
+  } else {
+    TBR_ROWS(key[q] = lds_u16_imm<rank_row_offset<S>(ROW0 + q)>(t.ka0))
+    TBR_ROWS(rank_root_one<WHOLE>(a[q], key[q], t, col))
+  }
 #define TBR_DECIDE(level)                                                                                           \
   if constexpr (D > level) {                                                                                        \
-    if constexpr (level > 1) TBR_ROWS(node[q] = lds_u32_imm<128 * ((1 << level) - 1)>(off[q]))                      \
-    TBR_ROWS(key[q] = lds_u16_imm<(ROW0 + q) * S>((node[q] >> 16) + kb))                                            \
-    TBR_ROWS((rank_step<WHOLE, (128u << level)>(off[q], key[q], node[q])))                                          \
+    if constexpr (level > 2) TBR_ROWS(a[q].node = lds_u32_imm<128 * ((1 << level) - 1)>(a[q].off))                  \
+    TBR_ROWS(key[q] = lds_u16_imm<rank_row_offset<S>(ROW0 + q)>((a[q].node >> 16) + kb))                            \
+    if constexpr (level == 1) TBR_ROWS(rank_step1<WHOLE>(a[q], key[q]))                                             \
+    else TBR_ROWS((rank_step<WHOLE, (128u << level)>(a[q].off, key[q], a[q].node)))                                 \
   }
   TBR_DECIDE(1) TBR_DECIDE(2) TBR_DECIDE(3) TBR_DECIDE(4) TBR_DECIDE(5) TBR_DECIDE(6) TBR_DECIDE(7)
-  TBR_ROWS(v[q] = lds_u32_imm<(128 << D)>(off[q]))
+  TBR_ROWS(v[q] = lds_u32_imm<(128 << D)>(a[q].off))
 #undef TBR_DECIDE
 #undef TBR_ROWS
 }
 
-// Adds up v over the 32 lanes for every of R rows: afterwards lane l holds the sum of row
-// l * R / 32 (32 / R neighbouring lanes hold the same row).
-template <int R> __device__ __forceinline__ float rank_reduce_rows(float (&v)[R], int lane) {
+// Adds up v over the 32 lanes for every of 16 rows: afterwards lanes 2i and 2i + 1 hold the sum
+// of row i.
+__device__ __forceinline__ float rank_reduce_rows(float (&v)[16], int lane) {
   int bit = 16;
 #pragma unroll
-  for (int half = R / 2; half >= 1; half /= 2, bit /= 2) {
+  for (int half = 8; half >= 1; half /= 2, bit /= 2) {
     const bool up = lane & bit;
 #pragma unroll
     for (int i = 0; i < half; ++i) {
@@ -143,62 +191,70 @@ template <int R> __device__ __forceinline__ float rank_reduce_rows(float (&v)[R]
       v[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
     }
   }
-  float s = v[0];
-  for (; bit >= 1; bit /= 2) s += __shfl_xor_sync(0xffffffffu, s, bit);
-  return s;
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
-// One group of depth D for all R rows of the warp; use(c, v) takes the leaf words of rows 4c .. 4c+3.
-template <int D, int S, int R, bool WHOLE, typename Use>
-__device__ __forceinline__ void rank_walk_rows(uint32_t col, uint32_t kb, Use use) {
-  const uint32_t root = lds_u32_imm<0>(col), ka0 = (root >> 16) + kb;
-  uint32_t left = 0, right = 0, v[4];
+// One group of depth D for the warp's rows, four times `fours` of them; use(c, v) takes the leaf
+// words of rows 4c .. 4c+3.
+template <int D, int S, bool WHOLE, typename Use>
+__device__ __forceinline__ void rank_walk_rows(int fours, uint32_t col, uint32_t kb, Use use) {
+  RankTop t{};
+  uint32_t v[4];
+  t.root = lds_u32_imm<0>(col);
+  t.ka0 = (t.root >> 16) + kb;
+  if constexpr (S == 64 && !WHOLE) t.root = __byte_perm(t.root, t.root, 0x1010);
   if constexpr (D > 1) {
-    left = lds_u32_imm<128>(col);
-    right = lds_u32_imm<256>(col);
+    t.n1[0] = lds_u32_imm<128>(col);
+    t.n1[1] = lds_u32_imm<256>(col);
   }
-  rank_walk4<D, S, 0, WHOLE>(v, col, kb, root, ka0, left, right);
+  if constexpr (D > 2) {
+    t.n2[0] = lds_u32_imm<384>(col);
+    t.n2[1] = lds_u32_imm<512>(col);
+    t.n2[2] = lds_u32_imm<640>(col);
+    t.n2[3] = lds_u32_imm<768>(col);
+  }
+  rank_walk4<D, S, 0, WHOLE>(v, col, kb, t);
   use(0, v);
-  if constexpr (R > 4) {
-    rank_walk4<D, S, 4, WHOLE>(v, col, kb, root, ka0, left, right);
-    use(1, v);
-  }
-  if constexpr (R > 8) {
-    rank_walk4<D, S, 8, WHOLE>(v, col, kb, root, ka0, left, right);
-    use(2, v);
-    rank_walk4<D, S, 12, WHOLE>(v, col, kb, root, ka0, left, right);
-    use(3, v);
-  }
+  if (fours == 1) return;
+  rank_walk4<D, S, 4, WHOLE>(v, col, kb, t);
+  use(1, v);
+  if (fours == 2) return;
+  rank_walk4<D, S, 8, WHOLE>(v, col, kb, t);
+  use(2, v);
+  if (fours == 3) return;
+  rank_walk4<D, S, 12, WHOLE>(v, col, kb, t);
+  use(3, v);
 }
-template <int S, int R, bool WHOLE, typename Use>
-__device__ __forceinline__ void rank_walk_group(uint32_t depth, uint32_t col, uint32_t kb, Use use) {
+template <int S, bool WHOLE, typename Use>
+__device__ __forceinline__ void rank_walk_group(uint32_t depth, int fours, uint32_t col, uint32_t kb, Use use) {
   switch (depth) {
-  case 1: return rank_walk_rows<1, S, R, WHOLE>(col, kb, use);
-  case 2: return rank_walk_rows<2, S, R, WHOLE>(col, kb, use);
-  case 3: return rank_walk_rows<3, S, R, WHOLE>(col, kb, use);
-  case 4: return rank_walk_rows<4, S, R, WHOLE>(col, kb, use);
-  case 5: return rank_walk_rows<5, S, R, WHOLE>(col, kb, use);
-  case 6: return rank_walk_rows<6, S, R, WHOLE>(col, kb, use);
-  case 7: return rank_walk_rows<7, S, R, WHOLE>(col, kb, use);
-  default: return rank_walk_rows<8, S, R, WHOLE>(col, kb, use);
+  case 1: return rank_walk_rows<1, S, WHOLE>(fours, col, kb, use);
+  case 2: return rank_walk_rows<2, S, WHOLE>(fours, col, kb, use);
+  case 3: return rank_walk_rows<3, S, WHOLE>(fours, col, kb, use);
+  case 4: return rank_walk_rows<4, S, WHOLE>(fours, col, kb, use);
+  case 5: return rank_walk_rows<5, S, WHOLE>(fours, col, kb, use);
+  case 6: return rank_walk_rows<6, S, WHOLE>(fours, col, kb, use);
+  case 7: return rank_walk_rows<7, S, WHOLE>(fours, col, kb, use);
+  default: return rank_walk_rows<8, S, WHOLE>(fours, col, kb, use);
   }
 }
 
 enum RankMode { kRankSums, kRankClasses, kRankLeafIds };
 
-// S: bytes per row of keys; R: rows per warp.
-template <int S, int R, bool WHOLE, int MODE>
+// S: bytes per row of keys.
+template <int S, bool WHOLE, int MODE>
 __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankWalkParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); // uniform by construction
-  constexpr int RB = kRWWalkers * R;                      // rows per batch
   const uint32_t bars_s = smem_u32(smem_raw);
   const uint32_t full_s = bars_s, empty_s = bars_s + 64u, keys_full_s = bars_s + 128u, keys_empty_s = bars_s + 144u;
   volatile uint32_t *last_flag = reinterpret_cast<volatile uint32_t *>(smem_raw + 192);
   unsigned char *keys = smem_raw + kRWBarBytes;           // two batches of keys
-  unsigned char *ring = keys + 2 * RB * S;
-  const int num_batches = (int)((p.n_rows + RB - 1) / RB);
-  const int my_batches = (num_batches - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  unsigned char *ring = keys + 2 * kRWBatchRows * S;
+  // this block's units of rows, in batches of up to four
+  const long long units = (p.n_rows + kRWUnitRows - 1) / kRWUnitRows;
+  const int unit0 = (int)(units * blockIdx.x / gridDim.x), unit1 = (int)(units * (blockIdx.x + 1) / gridDim.x);
+  const int my_batches = (unit1 - unit0 + kRWBatchUnits - 1) / kRWBatchUnits;
   // this chunk's groups; with classes: those that hold the columns of classes c0 .. c1 - 1
   int g0 = (int)blockIdx.y * p.groups_per_chunk, g1 = min(p.num_groups, g0 + p.groups_per_chunk);
   [[maybe_unused]] int c0 = 0, c1 = 0, col0 = 0;
@@ -261,31 +317,31 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
       if (it >= 2) ok = wait(keys_empty_s + 8u * buf, (uint32_t)((it >> 1) - 1) & 1u);
       issued += ok;
       if (ok && lane == 0) {
-        const long long row0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * RB;
-        const uint32_t bytes = (uint32_t)min((long long)RB, p.n_rows - row0) * (uint32_t)S;
+        const int u = unit0 + it * kRWBatchUnits;
+        const long long row0 = (long long)u * kRWUnitRows, end = (long long)min(unit1, u + kRWBatchUnits) * kRWUnitRows;
+        const uint32_t bytes = ((uint32_t)(min(end, p.n_rows) - row0) + 1u & ~1u) * (uint32_t)S; // (rows may lie in pairs)
         uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw) + 16 + buf;
         mbar_expect_tx(bar, bytes);
-        bulk_g2s_hint(keys + (size_t)buf * RB * S, p.keys + row0 * S, bytes, bar, stream);
+        bulk_g2s_hint(keys + (size_t)buf * kRWBatchRows * S, p.keys + row0 * S, bytes, bar, stream);
       }
     }
   } else {
     // ---- the walkers
     const bool elected = lane == 0;
     const uint32_t ring_col = smem_u32(ring) + (uint32_t)lane * 4u;
-    const int my_row = warp * R + lane * R / 32;       // the row whose sum this lane ends up with
-    const bool writer = (lane & (32 / R - 1)) == 0;
     int slot = 0;
     uint32_t parity = 0;
     for (int it = 0; it < my_batches && ok; ++it) {
-      const long long row0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * RB;
-      const long long row = row0 + my_row;
-      const bool live = writer && row < p.n_rows;
+      const int fours = min(unit1 - unit0 - it * kRWBatchUnits, kRWBatchUnits); // rows per warp / 4
+      const long long row0 = (long long)(unit0 + it * kRWBatchUnits) * kRWUnitRows + warp * fours * 4;
+      const long long row = row0 + (lane >> 1); // the row whose sum this lane ends up with
+      const bool live = (lane & 1) == 0 && lane < 8 * fours && row < p.n_rows;
       ok = wait(keys_full_s + 8u * ((uint32_t)it & 1u), (uint32_t)(it >> 1) & 1u);
       if (!ok) break;
-      const uint32_t kb = smem_u32(keys) + ((uint32_t)it & 1u) * (uint32_t)(RB * S) + (uint32_t)(warp * R * S);
-      float acc[R];
+      const uint32_t kb = smem_u32(keys) + ((uint32_t)it & 1u) * (uint32_t)(kRWBatchRows * S) + (uint32_t)(warp * fours * 4 * S);
+      float acc[16];
 #pragma unroll
-      for (int i = 0; i < R; ++i) acc[i] = 0.f;
+      for (int i = 0; i < 16; ++i) acc[i] = 0.f;
       [[maybe_unused]] int cls = c0, lo = col0 & 31, best_class = c0;
       [[maybe_unused]] float sum = 0.f, best = -INFINITY;
       // class `cls` is complete, its sum for this lane's row in `sum`
@@ -309,9 +365,9 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
         const uint32_t col = ring_col + (uint32_t)slot * p.stage_bytes;
         if constexpr (MODE == kRankLeafIds) {
           const int t = p.tree_index[(g0 + k) * 32 + lane];
-          int32_t *dst = p.leaf_ids + (row0 + warp * R) * p.num_trees + t;
-          const int rows = (int)min((long long)R, p.n_rows - (row0 + warp * R));
-          rank_walk_group<S, R, WHOLE>(depth, col, kb, [&](int c, const uint32_t(&v)[4]) {
+          int32_t *dst = p.leaf_ids + row0 * p.num_trees + t;
+          const int rows = (int)min(16ll, p.n_rows - row0);
+          rank_walk_group<S, WHOLE>(depth, fours, col, kb, [&](int c, const uint32_t(&v)[4]) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               if (t >= 0 && 4 * c + q < rows) dst[(4 * c + q) * p.num_trees] = (int32_t)v[q];
@@ -323,28 +379,51 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
           };
           if constexpr (MODE == kRankClasses) {
             int next = p.class_begin[cls + 1] - (g0 + k) * 32; // first column of the next class
-            const bool pure = lo == 0 && next >= 32;
-            if (!pure && lo == 0) { // the group starts in this class and ends in another
-              sum += rank_reduce_rows<R>(acc, lane);
+            auto combine = [&](float(&v)[16]) { sum += rank_reduce_rows(v, lane); };
+            if (lo == 0 && next >= 32) { // one class
+              rank_walk_group<S, WHOLE>(depth, fours, col, kb, add);
+              if (next == 32) {
+                combine(acc);
+                finish();
 #pragma unroll
-              for (int i = 0; i < R; ++i) acc[i] = 0.f;
-            }
-            rank_walk_group<S, R, WHOLE>(depth, col, kb, add);
-            while (cls < c1 && next <= 32) { // classes that end in this group
-              float part[R];
+                for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+              }
+            } else if (lo == 0 && cls + 1 < c1 && p.class_begin[cls + 2] - (g0 + k) * 32 > 32) {
+              // two classes: this one's columns complete its sums, the others start the next one's
+              float other[16];
 #pragma unroll
-              for (int i = 0; i < R; ++i) part[i] = lane >= lo && lane < next ? acc[i] : 0.f;
-              sum += rank_reduce_rows<R>(part, lane);
+              for (int i = 0; i < 16; ++i) other[i] = 0.f;
+              rank_walk_group<S, WHOLE>(depth, fours, col, kb, [&](int c, const uint32_t(&v)[4]) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  acc[4 * c + q] += lane < next ? __uint_as_float(v[q]) : 0.f;
+                  other[4 * c + q] = lane < next ? 0.f : __uint_as_float(v[q]);
+                }
+              });
+              combine(acc);
               finish();
-              lo = next;
-              if (cls < c1) next = p.class_begin[cls + 1] - (g0 + k) * 32;
-            }
-            if (lo > 0)
 #pragma unroll
-              for (int i = 0; i < R; ++i) acc[i] = lane >= lo ? acc[i] : 0.f;
-            lo = 0;
+              for (int i = 0; i < 16; ++i) acc[i] = other[i];
+            } else { // several, or a chunk that starts or ends inside the group
+              if (lo == 0) combine(acc);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+              rank_walk_group<S, WHOLE>(depth, fours, col, kb, add);
+              while (cls < c1 && next <= 32) { // classes that end in this group
+                float part[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) part[i] = lane >= lo && lane < next ? acc[i] : 0.f;
+                combine(part);
+                finish();
+                lo = next;
+                if (cls < c1) next = p.class_begin[cls + 1] - (g0 + k) * 32;
+              }
+#pragma unroll
+              for (int i = 0; i < 16; ++i) acc[i] = lane >= lo ? acc[i] : 0.f;
+              lo = 0;
+            }
           } else {
-            rank_walk_group<S, R, WHOLE>(depth, col, kb, add);
+            rank_walk_group<S, WHOLE>(depth, fours, col, kb, add);
           }
         }
         __syncwarp();
@@ -358,7 +437,7 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
       if (elected) mbar_arrive(keys_empty_s + 8u * ((uint32_t)it & 1u));
       // ---- the batch's results
       if constexpr (MODE == kRankSums) {
-        const float s = rank_reduce_rows<R>(acc, lane);
+        const float s = rank_reduce_rows(acc, lane);
         if (live) {
           if (gridDim.y > 1) p.scratch[(long long)blockIdx.y * p.n_rows + row] = s;
           else if (p.write_partial) p.partial[row] = s;
@@ -395,8 +474,8 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
   __syncthreads();
   if (!*last_flag) return;
   __threadfence();
-  const long long row = (long long)blockIdx.x * RB + tid;
-  if (tid >= RB || row >= p.n_rows) return;
+  const long long row = (long long)unit0 * kRWUnitRows + tid;
+  if (row >= min((long long)unit1 * kRWUnitRows, p.n_rows)) return;
   if constexpr (MODE == kRankClasses) {
     float best = -INFINITY;
     int best_class = 0;
