@@ -434,12 +434,7 @@ void run_batch(InferenceRunner *r, void *inputs, void *results, int64_t rows) {
         if (us > 0) r->kernelMicros += us;
       }
     }
-    if (rc == TBK_OK && cudaDeviceSynchronize() != cudaSuccess) {
-      rc = TBK_ERR_CUDA;
-      set_error(rc, "cudaDeviceSynchronize failed after the walk");
-      return;
-    }
-    if (rc == TBK_OK) rc = tbk_check_status(r->forest);
+    if (rc == TBK_OK) rc = tbk_check_status(r->forest); // (synchronises)
   } else if (g_measure_kernel_time) {
     // timed mode: copy once, then time the kernel alone, as the reference's
     // generated host code does around its launch

@@ -76,7 +76,7 @@ struct tbk_forest {
   int32_t *d_orig_node = nullptr;
   unsigned long long *d_orig_off = nullptr;
   int8_t *d_lut = nullptr;
-  int32_t *d_status = nullptr;
+  int32_t *h_status = nullptr, *d_status = nullptr; // status word in mapped host memory, both addresses
   float *d_scratch = nullptr; // tree-chunk partials, two slots
   size_t scratch_bytes = 0;
   // a slot's last user: a call on another stream waits for it before reusing the slot
@@ -123,14 +123,15 @@ struct tbk_forest {
   tb::DeepForest df;
   int deep_row_warps = 0, deep_slots = 0;
   int uniform_depth = 0; // key layouts: depth shared by all groups / pairs, 0 = mixed
-  // host pipeline
-  float *d_in[2] = {nullptr, nullptr};
-  unsigned char *d_res[2] = {nullptr, nullptr};
-  float *h_pin[2] = {nullptr, nullptr};
-  unsigned char *h_res = nullptr;
-  size_t pipe_rows = 0, pipe_ld = 0, h_res_bytes = 0;
+  // host pipeline: slots of device buffers and pinned staging that a large batch streams through,
+  // and one pinned buffer that the kernels read and write directly for small batches
+  static constexpr int kPipeSlots = 4;
+  unsigned char *d_in[kPipeSlots] = {}, *d_res[kPipeSlots] = {}, *h_pin[kPipeSlots] = {}, *h_res[kPipeSlots] = {};
+  size_t pipe_bytes = 0, pipe_rows = 0; // capacity of a slot
+  unsigned char *h_small = nullptr, *d_small = nullptr, *d_small_in = nullptr;
   cudaStream_t streams[2] = {nullptr, nullptr};
-  cudaEvent_t in_free[2] = {nullptr, nullptr};
+  cudaEvent_t slot_done[kPipeSlots] = {};
+  int64_t host_batch_rows = 0; // rows of the host batch whose chunks are being predicted
   // timing
   bool timing = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -824,9 +825,13 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
   tb::ForestShape shape{pk.num_features, pk.num_classes, (int64_t)pk.groups.size(), pk.max_group_bytes,
                         (int32_t)pk.lut.size(), pk.representation, pk.tile_size};
   tb::LaunchPlan plan;
-  std::string why = tb::select_launch(shape, f->user, n_rows, f->max_smem_optin, f->num_sms, mode == kLeafIds, &plan,
-                                      mode == kPartial);
+  // (a chunk of a host batch is walked in the shape of the whole batch: its sums then have the
+  // order, and so every bit, of the same batch in device memory)
+  std::string why = tb::select_launch(shape, f->user, std::max(n_rows, f->host_batch_rows), f->max_smem_optin, f->num_sms,
+                                      mode == kLeafIds, &plan, mode == kPartial);
   if (!why.empty()) return fail(TBK_ERR_UNSUPPORTED, "%s", why.c_str());
+  const int64_t rows_per_block = (int64_t)plan.row_warps * 32 * plan.rows_per_lane;
+  plan.grid_x = (n_rows + rows_per_block - 1) / rows_per_block;
   f->last_plan = plan;
 
   const int W = std::max(1, pk.num_classes);
@@ -916,12 +921,12 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
   return TBK_OK;
 }
 
+// (after a synchronisation with the forest's launches)
 int check_status(tbk_forest *f) {
-  int32_t st = 0;
-  CUDA_TRY(cudaMemcpy(&st, f->d_status, 4, cudaMemcpyDeviceToHost));
+  volatile int32_t *word = f->h_status;
+  const int32_t st = *word;
   if (st != 0) {
-    int32_t zero = 0;
-    cudaMemcpy(f->d_status, &zero, 4, cudaMemcpyHostToDevice);
+    *word = 0;
     return fail(TBK_ERR_DEVICE_WAIT, "a bounded wait on a bulk copy expired inside the walk kernel (status %d)", st);
   }
   return TBK_OK;
@@ -973,15 +978,65 @@ int upload_key_planes(tbk_forest *f, const std::vector<uint32_t> &node, const st
 }
 
 void free_pipeline(tbk_forest *f) {
-  for (int i = 0; i < 2; ++i) {
-    if (f->d_in[i]) cudaFree(f->d_in[i]);
-    if (f->d_res[i]) cudaFree(f->d_res[i]);
-    if (f->h_pin[i]) cudaFreeHost(f->h_pin[i]);
-    f->d_in[i] = nullptr; f->d_res[i] = nullptr; f->h_pin[i] = nullptr;
+  for (int i = 0; i < tbk_forest::kPipeSlots; ++i) {
+    cudaFree(f->d_in[i]);
+    cudaFree(f->d_res[i]);
+    cudaFreeHost(f->h_pin[i]);
+    cudaFreeHost(f->h_res[i]);
+    f->d_in[i] = f->d_res[i] = f->h_pin[i] = f->h_res[i] = nullptr;
   }
-  if (f->h_res) cudaFreeHost(f->h_res);
-  f->h_res = nullptr;
-  f->pipe_rows = f->pipe_ld = f->h_res_bytes = 0;
+  f->pipe_bytes = f->pipe_rows = 0;
+}
+
+bool is_pinned(const void *ptr) {
+  cudaPointerAttributes attr{};
+  const bool pinned = cudaPointerGetAttributes(&attr, ptr) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return pinned;
+}
+
+// memcpy by several threads: one core copies at about 10 GB/s, PCIe takes five times that.
+void copy_parallel(void *dst, const void *src, size_t bytes) {
+  const int threads = (int)std::min<size_t>({16, (size_t)tb::pack_threads(), bytes >> 18});
+  if (threads <= 1) {
+    std::memcpy(dst, src, bytes);
+    return;
+  }
+  const size_t part = (bytes / threads + 4095) / 4096 * 4096;
+#pragma omp parallel for schedule(static, 1) num_threads(threads)
+  for (int t = 0; t < threads; ++t) {
+    const size_t lo = std::min(bytes, t * part), hi = std::min(bytes, lo + part);
+    std::memcpy(static_cast<char *>(dst) + lo, static_cast<const char *>(src) + lo, hi - lo);
+  }
+}
+
+// Small host batches: everything but the walk itself is latency, so there are no copies to
+// enqueue and wait for.  The rows go through one pinned buffer that a ranking kernel reads over
+// PCIe (every value once); other kernels read rows more than once and get them copied.  Results
+// are written to pinned memory by the kernel that computes them, and the status word is mapped
+// host memory as well: one synchronisation ends the call.
+constexpr size_t kSmallRows = (size_t)512 << 10, kSmallDirect = (size_t)128 << 10, kSmallResults = (size_t)512 << 10;
+int predict_host_small(tbk_forest *f, const float *h_rows, int64_t n_rows, int64_t ld, void *h_out, int32_t out_kind) {
+  const size_t bytes = ((size_t)(n_rows - 1) * ld + f->packed.num_features) * 4; // (nothing behind the last row's values)
+  const size_t out_bytes = (size_t)n_rows * (out_kind == TBK_OUT_I8 ? 1 : 4);
+  if (!f->h_small) {
+    CUDA_TRY(cudaHostAlloc(&f->h_small, kSmallRows + kSmallResults, cudaHostAllocMapped));
+    CUDA_TRY(cudaHostGetDevicePointer(&f->d_small, f->h_small, 0));
+    CUDA_TRY(cudaMalloc(&f->d_small_in, kSmallRows));
+  }
+  std::memcpy(f->h_small, h_rows, bytes);
+  const unsigned char *rows = f->d_small;
+  if (!f->rank || bytes > kSmallDirect) {
+    CUDA_TRY(cudaMemcpyAsync(f->d_small_in, f->h_small, bytes, cudaMemcpyHostToDevice, f->streams[0]));
+    rows = f->d_small_in;
+  }
+  const int rc = run(f, kPredict, reinterpret_cast<const float *>(rows), n_rows, ld, f->d_small + kSmallRows, out_kind, nullptr,
+                     nullptr, f->streams[0], 0);
+  const cudaError_t e = cudaStreamSynchronize(f->streams[0]);
+  if (rc != TBK_OK) return rc;
+  if (e != cudaSuccess) return fail(TBK_ERR_CUDA, "cudaStreamSynchronize: %s", cudaGetErrorString(e));
+  std::memcpy(h_out, f->h_small + kSmallRows, out_bytes);
+  return check_status(f);
 }
 
 } // namespace
@@ -1221,8 +1276,9 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
   if (im.smem_limit > f->max_smem_optin)
     return bail(fail(TBK_ERR_UNSUPPORTED, "the packed image was laid out for %d bytes of shared memory per block, this device has %d",
                      im.smem_limit, f->max_smem_optin));
-  CUDA_TRY_F(cudaMalloc(&f->d_status, 4));
-  CUDA_TRY_F(cudaMemset(f->d_status, 0, 4));
+  CUDA_TRY_F(cudaHostAlloc(&f->h_status, 4, cudaHostAllocMapped));
+  *f->h_status = 0;
+  CUDA_TRY_F(cudaHostGetDevicePointer(&f->d_status, f->h_status, 0));
   CUDA_TRY_F(cudaEventCreate(&f->ev0));
   CUDA_TRY_F(cudaEventCreate(&f->ev1));
 
@@ -1391,10 +1447,10 @@ int tbk_forest_free(tbk_forest *f) {
   if (!f) return TBK_OK;
   cudaSetDevice(f->device);
   free_pipeline(f);
-  for (int i = 0; i < 2; ++i) {
-    if (f->streams[i]) cudaStreamDestroy(f->streams[i]);
-    if (f->in_free[i]) cudaEventDestroy(f->in_free[i]);
-  }
+  for (cudaStream_t st : f->streams)
+    if (st) cudaStreamDestroy(st);
+  for (cudaEvent_t e : f->slot_done)
+    if (e) cudaEventDestroy(e);
   cudaFree(f->d_blob);
   cudaFree(f->d_groups);
   cudaFree(f->d_tree_class);
@@ -1402,7 +1458,9 @@ int tbk_forest_free(tbk_forest *f) {
   cudaFree(f->d_orig_node);
   cudaFree(f->d_orig_off);
   cudaFree(f->d_lut);
-  cudaFree(f->d_status);
+  cudaFreeHost(f->h_status);
+  cudaFreeHost(f->h_small);
+  cudaFree(f->d_small_in);
   cudaFree(f->d_scratch);
   cudaFree(f->d_qnode);
   cudaFree(f->d_qleaf);
@@ -1517,74 +1575,93 @@ int tbk_predict_host(tbk_forest *f, const float *h_rows, int64_t n_rows, int64_t
   if (!f) return fail(TBK_ERR_INVALID, "null forest");
   if (n_rows == 0) return TBK_OK;
   if (!h_rows || !h_out) return fail(TBK_ERR_INVALID, "null pointer");
+  if (n_rows < 0 || ld < f->packed.num_features)
+    return fail(TBK_ERR_INVALID, "ld (%lld) is smaller than the row size (%d)", (long long)ld, f->packed.num_features);
   std::lock_guard<std::mutex> lock(f->mu);
   CUDA_TRY(cudaSetDevice(f->device));
-  const size_t out_elt = out_kind == TBK_OUT_I8 ? 1 : 4;
-  // chunk size: about 64 MiB of features, a multiple of 1024 rows
-  size_t chunk = std::max<size_t>(1024, ((size_t)64 << 20) / ((size_t)ld * 4) / 1024 * 1024);
-  chunk = std::min<size_t>(chunk, ((size_t)n_rows + 1023) / 1024 * 1024);
   if (!f->streams[0]) {
-    for (int i = 0; i < 2; ++i) {
-      CUDA_TRY(cudaStreamCreateWithFlags(&f->streams[i], cudaStreamNonBlocking));
-      CUDA_TRY(cudaEventCreateWithFlags(&f->in_free[i], cudaEventDisableTiming));
-    }
+    for (cudaStream_t &st : f->streams) CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    for (cudaEvent_t &e : f->slot_done) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
-  cudaPointerAttributes attr{};
-  const bool in_pinned = cudaPointerGetAttributes(&attr, h_rows) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-  cudaGetLastError();
-  cudaPointerAttributes oattr{};
-  const bool out_pinned = cudaPointerGetAttributes(&oattr, h_out) == cudaSuccess && oattr.type == cudaMemoryTypeHost;
-  cudaGetLastError();
-  if (f->pipe_rows < chunk || f->pipe_ld != (size_t)ld) {
-    free_pipeline(f);
-    for (int i = 0; i < 2; ++i) {
-      CUDA_TRY(cudaMalloc(&f->d_in[i], chunk * ld * 4));
-      CUDA_TRY(cudaMalloc(&f->d_res[i], chunk * 4));
-    }
-    f->pipe_rows = chunk;
-    f->pipe_ld = (size_t)ld;
-  }
-  if (!in_pinned && !f->h_pin[0])
-    for (int i = 0; i < 2; ++i) CUDA_TRY(cudaMallocHost(&f->h_pin[i], f->pipe_rows * ld * 4));
-  if (!out_pinned && f->h_res_bytes < (size_t)n_rows * out_elt) {
-    if (f->h_res) CUDA_TRY(cudaFreeHost(f->h_res));
-    f->h_res = nullptr;
-    CUDA_TRY(cudaMallocHost(&f->h_res, (size_t)n_rows * out_elt));
-    f->h_res_bytes = (size_t)n_rows * out_elt;
-  }
-  unsigned char *res_dst = out_pinned ? static_cast<unsigned char *>(h_out) : f->h_res;
+  const size_t out_elt = out_kind == TBK_OUT_I8 ? 1 : 4, row_bytes = (size_t)ld * 4;
   const bool was_timing = f->timing;
   f->timing = false; // per-chunk launches overlap on two streams; event timing does not apply
+  struct Restore { // (on every way out)
+    tbk_forest *f;
+    bool timing;
+    ~Restore() {
+      f->timing = timing;
+      f->host_batch_rows = 0;
+    }
+  } restore{f, was_timing};
+  f->host_batch_rows = n_rows;
+  if ((size_t)n_rows * row_bytes <= kSmallRows && (size_t)n_rows * out_elt <= kSmallResults)
+    return predict_host_small(f, h_rows, n_rows, ld, h_out, out_kind);
+
+  // Chunks of about a twelfth of the batch, 4 to 32 MiB: small enough that filling and draining
+  // the pipeline is a small part of the whole and that a staging slot stays in the cores' caches.
+  size_t chunk_bytes = std::min<size_t>((size_t)32 << 20, std::max<size_t>((size_t)4 << 20, (size_t)n_rows * row_bytes / 12));
+  const int64_t chunk = std::max<int64_t>(1024, (int64_t)(chunk_bytes / row_bytes) / 1024 * 1024);
+  chunk_bytes = (size_t)chunk * row_bytes;
+  const bool in_pinned = is_pinned(h_rows), out_pinned = is_pinned(h_out);
+  if (f->pipe_bytes < chunk_bytes || f->pipe_rows < (size_t)chunk) {
+    free_pipeline(f);
+    for (int i = 0; i < tbk_forest::kPipeSlots; ++i) {
+      CUDA_TRY(cudaMalloc(&f->d_in[i], chunk_bytes));
+      CUDA_TRY(cudaMalloc(&f->d_res[i], (size_t)chunk * 4));
+    }
+    f->pipe_bytes = chunk_bytes;
+    f->pipe_rows = (size_t)chunk;
+  }
+  for (int i = 0; i < tbk_forest::kPipeSlots; ++i) {
+    if (!in_pinned && !f->h_pin[i]) CUDA_TRY(cudaMallocHost(&f->h_pin[i], f->pipe_bytes));
+    if (!out_pinned && !f->h_res[i]) CUDA_TRY(cudaMallocHost(&f->h_res[i], f->pipe_rows * 4));
+  }
+  unsigned char *out = static_cast<unsigned char *>(h_out);
   int rc = TBK_OK;
-  int64_t done = 0;
-  for (int it = 0; done < n_rows && rc == TBK_OK; ++it) {
-    const int s = it & 1;
-    const int64_t n = std::min<int64_t>((int64_t)chunk, n_rows - done);
-    const float *src = h_rows + done * ld;
+  int64_t held[tbk_forest::kPipeSlots] = {}, held_at[tbk_forest::kPipeSlots] = {}; // rows whose results a slot holds
+  auto collect = [&](int s) { // waits for the chunk in slot s and hands its results over
+    if (held[s] == 0) return;
+    const cudaError_t e = cudaEventSynchronize(f->slot_done[s]);
+    if (e != cudaSuccess && rc == TBK_OK) rc = fail(TBK_ERR_CUDA, "cudaEventSynchronize: %s", cudaGetErrorString(e));
+    if (!out_pinned && rc == TBK_OK) std::memcpy(out + (size_t)held_at[s] * out_elt, f->h_res[s], (size_t)held[s] * out_elt);
+    held[s] = 0;
+  };
+  int s = 0;
+  for (int64_t done = 0; done < n_rows && rc == TBK_OK; s = (s + 1) % tbk_forest::kPipeSlots) {
+    const int64_t n = std::min<int64_t>(chunk, n_rows - done);
+    const size_t bytes = ((size_t)(n - 1) * ld + f->packed.num_features) * 4; // (nothing behind the last row's values)
+    cudaStream_t stream = f->streams[s & 1];
+    collect(s);
+    if (rc != TBK_OK) break;
+    const void *src = h_rows + done * ld;
     if (!in_pinned) {
-      // the staging buffer is free once the copy that last read it has finished
-      cudaError_t e = cudaEventSynchronize(f->in_free[s]);
-      if (e != cudaSuccess) { rc = fail(TBK_ERR_CUDA, "cudaEventSynchronize: %s", cudaGetErrorString(e)); break; }
-      std::memcpy(f->h_pin[s], src, (size_t)n * ld * 4);
+      copy_parallel(f->h_pin[s], src, bytes);
       src = f->h_pin[s];
     }
-    cudaError_t e = cudaMemcpyAsync(f->d_in[s], src, (size_t)n * ld * 4, cudaMemcpyHostToDevice, f->streams[s]);
-    if (e == cudaSuccess) e = cudaEventRecord(f->in_free[s], f->streams[s]);
-    if (e != cudaSuccess) { rc = fail(TBK_ERR_CUDA, "host-to-device copy: %s", cudaGetErrorString(e)); break; }
-    rc = run(f, kPredict, f->d_in[s], n, ld, f->d_res[s], out_kind, nullptr, nullptr, f->streams[s], s);
+    cudaError_t e = cudaMemcpyAsync(f->d_in[s], src, bytes, cudaMemcpyHostToDevice, stream);
+    if (e != cudaSuccess) {
+      rc = fail(TBK_ERR_CUDA, "host-to-device copy: %s", cudaGetErrorString(e));
+      break;
+    }
+    rc = run(f, kPredict, reinterpret_cast<const float *>(f->d_in[s]), n, ld, f->d_res[s], out_kind, nullptr, nullptr, stream, s & 1);
     if (rc != TBK_OK) break;
-    e = cudaMemcpyAsync(res_dst + done * out_elt, f->d_res[s], (size_t)n * out_elt, cudaMemcpyDeviceToHost, f->streams[s]);
-    if (e != cudaSuccess) { rc = fail(TBK_ERR_CUDA, "device-to-host copy: %s", cudaGetErrorString(e)); break; }
+    e = cudaMemcpyAsync(out_pinned ? out + (size_t)done * out_elt : f->h_res[s], f->d_res[s], (size_t)n * out_elt, cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaEventRecord(f->slot_done[s], stream);
+    if (e != cudaSuccess) {
+      rc = fail(TBK_ERR_CUDA, "device-to-host copy: %s", cudaGetErrorString(e));
+      break;
+    }
+    held[s] = n;
+    held_at[s] = done;
     done += n;
   }
-  for (int i = 0; i < 2; ++i) {
-    cudaError_t e = cudaStreamSynchronize(f->streams[i]);
+  for (int i = 0; i < tbk_forest::kPipeSlots; ++i) collect((s + i) % tbk_forest::kPipeSlots);
+  for (cudaStream_t st : f->streams) {
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess && rc == TBK_OK) rc = fail(TBK_ERR_CUDA, "cudaStreamSynchronize: %s", cudaGetErrorString(e));
   }
-  f->timing = was_timing;
-  if (rc != TBK_OK) return rc;
-  if (!out_pinned) std::memcpy(h_out, f->h_res, (size_t)n_rows * out_elt);
-  return check_status(f);
+  return rc != TBK_OK ? rc : check_status(f);
 }
 
 int tbk_set_timing(tbk_forest *f, int32_t enable) {
@@ -1606,6 +1683,8 @@ int64_t tbk_launch_count(const tbk_forest *f) { return f ? f->launches : 0; }
 
 int tbk_check_status(tbk_forest *f) {
   if (!f) return fail(TBK_ERR_INVALID, "null forest");
+  CUDA_TRY(cudaSetDevice(f->device));
+  CUDA_TRY(cudaDeviceSynchronize());
   return check_status(f);
 }
 

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
         ++round;
       }
     }
-    if (__syncthreads_or(!ok) && lane == 0) atomicExch(p.status, 4);
+    if (__syncthreads_or(!ok) && lane == 0) set_status(p.status, 4);
     return;
   }
 
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   // every wait above is bounded: a wait that gave up ends the launch with a status word
   const bool failed = __syncthreads_or(!ok) != 0;
   if (failed) {
-    if (tid == 0) atomicExch(p.status, 4);
+    if (tid == 0) set_status(p.status, 4);
     return;
   }
   acc += (double)pend0 + (double)pend1;

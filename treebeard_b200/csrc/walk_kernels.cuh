@@ -108,6 +108,12 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// The status word lies in mapped host memory: the host reads it after a synchronisation it needs
+// anyway, without a copy.
+__device__ __forceinline__ void set_status(int32_t *status, int32_t value) {
+  *reinterpret_cast<volatile int32_t *>(status) = value;
+  __threadfence_system();
+}
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -338,7 +344,7 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
       const uint32_t parity = ((g - g0) >> 1) & 1;
       const bool ok = mbar_wait_bounded(&mbar[s], parity, p.wait_limit ? p.wait_limit : kWaitLimit);
       if (__syncthreads_or(!ok)) {
-        if (tid == 0) atomicExch(p.status, 4);
+        if (tid == 0) set_status(p.status, 4);
         return;
       }
       gbase = stage0 + (size_t)s * p.stage_bytes;

@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(kQThreads, 1) tb_walk_quant_kernel(const Quant
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kQTmemCols) : "memory");
   }
   if (failed) {
-    if (tid == 0) atomicExch(p.status, 4);
+    if (tid == 0) set_status(p.status, 4);
     return;
   }
   if (p.tie_count != nullptr && tie_count) atomicAdd(p.tie_count, (unsigned long long)tie_count);

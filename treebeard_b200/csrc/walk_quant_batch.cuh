@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kQBMaxThreads, 1) tb_walk_quant_batch_kernel(c
   // every wait above is bounded: a wait that gave up ends the launch with a status word
   const bool failed = __syncthreads_or(!ok) != 0;
   if (failed) {
-    if (tid == 0) atomicExch(p.status, 4);
+    if (tid == 0) set_status(p.status, 4);
     return;
   }
   if (p.tie_count != nullptr && tie_count) atomicAdd(p.tie_count, (unsigned long long)tie_count);

@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
   const bool chunked = gridDim.y > 1 && MODE != kRankLeafIds && !(MODE == kRankClasses && p.write_partial);
   if (chunked) __threadfence();
   if (__syncthreads_or(!ok)) {
-    if (tid == 0) atomicExch(p.status, 4);
+    if (tid == 0) set_status(p.status, 4);
     if (warp >= kRWWalkers) { // no copy may land after the block is gone
       const uint32_t bars = warp == kRWWalkers ? full_s : keys_full_s, n = warp == kRWWalkers ? (uint32_t)p.stages : 2u;
       for (uint32_t s = 0; s < min(n, issued); ++s) wait(bars + 8u * s, ((issued - 1u - s) / n) & 1u);

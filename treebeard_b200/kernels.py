@@ -116,10 +116,18 @@ def _torch():
     return torch
 
 
-def _stream_ptr(stream) -> Optional[int]:
-    if stream is None:
-        return _torch().cuda.current_stream().cuda_stream
-    return stream.cuda_stream
+_raw_stream = None
+
+
+def _stream_ptr(stream, device) -> Optional[int]:
+    if stream is not None:
+        return stream.cuda_stream
+    global _raw_stream
+    if _raw_stream is None:   # the stream's handle without a Stream object, where torch has that call
+        torch = _torch()
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or \
+            (lambda index: torch.cuda.current_stream(index).cuda_stream)
+    return _raw_stream(device)
 
 
 class DeviceForest:
@@ -164,9 +172,11 @@ class DeviceForest:
 
     def _rows(self, rows):
         torch = _torch()
-        assert rows.is_cuda and rows.dtype == torch.float32 and rows.dim() == 2
-        assert rows.stride(1) == 1 and rows.shape[1] == self.num_features
-        return rows.data_ptr(), rows.shape[0], rows.stride(0)
+        n, features = rows.shape
+        ld, step = rows.stride()
+        assert rows.is_cuda and rows.dtype is torch.float32
+        assert step == 1 and features == self.num_features
+        return rows.data_ptr(), n, ld
 
     def predict(self, rows, out=None, int8: bool = False, stream=None):
         """rows: CUDA float32 [n, F] (row stride free).  Returns a CUDA tensor [n]."""
@@ -175,7 +185,7 @@ class DeviceForest:
         if out is None:
             out = torch.empty(n, device=rows.device, dtype=torch.int8 if int8 else torch.float32)
         _check(lib().tbk_predict(self._h, ptr, n, ld, out.data_ptr(), OUT_I8 if int8 else OUT_F32,
-                                 _stream_ptr(stream)))
+                                 _stream_ptr(stream, self.device)))
         return out
 
     def predict_partial(self, rows, out=None, stream=None):
@@ -184,7 +194,7 @@ class DeviceForest:
         ptr, n, ld = self._rows(rows)
         if out is None:
             out = torch.empty((n, max(1, self.num_classes)), device=rows.device, dtype=torch.float32)
-        _check(lib().tbk_predict_partial(self._h, ptr, n, ld, out.data_ptr(), _stream_ptr(stream)))
+        _check(lib().tbk_predict_partial(self._h, ptr, n, ld, out.data_ptr(), _stream_ptr(stream, self.device)))
         return out
 
     def finalize(self, partial, out=None, int8: bool = False, stream=None):
@@ -193,14 +203,14 @@ class DeviceForest:
         if out is None:
             out = torch.empty(n, device=partial.device, dtype=torch.int8 if int8 else torch.float32)
         _check(lib().tbk_finalize(self._h, partial.data_ptr(), n, out.data_ptr(),
-                                  OUT_I8 if int8 else OUT_F32, _stream_ptr(stream)))
+                                  OUT_I8 if int8 else OUT_F32, _stream_ptr(stream, self.device)))
         return out
 
     def predict_leaf_ids(self, rows, stream=None):
         torch = _torch()
         ptr, n, ld = self._rows(rows)
         out = torch.empty((n, self.num_trees), device=rows.device, dtype=torch.int32)
-        _check(lib().tbk_predict_leaf_ids(self._h, ptr, n, ld, out.data_ptr(), _stream_ptr(stream)))
+        _check(lib().tbk_predict_leaf_ids(self._h, ptr, n, ld, out.data_ptr(), _stream_ptr(stream, self.device)))
         return out
 
     def predict_host(self, rows: np.ndarray, out: Optional[np.ndarray] = None, int8: bool = False):

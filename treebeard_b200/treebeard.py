@@ -294,6 +294,11 @@ class TreebeardInferenceRunner:
         r.inferenceRunner = handle
         r.rowSize = treebeardAPI.GetRowSize(handle)
         r.batchSize = treebeardAPI.GetBatchSize(handle)
+        # numpy types of the host buffers: what the runner was compiled for (32- or 64-bit
+        # inputs; fp32, fp64 or int8 results)
+        r._inType = numpy.dtype(numpy.float64 if _rt.TB_GetInputTypeBitWidth(handle) == 64 else numpy.float32)
+        width = _rt.TB_GetReturnTypeBitWidth(handle)
+        r._outType = numpy.dtype(numpy.int8 if width == 8 else numpy.float64 if width == 64 else numpy.float32)
         return r
 
     @classmethod
@@ -339,9 +344,6 @@ class TreebeardInferenceRunner:
             self.treebeardAPI.DeleteInferenceRunner(self.inferenceRunner)
             self.inferenceRunner = 0
 
-    def _is_int8(self):
-        return _rt.TB_GetReturnTypeBitWidth(self.inferenceRunner) == 8
-
     def _check_shape(self, inputs, rows):
         """The library reads rows x GetRowSize floats: a smaller buffer would be overrun."""
         shape = tuple(inputs.shape)
@@ -351,41 +353,33 @@ class TreebeardInferenceRunner:
             want = f"({rows if rows is not None else 'n'}, {self.rowSize})"
             raise TreebeardRuntimeError(f"inputs have shape {shape}, the runner expects {want}")
 
-    def _host_types(self, resultType):
-        """numpy types of the host buffers: what the runner was compiled for (32- or 64-bit
-        inputs; fp32, fp64 or int8 results)."""
-        in_type = numpy.float64 if _rt.TB_GetInputTypeBitWidth(self.inferenceRunner) == 64 else numpy.float32
-        width = _rt.TB_GetReturnTypeBitWidth(self.inferenceRunner)
-        out_type = numpy.int8 if width == 8 else numpy.float64 if width == 64 else numpy.float32
-        if numpy.dtype(resultType) != numpy.dtype(out_type):
-            raise TreebeardRuntimeError(f"the runner returns {numpy.dtype(out_type)}, not {numpy.dtype(resultType)}")
-        return in_type, out_type
+    def _host_buffers(self, inputs, rows, resultType):
+        """Checks a host batch; returns the array its results will be written to."""
+        if numpy.dtype(resultType) != self._outType:
+            raise TreebeardRuntimeError(f"the runner returns {self._outType}, not {numpy.dtype(resultType)}")
+        assert inputs.dtype == self._inType and inputs.flags.c_contiguous
+        self._check_shape(inputs, rows)
+        return numpy.empty(inputs.shape[0] if rows is None else rows, self._outType)
 
     def RunInference(self, inputs, resultType=numpy.float32):
         if isinstance(inputs, numpy.ndarray):
-            in_type, resultType = self._host_types(resultType)
-            assert inputs.dtype == in_type and inputs.flags.c_contiguous
-            self._check_shape(inputs, self.batchSize)
-            results = numpy.zeros((self.batchSize), resultType)
-            self.treebeardAPI.RunInference(self.inferenceRunner, inputs.ctypes.data, results.ctypes.data)
+            results = self._host_buffers(inputs, self.batchSize, resultType)
+            self.treebeardAPI.RunInference(self.inferenceRunner, inputs.__array_interface__["data"][0],
+                                           results.__array_interface__["data"][0])
             return results
         import torch  # device-resident path
         assert inputs.is_cuda and inputs.dtype == torch.float32 and inputs.is_contiguous()
         self._check_shape(inputs, self.batchSize)
-        results = torch.zeros(self.batchSize, device=inputs.device,
-                              dtype=torch.int8 if self._is_int8() else torch.float32)
+        results = torch.empty(self.batchSize, device=inputs.device,
+                              dtype=torch.int8 if self._outType.itemsize == 1 else torch.float32)
         self.treebeardAPI.RunInference(self.inferenceRunner, inputs.data_ptr(), results.data_ptr())
         return results
 
     def RunInferenceOnMultipleBatches(self, inputs, resultType=numpy.float32):
         assert type(inputs) is numpy.ndarray
-        in_type, resultType = self._host_types(resultType)
-        assert inputs.dtype == in_type and inputs.flags.c_contiguous
-        self._check_shape(inputs, None)
-        numRows = inputs.shape[0]
-        results = numpy.zeros((numRows), resultType)
-        self.treebeardAPI.RunInferenceOnMultipleBatches(self.inferenceRunner, inputs.ctypes.data,
-                                                        results.ctypes.data, numRows)
+        results = self._host_buffers(inputs, None, resultType)
+        self.treebeardAPI.RunInferenceOnMultipleBatches(self.inferenceRunner, inputs.__array_interface__["data"][0],
+                                                        results.__array_interface__["data"][0], inputs.shape[0])
         return results
 
     def device_count(self) -> int:
