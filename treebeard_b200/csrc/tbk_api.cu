@@ -14,7 +14,12 @@
 #include "walk_rank.cuh"
 #include "packed_image.h"
 
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
 #include <algorithm>
+#include <atomic>
+#include <condition_variable>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -22,6 +27,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace {
@@ -47,6 +53,115 @@ int fail(int code, const char *fmt, ...) {
   } while (0)
 
 } // namespace
+
+// Copies pageable batches into staging slots, chunk after chunk, on a few threads that a forest
+// keeps from its first such batch on: one core moves about 20 GB/s, PCIe takes 55, and starting
+// threads for every call costs more than the copy.  The calling thread enqueues GPU work meanwhile
+// and copies pieces when it has nothing else to do.
+//
+// The copies bypass the caches: the DMA engine reads lines that are still dirty in some core's cache
+// at a quarter of its rate (a bulk call of 524288 x 28 rows took 2.5 ms with plain copies).
+void copy_past_caches(unsigned char *dst, const unsigned char *src, size_t n) {
+#ifdef __SSE2__
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+    size_t i = 0;
+    for (; i + 64 <= n; i += 64) {
+      const __m128i *from = reinterpret_cast<const __m128i *>(src + i);
+      __m128i *to = reinterpret_cast<__m128i *>(dst + i);
+      const __m128i a = _mm_loadu_si128(from), b = _mm_loadu_si128(from + 1), c = _mm_loadu_si128(from + 2), d = _mm_loadu_si128(from + 3);
+      _mm_stream_si128(to, a);
+      _mm_stream_si128(to + 1, b);
+      _mm_stream_si128(to + 2, c);
+      _mm_stream_si128(to + 3, d);
+    }
+    std::memcpy(dst + i, src + i, n - i);
+    _mm_sfence();
+    return;
+  }
+#endif
+  std::memcpy(dst, src, n);
+}
+class Stager {
+public:
+  explicit Stager(int threads) {
+    for (int t = 0; t < threads; ++t) workers_.emplace_back([this] { work(); });
+  }
+  ~Stager() {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      quit_ = true;
+    }
+    wake_.notify_all();
+    for (std::thread &w : workers_) w.join();
+  }
+  void start(const void *rows, size_t bytes, unsigned char *const *slots, int num_slots, size_t chunk_bytes) {
+    std::lock_guard<std::mutex> lock(mu_);
+    src_ = static_cast<const unsigned char *>(rows);
+    total_ = bytes;
+    slots_ = slots;
+    num_slots_ = num_slots;
+    chunk_bytes_ = chunk_bytes;
+    per_chunk_ = (int64_t)((chunk_bytes + kPiece - 1) / kPiece);
+    const size_t chunks = (bytes + chunk_bytes - 1) / chunk_bytes;
+    done_ = std::vector<std::atomic<int64_t>>(chunks);
+    num_pieces_ = per_chunk_ * (int64_t)chunks;
+    next_ = 0;
+    allowed_ = num_slots - 1;
+    active_ = true;
+    wake_.notify_all();
+  }
+  void allow(int64_t chunk) { allowed_.store(chunk, std::memory_order_release); } // chunks up to this one have a free slot
+  bool ready(int64_t chunk) const { return done_[chunk].load(std::memory_order_acquire) == per_chunk_; }
+  // Copies one piece, if one is left whose slot is free.
+  bool copy_one() {
+    int64_t p = next_.load(std::memory_order_relaxed);
+    do {
+      if (p >= num_pieces_ || p / per_chunk_ > allowed_.load(std::memory_order_acquire)) return false;
+    } while (!next_.compare_exchange_weak(p, p + 1));
+    const int64_t chunk = p / per_chunk_;
+    const size_t lo = (size_t)(p % per_chunk_) * kPiece, begin = (size_t)chunk * chunk_bytes_ + lo;
+    const size_t end = std::min(total_, std::min(begin + kPiece, (size_t)(chunk + 1) * chunk_bytes_));
+    if (begin < end) copy_past_caches(slots_[chunk % num_slots_] + lo, src_ + begin, end - begin);
+    done_[chunk].fetch_add(1, std::memory_order_release);
+    return true;
+  }
+  // The batch is over (or given up): returns once no worker looks at it any more.
+  void finish() {
+    active_ = false;
+    while (busy_.load() != 0) std::this_thread::yield();
+  }
+
+private:
+  static constexpr size_t kPiece = (size_t)256 << 10;
+  void work() {
+    std::unique_lock<std::mutex> lock(mu_);
+    while (!quit_) {
+      if (!active_ || next_.load() >= num_pieces_) {
+        wake_.wait(lock);
+        continue;
+      }
+      ++busy_;
+      lock.unlock();
+      while (active_ && next_.load(std::memory_order_relaxed) < num_pieces_)
+        if (!copy_one()) std::this_thread::yield();
+      lock.lock();
+      --busy_;
+    }
+  }
+  std::mutex mu_;
+  std::condition_variable wake_;
+  std::vector<std::thread> workers_;
+  const unsigned char *src_ = nullptr;
+  unsigned char *const *slots_ = nullptr;
+  size_t total_ = 0, chunk_bytes_ = 0;
+  int num_slots_ = 0;
+  int64_t per_chunk_ = 1, num_pieces_ = 0;
+  std::vector<std::atomic<int64_t>> done_; // pieces of every chunk that are in place
+  std::atomic<int64_t> next_{0}, allowed_{0};
+  std::atomic<int> busy_{0};
+  std::atomic<bool> active_{false};
+  bool quit_ = false;
+};
 
 struct tbk_image {
   tb::PackedImage im;
@@ -128,9 +243,10 @@ struct tbk_forest {
   static constexpr int kPipeSlots = 4;
   unsigned char *d_in[kPipeSlots] = {}, *d_res[kPipeSlots] = {}, *h_pin[kPipeSlots] = {}, *h_res[kPipeSlots] = {};
   size_t pipe_bytes = 0, pipe_rows = 0; // capacity of a slot
+  std::unique_ptr<Stager> stager;
   unsigned char *h_small = nullptr, *d_small = nullptr, *d_small_in = nullptr;
   cudaStream_t streams[2] = {nullptr, nullptr};
-  cudaEvent_t slot_done[kPipeSlots] = {};
+  cudaEvent_t slot_read[kPipeSlots] = {}, slot_done[kPipeSlots] = {}; // a chunk's rows are copied / its results are there
   int64_t host_batch_rows = 0; // rows of the host batch whose chunks are being predicted
   // timing
   bool timing = false;
@@ -995,21 +1111,6 @@ bool is_pinned(const void *ptr) {
   return pinned;
 }
 
-// memcpy by several threads: one core copies at about 10 GB/s, PCIe takes five times that.
-void copy_parallel(void *dst, const void *src, size_t bytes) {
-  const int threads = (int)std::min<size_t>({16, (size_t)tb::pack_threads(), bytes >> 18});
-  if (threads <= 1) {
-    std::memcpy(dst, src, bytes);
-    return;
-  }
-  const size_t part = (bytes / threads + 4095) / 4096 * 4096;
-#pragma omp parallel for schedule(static, 1) num_threads(threads)
-  for (int t = 0; t < threads; ++t) {
-    const size_t lo = std::min(bytes, t * part), hi = std::min(bytes, lo + part);
-    std::memcpy(static_cast<char *>(dst) + lo, static_cast<const char *>(src) + lo, hi - lo);
-  }
-}
-
 // Small host batches: everything but the walk itself is latency, so there are no copies to
 // enqueue and wait for.  The rows go through one pinned buffer that a ranking kernel reads over
 // PCIe (every value once); other kernels read rows more than once and get them copied.  Results
@@ -1024,7 +1125,7 @@ int predict_host_small(tbk_forest *f, const float *h_rows, int64_t n_rows, int64
     CUDA_TRY(cudaHostGetDevicePointer(&f->d_small, f->h_small, 0));
     CUDA_TRY(cudaMalloc(&f->d_small_in, kSmallRows));
   }
-  std::memcpy(f->h_small, h_rows, bytes);
+  copy_past_caches(f->h_small, reinterpret_cast<const unsigned char *>(h_rows), bytes);
   const unsigned char *rows = f->d_small;
   if (!f->rank || bytes > kSmallDirect) {
     CUDA_TRY(cudaMemcpyAsync(f->d_small_in, f->h_small, bytes, cudaMemcpyHostToDevice, f->streams[0]));
@@ -1449,8 +1550,10 @@ int tbk_forest_free(tbk_forest *f) {
   free_pipeline(f);
   for (cudaStream_t st : f->streams)
     if (st) cudaStreamDestroy(st);
-  for (cudaEvent_t e : f->slot_done)
-    if (e) cudaEventDestroy(e);
+  for (int i = 0; i < tbk_forest::kPipeSlots; ++i) {
+    if (f->slot_done[i]) cudaEventDestroy(f->slot_done[i]);
+    if (f->slot_read[i]) cudaEventDestroy(f->slot_read[i]);
+  }
   cudaFree(f->d_blob);
   cudaFree(f->d_groups);
   cudaFree(f->d_tree_class);
@@ -1582,6 +1685,7 @@ int tbk_predict_host(tbk_forest *f, const float *h_rows, int64_t n_rows, int64_t
   if (!f->streams[0]) {
     for (cudaStream_t &st : f->streams) CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     for (cudaEvent_t &e : f->slot_done) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (cudaEvent_t &e : f->slot_read) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
   const size_t out_elt = out_kind == TBK_OUT_I8 ? 1 : 4, row_bytes = (size_t)ld * 4;
   const bool was_timing = f->timing;
@@ -1618,45 +1722,63 @@ int tbk_predict_host(tbk_forest *f, const float *h_rows, int64_t n_rows, int64_t
     if (!out_pinned && !f->h_res[i]) CUDA_TRY(cudaMallocHost(&f->h_res[i], f->pipe_rows * 4));
   }
   unsigned char *out = static_cast<unsigned char *>(h_out);
+  constexpr int NS = tbk_forest::kPipeSlots;
+  const int64_t num_chunks = (n_rows + chunk - 1) / chunk;
+  Stager *stager = nullptr;
+  if (!in_pinned) {
+    if (!f->stager) f->stager.reset(new Stager(std::max(0, std::min(6, tb::pack_threads() - 1))));
+    stager = f->stager.get();
+    stager->start(h_rows, ((size_t)(n_rows - 1) * ld + f->packed.num_features) * 4, f->h_pin, NS, chunk_bytes);
+  }
   int rc = TBK_OK;
-  int64_t held[tbk_forest::kPipeSlots] = {}, held_at[tbk_forest::kPipeSlots] = {}; // rows whose results a slot holds
-  auto collect = [&](int s) { // waits for the chunk in slot s and hands its results over
-    if (held[s] == 0) return;
-    const cudaError_t e = cudaEventSynchronize(f->slot_done[s]);
-    if (e != cudaSuccess && rc == TBK_OK) rc = fail(TBK_ERR_CUDA, "cudaEventSynchronize: %s", cudaGetErrorString(e));
-    if (!out_pinned && rc == TBK_OK) std::memcpy(out + (size_t)held_at[s] * out_elt, f->h_res[s], (size_t)held[s] * out_elt);
-    held[s] = 0;
+  int64_t copied = 0, collected = 0, issued = 0; // chunks whose rows have left their slot / whose results are out / in flight
+  auto rows_of = [&](int64_t c) { return std::min<int64_t>(chunk, n_rows - c * chunk); };
+  // Takes note of what the GPU has finished; wait: until the oldest chunk's results are there.
+  auto advance = [&](bool wait) {
+    while (copied < issued && cudaEventQuery(f->slot_read[copied % NS]) == cudaSuccess) {
+      ++copied;
+      if (stager) stager->allow(copied + NS - 1);
+    }
+    while (collected < issued) {
+      const int s = (int)(collected % NS);
+      const cudaError_t e = wait ? cudaEventSynchronize(f->slot_done[s]) : cudaEventQuery(f->slot_done[s]);
+      if (e == cudaErrorNotReady) break;
+      if (e != cudaSuccess && rc == TBK_OK) rc = fail(TBK_ERR_CUDA, "host pipeline: %s", cudaGetErrorString(e));
+      if (!out_pinned && rc == TBK_OK)
+        std::memcpy(out + (size_t)(collected * chunk) * out_elt, f->h_res[s], (size_t)rows_of(collected) * out_elt);
+      ++collected;
+      if (wait) break;
+    }
   };
-  int s = 0;
-  for (int64_t done = 0; done < n_rows && rc == TBK_OK; s = (s + 1) % tbk_forest::kPipeSlots) {
-    const int64_t n = std::min<int64_t>(chunk, n_rows - done);
+  for (int64_t c = 0; c < num_chunks && rc == TBK_OK; ++c) {
+    const int s = (int)(c % NS);
+    const int64_t n = rows_of(c);
     const size_t bytes = ((size_t)(n - 1) * ld + f->packed.num_features) * 4; // (nothing behind the last row's values)
     cudaStream_t stream = f->streams[s & 1];
-    collect(s);
+    while (stager && !stager->ready(c) && rc == TBK_OK)
+      if (!stager->copy_one()) advance(false);
+    while (collected + NS <= c && rc == TBK_OK) advance(true); // the slot's results must be out
     if (rc != TBK_OK) break;
-    const void *src = h_rows + done * ld;
-    if (!in_pinned) {
-      copy_parallel(f->h_pin[s], src, bytes);
-      src = f->h_pin[s];
-    }
+    const void *src = stager ? static_cast<const void *>(f->h_pin[s]) : h_rows + c * chunk * ld;
     cudaError_t e = cudaMemcpyAsync(f->d_in[s], src, bytes, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaEventRecord(f->slot_read[s], stream);
     if (e != cudaSuccess) {
       rc = fail(TBK_ERR_CUDA, "host-to-device copy: %s", cudaGetErrorString(e));
       break;
     }
     rc = run(f, kPredict, reinterpret_cast<const float *>(f->d_in[s]), n, ld, f->d_res[s], out_kind, nullptr, nullptr, stream, s & 1);
     if (rc != TBK_OK) break;
-    e = cudaMemcpyAsync(out_pinned ? out + (size_t)done * out_elt : f->h_res[s], f->d_res[s], (size_t)n * out_elt, cudaMemcpyDeviceToHost, stream);
+    e = cudaMemcpyAsync(out_pinned ? out + (size_t)(c * chunk) * out_elt : f->h_res[s], f->d_res[s], (size_t)n * out_elt, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaEventRecord(f->slot_done[s], stream);
     if (e != cudaSuccess) {
       rc = fail(TBK_ERR_CUDA, "device-to-host copy: %s", cudaGetErrorString(e));
       break;
     }
-    held[s] = n;
-    held_at[s] = done;
-    done += n;
+    ++issued;
+    advance(false);
   }
-  for (int i = 0; i < tbk_forest::kPipeSlots; ++i) collect((s + i) % tbk_forest::kPipeSlots);
+  if (stager) stager->finish();
+  while (collected < issued && rc == TBK_OK) advance(true);
   for (cudaStream_t st : f->streams) {
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess && rc == TBK_OK) rc = fail(TBK_ERR_CUDA, "cudaStreamSynchronize: %s", cudaGetErrorString(e));
