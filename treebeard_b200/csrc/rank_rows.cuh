@@ -32,6 +32,23 @@ struct RankRowsParams {
   unsigned long long *searched; // statistics: values that were compared with thresholds
 };
 
+// Rank of one value, tables in global memory (see tb_rank_rows, which ranks several in lock-step).
+__device__ __forceinline__ uint32_t rank_value(float x, const DevRankFeature *feature, const uint16_t *lut, const float *thr,
+                                               unsigned &searched) {
+  const uint4 a = __ldg(reinterpret_cast<const uint4 *>(feature)), b = __ldg(reinterpret_cast<const uint4 *>(feature) + 1);
+  const float lo = __uint_as_float(a.x), scale = __uint_as_float(a.y), top = __uint_as_float(a.z);
+  const float y = fmaxf(fminf(__fmul_rn(__fsub_rn(x, lo), scale), top), 0.f);
+  const uint16_t *l = lut + a.w + (uint32_t)y;
+  uint32_t s = __ldg(l), e = __ldg(l + 1);
+  if (b.w && x == floorf(x)) return x < lo ? 0u : e;
+  searched += s < e;
+  for (uint32_t step = s < e ? 1u << (31 - __clz(e - s)) : 0u; step; step >>= 1) {
+    const uint32_t m = s + step;
+    if (m <= e && !(x < __ldg(thr + b.x + m - 1u))) s = m;
+  }
+  return s;
+}
+
 template <int FW, bool PAIR, bool SMEM>
 __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankRowsParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];

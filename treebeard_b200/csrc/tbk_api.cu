@@ -225,7 +225,8 @@ struct tbk_forest {
     bool used = false;
     cudaEvent_t done = nullptr;
   };
-  static constexpr int kWorkspaces = 4;
+  static constexpr int kWorkspaces = 8;
+  bool mark_uses = false;
   Workspace workspace[kWorkspaces];
   int next_victim = 0;
   std::list<Workspace> captured; // of calls that were captured into graphs
@@ -245,6 +246,7 @@ struct tbk_forest {
   size_t pipe_bytes = 0, pipe_rows = 0; // capacity of a slot
   std::unique_ptr<Stager> stager;
   unsigned char *h_small = nullptr, *d_small = nullptr, *d_small_in = nullptr;
+  const float *inline_rows = nullptr; // rows of the small host batch being predicted, which may travel with the launch
   cudaStream_t streams[2] = {nullptr, nullptr};
   cudaEvent_t slot_read[kPipeSlots] = {}, slot_done[kPipeSlots] = {}; // a chunk's rows are copied / its results are there
   int64_t host_batch_rows = 0; // rows of the host batch whose chunks are being predicted
@@ -640,6 +642,11 @@ int workspace_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_fore
     for (auto &c : f->workspace)
       if (!c.used && (!w || c.bytes > w->bytes)) w = &c;
   if (!w) {
+    if (!f->mark_uses) {
+      CUDA_TRY(cudaDeviceSynchronize()); // (earlier uses have left no mark)
+      f->mark_uses = true;
+      for (auto &c : f->workspace) CUDA_TRY(cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming));
+    }
     w = &f->workspace[f->next_victim++ % tbk_forest::kWorkspaces];
     CUDA_TRY(cudaStreamWaitEvent(stream, w->done, 0));
   }
@@ -653,7 +660,6 @@ int workspace_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_fore
     w->bytes = bytes;
     CUDA_TRY(cudaMemsetAsync(w->mem, 0, tb::kRankArrivalBytes, stream));
   }
-  if (!w->done) CUDA_TRY(cudaEventCreateWithFlags(&w->done, cudaEventDisableTiming));
   *out = w;
   return TBK_OK;
 }
@@ -671,14 +677,15 @@ int allow_smem(tbk_forest *f, const void *kernel) {
 int rank_stride(int num_features) { return num_features <= tb::kRankPairFeatures ? 64 : 128; }
 
 using RankKernel = void (*)(const tb::RankWalkParams);
-template <int S, bool WHOLE> RankKernel pick_rank(int mode) {
-  return mode == tb::kRankLeafIds ? tb::tb_walk_rank_kernel<S, WHOLE, tb::kRankLeafIds>
-         : mode == tb::kRankClasses ? tb::tb_walk_rank_kernel<S, WHOLE, tb::kRankClasses>
-                                    : tb::tb_walk_rank_kernel<S, WHOLE, tb::kRankSums>;
+template <int S, int NR, bool WHOLE> RankKernel pick_rank(int mode) {
+  return mode == tb::kRankLeafIds ? tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankLeafIds>
+         : mode == tb::kRankClasses ? tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankClasses>
+                                    : tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankSums>;
 }
-RankKernel pick_rank_kernel(int stride, bool whole, int mode) {
-  if (stride == 64) return whole ? pick_rank<64, true>(mode) : pick_rank<64, false>(mode);
-  return whole ? pick_rank<128, true>(mode) : pick_rank<128, false>(mode);
+RankKernel pick_rank_kernel(int stride, bool small, bool whole, int mode) {
+  if (small) return stride == 64 ? pick_rank<64, 4, true>(mode) : pick_rank<128, 4, true>(mode);
+  if (stride == 64) return whole ? pick_rank<64, 16, true>(mode) : pick_rank<64, 16, false>(mode);
+  return whole ? pick_rank<128, 16, true>(mode) : pick_rank<128, 16, false>(mode);
 }
 
 // Launch shape of the walk over `n_rows` rows: blocks along the rows and tree chunks, by what the
@@ -772,8 +779,7 @@ size_t rank_workspace_bytes(const tbk_forest *f, const RankPlan &plan, int64_t r
   return bytes;
 }
 
-// The kernel that ranks `n` rows into `keys`.
-int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, uint16_t *keys, cudaStream_t stream) {
+tb::RankRowsParams rank_rows_params(const tbk_forest *f, const float *rows, int64_t n, int64_t ld, uint16_t *keys) {
   const auto &q = f->rf;
   const int F = q.num_features;
   tb::RankRowsParams p{};
@@ -789,6 +795,13 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
   p.vec4_ok = F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
   p.lattice = q.lattice;
   p.searched = f->d_ties;
+  return p;
+}
+
+// The kernel that ranks `n` rows into `keys`.
+int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, uint16_t *keys, cudaStream_t stream) {
+  const int F = f->rf.num_features;
+  tb::RankRowsParams p = rank_rows_params(f, rows, n, ld, keys);
   const bool pair = F <= tb::kRankPairFeatures;
   const int64_t lines = pair ? (n + 1) / 2 : n;
   // Tables in shared memory pay once every SM has a few thousand values to rank: loading them
@@ -861,7 +874,13 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   int rc = workspace_acquire(f, stream, rank_workspace_bytes(f, plan, pass), &ws);
   if (rc) return rc;
   unsigned char *keys = ws->mem + tb::kRankArrivalBytes;
-  const RankKernel kernel = pick_rank_kernel(S, q.whole_compare != 0, kmode);
+  // one unit of rows per block: the variant for small batches, with only as many walker warps as
+  // the rows -- or ranking them with two values per thread -- can use
+  const bool small = plan.units == 1;
+  int walkers = tb::kRWWalkers;
+  if (n_rows < tb::kRWUnitRows) walkers = (int)std::min<int64_t>(walkers, std::max((n_rows + 3) / 4, (n_rows * q.num_features + 63) / 64));
+  const int unit_rows = 4 * walkers;
+  const RankKernel kernel = pick_rank_kernel(S, small, q.whole_compare != 0, kmode);
   rc = allow_smem(f, (const void *)kernel);
   if (rc) return rc;
   tb::RankWalkParams p{};
@@ -883,14 +902,32 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   p.out_kind = out_kind == TBK_OUT_I8 ? 1 : 0;
   p.transform = q.transform;
   p.initial_value = (float)q.initial_value;
+  p.uniform_depth = f->uniform_depth;
   p.stages = plan.stages;
   p.stage_bytes = plan.stage_bytes;
   p.status = f->d_status;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   for (int64_t done = 0; done < n_rows; done += pass) {
     const int64_t n = std::min(pass, n_rows - done);
-    rc = launch_rank_rows(f, d_rows + done * ld, n, ld, reinterpret_cast<uint16_t *>(keys), stream);
-    if (rc) return rc;
+    const int64_t units = (n + unit_rows - 1) / unit_rows; // (chunks: at most four units to a block)
+    const int64_t batches = std::min(units, plan.grid_x);
+    // Up to four values per walker thread: the walk ranks its rows itself.  (Every chunk's blocks
+    // read the rows again, which host memory is too slow for.)
+    const int64_t block_rows = std::min<int64_t>(n, (int64_t)plan.units * unit_rows);
+    const bool inlined = f->inline_rows && batches == 1 && n * q.num_features <= tb::kRankInline;
+    const bool fused = pass == n_rows && plan.units < tb::kRWBatchUnits && block_rows * q.num_features <= 128 * walkers &&
+                       (!f->inline_rows || inlined || plan.chunks == 1);
+    if (fused) {
+      p.ranking = rank_rows_params(f, d_rows, n, ld, nullptr);
+      if (inlined) {
+        p.inline_values = (uint32_t)(n * q.num_features);
+        for (int64_t r = 0; r < n; ++r)
+          std::memcpy(p.inline_rows + r * q.num_features, f->inline_rows + r * ld, (size_t)q.num_features * 4);
+      }
+    } else {
+      rc = launch_rank_rows(f, d_rows + done * ld, n, ld, reinterpret_cast<uint16_t *>(keys), stream);
+      if (rc) return rc;
+    }
     p.n_rows = n;
     p.partial = d_partial ? d_partial + done * W : nullptr;
     p.out = d_out ? static_cast<unsigned char *>(d_out) + done * (out_kind == TBK_OUT_I8 ? 1 : 4) : nullptr;
@@ -898,10 +935,9 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     p.skip_first_copy = f->expire_next_wait ? 1 : 0;
     p.wait_tries = f->expire_next_wait ? 2000u : 0u;
     f->expire_next_wait = false;
-    const int64_t units = (n + tb::kRWUnitRows - 1) / tb::kRWUnitRows; // (chunks: at most four units to a block)
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)std::min(units, plan.grid_x), (unsigned)plan.chunks);
-    cfg.blockDim = dim3(tb::kRWThreads);
+    cfg.gridDim = dim3((unsigned)batches, (unsigned)plan.chunks);
+    cfg.blockDim = dim3(32u * (unsigned)(walkers + 2));
     cfg.dynamicSmemBytes = (size_t)plan.smem;
     cfg.stream = stream;
     // the walk starts its tree copies while the rows are still being ranked
@@ -909,7 +945,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = fused ? 0 : 1;
     CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
     ++f->launches;
   }
@@ -917,7 +953,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     CUDA_TRY(cudaEventRecord(f->ev1, stream));
     f->ev_pending = true;
   }
-  if (ws->done) CUDA_TRY(cudaEventRecord(ws->done, stream));
+  if (ws->done) CUDA_TRY(cudaEventRecord(ws->done, stream)); // (uses are marked)
   return TBK_OK;
 }
 
@@ -1113,30 +1149,52 @@ bool is_pinned(const void *ptr) {
 
 // Small host batches: everything but the walk itself is latency, so there are no copies to
 // enqueue and wait for.  The rows go through one pinned buffer that a ranking kernel reads over
-// PCIe (every value once); other kernels read rows more than once and get them copied.  Results
-// are written to pinned memory by the kernel that computes them, and the status word is mapped
-// host memory as well: one synchronisation ends the call.
+// PCIe (every value once) -- or, up to 256 values, with the launch itself; other kernels read rows
+// more than once and get them copied.  Results are written to pinned memory by the kernel that
+// computes them, over a value that no prediction has; the call ends when the last one has been
+// overwritten, several microseconds before fences in the kernel or the stream's end would tell.
+// The status word is mapped host memory as well.
 constexpr size_t kSmallRows = (size_t)512 << 10, kSmallDirect = (size_t)128 << 10, kSmallResults = (size_t)512 << 10;
+constexpr uint32_t kNoResult = 0x7fa5c3e1u; // as a float: a NaN that no arithmetic returns
+constexpr uint8_t kNoClass = 0xff;          // (class ids are at most 126)
 int predict_host_small(tbk_forest *f, const float *h_rows, int64_t n_rows, int64_t ld, void *h_out, int32_t out_kind) {
   const size_t bytes = ((size_t)(n_rows - 1) * ld + f->packed.num_features) * 4; // (nothing behind the last row's values)
-  const size_t out_bytes = (size_t)n_rows * (out_kind == TBK_OUT_I8 ? 1 : 4);
+  const bool classes = out_kind == TBK_OUT_I8;
+  const size_t out_bytes = (size_t)n_rows * (classes ? 1 : 4);
+  cudaStream_t stream = f->streams[0];
   if (!f->h_small) {
     CUDA_TRY(cudaHostAlloc(&f->h_small, kSmallRows + kSmallResults, cudaHostAllocMapped));
     CUDA_TRY(cudaHostGetDevicePointer(&f->d_small, f->h_small, 0));
     CUDA_TRY(cudaMalloc(&f->d_small_in, kSmallRows));
   }
+  unsigned char *results = f->h_small + kSmallRows;
+  if (classes) std::memset(results, kNoClass, out_bytes);
+  else std::fill_n(reinterpret_cast<uint32_t *>(results), n_rows, kNoResult);
   copy_past_caches(f->h_small, reinterpret_cast<const unsigned char *>(h_rows), bytes);
   const unsigned char *rows = f->d_small;
   if (!f->rank || bytes > kSmallDirect) {
-    CUDA_TRY(cudaMemcpyAsync(f->d_small_in, f->h_small, bytes, cudaMemcpyHostToDevice, f->streams[0]));
+    CUDA_TRY(cudaMemcpyAsync(f->d_small_in, f->h_small, bytes, cudaMemcpyHostToDevice, stream));
     rows = f->d_small_in;
   }
+  f->inline_rows = h_rows;
   const int rc = run(f, kPredict, reinterpret_cast<const float *>(rows), n_rows, ld, f->d_small + kSmallRows, out_kind, nullptr,
-                     nullptr, f->streams[0], 0);
-  const cudaError_t e = cudaStreamSynchronize(f->streams[0]);
-  if (rc != TBK_OK) return rc;
-  if (e != cudaSuccess) return fail(TBK_ERR_CUDA, "cudaStreamSynchronize: %s", cudaGetErrorString(e));
-  std::memcpy(h_out, f->h_small + kSmallRows, out_bytes);
+                     nullptr, stream, 0);
+  f->inline_rows = nullptr;
+  bool idle = rc != TBK_OK;
+  for (int64_t r = 0; r < n_rows && !idle; ++r)
+    for (int spin = 1; !idle; ++spin) {
+      if (classes ? reinterpret_cast<volatile uint8_t *>(results)[r] != kNoClass
+                  : reinterpret_cast<volatile uint32_t *>(results)[r] != kNoResult)
+        break;
+      idle = spin % 1024 == 0 && cudaStreamQuery(stream) != cudaErrorNotReady; // done without it, or an error
+    }
+  if (idle) {
+    const cudaError_t e = cudaStreamSynchronize(stream);
+    if (rc != TBK_OK) return rc;
+    if (e != cudaSuccess) return fail(TBK_ERR_CUDA, "cudaStreamSynchronize: %s", cudaGetErrorString(e));
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  std::memcpy(h_out, results, out_bytes);
   return check_status(f);
 }
 
@@ -1451,6 +1509,9 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     f->rf.lattice = q.lattice;
     f->rf.whole_compare = q.whole_compare;
     f->rf.groups = q.groups;
+    f->uniform_depth = (int)q.groups[0].depth;
+    for (const auto &g : q.groups)
+      if ((int)g.depth != f->uniform_depth) f->uniform_depth = 0;
     f->rf.features = q.features;
     plan_rank_tables(f);
     const int64_t rows = std::min(batch_hint > 0 ? batch_hint : 65536, rank_rows_per_pass(f));

@@ -26,6 +26,11 @@
 // the last block to finish with a batch adds them up in chunk order -- one launch, and the same
 // result every time.
 //
+// The smallest batches are ranked by the walkers themselves (every tree chunk's blocks rank their
+// rows again): a launch of its own takes longer than a few values per thread.  They also take a
+// variant of the kernel (NR = 4) with at most 20 walker warps of four rows each and every loop
+// rolled up: the code of such a launch is executed once.
+//
 // Multiclass: the running sums belong to one class at a time (a class owns consecutive columns);
 // when the class changes they are combined across the lanes -- afterwards a lane holds the class
 // sum of ONE row -- and the best class so far is updated with the reference's tie rule (ties go
@@ -36,9 +41,12 @@
 // tree caches src/gpu/GPURepresentations.cpp:279-399, :630-715, the cross-thread reduction
 // src/reduction/LowerReduceOps.cpp:921-1003.
 #pragma once
+#include "rank_rows.cuh"
 #include "walk_quant.cuh"
 
 namespace tb {
+
+constexpr int kRankInline = 256; // row values that travel with the launch
 
 struct RankWalkParams {
   const uint32_t *node_plane;
@@ -47,6 +55,7 @@ struct RankWalkParams {
   const int32_t *tree_index;
   const int32_t *class_begin; // multiclass
   const unsigned char *keys;  // [n_rows][S]
+  RankRowsParams ranking;     // rows != null: a block ranks the rows of its only batch itself
   long long n_rows;
   float *partial;             // where write_partial asks for raw sums
   float *scratch;             // [chunks][n_rows] partial sums, or (best sum, class) pairs
@@ -55,6 +64,7 @@ struct RankWalkParams {
   unsigned int *arrivals;     // per row batch: chunks that are done (zero between launches)
   long long num_trees;
   int32_t num_groups, groups_per_chunk, num_classes, classes_per_chunk;
+  int32_t uniform_depth;      // of all groups; 0: they differ
   int32_t write_partial, out_kind, transform;
   float initial_value;
   int32_t stages;
@@ -62,6 +72,8 @@ struct RankWalkParams {
   int32_t *status;
   int32_t skip_first_copy; // failure drill
   uint32_t wait_tries;
+  uint32_t inline_values; // > 0: the rows are these, one after another
+  float inline_rows[kRankInline];
 };
 
 constexpr int kRWWalkers = 20, kRWThreads = 32 * (kRWWalkers + 2);
@@ -178,12 +190,31 @@ __device__ __forceinline__ void rank_walk4(uint32_t (&v)[4], uint32_t col, uint3
 #undef TBR_ROWS
 }
 
-// Adds up v over the 32 lanes for every of 16 rows: afterwards lanes 2i and 2i + 1 hold the sum
-// of row i.
-__device__ __forceinline__ float rank_reduce_rows(float (&v)[16], int lane) {
+// The same walk with the levels rolled up; the offset moves from level to level with the loop.
+template <int S> __device__ __forceinline__ void rank_walk4_rolled(uint32_t (&v)[4], uint32_t depth, uint32_t col, uint32_t kb) {
+  uint32_t off[4] = {col, col, col, col}, step = 128;
+#pragma unroll 1
+  for (uint32_t d = 0; d < depth; ++d, step *= 2) {
+    uint32_t node[4], key[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) node[q] = lds_u32(off[q]);
+    key[0] = lds_u16_imm<rank_row_offset<S>(0)>((node[0] >> 16) + kb);
+    key[1] = lds_u16_imm<rank_row_offset<S>(1)>((node[1] >> 16) + kb);
+    key[2] = lds_u16_imm<rank_row_offset<S>(2)>((node[2] >> 16) + kb);
+    key[3] = lds_u16_imm<rank_row_offset<S>(3)>((node[3] >> 16) + kb);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) off[q] += step + (key[q] >= (node[q] & 0xffffu) ? step : 0u);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = lds_u32_imm<128>(off[q]); // past the node plane's last, unused slot
+}
+
+// Adds up v over the 32 lanes for every of NR rows: afterwards lane l holds the sum of row
+// l * NR / 32 (32 / NR neighbouring lanes hold the same row).
+template <int NR> __device__ __forceinline__ float rank_reduce_rows(float (&v)[NR], int lane) {
   int bit = 16;
 #pragma unroll
-  for (int half = 8; half >= 1; half /= 2, bit /= 2) {
+  for (int half = NR / 2; half >= 1; half /= 2, bit /= 2) {
     const bool up = lane & bit;
 #pragma unroll
     for (int i = 0; i < half; ++i) {
@@ -191,7 +222,9 @@ __device__ __forceinline__ float rank_reduce_rows(float (&v)[16], int lane) {
       v[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
     }
   }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+  float s = v[0];
+  for (; bit >= 1; bit /= 2) s += __shfl_xor_sync(0xffffffffu, s, bit);
+  return s;
 }
 // One group of depth D for the warp's rows, four times `fours` of them; use(c, v) takes the leaf
 // words of rows 4c .. 4c+3.
@@ -224,8 +257,13 @@ __device__ __forceinline__ void rank_walk_rows(int fours, uint32_t col, uint32_t
   rank_walk4<D, S, 12, WHOLE>(v, col, kb, t);
   use(3, v);
 }
-template <int S, bool WHOLE, typename Use>
+template <int S, int NR, bool WHOLE, typename Use>
 __device__ __forceinline__ void rank_walk_group(uint32_t depth, int fours, uint32_t col, uint32_t kb, Use use) {
+  if constexpr (NR == 4) {
+    uint32_t v[4];
+    rank_walk4_rolled<S>(v, depth, col, kb);
+    return use(0, v);
+  }
   switch (depth) {
   case 1: return rank_walk_rows<1, S, WHOLE>(fours, col, kb, use);
   case 2: return rank_walk_rows<2, S, WHOLE>(fours, col, kb, use);
@@ -240,19 +278,22 @@ __device__ __forceinline__ void rank_walk_group(uint32_t depth, int fours, uint3
 
 enum RankMode { kRankSums, kRankClasses, kRankLeafIds };
 
-// S: bytes per row of keys.
-template <int S, bool WHOLE, int MODE>
-__global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankWalkParams p) {
+// S: bytes per row of keys; NR: most rows per warp (16, or 4 where a block has one unit of rows;
+// that variant compares whole numbers whatever the ranks).
+template <int S, int NR, bool WHOLE, int MODE>
+__global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const __grid_constant__ RankWalkParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0); // uniform by construction
+  const int NW = NR == 4 ? (int)(blockDim.x >> 5) - 2 : kRWWalkers; // walker warps
+  const int UR = 4 * NW;                                           // rows per unit
   const uint32_t bars_s = smem_u32(smem_raw);
   const uint32_t full_s = bars_s, empty_s = bars_s + 64u, keys_full_s = bars_s + 128u, keys_empty_s = bars_s + 144u;
   volatile uint32_t *last_flag = reinterpret_cast<volatile uint32_t *>(smem_raw + 192);
   unsigned char *keys = smem_raw + kRWBarBytes;           // two batches of keys
   unsigned char *ring = keys + 2 * kRWBatchRows * S;
   // this block's units of rows, in batches of up to four
-  const long long units = (p.n_rows + kRWUnitRows - 1) / kRWUnitRows;
+  const long long units = (p.n_rows + UR - 1) / UR;
   const int unit0 = (int)(units * blockIdx.x / gridDim.x), unit1 = (int)(units * (blockIdx.x + 1) / gridDim.x);
   const int my_batches = (unit1 - unit0 + kRWBatchUnits - 1) / kRWBatchUnits;
   // this chunk's groups; with classes: those that hold the columns of classes c0 .. c1 - 1
@@ -271,9 +312,9 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
   if (tid == 0) {
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
     for (int i = 0; i < kRWMaxStages; ++i) mbar_init(bars + i, 1);              // full: the copies' bytes
-    for (int i = 0; i < kRWMaxStages; ++i) mbar_init(bars + 8 + i, kRWWalkers); // empty: one arrival per walker warp
+    for (int i = 0; i < kRWMaxStages; ++i) mbar_init(bars + 8 + i, NW); // empty: one arrival per walker warp
     for (int i = 0; i < 2; ++i) mbar_init(bars + 16 + i, 1);                    // keys_full
-    for (int i = 0; i < 2; ++i) mbar_init(bars + 18 + i, kRWWalkers);           // keys_empty
+    for (int i = 0; i < 2; ++i) mbar_init(bars + 18 + i, NW);           // keys_empty
     fence_barrier_init();
   }
   __syncthreads();
@@ -284,7 +325,7 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
   // (the warp agrees on the outcome: shuffles follow)
   auto wait = [tries](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_all_lanes(bar, parity, tries)) != 0; };
 
-  if (warp == kRWWalkers) {
+  if (warp == NW) {
     // ---- tree groups, batch after batch
     const uint64_t keep = l2_policy_keep();
     int slot = 0;
@@ -294,31 +335,32 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
         if (round > 0) ok = wait(empty_s + 8u * (uint32_t)slot, (round - 1u) & 1u);
         issued += ok;
         if (ok && lane == 0 && !(p.skip_first_copy && it == 0 && k == 0)) {
-          const DevQuantGroup gm = p.groups[g0 + k];
-          const uint32_t bytes = gm.slots * 128u;
+          const uint32_t d = p.uniform_depth;
+          const unsigned long long elem = d ? (unsigned long long)(g0 + k) << (d + 5) : p.groups[g0 + k].elem_off;
+          const uint32_t bytes = 128u << (d ? d : p.groups[g0 + k].depth);
           unsigned char *dst = ring + (size_t)slot * p.stage_bytes;
           uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw) + slot;
           mbar_expect_tx(bar, 2u * bytes);
-          bulk_g2s_hint(dst, p.node_plane + gm.elem_off, bytes, bar, keep);
-          bulk_g2s_hint(dst + bytes, p.leaf_plane + gm.elem_off, bytes, bar, keep);
+          bulk_g2s_hint(dst, p.node_plane + elem, bytes, bar, keep);
+          bulk_g2s_hint(dst + bytes, p.leaf_plane + elem, bytes, bar, keep);
         }
         if (++slot == p.stages) {
           slot = 0;
           ++round;
         }
       }
-  } else if (warp == kRWWalkers + 1) {
+  } else if (warp == NW + 1) {
     // ---- the batches' keys, one batch ahead of the walk; the kernel that ranks the rows may
     // still be running when this one starts
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint64_t stream = l2_policy_stream();
-    for (int it = 0; it < my_batches && ok; ++it) {
+    for (int it = 0; it < my_batches && ok && !p.ranking.rows; ++it) {
       const uint32_t buf = (uint32_t)it & 1u;
       if (it >= 2) ok = wait(keys_empty_s + 8u * buf, (uint32_t)((it >> 1) - 1) & 1u);
       issued += ok;
       if (ok && lane == 0) {
         const int u = unit0 + it * kRWBatchUnits;
-        const long long row0 = (long long)u * kRWUnitRows, end = (long long)min(unit1, u + kRWBatchUnits) * kRWUnitRows;
+        const long long row0 = (long long)u * UR, end = (long long)min(unit1, u + kRWBatchUnits) * UR;
         const uint32_t bytes = ((uint32_t)(min(end, p.n_rows) - row0) + 1u & ~1u) * (uint32_t)S; // (rows may lie in pairs)
         uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw) + 16 + buf;
         mbar_expect_tx(bar, bytes);
@@ -333,15 +375,33 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
     uint32_t parity = 0;
     for (int it = 0; it < my_batches && ok; ++it) {
       const int fours = min(unit1 - unit0 - it * kRWBatchUnits, kRWBatchUnits); // rows per warp / 4
-      const long long row0 = (long long)(unit0 + it * kRWBatchUnits) * kRWUnitRows + warp * fours * 4;
-      const long long row = row0 + (lane >> 1); // the row whose sum this lane ends up with
-      const bool live = (lane & 1) == 0 && lane < 8 * fours && row < p.n_rows;
-      ok = wait(keys_full_s + 8u * ((uint32_t)it & 1u), (uint32_t)(it >> 1) & 1u);
-      if (!ok) break;
+      const long long row0 = (long long)(unit0 + it * kRWBatchUnits) * UR + warp * fours * 4;
+      const long long row = row0 + lane * NR / 32; // the row whose sum this lane ends up with
+      const bool live = (lane & (32 / NR - 1)) == 0 && lane * NR / 32 < 4 * fours && row < p.n_rows;
+      if (p.ranking.rows) {
+        const RankRowsParams &r = p.ranking;
+        const int F = r.num_features;
+        const uint32_t values = (uint32_t)(min((long long)unit1 * UR, p.n_rows) - (long long)unit0 * UR) * (uint32_t)F;
+        unsigned searched = 0;
+        for (uint32_t i = tid; i < values; i += 32 * NW) {
+          const uint32_t q = i / (uint32_t)F, f = i - q * (uint32_t)F;
+          const float x = p.inline_values ? p.inline_rows[i] : __ldg(r.rows + ((long long)unit0 * UR + q) * r.ld + f);
+          const uint32_t at = S == 64 ? (q >> 1) * 128u + 4u * f + (q & 1u) * 2u : q * S + 2u * f;
+          sts_u16(smem_u32(keys) + at, rank_value(x, r.features + f, r.lut, r.thr, searched));
+        }
+        if (blockIdx.y == 0) {
+          searched = __reduce_add_sync(0xffffffffu, searched);
+          if (elected && searched) atomicAdd(r.searched, (unsigned long long)searched);
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(32 * NW) : "memory");
+      } else {
+        ok = wait(keys_full_s + 8u * ((uint32_t)it & 1u), (uint32_t)(it >> 1) & 1u);
+        if (!ok) break;
+      }
       const uint32_t kb = smem_u32(keys) + ((uint32_t)it & 1u) * (uint32_t)(kRWBatchRows * S) + (uint32_t)(warp * fours * 4 * S);
-      float acc[16];
+      float acc[NR];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+      for (int i = 0; i < NR; ++i) acc[i] = 0.f;
       [[maybe_unused]] int cls = c0, lo = col0 & 31, best_class = c0;
       [[maybe_unused]] float sum = 0.f, best = -INFINITY;
       // class `cls` is complete, its sum for this lane's row in `sum`
@@ -356,18 +416,18 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
         sum = 0.f;
         ++cls;
       };
-      uint32_t next_depth = NG > 0 ? p.groups[g0].depth : 0u;
+      uint32_t next_depth = p.uniform_depth ? (uint32_t)p.uniform_depth : NG > 0 ? p.groups[g0].depth : 0u;
       for (int k = 0; k < NG; ++k) {
         const uint32_t depth = next_depth;
-        next_depth = p.groups[min(g0 + k + 1, g1 - 1)].depth;
+        if (!p.uniform_depth) next_depth = p.groups[min(g0 + k + 1, g1 - 1)].depth;
         ok = wait(full_s + 8u * (uint32_t)slot, parity);
         if (!ok) break;
         const uint32_t col = ring_col + (uint32_t)slot * p.stage_bytes;
         if constexpr (MODE == kRankLeafIds) {
           const int t = p.tree_index[(g0 + k) * 32 + lane];
           int32_t *dst = p.leaf_ids + row0 * p.num_trees + t;
-          const int rows = (int)min(16ll, p.n_rows - row0);
-          rank_walk_group<S, WHOLE>(depth, fours, col, kb, [&](int c, const uint32_t(&v)[4]) {
+          const int rows = (int)min((long long)NR, p.n_rows - row0);
+          rank_walk_group<S, NR, WHOLE>(depth, fours, col, kb, [&](int c, const uint32_t(&v)[4]) {
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               if (t >= 0 && 4 * c + q < rows) dst[(4 * c + q) * p.num_trees] = (int32_t)v[q];
@@ -379,21 +439,21 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
           };
           if constexpr (MODE == kRankClasses) {
             int next = p.class_begin[cls + 1] - (g0 + k) * 32; // first column of the next class
-            auto combine = [&](float(&v)[16]) { sum += rank_reduce_rows(v, lane); };
-            if (lo == 0 && next >= 32) { // one class
-              rank_walk_group<S, WHOLE>(depth, fours, col, kb, add);
+            auto combine = [&](float(&v)[NR]) { sum += rank_reduce_rows<NR>(v, lane); };
+            if (NR > 4 && lo == 0 && next >= 32) { // one class
+              rank_walk_group<S, NR, WHOLE>(depth, fours, col, kb, add);
               if (next == 32) {
                 combine(acc);
                 finish();
 #pragma unroll
-                for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+                for (int i = 0; i < NR; ++i) acc[i] = 0.f;
               }
-            } else if (lo == 0 && cls + 1 < c1 && p.class_begin[cls + 2] - (g0 + k) * 32 > 32) {
+            } else if (NR > 4 && lo == 0 && cls + 1 < c1 && p.class_begin[cls + 2] - (g0 + k) * 32 > 32) {
               // two classes: this one's columns complete its sums, the others start the next one's
-              float other[16];
+              float other[NR];
 #pragma unroll
-              for (int i = 0; i < 16; ++i) other[i] = 0.f;
-              rank_walk_group<S, WHOLE>(depth, fours, col, kb, [&](int c, const uint32_t(&v)[4]) {
+              for (int i = 0; i < NR; ++i) other[i] = 0.f;
+              rank_walk_group<S, NR, WHOLE>(depth, fours, col, kb, [&](int c, const uint32_t(&v)[4]) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                   acc[4 * c + q] += lane < next ? __uint_as_float(v[q]) : 0.f;
@@ -403,27 +463,27 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
               combine(acc);
               finish();
 #pragma unroll
-              for (int i = 0; i < 16; ++i) acc[i] = other[i];
+              for (int i = 0; i < NR; ++i) acc[i] = other[i];
             } else { // several, or a chunk that starts or ends inside the group
               if (lo == 0) combine(acc);
 #pragma unroll
-              for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-              rank_walk_group<S, WHOLE>(depth, fours, col, kb, add);
+              for (int i = 0; i < NR; ++i) acc[i] = 0.f;
+              rank_walk_group<S, NR, WHOLE>(depth, fours, col, kb, add);
               while (cls < c1 && next <= 32) { // classes that end in this group
-                float part[16];
+                float part[NR];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) part[i] = lane >= lo && lane < next ? acc[i] : 0.f;
+                for (int i = 0; i < NR; ++i) part[i] = lane >= lo && lane < next ? acc[i] : 0.f;
                 combine(part);
                 finish();
                 lo = next;
                 if (cls < c1) next = p.class_begin[cls + 1] - (g0 + k) * 32;
               }
 #pragma unroll
-              for (int i = 0; i < 16; ++i) acc[i] = lane >= lo ? acc[i] : 0.f;
+              for (int i = 0; i < NR; ++i) acc[i] = lane >= lo ? acc[i] : 0.f;
               lo = 0;
             }
           } else {
-            rank_walk_group<S, WHOLE>(depth, fours, col, kb, add);
+            rank_walk_group<S, NR, WHOLE>(depth, fours, col, kb, add);
           }
         }
         __syncwarp();
@@ -437,7 +497,7 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
       if (elected) mbar_arrive(keys_empty_s + 8u * ((uint32_t)it & 1u));
       // ---- the batch's results
       if constexpr (MODE == kRankSums) {
-        const float s = rank_reduce_rows(acc, lane);
+        const float s = rank_reduce_rows<NR>(acc, lane);
         if (live) {
           if (gridDim.y > 1) p.scratch[(long long)blockIdx.y * p.n_rows + row] = s;
           else if (p.write_partial) p.partial[row] = s;
@@ -459,8 +519,8 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
   if (chunked) __threadfence();
   if (__syncthreads_or(!ok)) {
     if (tid == 0) set_status(p.status, 4);
-    if (warp >= kRWWalkers) { // no copy may land after the block is gone
-      const uint32_t bars = warp == kRWWalkers ? full_s : keys_full_s, n = warp == kRWWalkers ? (uint32_t)p.stages : 2u;
+    if (warp >= NW) { // no copy may land after the block is gone
+      const uint32_t bars = warp == NW ? full_s : keys_full_s, n = warp == NW ? (uint32_t)p.stages : 2u;
       for (uint32_t s = 0; s < min(n, issued); ++s) wait(bars + 8u * s, ((issued - 1u - s) / n) & 1u);
     }
   }
@@ -474,24 +534,36 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const RankW
   __syncthreads();
   if (!*last_flag) return;
   __threadfence();
-  const long long row = (long long)unit0 * kRWUnitRows + tid;
-  if (row >= min((long long)unit1 * kRWUnitRows, p.n_rows)) return;
+  const long long row = (long long)unit0 * UR + tid;
+  if (row >= min((long long)unit1 * UR, p.n_rows)) return;
+  // (many loads at a time: their round trip is what this costs)
   if constexpr (MODE == kRankClasses) {
     float best = -INFINITY;
     int best_class = 0;
-    for (int y = 0; y < (int)gridDim.y; ++y) { // (classes rise with the chunks: a later one wins ties)
-      const float2 b = __ldcg(reinterpret_cast<const float2 *>(p.scratch) + (long long)y * p.n_rows + row);
-      if (b.x >= best) {
-        best = b.x;
-        best_class = __float_as_int(b.y);
-      }
+    for (int y = 0; y < (int)gridDim.y; y += 8) {
+      float2 b[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        b[i] = y + i < (int)gridDim.y ? __ldcg(reinterpret_cast<const float2 *>(p.scratch) + (long long)(y + i) * p.n_rows + row)
+                                      : make_float2(__int_as_float(0x7fffffff), 0.f); // (NaN wins nothing)
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (b[i].x >= best) { // (classes rise with the chunks: a later one wins ties)
+          best = b[i].x;
+          best_class = __float_as_int(b[i].y);
+        }
     }
     if (p.out_kind == 1) reinterpret_cast<int8_t *>(p.out)[row] = (int8_t)best_class;
     else reinterpret_cast<float *>(p.out)[row] = (float)best_class;
   } else {
     float s = 0.f;
-#pragma unroll 4
-    for (int y = 0; y < (int)gridDim.y; ++y) s += __ldcg(p.scratch + (long long)y * p.n_rows + row);
+    for (int y = 0; y < (int)gridDim.y; y += 16) {
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = y + i < (int)gridDim.y ? __ldcg(p.scratch + (long long)(y + i) * p.n_rows + row) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) s += v[i];
+    }
     if (p.write_partial) p.partial[row] = s;
     else reinterpret_cast<float *>(p.out)[row] = apply_transform(p.initial_value + s, p.transform);
   }
