@@ -1,5 +1,5 @@
-"""Rank keys (forests of at most 8 levels over at most 64 features) at the edges of their kernels:
-unit and batch sizes of the walk, rows in pairs and one by one, groups of mixed depth, classes that
+"""Rank keys (forests of at most 8 levels) at the edges of their kernels:
+unit and batch sizes of the walks, rows in pairs, one by one and in tiles, groups of mixed depth, classes that
 share a group of trees, more thresholds than the half-precision comparison holds, and the direct
 and the shared-memory ranking of rows."""
 import numpy as np
@@ -39,7 +39,8 @@ def _rows(f, marg, n, seed=9):
 @pytest.mark.parametrize("trees,levels,features,classes,rows", [
     (1, 1, 1, 0, 1), (31, 2, 32, 0, 79), (33, 3, 33, 0, 81), (100, 6, 8, 0, 320), (97, 8, 64, 0, 321),
     (300, 7, 20, 0, 148 * 80 * 4 + 77), (64, 8, 28, 3, 5), (45, 5, 16, 7, 12003), (400, 8, 40, 26, 2500),
-    (140, 8, 1, 0, 4000)])
+    (140, 8, 1, 0, 4000), (1, 3, 65, 0, 1), (33, 8, 90, 0, 129), (90, 7, 111, 0, 148 * 128 * 3 + 5),
+    (70, 6, 511, 0, 2000), (40, 8, 300, 0, 30011)])
 def test_rank_key_walk_is_exact(trees, levels, features, classes, rows):
     f, marg = _forest(trees, levels, features, classes, p=0.0 if features == 1 and trees > 1 else 0.2)
     X = _rows(f, marg, rows)

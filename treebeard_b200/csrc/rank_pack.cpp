@@ -28,6 +28,8 @@ std::string pack_rank(const Forest &f, RankForest *out) {
   const int64_t T = f.num_trees(), N = f.num_nodes();
   const int F = f.num_features;
   if (F > kRankMaxFeatures) return "more than " + std::to_string(kRankMaxFeatures) + " features";
+  const bool tiles = F > kRankRowFeatures;
+  if (tiles && f.num_classes > 0) return "multiclass forests over more than " + std::to_string(kRankRowFeatures) + " features";
   RankForest &q = *out;
   q = RankForest();
   q.num_features = F;
@@ -67,7 +69,8 @@ std::string pack_rank(const Forest &f, RankForest *out) {
     uint32_t seen = most.load();
     while (d.size() > seen && !most.compare_exchange_weak(seen, (uint32_t)d.size())) {}
   }
-  if (most > kRankMax) return "a feature has more than " + std::to_string(kRankMax) + " distinct thresholds";
+  const uint32_t limit = tiles ? kRankHalfMax : kRankMax;
+  if (most > limit) return "a feature has more than " + std::to_string(limit) + " distinct thresholds";
   q.whole_compare = most > kRankHalfMax;
 
   // ---- rank tables
@@ -211,7 +214,7 @@ void walk_rank_on_host(const RankForest &q, const float *rows, int64_t n_rows, i
       uint32_t path = 0;
       for (uint32_t d = 0; d < gm.depth; ++d) {
         const uint32_t node = q.node_plane[base + (uint64_t)((1u << d) - 1 + path) * kRankCols];
-        if (key[(node >> 16) / rank_key_offset(q.num_features, 1)] >= (node & 0xffffu)) path |= 1u << d;
+        if (key[rank_feature_at(q.num_features, node >> 16)] >= (node & 0xffffu)) path |= 1u << d;
       }
       const uint64_t e = base + (uint64_t)path * kRankCols;
       while (q.num_classes > 0 && (int32_t)k >= q.class_begin[cls + 1]) ++cls;

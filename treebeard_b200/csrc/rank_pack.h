@@ -18,7 +18,8 @@
 //
 // Planes, per group of 32 trees of (padded) depth D, 2^D slots x 32 columns each:
 //   node plane  u32  (key offset << 16) | (j + 1); the offset is the byte offset of the feature's
-//                    key in a row of keys (2 f) or, for at most 32 features, in a pair of rows (4 f)
+//                    key in a row of keys (2 f), in a pair of rows (up to 32 features: 4 f) or in
+//                    a tile of 32 rows (more than 64 features: (f / 2) 128 + (f mod 2) 2)
 //   leaf plane  f32  leaf values
 // Slots: node on level d reached by the decisions r_0 .. r_(d-1) (1 = right) is slot
 // 2^d - 1 + sum r_i 2^i, leaf sum r_i 2^i.  With the decision of level i worth 2^i slots on EVERY
@@ -40,10 +41,15 @@ constexpr int kRankCols = 32, kRankMaxDepth = 8;
 // comparison, which needs no masking (one instruction per decision less than whole numbers).
 constexpr uint32_t kRankHalfMax = 31742, kRankMax = 65534;
 constexpr int kRankPairFeatures = 32; // up to here the keys of two rows lie side by side
-constexpr int kRankMaxFeatures = 64; // 16-bit keys of a row in 32 four-byte words: one bank each
-
+constexpr int kRankRowFeatures = 64;  // up to here the keys of a row have a bank each
+constexpr int kRankMaxFeatures = 511; // up to here four tiles of keys fit beside the ring (walk_rank_tiles.cuh)
 inline uint32_t rank_key_offset(int32_t num_features, uint32_t feature) {
+  if (num_features > kRankRowFeatures) return (feature >> 1) * 128 + (feature & 1) * 2;
   return num_features <= kRankPairFeatures ? 4 * feature : 2 * feature;
+}
+inline uint32_t rank_feature_at(int32_t num_features, uint32_t offset) {
+  if (num_features > kRankRowFeatures) return (offset >> 7) * 2 + (offset >> 1 & 1);
+  return num_features <= kRankPairFeatures ? offset / 4 : offset / 2;
 }
 
 struct RankFeature { // 32 bytes, the same on the device
@@ -76,8 +82,9 @@ struct RankForest {
 };
 
 // Empty string on success; fails (so that the caller can take another layout) for trees deeper
-// than 8 levels, more than kRankMaxFeatures features, non-finite thresholds or leaves, or a
-// feature with more than kRankMax distinct thresholds.
+// than 8 levels, more than kRankMaxFeatures features (kRankRowFeatures for multiclass forests),
+// non-finite thresholds or leaves, or a feature with more than kRankMax distinct thresholds
+// (kRankHalfMax beyond kRankRowFeatures features).
 std::string pack_rank(const Forest &f, RankForest *out);
 
 // Rank of a row value; *searched: the value's bucket held thresholds it was compared with.

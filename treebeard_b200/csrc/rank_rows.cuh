@@ -1,6 +1,7 @@
 // Ranks the rows of a batch (rank_pack.h): fp32 row values -> 16-bit keys in the order in which the
 // walk (walk_rank.cuh) copies them into shared memory: rows of at most 32 features in pairs
-// (PAIR: word f of a line = keys of feature f of rows 2i and 2i + 1), wider rows one by one.
+// (word f of a line = keys of feature f of rows 2i and 2i + 1), rows of at most 64 one by one, wider
+// rows in tiles of 32 (word j of line m = keys of features 2m and 2m + 1 of row j).
 //
 // A thread ranks FW neighbouring features of a row or of a pair of rows, all in lock-step: the
 // look-ups and search steps of different values are independent, so their latencies overlap.
@@ -49,7 +50,9 @@ __device__ __forceinline__ uint32_t rank_value(float x, const DevRankFeature *fe
   return s;
 }
 
-template <int FW, bool PAIR, bool SMEM>
+enum RankLayout { kRankPairs, kRankRows, kRankTiles };
+
+template <int FW, int LAYOUT, bool SMEM>
 __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankRowsParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -80,13 +83,16 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
     __syncthreads();
   }
   const int pieces = p.pieces; // without tables in shared memory: of the whole row
+  constexpr bool PAIR = LAYOUT == kRankPairs, TILES = LAYOUT == kRankTiles;
   constexpr int RPT = PAIR ? 2 : 1, N = RPT * FW; // rows and values per thread
   const uint32_t n_rows = (uint32_t)p.n_rows;     // (the host bounds a batch by the bytes of its keys)
-  const uint32_t items = (n_rows + RPT - 1) / RPT * (uint32_t)pieces;
+  // lines: rows, or pairs of rows, or all rows of the tiles; a warp takes one piece of a tile's rows
+  const uint32_t items = (TILES ? (n_rows + 31) & ~31u : (n_rows + RPT - 1) / RPT) * (uint32_t)pieces;
   unsigned searched = 0;
   for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < items; it += gridDim.x * blockDim.x) {
-    const uint32_t line = pieces == 1 ? it : it / (uint32_t)pieces; // a row, or a pair of rows
-    const int f0 = f_first + (int)(it - line * (uint32_t)pieces) * FW;
+    const uint32_t unit = TILES ? it >> 5 : it, whole = pieces == 1 ? unit : unit / (uint32_t)pieces;
+    const uint32_t line = TILES ? whole * 32u + (it & 31u) : whole;
+    const int f0 = f_first + (int)(unit - whole * (uint32_t)pieces) * FW;
     if (f0 >= F) continue;
     float x[N];
 #pragma unroll
@@ -163,7 +169,16 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
       if constexpr (PAIR) w[k] = s[k] | s[FW + k] << 16;
       else w[k] = 2 * k + 1 < N ? s[2 * k] | s[2 * k + 1] << 16 : s[2 * k];
     }
-    if constexpr (N == 8) *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    if constexpr (TILES) {
+      unsigned char *tile = reinterpret_cast<unsigned char *>(p.keys) + (size_t)whole * (32 * p.stride) + (it & 31u) * 4u;
+      if constexpr (FW == 1) {
+        *reinterpret_cast<uint16_t *>(tile + (f0 >> 1) * 128 + (f0 & 1) * 2) = (uint16_t)s[0];
+      } else {
+#pragma unroll
+        for (int k = 0; k < N / 2; ++k)
+          if (f0 + 2 * k < F) *reinterpret_cast<uint32_t *>(tile + (f0 / 2 + k) * 128) = w[k];
+      }
+    } else if constexpr (N == 8) *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
     else if constexpr (N == 4) *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
     else if constexpr (N == 2) *reinterpret_cast<uint32_t *>(dst) = w[0];
     else *reinterpret_cast<uint16_t *>(dst) = (uint16_t)w[0];

@@ -12,6 +12,7 @@
 #include "walk_deep.cuh"
 #include "rank_rows.cuh"
 #include "walk_rank.cuh"
+#include "walk_rank_tiles.cuh"
 #include "packed_image.h"
 
 #ifdef __SSE2__
@@ -169,6 +170,7 @@ struct tbk_image {
 
 struct RankPlan {
   int units = tb::kRWBatchUnits; // units of rows in a block's (first) batch
+  int quads = 0, walkers = 0;    // tiled keys: quads of tiles per batch, walker warps
   int chunks = 1, per_chunk = 1; // per_chunk: groups, or classes of a multiclass forest
   int stages = 2, smem = 0;
   uint32_t stage_bytes = 0;
@@ -674,7 +676,10 @@ int allow_smem(tbk_forest *f, const void *kernel) {
 }
 
 // bytes of keys per row
-int rank_stride(int num_features) { return num_features <= tb::kRankPairFeatures ? 64 : 128; }
+bool rank_tiled(int num_features) { return num_features > tb::kRankRowFeatures; }
+int rank_stride(int num_features) {
+  return rank_tiled(num_features) ? (num_features + 1) / 2 * 4 : num_features <= tb::kRankPairFeatures ? 64 : 128;
+}
 
 using RankKernel = void (*)(const tb::RankWalkParams);
 template <int S, int NR, bool WHOLE> RankKernel pick_rank(int mode) {
@@ -686,6 +691,49 @@ RankKernel pick_rank_kernel(int stride, bool small, bool whole, int mode) {
   if (small) return stride == 64 ? pick_rank<64, 4, true>(mode) : pick_rank<128, 4, true>(mode);
   if (stride == 64) return whole ? pick_rank<64, 16, true>(mode) : pick_rank<64, 16, false>(mode);
   return whole ? pick_rank<128, 16, true>(mode) : pick_rank<128, 16, false>(mode);
+}
+
+// The same for keys in tiles.  A block takes up to `quads` quads of tiles at a time with 16 to 24
+// walker warps; what fits beside a ring of at least three slots bounds them.
+RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
+  const auto &q = f->rf;
+  const int G = (int)q.groups.size(), D = q.max_depth;
+  const int tile_bytes = 32 * rank_stride(q.num_features);
+  const int64_t quads = (n_rows + 127) / 128;
+  struct Shape { int quads, walkers; };
+  RankPlan best;
+  double best_cost = -1.0;
+  for (const Shape sh : {Shape{1, 16}, Shape{2, 16}, Shape{3, 24}, Shape{4, 16}, Shape{5, 20}, Shape{6, 24}}) {
+    RankPlan p;
+    p.quads = sh.quads;
+    p.walkers = sh.walkers;
+    p.stage_bytes = 128u << D;
+    const int room = f->max_smem_optin - tb::rank_tiles_smem_bytes(tile_bytes, 4 * sh.quads, sh.walkers, 4, 0, 0);
+    p.stages = std::min(tb::kRTMaxSlots, room / (int)p.stage_bytes);
+    if (p.stages < 3) continue;
+    p.smem = tb::rank_tiles_smem_bytes(tile_bytes, 4 * sh.quads, sh.walkers, 4, p.stages, p.stage_bytes);
+    // clocks of a group of trees for a batch of b quads (2 D - 0.25 wavefronts per 32 rows and tree)
+    auto group = [&](int64_t b) {
+      return std::max(1.15 * 4 * 32 * (double)b * (2 * D - 0.25) + 300.0, std::max(2.0 * p.stage_bytes / 70.0, 32.0 / (sh.walkers / sh.quads) * 90.0 * D));
+    };
+    auto block = [&](int64_t mine) { return (double)(mine / sh.quads) * group(sh.quads) + (mine % sh.quads ? group(mine % sh.quads) : 0.0); };
+    const int most = f->user.tree_chunks > 0 ? std::min(G, f->user.tree_chunks) : std::min(G, 64);
+    for (int c = f->user.tree_chunks > 0 ? most : 1; c <= most; ++c) {
+      const int per = (G + c - 1) / c, chunks = (G + per - 1) / per;
+      const int64_t x = chunks > 1 ? (quads + sh.quads - 1) / sh.quads : std::min<int64_t>(quads, f->num_sms);
+      if (chunks > 1 && x >= f->num_sms && f->user.tree_chunks <= 0) break;
+      const double waves = chunks > 1 ? (double)((x * chunks + f->num_sms - 1) / f->num_sms) : 1.0;
+      const double cost = waves * (per * block((quads + x - 1) / x) + 4000.0) + (chunks > 1 ? 1500.0 : 0.0);
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best = p;
+        best.chunks = chunks;
+        best.per_chunk = per;
+        best.grid_x = x;
+      }
+    }
+  }
+  return best;
 }
 
 // Launch shape of the walk over `n_rows` rows: blocks along the rows and tree chunks, by what the
@@ -739,7 +787,7 @@ RankPlan make_rank_plan(const tbk_forest *f, int64_t n_rows, bool leaf_ids) {
 
 RankPlan plan_rank(tbk_forest *f, int64_t n_rows, bool leaf_ids) { // (a server's batches are mostly alike)
   if (f->rank_plan_rows != n_rows || f->rank_plan_ids != leaf_ids) {
-    f->rank_plan = make_rank_plan(f, n_rows, leaf_ids);
+    f->rank_plan = rank_tiled(f->rf.num_features) ? make_rank_tiles_plan(f, n_rows) : make_rank_plan(f, n_rows, leaf_ids);
     f->rank_plan_rows = n_rows;
     f->rank_plan_ids = leaf_ids;
   }
@@ -748,7 +796,7 @@ RankPlan plan_rank(tbk_forest *f, int64_t n_rows, bool leaf_ids) { // (a server'
 
 tb::LaunchPlan rank_launch_plan(const RankPlan &r) {
   tb::LaunchPlan plan;
-  plan.row_warps = std::max(1, tb::kRWUnitRows * r.units / 32);
+  plan.row_warps = r.quads ? 4 * r.quads : std::max(1, tb::kRWUnitRows * r.units / 32);
   plan.tree_threads = tb::kRWWalkers;
   plan.rows_per_lane = 1;
   plan.chunks = r.chunks;
@@ -766,12 +814,12 @@ tb::LaunchPlan rank_launch_plan(const RankPlan &r) {
 // chunks has an arrival counter for every row batch.
 int64_t rank_rows_per_pass(const tbk_forest *f) {
   const int64_t by_keys = ((int64_t)96 << 20) / rank_stride(f->rf.num_features);
-  const int64_t round = (int64_t)tb::kRWBatchRows * f->num_sms;
+  const int64_t round = rank_tiled(f->rf.num_features) ? (int64_t)128 * f->num_sms : (int64_t)tb::kRWBatchRows * f->num_sms;
   return std::max(round, by_keys / round * round);
 }
 
-size_t rank_key_bytes(const tbk_forest *f, int64_t rows) { // (the last pair of rows may be half empty)
-  return ((size_t)(rows + 1) * rank_stride(f->rf.num_features) + 255) / 256 * 256;
+size_t rank_key_bytes(const tbk_forest *f, int64_t rows) { // (whole tiles)
+  return ((size_t)((rows + 31) / 32 * 32) * rank_stride(f->rf.num_features) + 255) / 256 * 256;
 }
 size_t rank_workspace_bytes(const tbk_forest *f, const RankPlan &plan, int64_t rows) {
   size_t bytes = tb::kRankArrivalBytes + rank_key_bytes(f, rows);
@@ -802,8 +850,8 @@ tb::RankRowsParams rank_rows_params(const tbk_forest *f, const float *rows, int6
 int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, uint16_t *keys, cudaStream_t stream) {
   const int F = f->rf.num_features;
   tb::RankRowsParams p = rank_rows_params(f, rows, n, ld, keys);
-  const bool pair = F <= tb::kRankPairFeatures;
-  const int64_t lines = pair ? (n + 1) / 2 : n;
+  const bool pair = F <= tb::kRankPairFeatures, tiled = rank_tiled(F);
+  const int64_t lines = pair ? (n + 1) / 2 : tiled ? (n + 31) / 32 * 32 : n;
   // Tables in shared memory pay once every SM has a few thousand values to rank: loading them
   // takes about as long as ranking 2000 values through L2 (a gather there costs a wavefront per lane).
   if (f->rank_width > 0 && n * F > (int64_t)f->num_sms * 2048) {
@@ -812,11 +860,15 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
     const int64_t want = (lines * p.pieces + 1023) / 1024;
     const dim3 grid((unsigned)std::min<int64_t>(want, std::max(1, f->num_sms / slabs)), (unsigned)slabs);
     using K = void (*)(const tb::RankRowsParams);
-    const K k = pair ? (w == 4 ? tb::tb_rank_rows<4, true, true> : w == 2 ? tb::tb_rank_rows<2, true, true> : tb::tb_rank_rows<1, true, true>)
-                     : (w == 8   ? tb::tb_rank_rows<8, false, true>
-                        : w == 4 ? tb::tb_rank_rows<4, false, true>
-                        : w == 2 ? tb::tb_rank_rows<2, false, true>
-                                 : tb::tb_rank_rows<1, false, true>);
+    using tb::kRankPairs, tb::kRankRows, tb::kRankTiles;
+    const K k = tiled  ? tb::tb_rank_rows<8, kRankTiles, true>
+                : pair ? (w == 4   ? tb::tb_rank_rows<4, kRankPairs, true>
+                          : w == 2 ? tb::tb_rank_rows<2, kRankPairs, true>
+                                   : tb::tb_rank_rows<1, kRankPairs, true>)
+                       : (w == 8   ? tb::tb_rank_rows<8, kRankRows, true>
+                          : w == 4 ? tb::tb_rank_rows<4, kRankRows, true>
+                          : w == 2 ? tb::tb_rank_rows<2, kRankRows, true>
+                                   : tb::tb_rank_rows<1, kRankRows, true>);
     const int rc = allow_smem(f, (const void *)k);
     if (rc) return rc;
     k<<<grid, 1024, f->rank_smem, stream>>>(p);
@@ -824,8 +876,9 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
     // (one feature per thread: a small batch is all latency)
     p.pieces = F;
     const unsigned grid = (unsigned)std::min<int64_t>((lines * p.pieces + 255) / 256, 8ll * f->num_sms);
-    if (pair) tb::tb_rank_rows<1, true, false><<<grid, 256, 0, stream>>>(p);
-    else tb::tb_rank_rows<1, false, false><<<grid, 256, 0, stream>>>(p);
+    if (tiled) tb::tb_rank_rows<1, tb::kRankTiles, false><<<grid, 256, 0, stream>>>(p);
+    else if (pair) tb::tb_rank_rows<1, tb::kRankPairs, false><<<grid, 256, 0, stream>>>(p);
+    else tb::tb_rank_rows<1, tb::kRankRows, false><<<grid, 256, 0, stream>>>(p);
   }
   CUDA_TRY(cudaGetLastError());
   ++f->launches;
@@ -844,7 +897,7 @@ void plan_rank_tables(tbk_forest *f) {
     return b;
   };
   f->rank_width = 0;
-  for (int w = F <= tb::kRankPairFeatures ? 4 : 8; w >= 1; w /= 2) {
+  for (int w = F <= tb::kRankPairFeatures ? 4 : 8; w >= (rank_tiled(F) ? 8 : 1); w /= 2) {
     for (int pieces = (F + w - 1) / w; pieces >= 1; --pieces) {
       size_t most = 0;
       for (int first = 0; first < F; first += w * pieces) most = std::max(most, bytes(first, std::min(F, first + w * pieces)));
@@ -866,7 +919,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   int64_t pass = std::min(n_rows, rank_rows_per_pass(f));
   RankPlan plan = plan_rank(f, pass, mode == kLeafIds);
   if (plan.chunks > 1) {
-    pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * tb::kRWUnitRows);
+    pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * 64); // (units of at least 80 rows)
     plan = plan_rank(f, pass, mode == kLeafIds);
   }
   f->last_plan = rank_launch_plan(plan);
@@ -876,11 +929,13 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   unsigned char *keys = ws->mem + tb::kRankArrivalBytes;
   // one unit of rows per block: the variant for small batches, with only as many walker warps as
   // the rows -- or ranking them with two values per thread -- can use
-  const bool small = plan.units == 1;
+  const bool tiled = rank_tiled(q.num_features), small = !tiled && plan.units == 1;
   int walkers = tb::kRWWalkers;
-  if (n_rows < tb::kRWUnitRows) walkers = (int)std::min<int64_t>(walkers, std::max((n_rows + 3) / 4, (n_rows * q.num_features + 63) / 64));
-  const int unit_rows = 4 * walkers;
-  const RankKernel kernel = pick_rank_kernel(S, small, q.whole_compare != 0, kmode);
+  if (tiled) walkers = plan.walkers;
+  else if (n_rows < tb::kRWUnitRows) walkers = (int)std::min<int64_t>(walkers, std::max((n_rows + 3) / 4, (n_rows * q.num_features + 63) / 64));
+  const int unit_rows = tiled ? 128 : 4 * walkers;
+  const RankKernel kernel = tiled ? (mode == kLeafIds ? tb::tb_walk_rank_tiles_kernel<4, true> : tb::tb_walk_rank_tiles_kernel<4, false>)
+                            : pick_rank_kernel(S, small, q.whole_compare != 0, kmode);
   rc = allow_smem(f, (const void *)kernel);
   if (rc) return rc;
   tb::RankWalkParams p{};
@@ -903,6 +958,8 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   p.transform = q.transform;
   p.initial_value = (float)q.initial_value;
   p.uniform_depth = f->uniform_depth;
+  p.quads = plan.quads;
+  p.tile_bytes = 32 * S;
   p.stages = plan.stages;
   p.stage_bytes = plan.stage_bytes;
   p.status = f->d_status;
@@ -915,7 +972,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     // read the rows again, which host memory is too slow for.)
     const int64_t block_rows = std::min<int64_t>(n, (int64_t)plan.units * unit_rows);
     const bool inlined = f->inline_rows && batches == 1 && n * q.num_features <= tb::kRankInline;
-    const bool fused = pass == n_rows && plan.units < tb::kRWBatchUnits && block_rows * q.num_features <= 128 * walkers &&
+    const bool fused = !tiled && pass == n_rows && plan.units < tb::kRWBatchUnits && block_rows * q.num_features <= 128 * walkers &&
                        (!f->inline_rows || inlined || plan.chunks == 1);
     if (fused) {
       p.ranking = rank_rows_params(f, d_rows, n, ld, nullptr);
@@ -1274,8 +1331,9 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
                     (bits == 0 && (rep == TBK_REP_AUTO || rep == TBK_REP_REORG) && ts == 1 && !fp32_tile_fits &&
                      host.num_classes == 0) ||
                     (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && batch_fits && max_depth <= tb::kQuantMaxDepth);
-  // rank keys: whatever the batch kernel would take, over at most 64 features
-  if (want_quant && batch_fits && host.num_features <= tb::kRankMaxFeatures) {
+  // rank keys: whatever the key kernels would take, over at most kRankMaxFeatures features
+  const bool want_rank = want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth);
+  if (want_rank && host.num_features <= tb::kRankMaxFeatures) {
     if (tb::pack_rank(host, &im.rf).empty()) {
       im.kind = tb::PackedImage::kRank;
       im.user.representation = TBK_REP_REORG;

@@ -65,6 +65,7 @@ struct RankWalkParams {
   long long num_trees;
   int32_t num_groups, groups_per_chunk, num_classes, classes_per_chunk;
   int32_t uniform_depth;      // of all groups; 0: they differ
+  int32_t quads, tile_bytes;  // tiles of rows (walk_rank_tiles.cuh)
   int32_t write_partial, out_kind, transform;
   float initial_value;
   int32_t stages;
@@ -274,6 +275,20 @@ __device__ __forceinline__ void rank_walk_group(uint32_t depth, int fours, uint3
   case 7: return rank_walk_rows<7, S, WHOLE>(fours, col, kb, use);
   default: return rank_walk_rows<8, S, WHOLE>(fours, col, kb, use);
   }
+}
+
+// The chunks' partial sums of a row, in chunk order.  (Many loads at a time: their round trip is
+// what this costs.)
+__device__ __forceinline__ float rank_sum_chunks(const RankWalkParams &p, long long row) {
+  float s = 0.f;
+  for (int y = 0; y < (int)gridDim.y; y += 16) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = y + i < (int)gridDim.y ? __ldcg(p.scratch + (long long)(y + i) * p.n_rows + row) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s += v[i];
+  }
+  return s;
 }
 
 enum RankMode { kRankSums, kRankClasses, kRankLeafIds };
@@ -536,7 +551,6 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const __gri
   __threadfence();
   const long long row = (long long)unit0 * UR + tid;
   if (row >= min((long long)unit1 * UR, p.n_rows)) return;
-  // (many loads at a time: their round trip is what this costs)
   if constexpr (MODE == kRankClasses) {
     float best = -INFINITY;
     int best_class = 0;
@@ -556,14 +570,7 @@ __global__ void __launch_bounds__(kRWThreads, 1) tb_walk_rank_kernel(const __gri
     if (p.out_kind == 1) reinterpret_cast<int8_t *>(p.out)[row] = (int8_t)best_class;
     else reinterpret_cast<float *>(p.out)[row] = (float)best_class;
   } else {
-    float s = 0.f;
-    for (int y = 0; y < (int)gridDim.y; y += 16) {
-      float v[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = y + i < (int)gridDim.y ? __ldcg(p.scratch + (long long)(y + i) * p.n_rows + row) : 0.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) s += v[i];
-    }
+    const float s = rank_sum_chunks(p, row);
     if (p.write_partial) p.partial[row] = s;
     else reinterpret_cast<float *>(p.out)[row] = apply_transform(p.initial_value + s, p.transform);
   }
