@@ -91,9 +91,9 @@ std::string pack_rank(const Forest &f, RankForest *out) {
         rf.buckets = (uint32_t)(hi - rf.lo) + 1;
         rf.scale = 1.f;
       } else {
-        // a bucket per threshold: the table takes half the thresholds' bytes, and three or four
-        // steps finish the search of the fullest bucket that a warp meets
-        rf.buckets = (uint32_t)d.size();
+        // two buckets per threshold: the table takes as much room as the thresholds, and three steps
+        // finish the search of the fullest bucket that a warp usually meets
+        rf.buckets = 2 * (uint32_t)d.size();
         const float range = hi - rf.lo;
         rf.scale = range > 0.f && std::isfinite(range) ? (float)rf.buckets / range : 0.f;
         if (!std::isfinite(rf.scale) || rf.scale == 0.f) { // a range that fp32 cannot cut up: one bucket

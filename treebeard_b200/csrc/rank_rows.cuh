@@ -30,6 +30,7 @@ struct RankRowsParams {
   int32_t pieces;               // pieces per slab
   int32_t vec4_ok;
   int32_t lattice;              // some feature is a lattice feature
+  uint32_t turn_off;            // tiles: the warps' buffers, behind the tables
   unsigned long long *searched; // statistics: values that were compared with thresholds
 };
 
@@ -50,6 +51,10 @@ __device__ __forceinline__ uint32_t rank_value(float x, const DevRankFeature *fe
   return s;
 }
 
+// A warp that ranks a piece of a tile reads its 32 x 8 values as 32-byte stretches of rows and turns
+// them around in a buffer of its own: one row per lane would take 32 wavefronts a load.
+constexpr int kRankTurnBytes = 32 * 32 * 9 * 4;
+
 enum RankLayout { kRankPairs, kRankRows, kRankTiles };
 
 template <int FW, int LAYOUT, bool SMEM>
@@ -61,6 +66,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
   const int f_end = SMEM ? min(F, f_first + p.pieces * FW) : F;
   const DevRankFeature *feat = p.features;
   const unsigned char *lut = reinterpret_cast<const unsigned char *>(p.lut), *thr = reinterpret_cast<const unsigned char *>(p.thr);
+  [[maybe_unused]] uint32_t thr_lane = 0; // shared-memory address of the threshold before offset 0
   if constexpr (SMEM) {
     // the block's own copies: descriptors (offsets now from smem_raw), thresholds, bucket tables
     const DevRankFeature a = p.features[f_first], z = p.features[f_end - 1];
@@ -80,6 +86,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
       *reinterpret_cast<uint4 *>(smem_raw + lut_s + 16 * i) = __ldg(reinterpret_cast<const uint4 *>(p.lut + lut0) + i);
     feat = feat_s - f_first;
     lut = thr = smem_raw;
+    thr_lane = smem_u32(smem_raw) - 4u;
     __syncthreads();
   }
   const int pieces = p.pieces; // without tables in shared memory: of the whole row
@@ -95,6 +102,21 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
     const int f0 = f_first + (int)(unit - whole * (uint32_t)pieces) * FW;
     if (f0 >= F) continue;
     float x[N];
+    if constexpr (TILES && SMEM) {
+      static_assert(FW == 8, "a piece is 8 features");
+      float *turn = reinterpret_cast<float *>(smem_raw + p.turn_off) + (threadIdx.x >> 5) * (32 * 9);
+      const uint32_t lane = it & 31u, i = lane & 7u;
+      const bool in = f0 + (int)i < F;
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t r = 4u * k + (lane >> 3), row = min(whole * 32u + r, n_rows - 1);
+        turn[r * 9 + i] = in ? __ldg(p.rows + (long long)row * p.ld + f0 + i) : 0.f;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = turn[lane * 9 + k];
+    } else
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       const float *src = p.rows + (long long)min(line * RPT + r, n_rows - 1) * p.ld + f0;
@@ -154,9 +176,13 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
 #pragma unroll
       for (int k = 0; k < N; ++k) {
         const uint32_t m = s[k] + step;
-        if (m <= e[k]) {
+        if constexpr (SMEM) { // (without a branch: a value's next threshold, the comparison, the step)
+          asm volatile("{\n .reg .pred p, q;\n .reg .f32 t;\n setp.le.u32 p, %1, %2;\n mov.f32 t, 0f00000000;\n"
+                       " @p ld.shared.f32 t, [%3];\n setp.geu.and.f32 q, %4, t, p;\n @q mov.b32 %0, %1;\n}"
+                       : "+r"(s[k]) : "r"(m), "r"(e[k]), "r"(thr_lane + m), "f"(x[k]));
+        } else if (m <= e[k]) {
           const float *t = reinterpret_cast<const float *>(thr + m - 4u);
-          if (!(x[k] < (SMEM ? *t : __ldg(t)))) s[k] = m;
+          if (!(x[k] < __ldg(t))) s[k] = m;
         }
       }
     }

@@ -693,7 +693,7 @@ RankKernel pick_rank_kernel(int stride, bool small, bool whole, int mode) {
   return whole ? pick_rank<128, 16, true>(mode) : pick_rank<128, 16, false>(mode);
 }
 
-// The same for keys in tiles.  A block takes up to `quads` quads of tiles at a time with 16 to 24
+// The same for keys in tiles.  A block takes up to `quads` quads of tiles at a time with 12 to 20
 // walker warps; what fits beside a ring of at least three slots bounds them.
 RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
   const auto &q = f->rf;
@@ -703,7 +703,7 @@ RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
   struct Shape { int quads, walkers; };
   RankPlan best;
   double best_cost = -1.0;
-  for (const Shape sh : {Shape{1, 16}, Shape{2, 16}, Shape{3, 24}, Shape{4, 16}, Shape{5, 20}, Shape{6, 24}}) {
+  for (const Shape sh : {Shape{1, 16}, Shape{2, 16}, Shape{3, 12}, Shape{4, 16}, Shape{5, 20}, Shape{6, 12}}) {
     RankPlan p;
     p.quads = sh.quads;
     p.walkers = sh.walkers;
@@ -714,7 +714,7 @@ RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
     p.smem = tb::rank_tiles_smem_bytes(tile_bytes, 4 * sh.quads, sh.walkers, 4, p.stages, p.stage_bytes);
     // clocks of a group of trees for a batch of b quads (2 D - 0.25 wavefronts per 32 rows and tree)
     auto group = [&](int64_t b) {
-      return std::max(1.15 * 4 * 32 * (double)b * (2 * D - 0.25) + 300.0, std::max(2.0 * p.stage_bytes / 70.0, 32.0 / (sh.walkers / sh.quads) * 90.0 * D));
+      return std::max(1.15 * 4 * 32 * (double)b * (2 * D - 0.25) + 300.0, std::max(2.0 * p.stage_bytes / 70.0, 32.0 / (sh.walkers / sh.quads) * 50.0 * D));
     };
     auto block = [&](int64_t mine) { return (double)(mine / sh.quads) * group(sh.quads) + (mine % sh.quads ? group(mine % sh.quads) : 0.0); };
     const int most = f->user.tree_chunks > 0 ? std::min(G, f->user.tree_chunks) : std::min(G, 64);
@@ -857,6 +857,7 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
   if (f->rank_width > 0 && n * F > (int64_t)f->num_sms * 2048) {
     const int w = f->rank_width, slabs = (F + w * f->rank_pieces - 1) / (w * f->rank_pieces);
     p.pieces = f->rank_pieces;
+    p.turn_off = (uint32_t)f->rank_smem;
     const int64_t want = (lines * p.pieces + 1023) / 1024;
     const dim3 grid((unsigned)std::min<int64_t>(want, std::max(1, f->num_sms / slabs)), (unsigned)slabs);
     using K = void (*)(const tb::RankRowsParams);
@@ -871,7 +872,7 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
                                    : tb::tb_rank_rows<1, kRankRows, true>);
     const int rc = allow_smem(f, (const void *)k);
     if (rc) return rc;
-    k<<<grid, 1024, f->rank_smem, stream>>>(p);
+    k<<<grid, 1024, f->rank_smem + (tiled ? tb::kRankTurnBytes : 0), stream>>>(p);
   } else {
     // (one feature per thread: a small batch is all latency)
     p.pieces = F;
@@ -889,7 +890,7 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
 // together) and then the most pieces per block whose tables fit; rank_width 0: not even one feature's.
 void plan_rank_tables(tbk_forest *f) {
   const auto &q = f->rf;
-  const int F = q.num_features, room = 200 * 1024;
+  const int F = q.num_features, room = 185 * 1024; // (beside the ranking kernel's buffers)
   auto bytes = [&](int first, int end) { // tables of the features [first, end)
     size_t b = 0;
     for (int i = first; i < end; ++i)

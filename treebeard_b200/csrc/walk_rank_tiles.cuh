@@ -4,10 +4,10 @@
 // 32 banks whatever the features are; at step i of a group lane l walks column (l + i) mod 32,
 // which makes node and leaf loads conflict-free.
 //
-// A warp walks T tiles in lock-step through 4 / T columns at a time.  With four tiles the nodes of
-// a column's two topmost levels are loaded once for the four; a tree of 8 levels then costs 15.75
-// shared-memory wavefronts per 32 rows (17 with one tile), which is what bounds the kernel.  Sums
-// stay in the lane that owns the row.
+// A warp walks four tiles in lock-step through two columns at a time: eight independent chains of
+// loads per lane keep the shared-memory pipe busy with 12 to 20 warps (one column at a time left it
+// a third idle).  The nodes of a column's two topmost levels are loaded once for the four tiles; a tree of 8
+// levels costs 15.75 wavefronts per 32 rows.  Sums stay in the lane that owns the row.
 //
 // A block has `quads` x `shares` walker warps (T x quads tiles at a time; the shares of a quad split
 // the 32 columns of every group), a warp that streams the groups (node plane and leaf plane take a
@@ -22,21 +22,21 @@
 
 namespace tb {
 
-constexpr int kRTMaxWalkers = 24, kRTBarBytes = 512, kRTMaxSlots = 16;
+constexpr int kRTMaxWalkers = 20, kRTBarBytes = 512, kRTMaxSlots = 16;
 // shared memory: barriers, what the shares of a quad hand over, the keys of T * quads tiles, the ring
 __host__ __device__ constexpr int rank_tiles_smem_bytes(int tile_bytes, int tiles, int walkers, int lockstep, int slots, uint32_t slot_bytes) {
   return kRTBarBytes + walkers * lockstep * 128 + tiles * tile_bytes + slots * (int)slot_bytes;
 }
 
-// T tiles through C = 4 / T columns (addresses col[c] in the node plane); kb[t]: this lane's keys in
+// T tiles through C columns (addresses col[c] in the node plane); kb[t]: this lane's keys in
 // tile t.  off: where the walks end, as offsets into the leaf plane plus the node plane's address.
-template <int D, int T> __device__ __forceinline__ void rank_tiles_walk(uint32_t (&off)[4], const uint32_t *col, const uint32_t *kb) {
-  constexpr int C = 4 / T;
-  uint32_t node[4], key[4], root[C];
+template <int D, int T, int C> __device__ __forceinline__ void rank_tiles_walk(uint32_t (&off)[T * C], const uint32_t *col, const uint32_t *kb) {
+  constexpr int W = T * C;
+  uint32_t node[W], key[W], root[C];
   [[maybe_unused]] uint32_t left[C], right[C];
 #define TBT_ALL(...)                                                                                                \
   {                                                                                                                 \
-    _Pragma("unroll") for (int q = 0; q < 4; ++q) {                                                                 \
+    _Pragma("unroll") for (int q = 0; q < W; ++q) {                                                                 \
       [[maybe_unused]] const int t = q % T, c = q / T;                                                              \
       __VA_ARGS__;                                                                                                  \
     }                                                                                                               \
@@ -67,23 +67,23 @@ template <int D, int T> __device__ __forceinline__ void rank_tiles_walk(uint32_t
 #undef TBT_LEVEL
 #undef TBT_ALL
 }
-template <int T> __device__ __forceinline__ void rank_tiles_walk_any(uint32_t depth, uint32_t (&off)[4], const uint32_t *col, const uint32_t *kb) {
+template <int T, int C> __device__ __forceinline__ void rank_tiles_walk_any(uint32_t depth, uint32_t (&off)[T * C], const uint32_t *col, const uint32_t *kb) {
   switch (depth) {
-  case 1: return rank_tiles_walk<1, T>(off, col, kb);
-  case 2: return rank_tiles_walk<2, T>(off, col, kb);
-  case 3: return rank_tiles_walk<3, T>(off, col, kb);
-  case 4: return rank_tiles_walk<4, T>(off, col, kb);
-  case 5: return rank_tiles_walk<5, T>(off, col, kb);
-  case 6: return rank_tiles_walk<6, T>(off, col, kb);
-  case 7: return rank_tiles_walk<7, T>(off, col, kb);
-  default: return rank_tiles_walk<8, T>(off, col, kb);
+  case 1: return rank_tiles_walk<1, T, C>(off, col, kb);
+  case 2: return rank_tiles_walk<2, T, C>(off, col, kb);
+  case 3: return rank_tiles_walk<3, T, C>(off, col, kb);
+  case 4: return rank_tiles_walk<4, T, C>(off, col, kb);
+  case 5: return rank_tiles_walk<5, T, C>(off, col, kb);
+  case 6: return rank_tiles_walk<6, T, C>(off, col, kb);
+  case 7: return rank_tiles_walk<7, T, C>(off, col, kb);
+  default: return rank_tiles_walk<8, T, C>(off, col, kb);
   }
 }
 
 template <int T, bool LEAF_IDS>
 __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tiles_kernel(const __grid_constant__ RankWalkParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  constexpr int C = 4 / T;
+  constexpr int C = 2, W = T * C;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int NW = (int)(blockDim.x >> 5) - 2, Q = p.quads, shares = NW / Q;
@@ -190,27 +190,27 @@ __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tile
         if (busy)
 #pragma unroll 1
           for (int i = 0; i < cols; i += C) {
-            uint32_t col[C], off[4];
+            uint32_t col[C], off[W];
 #pragma unroll
             for (int c = 0; c < C; ++c) col[c] = nodes + ((uint32_t)(lane + share * cols + i + c) & 31u) * 4u;
-            rank_tiles_walk_any<T>(depth, off, col, kb);
+            rank_tiles_walk_any<T, C>(depth, off, col, kb);
             if (!leaves_here) {
               leaves_here = ok = wait(full_s + 8u * sl, pl);
               if (!ok) break;
             }
-            uint32_t v[4];
+            uint32_t v[W];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = lds_u32(off[q] + leaves);
+            for (int q = 0; q < W; ++q) v[q] = lds_u32(off[q] + leaves);
             if constexpr (LEAF_IDS) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
+              for (int q = 0; q < W; ++q) {
                 const int tree = p.tree_index[(g0 + k) * 32 + (int)((uint32_t)(lane + share * cols + i + q / T) & 31u)];
                 const long long row = row0 + (q % T) * 32;
                 if (tree >= 0 && row < p.n_rows) p.leaf_ids[row * p.num_trees + tree] = (int32_t)v[q];
               }
             } else {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) sum[q % T] += __uint_as_float(v[q]);
+              for (int q = 0; q < W; ++q) sum[q % T] += __uint_as_float(v[q]);
             }
           }
         else
