@@ -40,11 +40,10 @@ std::string pack_deep(const Forest &f, DeepForest *out) {
   for (int64_t g = 0; g < P; ++g) {
     uint32_t d = kDeepMinDepth;
     for (int c = 0; c < 2 && 2 * g + c < T; ++c) d = std::max<uint32_t>(d, depth[order[2 * g + c]]);
-    q.pairs[g] = QuantGroup{elems, d, 1u << d};
-    elems += 2ull << d;
+    q.pairs[g] = QuantGroup{elems, d, deep_tree_words(d)};
+    elems += 2ull * deep_tree_words(d);
   }
-  const uint32_t pass_through = (uint32_t)F << 16; // sentinel feature, key 0: always left
-  q.node_plane.assign(elems, pass_through);
+  q.node_plane.assign(elems, 0); // key 0, below every row key: always left
   q.leaf_plane.assign(elems, 0.f);
   q.exact_plane.assign(elems, 0.f);
   q.orig_leaf.assign(elems, -1);
@@ -58,24 +57,25 @@ std::string pack_deep(const Forest &f, DeepForest *out) {
       const int64_t t = order[k], a = f.tree_off[t];
       const uint64_t base = gm.elem_off + (uint64_t)c * gm.slots;
       q.tree_index[k] = (int32_t)t;
-      struct Item { int32_t node; uint32_t heap, level; };
-      std::vector<Item> stack{{0, 1, 0}};
+      struct Item { int32_t node; uint32_t first, level; }; // first: leftmost leaf below
+      std::vector<Item> stack{{0, 0, 0}};
       while (!stack.empty()) {
         const Item it = stack.back();
         stack.pop_back();
         if (f.left[a + it.node] < 0) {
-          // the leftmost descendant on the leaf level holds the value
-          const uint64_t leaf = ((uint64_t)it.heap << (gm.depth - it.level)) - gm.slots;
-          q.leaf_plane[base + leaf] = f.thr[a + it.node];
-          q.orig_leaf[base + leaf] = it.node;
+          // all-left from here on
+          q.leaf_plane[base + deep_position(it.first)] = f.thr[a + it.node];
+          q.orig_leaf[base + deep_position(it.first)] = it.node;
           continue;
         }
         const int32_t ft = f.feat[a + it.node];
         const float thr = f.thr[a + it.node];
-            q.node_plane[base + it.heap] = ((uint32_t)ft << 16) | quant_threshold_key15(thr, q.lo[ft], q.scale[ft]);
-        q.exact_plane[base + it.heap] = thr;
-        stack.push_back({f.left[a + it.node], 2 * it.heap, it.level + 1});
-        stack.push_back({f.right[a + it.node], 2 * it.heap + 1, it.level + 1});
+        const uint32_t half = 1u << (gm.depth - 1 - it.level);
+        const uint64_t e = base + deep_position(it.first + half);
+        q.node_plane[e] = (deep_feature_code(F, (uint32_t)ft) << 16) | quant_threshold_key15(thr, q.lo[ft], q.scale[ft]);
+        q.exact_plane[e] = thr;
+        stack.push_back({f.left[a + it.node], it.first, it.level + 1});
+        stack.push_back({f.right[a + it.node], it.first + half, it.level + 1});
       }
     }
   }
@@ -98,18 +98,20 @@ void walk_deep_on_host(const DeepForest &q, const float *rows, int64_t n_rows, i
         const int32_t t = q.tree_index[g * 2 + c];
         if (t < 0) continue;
         const uint64_t base = gm.elem_off + (uint64_t)c * gm.slots;
-        uint32_t i = 1;
+        uint32_t first = 0;
         for (uint32_t d = 0; d < gm.depth; ++d) {
+          const uint32_t half = 1u << (gm.depth - 1 - d);
+          const uint64_t i = deep_position(first + half);
           const uint32_t node = q.node_plane[base + i];
-          const uint32_t ft = node >> 16, kt = node & 0xffffu, kx = keys[ft];
+          const uint32_t ft = (node >> 16) / deep_feature_code(F, 1), kt = node & 0xffffu, kx = keys[ft];
           bool right = kx < kt;
           if (kx == kt) {
             ++tie_count;
             right = !(row[ft] < q.exact_plane[base + i]);
           }
-          i = 2 * i + (right ? 1 : 0);
+          first += right ? half : 0u;
         }
-        const uint64_t e = base + (i - gm.slots);
+        const uint64_t e = base + deep_position(first);
         acc += q.leaf_plane[e];
         if (leaf_ids) leaf_ids[r * q.num_trees + t] = q.orig_leaf[e];
       }

@@ -5,18 +5,23 @@
 //
 // Every tree becomes a complete tree of its pair's depth D (trees are sorted by depth and
 // taken two at a time; a pair is what one thread walks in lock-step), stored as planes of
-// 2^D elements per tree, 16 KB at D = 12:
+// deep_tree_words(D) elements per tree, 16.5 KB at D = 12.  Nodes are numbered IN ORDER: the node
+// that prefix p of decisions leads to on level d has number (2p + 1) 2^(D-1-d), leaf l number l; so
+// a walk that keeps the number of the leftmost leaf below it finds the node 2^(D-1-d) further on,
+// and a right turn adds just that.  Positions are numbers with one element of padding after every
+// 32 and one after every 1024: still additive bit by bit, but the nodes of the upper levels and the
+// siblings of the lower ones spread over all shared-memory banks (19.2 wavefronts for the 12 node
+// loads of a warp on random trees; 21.4 in level order):
 //
-//   node plane   u32 [2^D]  word i = node with 1-based heap index i (children 2i, 2i+1, an
-//                           aligned 8-byte pair); (feature index << 16) | threshold key;
-//                           word 0 is unused
-//   leaf plane   f32 [2^D]  value of leaf j = i - 2^D after D steps
-//   exact plane  f32 [2^D]  fp32 thresholds, indexed like the node plane (global memory only)
+//   node plane   u32  (feature code << 16) | threshold key.  Feature code: the byte offset of the
+//                     feature's line in a key tile (128 f), or f itself where that does not fit 16 bits
+//   leaf plane   f32  leaf values
+//   exact plane  f32  fp32 thresholds, laid out like the node plane (global memory only)
 //
 // Rows are staged as the 15-bit order-preserving keys of quant_pack.h, so a block holds
 // 32 x row_warps rows (512 for 128 features) next to a ring of whole-tree pieces; key ties
 // are resolved on the exact fp32 values, which keeps leaf selection that of the fp32 walk.
-// A leaf above the bottom level is a chain of pass-through nodes (sentinel feature, key 0:
+// A leaf above the bottom level is a chain of pass-through nodes (key 0, below every row key:
 // always left) ending in the leaf slot that holds its value.
 #pragma once
 #include "forest.h"
@@ -30,13 +35,17 @@ namespace tb {
 
 constexpr int kDeepMaxDepth = 12;
 constexpr int kDeepMinDepth = 2; // pieces of at least 16 bytes
+constexpr uint32_t deep_position(uint32_t number) { return number + (number >> 5) + (number >> 10); }
+constexpr uint32_t deep_tree_words(uint32_t depth) { return (deep_position((1u << depth) - 1) + 1 + 3) / 4 * 4; }
+constexpr int kDeepNarrowFeatures = 511; // feature codes up to here are byte offsets
+inline uint32_t deep_feature_code(int32_t num_features, uint32_t f) { return num_features <= kDeepNarrowFeatures ? 128 * f : f; }
 
 struct DeepForest {
   int32_t num_features = 0, transform = 0;
   double initial_value = 0.0;
   int64_t num_trees = 0, num_nodes = 0;
   int32_t max_depth = 0;
-  std::vector<QuantGroup> pairs;    // elem_off of tree 0 of the pair (tree 1 follows at + slots)
+  std::vector<QuantGroup> pairs;    // elem_off of tree 0 of the pair; tree 1 follows at + slots = deep_tree_words(depth)
   std::vector<uint32_t> node_plane; // key field is filled on the device at upload
   std::vector<float> leaf_plane;
   std::vector<float> exact_plane;

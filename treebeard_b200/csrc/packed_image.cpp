@@ -289,7 +289,7 @@ std::string deserialize_image(const uint8_t *data, uint64_t size, PackedImage *i
                   q.scale.size() != q.lo.size()))
       in.ok = false;
     for (const QuantGroup &g : q.pairs)
-      if (in.ok && (g.depth > (uint32_t)kDeepMaxDepth || g.elem_off + 2ull * g.slots > n)) in.ok = false;
+      if (in.ok && (g.depth > (uint32_t)kDeepMaxDepth || g.slots != deep_tree_words(g.depth) || g.elem_off + 2ull * g.slots > n)) in.ok = false;
   } else {
     return "packed image: unknown layout kind";
   }

@@ -32,7 +32,7 @@ struct PackedImage {
   RankForest rf;       // kRank
 };
 
-constexpr uint32_t kPackedImageVersion = 7; // changes whenever a packer's output does
+constexpr uint32_t kPackedImageVersion = 8; // changes whenever a packer's output does
 
 void serialize_image(const PackedImage &im, std::vector<uint8_t> *out);
 uint64_t serialized_image_size(const PackedImage &im); // without serialising

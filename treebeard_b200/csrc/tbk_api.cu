@@ -484,10 +484,10 @@ int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
 // either way, and more rows per tile mean fewer passes over the forest and more walks in
 // flight) whose key tile leaves room for a ring of at least 4 whole-tree pieces.
 bool deep_plan(int num_features, int max_depth, int smem_limit, int *row_warps, int *slots) {
-  const int64_t slot = 4ll << std::max(max_depth, tb::kDeepMinDepth);
+  const int64_t slot = 4ll * tb::deep_tree_words((uint32_t)std::max(max_depth, tb::kDeepMinDepth));
   // four slots hold the node planes of the pair being walked and of the next one
   for (int rw = 30; rw >= 4; rw -= 2) { // (the block has one more warp, the ring producer)
-    const int64_t keys = (int64_t)(num_features + 1) * 64 * rw;
+    const int64_t keys = (int64_t)num_features * 64 * rw;
     const int64_t room = (int64_t)smem_limit - 128 - keys;
     const int64_t s = std::min<int64_t>(tb::kDeepMaxSlots, room / slot);
     if (s >= 4) {
@@ -499,8 +499,16 @@ bool deep_plan(int num_features, int max_depth, int smem_limit, int *row_warps, 
   return false;
 }
 int deep_smem_bytes(const tbk_forest *f) {
-  return 128 + f->deep_slots * (4 << std::max(f->df.max_depth, tb::kDeepMinDepth)) +
-         (f->df.num_features + 1) * 64 * f->deep_row_warps;
+  return 128 + f->deep_slots * 4 * (int)tb::deep_tree_words((uint32_t)std::max(f->df.max_depth, tb::kDeepMinDepth)) +
+         f->df.num_features * 64 * f->deep_row_warps;
+}
+
+template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb::DeepParams) {
+  if (small)
+    return d12 ? (ids ? tb::tb_walk_deep_kernel<768, 12, WIDE, true> : tb::tb_walk_deep_kernel<768, 12, WIDE, false>)
+               : (ids ? tb::tb_walk_deep_kernel<768, 0, WIDE, true> : tb::tb_walk_deep_kernel<768, 0, WIDE, false>);
+  return d12 ? (ids ? tb::tb_walk_deep_kernel<1024, 12, WIDE, true> : tb::tb_walk_deep_kernel<1024, 12, WIDE, false>)
+             : (ids ? tb::tb_walk_deep_kernel<1024, 0, WIDE, true> : tb::tb_walk_deep_kernel<1024, 0, WIDE, false>);
 }
 
 // One prediction with the deep-tree kernel (one block per 32 x row_warps rows).
@@ -508,9 +516,11 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot) {
   const auto &q = f->df;
   const int64_t G = (int64_t)q.pairs.size();
-  // small batches: fewer row warps per block, so that the tiles still cover the SMs
+  // as few row warps per block as do not cost another wave of blocks: the last wave is then as
+  // full as the others, and small batches still cover the SMs
   int rw = f->deep_row_warps;
-  while (rw > 4 && (n_rows + 32 * rw - 1) / (32 * rw) < f->num_sms) rw -= 2;
+  const int64_t row_tiles = (n_rows + 31) / 32, waves = (row_tiles + (int64_t)rw * f->num_sms - 1) / ((int64_t)rw * f->num_sms);
+  rw = std::max(4, (int)((row_tiles + waves * f->num_sms - 1) / (waves * f->num_sms)));
   const int64_t rows_per_block = 32 * rw;
   const int64_t grid_x = (n_rows + rows_per_block - 1) / rows_per_block;
   int64_t chunks = 1;
@@ -527,7 +537,7 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   plan.groups_per_chunk = gpc;
   plan.staged = 1;
   plan.cache_rows = 1;
-  plan.stage_bytes = 4u << std::max(q.max_depth, tb::kDeepMinDepth);
+  plan.stage_bytes = 4u * tb::deep_tree_words((uint32_t)std::max(q.max_depth, tb::kDeepMinDepth));
   plan.smem_bytes = deep_smem_bytes(f);
   plan.threads = 32 * (rw + 1); // row warps + the ring producer
   plan.grid_x = grid_x;
@@ -573,7 +583,8 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   p.initial_value = (float)q.initial_value;
   p.ring_slots = f->deep_slots;
   p.slot_bytes = plan.stage_bytes;
-  p.key_stride = 64u * (uint32_t)f->deep_row_warps; // the tile keeps its full width whatever rw is
+  p.tree_words = plan.stage_bytes / 4;
+  p.key_tile = 128u * (uint32_t)q.num_features;
   p.status = f->d_status;
   p.tie_count = f->d_ties;
   p.skip_first_copy = f->expire_next_wait ? 1 : 0;
@@ -583,11 +594,7 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   // specialised for forests whose pairs all have 12 levels; generic otherwise
   using DeepKernel = void (*)(const tb::DeepParams);
   const bool d12 = f->uniform_depth == 12, ids = mode == kLeafIds, small = plan.threads <= 768;
-  const DeepKernel kernel =
-      small ? (d12 ? (ids ? tb::tb_walk_deep_kernel<768, 12, true> : tb::tb_walk_deep_kernel<768, 12, false>)
-                   : (ids ? tb::tb_walk_deep_kernel<768, 0, true> : tb::tb_walk_deep_kernel<768, 0, false>))
-            : (d12 ? (ids ? tb::tb_walk_deep_kernel<1024, 12, true> : tb::tb_walk_deep_kernel<1024, 12, false>)
-                   : (ids ? tb::tb_walk_deep_kernel<1024, 0, true> : tb::tb_walk_deep_kernel<1024, 0, false>));
+  const DeepKernel kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
   CUDA_TRY(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
@@ -1180,7 +1187,7 @@ int upload_key_planes(tbk_forest *f, const std::vector<uint32_t> &node, const st
   CUDA_TRY(cudaMemcpy(f->d_qlo, lo.data(), lo.size() * 4, cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMemcpy(f->d_qscale, scale.data(), scale.size() * 4, cudaMemcpyHostToDevice));
   tb::tb_quant_fill_keys<<<(unsigned)((n + 255) / 256), 256>>>(f->d_qnode, f->d_qexact, f->d_qlo, f->d_qscale,
-                                                             (unsigned long long)n, num_features, wide ? 1 : 0);
+                                                             (unsigned long long)n, num_features, wide ? 1 : 0, tb::deep_feature_code(num_features, 1));
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaDeviceSynchronize());
   ++f->launches;
@@ -1523,7 +1530,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     std::vector<int32_t>().swap(q.orig_leaf);
     tb::LaunchPlan &pl = f->last_plan;
     pl.row_warps = f->deep_row_warps; pl.tree_threads = 1; pl.rows_per_lane = 1; pl.chunks = 1; pl.staged = 1; pl.cache_rows = 1;
-    pl.stage_bytes = 4u << std::max(q.max_depth, tb::kDeepMinDepth); pl.smem_bytes = deep_smem_bytes(f); pl.threads = 32 * (f->deep_row_warps + 1);
+    pl.stage_bytes = 4u * tb::deep_tree_words((uint32_t)std::max(q.max_depth, tb::kDeepMinDepth)); pl.smem_bytes = deep_smem_bytes(f); pl.threads = 32 * (f->deep_row_warps + 1);
     *out = f;
     return TBK_OK;
   }

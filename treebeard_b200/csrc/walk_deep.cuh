@@ -12,9 +12,11 @@
 // sectors per warp whatever the layout) and consumed one pair later.  Sums stay in the
 // owning thread's register: there is no cross-thread reduction.
 //
-// Keys of two row warps are interleaved (feature-major, 128 bytes per warp pair: word j =
-// row j of the even warp | row j of the odd warp << 16), so a warp's key load touches 32
-// distinct banks.  A key tie is only flagged on the fast path; the flagged (row, tree) is
+// Every two row warps have a key tile of their own (128 bytes per feature: word j = row j of the even
+// warp | row j of the odd warp << 16), so a warp's key load touches 32 distinct banks and the
+// upper half of a node word -- the byte offset of the feature's line -- is one shift-add away from
+// the key's address.  The in-order numbering of deep_pack.h makes a right turn one addition that
+// depends on the level alone.  A key tie is only flagged on the fast path; the flagged (row, tree) is
 // re-walked with exact fp32 comparisons at the tied steps.
 //
 // Reference counterparts: src/mlir/CodeGenStateMachine.cpp:149-243 (scalar walk),
@@ -44,8 +46,9 @@ struct DeepParams {
   int32_t num_pairs, pairs_per_chunk, num_features, transform;
   float initial_value;
   int32_t ring_slots;  // 4 .. 8
-  uint32_t slot_bytes; // 4 << max depth of the forest
-  uint32_t key_stride; // bytes per feature in the key tile: 64 * (row warps rounded up to even)
+  uint32_t slot_bytes; // of a tree of the forest's depth
+  uint32_t tree_words; // the same in words
+  uint32_t key_tile;   // bytes of the key tile of two row warps
   int32_t *status;
   unsigned long long *tie_count;
   int32_t skip_first_copy; // failure drill: the first piece's copy is never issued, so its wait expires
@@ -56,88 +59,107 @@ constexpr int kDeepMaxSlots = 8;
 
 // Fast walk of DEPTH levels of two trees in lock-step, in PTX (the step of walk_quant.cuh: keys
 // are 15-bit integers that compare as fp16 numbers, so one half2 comparison of (key, node word)
-// picks the child and a second one accumulates the tie flag; the node's address itself is
-// tracked: the children of the node at address A = base + 4 i sit at 2A - base and 2A - base + 4).
-// base0 / base1: shared-memory addresses of the node planes; returns the heap indices reached
-// (in [2^DEPTH, 2^(DEPTH+1))) and whether any key comparison on either path tied.
-//   %0, %1  node addresses (updated)   %2, %3  node words (scratch)   %4  tie flags (out)
-//   %5  the thread's base in the key tile   %6  key-tile bytes per feature   %7, %8  -base
+// picks the child and a second one accumulates the tie flag).  On a level whose distance to the
+// leaves is s (deep_position of a power of two, in bytes) the node lies s behind the current
+// address, and a right turn moves the address on by s.
+// base0 / base1: shared-memory addresses of the node planes; returns the leaf positions reached and
+// whether any key comparison on either path tied.
+//   %0, %1  addresses (updated)   %2, %3  node words (scratch)   %4  tie flags (out)
+//   %5  the thread's base in its key tile
 #define TBD_DECL ".reg .b32 ka0, ka1, kx0, kx1;\n .reg .pred p0, p1, t0, t1, q;\n"
-#define TBD_LOAD "ld.shared.u32 %2, [%0];\n ld.shared.u32 %3, [%1];\n"
-#define TBD_KEY(i, n) "shr.u32 ka" #i ", " n ", 16;\n mad.lo.u32 ka" #i ", ka" #i ", %6, %5;\n ld.shared.u16 kx" #i ", [ka" #i "];\n"
+#define TBD_KEY(i, n)                                                                                               \
+  "shr.u32 ka" #i ", " n ", 16;\n add.u32 ka" #i ", ka" #i ", %5;\n ld.shared.u16 kx" #i ", [ka" #i "];\n"
+// WIDE: the upper half of a node word is the feature's number, its line 128 bytes for each
+#define TBD_KEYW(i, n)                                                                                              \
+  "shr.u32 ka" #i ", " n ", 16;\n mad.lo.u32 ka" #i ", ka" #i ", 128, %5;\n ld.shared.u16 kx" #i ", [ka" #i "];\n"
 #define TBD_CMP0(i, n) "setp.lt.f16x2 p" #i "|q, kx" #i ", " n ";\n setp.eq.f16x2 t" #i "|q, kx" #i ", " n ";\n"
 #define TBD_CMP(i, n) "setp.lt.f16x2 p" #i "|q, kx" #i ", " n ";\n setp.eq.or.f16x2 t" #i "|q, kx" #i ", " n ", t" #i ";\n"
-#define TBD_ADV(i, a, c) "shl.b32 " a ", " a ", 1;\n add.u32 " a ", " a ", " c ";\n @p" #i " add.u32 " a ", " a ", 4;\n"
-#define TBD_KEYS TBD_KEY(0, "%2") TBD_KEY(1, "%3")
-#define TBD_ADVS TBD_ADV(0, "%0", "%7") TBD_ADV(1, "%1", "%8")
-#define TBD_FIRST TBD_KEYS TBD_CMP0(0, "%2") TBD_CMP0(1, "%3") TBD_ADVS
-#define TBD_NEXT TBD_LOAD TBD_KEYS TBD_CMP(0, "%2") TBD_CMP(1, "%3") TBD_ADVS
+#define TBD_LEVEL(K, C, step)                                                                                       \
+  "ld.shared.u32 %2, [%0+" step "];\n ld.shared.u32 %3, [%1+" step "];\n" K(0, "%2") K(1, "%3") C(0, "%2") C(1, "%3") \
+  "@p0 add.u32 %0, %0, " step ";\n @p1 add.u32 %1, %1, " step ";\n"
+#define TBD_R1(K) TBD_LEVEL(K, TBD_CMP, "4")
+#define TBD_R2(K) TBD_LEVEL(K, TBD_CMP, "8") TBD_R1(K)
+#define TBD_R3(K) TBD_LEVEL(K, TBD_CMP, "16") TBD_R2(K)
+#define TBD_R4(K) TBD_LEVEL(K, TBD_CMP, "32") TBD_R3(K)
+#define TBD_R5(K) TBD_LEVEL(K, TBD_CMP, "64") TBD_R4(K)
+#define TBD_R6(K) TBD_LEVEL(K, TBD_CMP, "132") TBD_R5(K)
+#define TBD_R7(K) TBD_LEVEL(K, TBD_CMP, "264") TBD_R6(K)
+#define TBD_R8(K) TBD_LEVEL(K, TBD_CMP, "528") TBD_R7(K)
+#define TBD_R9(K) TBD_LEVEL(K, TBD_CMP, "1056") TBD_R8(K)
+#define TBD_R10(K) TBD_LEVEL(K, TBD_CMP, "2112") TBD_R9(K)
+#define TBD_R11(K) TBD_LEVEL(K, TBD_CMP, "4228") TBD_R10(K)
+#define TBD_L2(K) TBD_LEVEL(K, TBD_CMP0, "8") TBD_R1(K)
+#define TBD_L3(K) TBD_LEVEL(K, TBD_CMP0, "16") TBD_R2(K)
+#define TBD_L4(K) TBD_LEVEL(K, TBD_CMP0, "32") TBD_R3(K)
+#define TBD_L5(K) TBD_LEVEL(K, TBD_CMP0, "64") TBD_R4(K)
+#define TBD_L6(K) TBD_LEVEL(K, TBD_CMP0, "132") TBD_R5(K)
+#define TBD_L7(K) TBD_LEVEL(K, TBD_CMP0, "264") TBD_R6(K)
+#define TBD_L8(K) TBD_LEVEL(K, TBD_CMP0, "528") TBD_R7(K)
+#define TBD_L9(K) TBD_LEVEL(K, TBD_CMP0, "1056") TBD_R8(K)
+#define TBD_L10(K) TBD_LEVEL(K, TBD_CMP0, "2112") TBD_R9(K)
+#define TBD_L11(K) TBD_LEVEL(K, TBD_CMP0, "4228") TBD_R10(K)
+#define TBD_L12(K) TBD_LEVEL(K, TBD_CMP0, "8456") TBD_R11(K)
 #define TBD_TIES "selp.u32 %4, 1, 0, t0;\n @t1 or.b32 %4, %4, 2;\n"
-#define TBD_N2 TBD_NEXT TBD_NEXT
-#define TBD_N4 TBD_N2 TBD_N2
-#define TBD_N8 TBD_N4 TBD_N4
-template <int DEPTH>
-__device__ __forceinline__ void deep_walk(uint32_t base0, uint32_t base1, uint32_t key_lane, uint32_t ks,
-                                          uint32_t *i0_out, uint32_t *i1_out, bool *tie0, bool *tie1) {
+template <int DEPTH, bool WIDE>
+__device__ __forceinline__ void deep_walk(uint32_t base0, uint32_t base1, uint32_t key_lane, uint32_t *j0, uint32_t *j1,
+                                          bool *tie0, bool *tie1) {
   static_assert(DEPTH >= 2 && DEPTH <= 12, "two to twelve levels");
-  uint32_t a0 = base0 + 4u, a1 = base1 + 4u, tb; // the root is heap node 1
+  uint32_t a0 = base0, a1 = base1, tb;
   [[maybe_unused]] uint32_t n0, n1;
-#define TBD_OPERANDS : "+r"(a0), "+r"(a1), "=&r"(n0), "=&r"(n1), "=&r"(tb) : "r"(key_lane), "r"(ks), "r"(0u - base0), "r"(0u - base1)
-  // DEPTH levels = the first one and DEPTH - 1 more, each of which loads its node first
-  if constexpr (DEPTH == 2) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_NEXT TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 3) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N2 TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 4) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N2 TBD_NEXT TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 5) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N4 TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 6) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N4 TBD_NEXT TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 7) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N4 TBD_N2 TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 8) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N4 TBD_N2 TBD_NEXT TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 9) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N8 TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 10) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N8 TBD_NEXT TBD_TIES "}" TBD_OPERANDS);
-  else if constexpr (DEPTH == 11) asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N8 TBD_N2 TBD_TIES "}" TBD_OPERANDS);
-  else asm volatile("{\n" TBD_DECL TBD_LOAD TBD_FIRST TBD_N8 TBD_N2 TBD_NEXT TBD_TIES "}" TBD_OPERANDS);
-#undef TBD_OPERANDS
-  *i0_out = (a0 - base0) >> 2;
-  *i1_out = (a1 - base1) >> 2;
+#define TBD_ASM(levels) asm volatile("{\n" TBD_DECL levels TBD_TIES "}" : "+r"(a0), "+r"(a1), "=&r"(n0), "=&r"(n1), "=&r"(tb) : "r"(key_lane))
+#define TBD_CASE(n)                                                                                                 \
+  if constexpr (DEPTH == n) {                                                                                       \
+    if constexpr (WIDE) TBD_ASM(TBD_L##n(TBD_KEYW));                                                                \
+    else TBD_ASM(TBD_L##n(TBD_KEY));                                                                                \
+  }
+  TBD_CASE(2) TBD_CASE(3) TBD_CASE(4) TBD_CASE(5) TBD_CASE(6) TBD_CASE(7) TBD_CASE(8) TBD_CASE(9) TBD_CASE(10) TBD_CASE(11) TBD_CASE(12)
+#undef TBD_CASE
+#undef TBD_ASM
+  *j0 = (a0 - base0) >> 2;
+  *j1 = (a1 - base1) >> 2;
   *tie0 = tb & 1u;
   *tie1 = tb & 2u;
 }
 
-__device__ __forceinline__ void deep_walk_any(uint32_t depth, uint32_t base0, uint32_t base1, uint32_t key_lane,
-                                              uint32_t ks, uint32_t *i0, uint32_t *i1, bool *t0, bool *t1) {
+template <bool WIDE>
+__device__ __forceinline__ void deep_walk_any(uint32_t depth, uint32_t base0, uint32_t base1, uint32_t key_lane, uint32_t *j0,
+                                              uint32_t *j1, bool *t0, bool *t1) {
   switch (depth) {
-  case 2: return deep_walk<2>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 3: return deep_walk<3>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 4: return deep_walk<4>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 5: return deep_walk<5>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 6: return deep_walk<6>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 7: return deep_walk<7>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 8: return deep_walk<8>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 9: return deep_walk<9>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 10: return deep_walk<10>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  case 11: return deep_walk<11>(base0, base1, key_lane, ks, i0, i1, t0, t1);
-  default: return deep_walk<12>(base0, base1, key_lane, ks, i0, i1, t0, t1);
+  case 2: return deep_walk<2, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 3: return deep_walk<3, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 4: return deep_walk<4, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 5: return deep_walk<5, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 6: return deep_walk<6, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 7: return deep_walk<7, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 8: return deep_walk<8, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 9: return deep_walk<9, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 10: return deep_walk<10, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  case 11: return deep_walk<11, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
+  default: return deep_walk<12, WIDE>(base0, base1, key_lane, j0, j1, t0, t1);
   }
 }
 
 // Re-walk of one (row, tree) behind a key tie: the staged keys decide wherever they can,
-// the tied comparisons read the exact fp32 values from global memory.
-__device__ __noinline__ uint32_t deep_walk_exact(uint32_t base, uint32_t key_lane, uint32_t ks, uint32_t depth,
+// the tied comparisons read the exact fp32 values from global memory.  Returns the leaf position.
+__device__ __noinline__ uint32_t deep_walk_exact(uint32_t base, uint32_t key_lane, bool wide, uint32_t depth,
                                                  const float *exact_tree, const float *rowp) {
-  uint32_t i = 1;
+  uint32_t at = 0;
   for (uint32_t d = 0; d < depth; ++d) {
-    const uint32_t node = lds_u32(base + i * 4u);
-    const uint32_t f = node >> 16, kt = node & 0xffffu;
-    const uint32_t kx = lds_u16(key_lane + f * ks);
+    const uint32_t x = 1u << (depth - 1 - d), step = x + (x >> 5) + (x >> 10); // (deep_position)
+    const uint32_t node = lds_u32(base + (at + step) * 4u);
+    const uint32_t f = wide ? node >> 16 : node >> 23, kt = node & 0x7fffu;
+    const uint32_t kx = lds_u16(key_lane + f * 128u);
     bool right = kx < kt;
-    if (kx == kt) right = !(__ldg(rowp + f) < __ldg(exact_tree + i));
-    i = 2u * i + (right ? 1u : 0u);
+    if (kx == kt) right = !(__ldg(rowp + f) < __ldg(exact_tree + at + step));
+    at += right ? step : 0u;
   }
-  return i;
+  return at;
 }
 
 // UD: depth shared by every pair of the forest (0 = mixed, decided per pair at run time).
 // LEAF_IDS: the launch records leaf ids instead of predictions.
-template <int MAX_THREADS, int UD, bool LEAF_IDS>
+// WIDE: more features than the byte offset of a 128-byte line in 16 bits reaches.
+template <int MAX_THREADS, int UD, bool WIDE, bool LEAF_IDS>
 __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const DeepParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -148,8 +170,8 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   unsigned char *ring = smem_raw + 128;
   const uint32_t ring_s = smem_u32(ring);
   const uint32_t keys_s = ring_s + (uint32_t)S * p.slot_bytes;
-  const uint32_t ks = p.key_stride;
-  const uint32_t key_lane = keys_s + (uint32_t)(warp >> 1) * 128u + (uint32_t)lane * 4u + (uint32_t)(warp & 1) * 2u;
+  constexpr uint32_t ks = 128;
+  const uint32_t key_lane = keys_s + (uint32_t)(warp >> 1) * p.key_tile + (uint32_t)lane * 4u + (uint32_t)(warp & 1) * 2u;
 
   const long long row = ((long long)blockIdx.x * RW + warp) * 32 + lane;
   const bool live = row < p.n_rows;
@@ -212,7 +234,6 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
       for (int f = 0; f < F; ++f)
         sts_u16(key_lane + (uint32_t)f * ks, quant_key15_lattice_dev(live ? __ldg(rowp + f) : 0.f, __ldg(p.lo + f), __ldg(p.scale + f)));
     }
-    sts_u16(key_lane + (uint32_t)F * ks, 0x7bffu); // sentinel feature: the largest key
   }
   // (each thread reads back only the keys it wrote: no barrier is needed for the tile)
 
@@ -237,25 +258,33 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
     return ring_s + (uint32_t)s * p.slot_bytes;
   };
 
+  // where pair k's planes start and its depth: computed where all pairs have the same depth, else
+  // loaded a pair ahead
+  auto pair_of = [&](int k) -> DevQuantGroup {
+    if constexpr (UD > 0) return DevQuantGroup{(unsigned long long)(g0 + k) * (2u * p.tree_words), (uint32_t)UD, p.tree_words};
+    return p.pairs[min(g0 + k, g1 - 1)];
+  };
+  DevQuantGroup next = pair_of(0);
   for (int k = 0; k < g1 - g0 && ok; ++k) {
-    const DevQuantGroup gm = p.pairs[g0 + k];
-    const uint32_t depth = UD ? (uint32_t)UD : gm.depth;
-    uint32_t i0 = gm.slots, i1 = gm.slots;
+    const DevQuantGroup gm = next;
+    next = pair_of(k + 1);
+    const uint32_t depth = gm.depth;
+    uint32_t j0 = 0, j1 = 0;
     int sl[2];
 
     const uint32_t n0 = take(&sl[0]), n1 = take(&sl[1]);
     if (ok) {
       bool t0, t1;
       if constexpr (UD > 0)
-        deep_walk<UD>(n0, n1, key_lane, ks, &i0, &i1, &t0, &t1);
+        deep_walk<UD, WIDE>(n0, n1, key_lane, &j0, &j1, &t0, &t1);
       else
-        deep_walk_any(depth, n0, n1, key_lane, ks, &i0, &i1, &t0, &t1);
+        deep_walk_any<WIDE>(depth, n0, n1, key_lane, &j0, &j1, &t0, &t1);
       if (t0) {
-        i0 = deep_walk_exact(n0, key_lane, ks, depth, p.exact_plane + gm.elem_off, rowp);
+        j0 = deep_walk_exact(n0, key_lane, WIDE, depth, p.exact_plane + gm.elem_off, rowp);
         ++ties;
       }
       if (t1) {
-        i1 = deep_walk_exact(n1, key_lane, ks, depth, p.exact_plane + gm.elem_off + gm.slots, rowp);
+        j1 = deep_walk_exact(n1, key_lane, WIDE, depth, p.exact_plane + gm.elem_off + gm.slots, rowp);
         ++ties;
       }
     }
@@ -263,8 +292,11 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
     // 32 leaves are scattered over the leaf plane (one sector each), which moves the same
     // bytes as staging the plane would, without taking ring slots.
     if (ok) {
-      const uint32_t j0 = i0 - gm.slots, j1 = i1 - gm.slots;
       if (!LEAF_IDS) {
+        // (tied to the walk's end by a condition that is never met: scheduled in front of the walk,
+        // the additions would wait for the loads)
+        asm volatile("{\n .reg .pred p;\n setp.eq.u32 p, %2, 0xffffffff;\n @p mov.f32 %0, 0f00000000;\n @p mov.f32 %1, 0f00000000;\n}"
+                     : "+f"(pend0), "+f"(pend1) : "r"(j0 & j1));
         acc += (double)pend0 + (double)pend1;
         pend0 = __ldg(p.leaf_plane + gm.elem_off + j0);
         pend1 = __ldg(p.leaf_plane + gm.elem_off + gm.slots + j1);
