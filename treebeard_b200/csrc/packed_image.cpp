@@ -133,6 +133,15 @@ void put_image(const PackedImage &im, Out &o) {
     o.vec(q.features);
     o.vec(q.lut);
     o.vec(q.thresholds);
+  } else if (im.kind == PackedImage::kLanes) {
+    const LaneForest &q = im.lf;
+    put_key_forest_head(o, q.num_features, q.transform, q.initial_value, q.num_trees, q.num_nodes, q.max_depth);
+    o.pod(q.num_classes);
+    o.vec(q.nodes);
+    o.vec(q.root);
+    o.vec(q.tree_index);
+    o.vec(q.orig_node);
+    o.vec(q.class_end);
   } else {
     const DeepForest &q = im.df;
     put_key_forest_head(o, q.num_features, q.transform, q.initial_value, q.num_trees, q.num_nodes, q.max_depth);
@@ -272,6 +281,27 @@ std::string deserialize_image(const uint8_t *data, uint64_t size, PackedImage *i
       if (in.ok && (g.depth < 1 || g.depth > (uint32_t)q.max_depth || g.slots != (1u << g.depth) ||
                     g.elem_off + (uint64_t)g.slots * kRankCols > n))
         in.ok = false;
+  } else if (im->kind == PackedImage::kLanes) {
+    LaneForest &q = im->lf;
+    key_head(&q.num_features, &q.transform, &q.initial_value, &q.num_trees, &q.num_nodes, &q.max_depth);
+    q.num_classes = in.pod<int32_t>();
+    in.vec(&q.nodes);
+    in.vec(&q.root);
+    in.vec(&q.tree_index);
+    in.vec(&q.orig_node);
+    in.vec(&q.class_end);
+    const size_t n = q.nodes.size();
+    if (in.ok && ((int64_t)n != q.num_nodes || q.orig_node.size() != n || (int64_t)q.tree_index.size() != q.num_trees ||
+                  (int64_t)q.root.size() != q.num_trees + 1 || q.root.back() != n || q.num_classes < 0 ||
+                  (int64_t)q.class_end.size() != q.num_classes))
+      in.ok = false;
+    for (size_t i = 0; in.ok && i < n; ++i) { // every distance must lead forward, to a node or to the end
+      const uint64_t to = i + (q.nodes[i].link >> 16);
+      const uint32_t f = q.nodes[i].link & 0xffffu;
+      if (to <= i || f > (uint32_t)q.num_features || (f == (uint32_t)q.num_features ? to > n : to + 1 >= n)) in.ok = false;
+    }
+    for (size_t c = 0; in.ok && c < q.class_end.size(); ++c)
+      if (q.class_end[c] > n || (c && q.class_end[c] < q.class_end[c - 1])) in.ok = false;
   } else if (im->kind == PackedImage::kDeep) {
     DeepForest &q = im->df;
     key_head(&q.num_features, &q.transform, &q.initial_value, &q.num_trees, &q.num_nodes, &q.max_depth);

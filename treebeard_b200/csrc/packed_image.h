@@ -1,12 +1,13 @@
 // A packed forest as it lies in host memory just before the upload: the layout that was
 // chosen for it (general tiles / rank keys for narrow rows / 16-bit keys for wide rows / one tree
-// per stage for deep trees) and that layout's buffers.  It can be serialised, which is what a compiled-model
+// per stage for deep trees / lanes for what is left) and that layout's buffers.  It can be serialised, which is what a compiled-model
 // file caches so that loading it skips the packer -- the counterpart of the buffers the
 // reference's serializer writes next to a compiled module and reloads
 // (src/utils/TreeTilingUtils.cpp:95-170, src/runtime/runtime.cpp:35-54).
 #pragma once
 #include "../../include/tbk.h"
 #include "deep_pack.h"
+#include "lane_pack.h"
 #include "pack.h"
 #include "quant_pack.h"
 #include "rank_pack.h"
@@ -18,7 +19,7 @@
 namespace tb {
 
 struct PackedImage {
-  enum Kind : int32_t { kGeneral = 0, kQuant = 1, kDeep = 2, kRank = 3 };
+  enum Kind : int32_t { kGeneral = 0, kQuant = 1, kDeep = 2, kRank = 3, kLanes = 4 };
   int32_t kind = kGeneral;
   // what was asked for (the key under which a cached image may be reused) ...
   int32_t requested_representation = 0, requested_tile_size = 1, requested_feature_bits = 0;
@@ -30,9 +31,10 @@ struct PackedImage {
   QuantForest qf;      // kQuant
   DeepForest df;       // kDeep
   RankForest rf;       // kRank
+  LaneForest lf;       // kLanes
 };
 
-constexpr uint32_t kPackedImageVersion = 8; // changes whenever a packer's output does
+constexpr uint32_t kPackedImageVersion = 9; // changes whenever a packer's output does
 
 void serialize_image(const PackedImage &im, std::vector<uint8_t> *out);
 uint64_t serialized_image_size(const PackedImage &im); // without serialising

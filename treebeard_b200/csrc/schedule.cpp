@@ -9,7 +9,7 @@ static int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 int64_t smem_needed(const ForestShape &fs, const LaunchPlan &p) {
   const int64_t rt = 32 * p.rows_per_lane;
   int64_t bytes = align_up(16 + fs.lut_bytes, 128);
-  if (p.staged) bytes += 2 * (int64_t)p.stage_bytes;
+  if (p.staged) bytes += p.stages * (int64_t)p.stage_bytes;
   if (p.cache_rows) bytes += (int64_t)p.row_warps * (fs.num_features + 1) * rt * 4;
   const int64_t warps = (int64_t)p.row_warps * p.tree_threads;
   if (fs.num_classes > 0 && !p.class_regs)
@@ -36,8 +36,11 @@ std::string select_launch(const ForestShape &fs, const tbk_schedule &user, int64
   bool have = false;
 
   const uint32_t stage_bytes = (uint32_t)align_up((int64_t)fs.max_group_bytes, 128);
-  // staging pays when two stages leave at least ~40% of shared memory to the rows
-  const bool can_stage = 2 * (int64_t)stage_bytes <= (int64_t)smem_limit * 6 / 10 && stage_bytes < (1u << 20);
+  // Staging pays when two stages leave at least ~40% of shared memory to the rows; a group that fits
+  // half of it once is copied and walked by turns (100 000 rows through 300 trees of 8 levels in tiles
+  // of two nodes: 706 us with nodes from global memory, where a gather costs a wavefront per lane, 540 us so).
+  const int stages = 2 * (int64_t)stage_bytes <= (int64_t)smem_limit * 6 / 10 ? 2 : 2 * (int64_t)stage_bytes <= (int64_t)smem_limit ? 1 : 0;
+  const bool can_stage = stages > 0 && stage_bytes < (1u << 20);
   const bool want_stage = user.cache_trees == 2 ? false : can_stage;
   if (user.cache_trees == 1 && !can_stage)
     return "tree groups of this forest do not fit the shared-memory stages (cache_trees = 1)";
@@ -64,6 +67,7 @@ std::string select_launch(const ForestShape &fs, const tbk_schedule &user, int64
         p.rows_per_lane = rpl;
         p.tree_threads = tt;
         p.staged = want_stage;
+        p.stages = want_stage ? stages : 0;
         p.stage_bytes = want_stage ? stage_bytes : 0;
         p.cache_rows = cached;
         // class sums can stay in registers when one warp walks all trees of its rows and

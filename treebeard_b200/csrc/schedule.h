@@ -30,6 +30,7 @@ struct LaunchPlan {
   int32_t chunks = 1;        // grid.y
   int32_t groups_per_chunk = 1;
   int32_t staged = 0;        // tree groups staged through shared memory
+  int32_t stages = 0;        // ... 2: the next group is copied while one is walked; 1: by turns
   int32_t cache_rows = 1;    // row tile transposed into shared memory
   int32_t class_regs = 0;    // multiclass: class sums in registers (no shared-memory class table)
   uint32_t stage_bytes = 0;

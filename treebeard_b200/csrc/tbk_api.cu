@@ -5,6 +5,7 @@
 #include "quant_pack.h"
 #include "rank_pack.h"
 #include "deep_pack.h"
+#include "lane_pack.h"
 #include "schedule.h"
 #include "walk_kernels.cuh"
 #include "walk_quant.cuh"
@@ -13,6 +14,7 @@
 #include "rank_rows.cuh"
 #include "walk_rank.cuh"
 #include "walk_rank_tiles.cuh"
+#include "walk_lanes.cuh"
 #include "packed_image.h"
 
 #ifdef __SSE2__
@@ -236,6 +238,11 @@ struct tbk_forest {
   RankPlan rank_plan;          // of the last batch size
   int64_t rank_plan_rows = -1;
   bool rank_plan_ids = false;
+  // lane layout (what is left)
+  bool lanes = false;
+  uint2 *d_lnodes = nullptr;
+  uint32_t *d_lroot = nullptr, *d_lclass_end = nullptr;
+  int32_t *d_ltree_index = nullptr, *d_lorig = nullptr;
   // one-tree-per-stage layout (deep trees); shares the device buffers of the key layout
   bool deep = false;
   tb::DeepForest df;
@@ -1022,6 +1029,122 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   return TBK_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Lane layout (lane_pack.h)
+
+struct LanePlan {
+  int tiles = 1, shares = 1, chunks = 1, smem = 0;
+  int64_t grid_x = 1;
+};
+
+// Enough warps for 48 on every SM, where there are that many: row tiles first, then shares of the
+// trees within a block (at least four trees each, or a class), then further chunks of them.
+LanePlan plan_lanes(const tbk_forest *f, int64_t n_rows, bool chunks_allowed) {
+  const auto &pk = f->packed;
+  const int64_t tiles = (n_rows + 31) / 32, wanted = std::max<int64_t>(1, 48ll * f->num_sms / tiles);
+  const int64_t parts = pk.num_classes > 0 ? pk.num_classes : std::max<int64_t>(1, pk.num_trees / 4);
+  LanePlan p;
+  while (p.shares < 16 && p.shares < wanted && 2 * p.shares <= parts) p.shares *= 2;
+  p.tiles = (int)std::min<int64_t>(tiles, 16 / p.shares);
+  auto bytes = [&] { return p.tiles * (pk.num_features + 1) * 128 + p.tiles * p.shares * 256; };
+  while (p.tiles > 1 && bytes() > 48 * 1024) --p.tiles;
+  p.smem = bytes();
+  p.grid_x = (tiles + p.tiles - 1) / p.tiles;
+  if (chunks_allowed) {
+    p.chunks = (int)std::min({(wanted + p.shares - 1) / p.shares, std::max<int64_t>(1, parts / p.shares), (int64_t)64});
+    if (f->user.tree_chunks > 0) p.chunks = (int)std::min<int64_t>(f->user.tree_chunks, std::max<int64_t>(1, pk.num_trees / p.shares));
+  }
+  return p;
+}
+
+tb::LaunchPlan lane_launch_plan(const LanePlan &l) {
+  tb::LaunchPlan plan;
+  plan.row_warps = l.tiles;
+  plan.tree_threads = l.shares;
+  plan.chunks = l.chunks;
+  plan.smem_bytes = l.smem;
+  plan.threads = 32 * l.tiles * l.shares;
+  plan.grid_x = l.grid_x;
+  return plan;
+}
+
+// fixed: the partial sums go to this memory, whatever the number of chunks (tbk_predict_noalloc).
+int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out, int32_t out_kind,
+              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot, float *fixed = nullptr, size_t fixed_floats = 0) {
+  const auto &pk = f->packed;
+  const int W = std::max(1, pk.num_classes);
+  const bool classes = pk.num_classes > 0;
+  // (a chunk of a host batch is walked in the shape of the whole batch, see run)
+  LanePlan plan = plan_lanes(f, std::max(n_rows, f->host_batch_rows), !classes || mode == kLeafIds);
+  plan.grid_x = ((n_rows + 31) / 32 + plan.tiles - 1) / plan.tiles;
+  f->last_plan = lane_launch_plan(plan);
+  const bool second_pass = fixed != nullptr || (mode != kLeafIds && plan.chunks > 1);
+  float *partial = d_partial;
+  bool uses_scratch = false;
+  if (fixed) {
+    partial = fixed;
+    if ((size_t)plan.chunks * n_rows * W > fixed_floats)
+      return fail(TBK_ERR_UNSUPPORTED, "tbk_predict_noalloc: %lld rows x %d tree chunks x %d outputs need %zu partial sums, the fixed "
+                  "scratch holds %zu; split the batch or use tbk_predict", (long long)n_rows, plan.chunks, W,
+                  (size_t)plan.chunks * n_rows * W, fixed_floats);
+  } else if (second_pass) {
+    const size_t need = ((size_t)plan.chunks * n_rows * sizeof(float) + 255) & ~(size_t)255;
+    int rc = ensure_scratch(f, 2 * need);
+    if (rc) return rc;
+    partial = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(f->d_scratch) + (size_t)slot * (f->scratch_bytes / 2));
+    rc = scratch_acquire(f, slot, stream);
+    if (rc) return rc;
+    uses_scratch = true;
+  }
+  tb::LaneParams p{};
+  p.nodes = f->d_lnodes;
+  p.root = f->d_lroot;
+  p.tree_index = f->d_ltree_index;
+  p.orig_node = f->d_lorig;
+  p.class_end = f->d_lclass_end;
+  p.rows = d_rows;
+  p.n_rows = n_rows;
+  p.ld = ld;
+  p.partial = partial;
+  p.out = d_out;
+  p.leaf_ids = d_leaf_ids;
+  p.num_trees = pk.num_trees;
+  p.num_features = pk.num_features;
+  p.num_classes = pk.num_classes;
+  p.transform = pk.transform;
+  p.out_kind = out_kind == TBK_OUT_I8 ? 1 : 0;
+  p.write_partial = mode == kPartial || second_pass ? 1 : 0;
+  p.initial_value = (float)pk.initial_value;
+  p.tiles = plan.tiles;
+  p.shares = plan.shares;
+  p.vec4_ok = (pk.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0) ? 1 : 0;
+  using K = void (*)(const tb::LaneParams);
+  const K k = classes ? (mode == kLeafIds ? tb::tb_walk_lanes_kernel<true, true> : tb::tb_walk_lanes_kernel<true, false>)
+                      : (mode == kLeafIds ? tb::tb_walk_lanes_kernel<false, true> : tb::tb_walk_lanes_kernel<false, false>);
+  int rc = allow_smem(f, (const void *)k);
+  if (rc) return rc;
+  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
+  k<<<dim3((unsigned)plan.grid_x, (unsigned)plan.chunks), f->last_plan.threads, plan.smem, stream>>>(p);
+  CUDA_TRY(cudaGetLastError());
+  ++f->launches;
+  if (second_pass) {
+    const int tpb = 256;
+    if (mode == kPartial)
+      tb::tb_sum_partials_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(partial, plan.chunks, n_rows, d_partial);
+    else
+      tb::tb_finalize_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(
+          partial, plan.chunks, n_rows, W, pk.num_classes, (float)pk.initial_value, pk.transform, d_out, out_kind);
+    CUDA_TRY(cudaGetLastError());
+    ++f->launches;
+  }
+  if (f->timing) {
+    CUDA_TRY(cudaEventRecord(f->ev1, stream));
+    f->ev_pending = true;
+  }
+  if (uses_scratch) return scratch_release(f, slot, stream);
+  return TBK_OK;
+}
+
 // One prediction over device-resident rows.
 int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
         int32_t out_kind, float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot = 0) {
@@ -1036,6 +1159,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
   }
   CUDA_TRY(cudaSetDevice(f->device));
   if (f->rank) return run_rank(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
+  if (f->lanes) return run_lanes(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream, slot);
   if (f->quant) return run_quant(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream, slot);
   if (f->deep) return run_deep(f, mode, d_rows, n_rows, ld, d_out, d_partial, d_leaf_ids, stream, slot);
 
@@ -1100,6 +1224,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
   p.row_warps = plan.row_warps;
   p.tree_threads = plan.tree_threads;
   p.stage_bytes = plan.staged ? plan.stage_bytes : 0;
+  p.stages = plan.stages;
   p.vec4_ok = (pk.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0) ? 1 : 0;
   p.status = f->d_status;
   p.skip_first_copy = (f->expire_next_wait && plan.staged) ? 1 : 0;
@@ -1420,6 +1545,16 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
     *out = img.release();
     return TBK_OK;
   }
+  // trees deeper than the key layouts reach (or than a shared-memory stage of tree groups could
+  // hold), layout left to the library: nodes in global memory, every lane at its own pace
+  if (im.user.representation == TBK_REP_AUTO && bits == 0 && ts == 1 && max_depth > tb::kQuantMaxDepth &&
+      im.user.cache_trees != 1 && (host.num_features + 1) * 128 <= 96 * 1024 && tb::pack_lanes(host, &im.lf).empty()) {
+    im.kind = tb::PackedImage::kLanes;
+    im.user.representation = rep;
+    *out = img.release();
+    return TBK_OK;
+  }
+  im.lf = tb::LaneForest();
   tb::PackOptions opt;
   opt.representation = rep;
   opt.tile_size = ts;
@@ -1534,6 +1669,34 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     *out = f;
     return TBK_OK;
   }
+  auto upload = [](auto **dst, const auto &v) { // (an empty vector gets a few bytes)
+    const size_t bytes = v.size() * sizeof(v[0]);
+    cudaError_t e = cudaMalloc((void **)dst, std::max<size_t>(16, bytes));
+    if (e == cudaSuccess && bytes) e = cudaMemcpy((void *)*dst, v.data(), bytes, cudaMemcpyHostToDevice);
+    return e;
+  };
+  if (im.kind == tb::PackedImage::kLanes) {
+    const auto &q = im.lf;
+    f->lanes = true;
+    f->packed.representation = tb::kSparse;
+    f->packed.tile_size = 1;
+    f->packed.num_features = q.num_features;
+    f->packed.num_classes = q.num_classes;
+    f->packed.transform = q.transform;
+    f->packed.initial_value = q.initial_value;
+    f->packed.num_trees = q.num_trees;
+    f->packed.num_nodes = q.num_nodes;
+    f->packed.max_depth = q.max_depth;
+    static_assert(sizeof(tb::LaneNode) == sizeof(uint2), "node layout");
+    CUDA_TRY_F(upload(&f->d_lnodes, q.nodes));
+    CUDA_TRY_F(upload(&f->d_lroot, q.root));
+    CUDA_TRY_F(upload(&f->d_ltree_index, q.tree_index));
+    CUDA_TRY_F(upload(&f->d_lorig, q.orig_node));
+    CUDA_TRY_F(upload(&f->d_lclass_end, q.class_end));
+    f->last_plan = lane_launch_plan(plan_lanes(f, batch_hint > 0 ? batch_hint : 65536, q.num_classes == 0));
+    *out = f;
+    return TBK_OK;
+  }
   if (im.kind == tb::PackedImage::kRank) {
     const auto &q = im.rf;
     f->rank = true;
@@ -1547,12 +1710,6 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     f->packed.num_nodes = q.num_nodes;
     f->packed.max_depth = q.max_depth;
     static_assert(sizeof(tb::RankFeature) == sizeof(tb::DevRankFeature) && sizeof(tb::RankFeature) == 32, "rank table layout");
-    auto upload = [](auto **dst, const auto &v) { // (an empty vector gets a few bytes)
-      const size_t bytes = v.size() * sizeof(v[0]);
-      cudaError_t e = cudaMalloc(dst, std::max<size_t>(16, bytes));
-      if (e == cudaSuccess && bytes) e = cudaMemcpy((void *)*dst, v.data(), bytes, cudaMemcpyHostToDevice);
-      return e;
-    };
     CUDA_TRY_F(upload(&f->d_rnode, q.node_plane));
     CUDA_TRY_F(upload(&f->d_rleaf, q.leaf_plane));
     CUDA_TRY_F(upload(&f->d_rorig, q.orig_leaf));
@@ -1704,7 +1861,8 @@ int tbk_forest_free(tbk_forest *f) {
   cudaFree(f->d_qscale);
   cudaFree(f->d_ties);
   for (void *d : {(void *)f->d_rnode, (void *)f->d_rleaf, (void *)f->d_rorig, (void *)f->d_rgroups, (void *)f->d_rtree_index,
-                  (void *)f->d_rclass_begin, (void *)f->d_rfeatures, (void *)f->d_rlut, (void *)f->d_rthr})
+                  (void *)f->d_rclass_begin, (void *)f->d_rfeatures, (void *)f->d_rlut, (void *)f->d_rthr, (void *)f->d_lnodes, (void *)f->d_lroot,
+                  (void *)f->d_ltree_index, (void *)f->d_lorig, (void *)f->d_lclass_end})
     cudaFree(d);
   for (auto &w : f->workspace) {
     cudaFree(w.mem);
@@ -1725,8 +1883,8 @@ int tbk_forest_get_info(const tbk_forest *f, tbk_forest_info *info) {
   const auto &p = f->packed;
   info->num_trees = p.num_trees;
   info->num_nodes = p.num_nodes;
-  info->num_groups = f->rank ? (int64_t)f->rf.groups.size() : f->quant ? (int64_t)f->qf.groups.size() : f->deep ? (int64_t)f->df.pairs.size() : (int64_t)p.groups.size();
-  info->packed_bytes = f->rank ? (int64_t)(8 * (f->rf.groups.back().elem_off + (uint64_t)f->rf.groups.back().slots * tb::kRankCols)) :
+  info->num_groups = f->lanes ? p.num_trees : f->rank ? (int64_t)f->rf.groups.size() : f->quant ? (int64_t)f->qf.groups.size() : f->deep ? (int64_t)f->df.pairs.size() : (int64_t)p.groups.size();
+  info->packed_bytes = f->lanes ? 8 * p.num_nodes : f->rank ? (int64_t)(8 * (f->rf.groups.back().elem_off + (uint64_t)f->rf.groups.back().slots * tb::kRankCols)) :
                        f->deep ? (int64_t)(f->df.pairs.empty() ? 0 : 8 * (f->df.pairs.back().elem_off + 2ull * f->df.pairs.back().slots)) :
                        f->quant ? (int64_t)(f->qf.groups.empty() ? 0 : 8 * (f->qf.groups.back().elem_off + (uint64_t)f->qf.groups.back().slots * tb::kQuantCols)) :
                        p.groups.empty() ? 0 : (int64_t)(p.groups.back().byte_off +
@@ -2007,6 +2165,8 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   float *scratch = nullptr;
   int rc = noalloc_scratch_address(f->device, &scratch);
   if (rc != TBK_OK) return rc;
+  if (f->lanes)
+    return run_lanes(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, 0, scratch, kNoAllocScratchFloats);
 
   tb::ForestShape shape{pk.num_features, pk.num_classes, (int64_t)pk.groups.size(), pk.max_group_bytes,
                         (int32_t)pk.lut.size(), pk.representation, pk.tile_size};
@@ -2049,6 +2209,7 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   p.row_warps = plan.row_warps;
   p.tree_threads = plan.tree_threads;
   p.stage_bytes = plan.staged ? plan.stage_bytes : 0;
+  p.stages = plan.stages;
   p.vec4_ok = (pk.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0) ? 1 : 0;
   p.status = f->d_status;
   p.class_regs = 0; // class sums go through the shared-memory table the plan has sized

@@ -20,7 +20,7 @@
 // 32 distinct banks.
 //
 // Tree groups are staged into shared memory with cp.async.bulk (the TMA unit's
-// untiled bulk copy) into a two-stage ring guarded by mbarriers; feature rows are
+// untiled bulk copy) into a ring of two stages, or one, guarded by mbarriers; feature rows are
 // read with 16-byte loads and transposed through shared memory.  The reference's
 // counterparts are the cooperative row cache (src/gpu/GPURepresentations.cpp:279-399)
 // and tree cache (:630-715).
@@ -63,6 +63,7 @@ struct WalkParams {
   int32_t row_warps;
   int32_t tree_threads;
   uint32_t stage_bytes; // capacity of one stage (0 when not staged)
+  int32_t stages;       // 1 or 2: groups that fit only once are copied and walked by turns
   int32_t vec4_ok;      // rows can be read with 16-byte loads
   int32_t class_regs;   // multiclass: class sums in registers, arg-max decided on the fly
   int32_t *status;      // device status word, 0 = ok
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
   int8_t *lut_s = reinterpret_cast<int8_t *>(smem_raw + 16);               // look-up table
   size_t off = (16 + (size_t)p.lut_bytes + 127) & ~(size_t)127;
   unsigned char *stage0 = smem_raw + off;
-  off += STAGED ? 2 * (size_t)p.stage_bytes : 0;
+  off += STAGED ? (size_t)p.stages * p.stage_bytes : 0;
   float *xs_all = reinterpret_cast<float *>(smem_raw + off);
   const size_t xs_floats = CACHED ? (size_t)(F + 1) * RT : 0;
   off += (size_t)RW * xs_floats * 4;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
   __syncthreads();
 
   if (STAGED && tid == 0) {
-    for (int s = p.skip_first_copy ? 1 : 0; s < 2 && g0 + s < g1; ++s) {
+    for (int s = p.skip_first_copy ? 1 : 0; s < p.stages && g0 + s < g1; ++s) {
       const DevGroupMeta gm = p.groups[g0 + s];
       const uint32_t bytes = (gm.slots * kCols * (REP == 2 ? 6u : (uint32_t)(TS == 1 ? 8 : TS == 2 ? 16 : TS == 3 ? 24 : 32)) + 15u) & ~15u;
       mbar_expect_tx(&mbar[s], bytes);
@@ -340,8 +341,8 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
     }
     const uint8_t *gbase;
     if (STAGED) {
-      const int s = (g - g0) & 1;
-      const uint32_t parity = ((g - g0) >> 1) & 1;
+      const int s = p.stages == 2 ? (g - g0) & 1 : 0;
+      const uint32_t parity = (p.stages == 2 ? (g - g0) >> 1 : g - g0) & 1;
       const bool ok = mbar_wait_bounded(&mbar[s], parity, p.wait_limit ? p.wait_limit : kWaitLimit);
       if (__syncthreads_or(!ok)) {
         if (tid == 0) set_status(p.status, 4);
@@ -380,9 +381,9 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
     }
     if (STAGED) {
       __syncthreads(); // every warp is done with this stage
-      if (tid == 0 && g + 2 < g1) {
-        const int s = (g - g0) & 1;
-        const DevGroupMeta nx = p.groups[g + 2];
+      if (tid == 0 && g + p.stages < g1) {
+        const int s = p.stages == 2 ? (g - g0) & 1 : 0;
+        const DevGroupMeta nx = p.groups[g + p.stages];
         const uint32_t bytes = (nx.slots * kCols * (REP == 2 ? 6u : (uint32_t)(TS == 1 ? 8 : TS == 2 ? 16 : TS == 3 ? 24 : 32)) + 15u) & ~15u;
         mbar_expect_tx(&mbar[s], bytes);
         bulk_g2s(stage0 + (size_t)s * p.stage_bytes, p.blob + nx.byte_off, bytes, &mbar[s]);

@@ -1,0 +1,151 @@
+// Walk kernel for the lane layout (lane_pack.h): every lane takes its row through the trees of a
+// range at its own pace.  A step follows the node's distance -- to a child, or from a leaf to the
+// next tree's root -- so a lane spends no step below a leaf and needs no tree counter; a fixed-depth
+// walk takes every row to the depth of the deepest tree of the group (16 steps where trees grown
+// until their leaves are pure need 5).  65536 rows through 200 such trees of up to 16 levels: 207 us at
+// fixed depth from interleaved groups, 83 us here.
+//
+// A warp = 32 rows and one of `shares` ranges of the trees; the row tile (transposed, bank = row) is
+// shared by the warps that split the trees, and their sums meet in shared memory in share order.
+// The kernel is bound by the latency of the nodes' gathers, so blocks are small and many fit an SM:
+// the trees being walked stay in L1.  blockIdx.y splits the trees further for small batches; a second
+// kernel adds those partial sums (walk_kernels.cuh).
+//
+// Reference counterparts: the scalar walk that stops at a leaf, src/mlir/CodeGenStateMachine.cpp:
+// 149-243; the tie rule of class ids, src/reduction/LowerReduceOps.cpp:148-189.
+#pragma once
+#include "walk_kernels.cuh"
+
+namespace tb {
+
+struct LaneParams {
+  const uint2 *nodes;
+  const uint32_t *root;       // [num_trees + 1]
+  const int32_t *tree_index;
+  const int32_t *orig_node;
+  const uint32_t *class_end;  // multiclass
+  const float *rows;
+  long long n_rows, ld;
+  float *partial;             // write_partial: [chunks][n_rows], or [n_rows][classes]
+  void *out;
+  int32_t *leaf_ids;
+  long long num_trees;
+  int32_t num_features, num_classes, transform, out_kind, write_partial;
+  float initial_value;
+  int32_t tiles, shares;      // of a block: row tiles, warps that split the trees of a tile
+  int32_t vec4_ok;
+};
+
+// Where part `i` of `n` of the trees begins; parts of a multiclass forest are whole classes.
+__device__ __forceinline__ uint32_t lane_part(const LaneParams &p, int i, int n) {
+  if (p.num_classes == 0) return p.root[p.num_trees * i / n];
+  const int c = (int)((long long)p.num_classes * i / n);
+  return c == 0 ? 0u : p.class_end[c - 1];
+}
+
+template <bool CLASSES, bool LEAF_IDS>
+__global__ void __launch_bounds__(512) tb_walk_lanes_kernel(const LaneParams p) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tile = warp % p.tiles, share = warp / p.tiles;
+  const int F = p.num_features;
+  float *xs = reinterpret_cast<float *>(smem_raw) + (size_t)tile * (F + 1) * 32;
+  float *sums = reinterpret_cast<float *>(smem_raw) + (size_t)p.tiles * (F + 1) * 32; // [warp][row], classes: [warp][2][row]
+  const long long row = ((long long)blockIdx.x * p.tiles + tile) * 32 + lane;
+  const bool live = row < p.n_rows;
+  {
+    const float *src = p.rows + (live ? row : 0) * p.ld;
+    if (p.vec4_ok) {
+      for (int k = share; k < F / 4; k += p.shares) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(src) + k);
+        xs[(4 * k + 0) * 32 + lane] = v.x;
+        xs[(4 * k + 1) * 32 + lane] = v.y;
+        xs[(4 * k + 2) * 32 + lane] = v.z;
+        xs[(4 * k + 3) * 32 + lane] = v.w;
+      }
+    } else {
+      for (int k = share; k < F; k += p.shares) xs[k * 32 + lane] = __ldg(src + k);
+    }
+    if (share == 0) xs[F * 32 + lane] = -INFINITY; // a leaf's feature: on to the next tree
+  }
+  __syncthreads();
+
+  const int part = (int)blockIdx.y * p.shares + share, parts = (int)gridDim.y * p.shares;
+  uint32_t n = lane_part(p, part, parts);
+  const uint32_t end = lane_part(p, part + 1, parts);
+  const float *mine = xs + lane;
+  float acc = 0.f;
+  [[maybe_unused]] float best = -INFINITY;
+  [[maybe_unused]] int cls = 0, best_class = 0, last_class = 0;
+  [[maybe_unused]] uint32_t class_end = 0, tree = 0;
+  if constexpr (CLASSES) {
+    cls = (int)((long long)p.num_classes * part / parts);
+    last_class = (int)((long long)p.num_classes * (part + 1) / parts);
+    class_end = cls < last_class ? p.class_end[cls] : end;
+  }
+  // the sum of class `cls` is complete (ties go to the higher class)
+  [[maybe_unused]] auto close = [&]() {
+    if (p.write_partial && live) p.partial[row * p.num_classes + cls] = acc;
+    if (acc >= best) {
+      best = acc;
+      best_class = cls;
+    }
+    acc = 0.f;
+    ++cls;
+    class_end = cls < last_class ? p.class_end[cls] : 0xffffffffu;
+  };
+  if constexpr (LEAF_IDS) { // the tree that this part begins with
+    uint32_t lo = 0, hi = (uint32_t)p.num_trees;
+    while (lo < hi) {
+      const uint32_t m = (lo + hi) / 2;
+      if (p.root[m] < n) lo = m + 1;
+      else hi = m;
+    }
+    tree = lo;
+  }
+  while (n < end) {
+    if constexpr (CLASSES && !LEAF_IDS)
+      while (n >= class_end) close();
+    const uint2 node = __ldg(p.nodes + n);
+    const uint32_t f = node.y & 0xffffu;
+    const float t = __uint_as_float(node.x), x = mine[f * 32];
+    const bool leaf = f == (uint32_t)F;
+    if constexpr (LEAF_IDS) {
+      if (leaf) {
+        if (live) p.leaf_ids[row * p.num_trees + p.tree_index[tree]] = p.orig_node[n];
+        ++tree;
+      }
+    } else {
+      acc += leaf ? t : 0.f;
+    }
+    n += (node.y >> 16) + (x < t || leaf ? 0u : 1u);
+  }
+  if constexpr (LEAF_IDS) return;
+  if constexpr (CLASSES) {
+    const bool empty = (int)((long long)p.num_classes * part / parts) == last_class; // (a part without classes wins nothing)
+    while (cls < last_class) close();
+    if (p.write_partial) return;
+    sums[(2 * warp) * 32 + lane] = empty ? __int_as_float(0x7fffffff) : best;
+    sums[(2 * warp + 1) * 32 + lane] = __int_as_float(best_class);
+    __syncthreads();
+    if (share != 0 || !live) return;
+    for (int s = 1; s < p.shares; ++s) { // (classes rise with the shares)
+      const float b = sums[2 * (s * p.tiles + tile) * 32 + lane];
+      if (b >= best) {
+        best = b;
+        best_class = __float_as_int(sums[(2 * (s * p.tiles + tile) + 1) * 32 + lane]);
+      }
+    }
+    if (p.out_kind == 1) reinterpret_cast<int8_t *>(p.out)[row] = (int8_t)best_class;
+    else reinterpret_cast<float *>(p.out)[row] = (float)best_class;
+  } else {
+    sums[warp * 32 + lane] = acc;
+    __syncthreads();
+    if (share != 0 || !live) return;
+    for (int s = 1; s < p.shares; ++s) acc += sums[(s * p.tiles + tile) * 32 + lane];
+    if (p.write_partial) p.partial[(long long)blockIdx.y * p.n_rows + row] = acc;
+    else reinterpret_cast<float *>(p.out)[row] = apply_transform(p.initial_value + acc, p.transform);
+  }
+}
+
+} // namespace tb
