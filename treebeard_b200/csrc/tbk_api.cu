@@ -1463,7 +1463,10 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
   bool want_quant = (bits == 16 && max_depth <= tb::kQuantMaxDepth && (host.num_classes == 0 || batch_fits)) ||
                     (bits == 0 && (rep == TBK_REP_AUTO || rep == TBK_REP_REORG) && ts == 1 && !fp32_tile_fits &&
                      host.num_classes == 0) ||
-                    (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && batch_fits && max_depth <= tb::kQuantMaxDepth);
+                    (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kQuantMaxDepth &&
+                     (batch_fits || (host.num_features > tb::kRankMaxFeatures && host.num_classes == 0)));
+  // (rows too wide for rank keys: the one-tile kernel; on fp32 tiles of 32 rows, one per block, 98431 rows
+  // of 1303 features took 3.3 ms)
   // rank keys: whatever the key kernels would take, over at most kRankMaxFeatures features
   const bool want_rank = want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth);
   if (want_rank && host.num_features <= tb::kRankMaxFeatures) {

@@ -144,65 +144,82 @@ template <bool CACHED, int RT> __device__ __forceinline__ float feature(const Ro
   return f == (uint32_t)ra.num_features ? __int_as_float(0xff800000) : __ldg(ra.grow + f);
 }
 
-// REP: 0 sparse, 1 array, 2 reorg.  Returns the leaf value after `depth` steps and
-// the final slot in *slot_out.
-template <int REP, int TS, bool SMEM, bool CACHED, int RT>
-__device__ __forceinline__ float walk_one(const uint8_t *gbase, uint32_t slots, uint32_t depth, uint32_t col,
-                                          const RowAccess &ra, const int8_t *lut, uint32_t *slot_out) {
-  uint32_t n = 0;
+// REP: 0 sparse, 1 array, 2 reorg.  Walks NC columns in lock-step (their loads are independent, so
+// that many are in flight per lane); returns the leaf values after `depth` steps and the final slots.
+template <int REP, int TS, bool SMEM, bool CACHED, int RT, int NC>
+__device__ __forceinline__ void walk_columns(const uint8_t *gbase, uint32_t slots, uint32_t depth, const uint32_t (&col)[NC],
+                                             const RowAccess &ra, const int8_t *lut, uint32_t (&n)[NC], float (&v)[NC]) {
+#define TBW_ALL _Pragma("unroll") for (int c = 0; c < NC; ++c)
+  TBW_ALL n[c] = 0;
   if (REP == 2) {
     const float *thr = reinterpret_cast<const float *>(gbase);
     const uint16_t *feat = reinterpret_cast<const uint16_t *>(gbase + (size_t)slots * kCols * 4);
     for (uint32_t d = 0; d < depth; ++d) {
-      const uint32_t i = n * kCols + col;
-      const float t = SMEM ? thr[i] : __ldg(thr + i);
-      const uint32_t f = SMEM ? feat[i] : __ldg(feat + i);
-      const float x = feature<CACHED, RT>(ra, f);
-      n = 2 * n + 1 + !(x < t);
+      float t[NC], x[NC];
+      uint32_t f[NC];
+      TBW_ALL {
+        const uint32_t i = n[c] * kCols + col[c];
+        t[c] = SMEM ? thr[i] : __ldg(thr + i);
+        f[c] = SMEM ? feat[i] : __ldg(feat + i);
+      }
+      TBW_ALL x[c] = feature<CACHED, RT>(ra, f[c]);
+      TBW_ALL n[c] = 2 * n[c] + 1 + !(x[c] < t[c]);
     }
-    *slot_out = n;
-    const uint32_t i = n * kCols + col;
-    return SMEM ? thr[i] : __ldg(thr + i);
+    TBW_ALL {
+      const uint32_t i = n[c] * kCols + col[c];
+      v[c] = SMEM ? thr[i] : __ldg(thr + i);
+    }
+    return;
   }
   constexpr int TB = TS == 1 ? 8 : TS == 2 ? 16 : TS == 3 ? 24 : 32;
   for (uint32_t d = 0; d < depth; ++d) {
-    const uint8_t *tp = gbase + (size_t)(n * kCols + col) * TB;
-    uint32_t k, child;
+    uint32_t k[NC], child[NC];
     if (TS == 1) {
-      const uint2 t = ld2<SMEM>(tp);
-      const float x = feature<CACHED, RT>(ra, t.y & 0xffffu);
-      child = t.y >> 16;
-      k = !(x < __uint_as_float(t.x));
-    } else {
-      float thr[TS];
-      uint32_t f[TS], shape;
-      if (TS == 2) {
-        const uint4 t = ld4<SMEM>(tp);
-        thr[0] = __uint_as_float(t.x); thr[1] = __uint_as_float(t.y);
-        f[0] = t.z & 0xffffu; f[1] = t.z >> 16;
-        shape = t.w & 0xffffu; child = t.w >> 16;
-      } else if (TS == 3) {
-        const uint2 a = ld2<SMEM>(tp), b = ld2<SMEM>(tp + 8), c = ld2<SMEM>(tp + 16);
-        thr[0] = __uint_as_float(a.x); thr[1] = __uint_as_float(a.y); thr[2] = __uint_as_float(b.x);
-        f[0] = b.y & 0xffffu; f[1] = b.y >> 16; f[2] = c.x & 0xffffu;
-        shape = c.x >> 16; child = c.y & 0xffffu;
-      } else {
-        const uint4 a = ld4<SMEM>(tp), b = ld4<SMEM>(tp + 16);
-        thr[0] = __uint_as_float(a.x); thr[1] = __uint_as_float(a.y);
-        thr[2] = __uint_as_float(a.z); thr[3] = __uint_as_float(a.w);
-        f[0] = b.x & 0xffffu; f[1] = b.x >> 16; f[2] = b.y & 0xffffu; f[3] = b.y >> 16;
-        shape = b.z & 0xffffu; child = b.z >> 16;
+      uint2 t[NC];
+      float x[NC];
+      TBW_ALL t[c] = ld2<SMEM>(gbase + (size_t)(n[c] * kCols + col[c]) * TB);
+      TBW_ALL x[c] = feature<CACHED, RT>(ra, t[c].y & 0xffffu);
+      TBW_ALL {
+        child[c] = t[c].y >> 16;
+        k[c] = !(x[c] < __uint_as_float(t[c].x));
       }
-      uint32_t bits = 0;
+    } else {
+      float thr[NC][TS];
+      uint32_t f[NC][TS], shape[NC], bits[NC];
+      TBW_ALL {
+        const uint8_t *tp = gbase + (size_t)(n[c] * kCols + col[c]) * TB;
+        if (TS == 2) {
+          const uint4 t = ld4<SMEM>(tp);
+          thr[c][0] = __uint_as_float(t.x); thr[c][1] = __uint_as_float(t.y);
+          f[c][0] = t.z & 0xffffu; f[c][1] = t.z >> 16;
+          shape[c] = t.w & 0xffffu; child[c] = t.w >> 16;
+        } else if (TS == 3) {
+          const uint2 a = ld2<SMEM>(tp), b = ld2<SMEM>(tp + 8), e = ld2<SMEM>(tp + 16);
+          thr[c][0] = __uint_as_float(a.x); thr[c][1] = __uint_as_float(a.y); thr[c][2] = __uint_as_float(b.x);
+          f[c][0] = b.y & 0xffffu; f[c][1] = b.y >> 16; f[c][2] = e.x & 0xffffu;
+          shape[c] = e.x >> 16; child[c] = e.y & 0xffffu;
+        } else {
+          const uint4 a = ld4<SMEM>(tp), b = ld4<SMEM>(tp + 16);
+          thr[c][0] = __uint_as_float(a.x); thr[c][1] = __uint_as_float(a.y);
+          thr[c][2] = __uint_as_float(a.z); thr[c][3] = __uint_as_float(a.w);
+          f[c][0] = b.x & 0xffffu; f[c][1] = b.x >> 16; f[c][2] = b.y & 0xffffu; f[c][3] = b.y >> 16;
+          shape[c] = b.z & 0xffffu; child[c] = b.z >> 16;
+        }
+      }
+      TBW_ALL {
+        bits[c] = 0;
 #pragma unroll
-      for (int i = 0; i < TS; ++i) bits |= (uint32_t)(feature<CACHED, RT>(ra, f[i]) < thr[i]) << i;
-      k = (uint32_t)lut[(shape << TS) + bits];
+        for (int i = 0; i < TS; ++i) bits[c] |= (uint32_t)(feature<CACHED, RT>(ra, f[c][i]) < thr[c][i]) << i;
+      }
+      TBW_ALL k[c] = (uint32_t)lut[(shape[c] << TS) + bits[c]];
     }
-    n = REP == 0 ? child + k : n * (TS + 1) + 1 + k;
+    TBW_ALL n[c] = REP == 0 ? child[c] + k[c] : n[c] * (TS + 1) + 1 + k[c];
   }
-  *slot_out = n;
-  const uint8_t *tp = gbase + (size_t)(n * kCols + col) * TB;
-  return SMEM ? *reinterpret_cast<const float *>(tp) : __ldg(reinterpret_cast<const float *>(tp));
+  TBW_ALL {
+    const uint8_t *tp = gbase + (size_t)(n[c] * kCols + col[c]) * TB;
+    v[c] = SMEM ? *reinterpret_cast<const float *>(tp) : __ldg(reinterpret_cast<const float *>(tp));
+  }
+#undef TBW_ALL
 }
 
 __device__ __forceinline__ float apply_transform(float v, int transform) {
@@ -352,31 +369,40 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
     } else {
       gbase = p.blob + gm.byte_off;
     }
-    for (int s = tt; s < kCols; s += TT) {
-      const uint32_t col = (lane + s) & (kCols - 1);
+    // what becomes of row q's value from column `col`
+    auto use = [&](uint32_t col, int q, float v, uint32_t slot) {
       const int k = g * kCols + (int)col;
-      uint32_t slot[RPL];
-      float v[RPL];
-#pragma unroll
-      for (int q = 0; q < RPL; ++q)
-        v[q] = walk_one<REP, TS, STAGED, CACHED, RT>(gbase, gm.slots, gm.depth, col, ra[q], lut_s, &slot[q]);
       if (p.leaf_ids != nullptr) {
         const int t = p.tree_index[k];
-        if (t >= 0) {
-#pragma unroll
-          for (int q = 0; q < RPL; ++q) {
-            const long long row = row_base + q * 32 + lane;
-            if (row < p.n_rows)
-              p.leaf_ids[row * p.num_trees + t] = p.orig_node[p.orig_off[g] + (size_t)slot[q] * kCols + col];
-          }
-        }
+        const long long row = row_base + q * 32 + lane;
+        if (t >= 0 && row < p.n_rows)
+          p.leaf_ids[row * p.num_trees + t] = p.orig_node[p.orig_off[g] + (size_t)slot * kCols + col];
       } else if (p.num_classes > 0 && !p.class_regs) {
-        const int cls = p.tree_class[k];
-#pragma unroll
-        for (int q = 0; q < RPL; ++q) cacc[cls * RT + q * 32 + lane] += v[q];
+        cacc[(int)p.tree_class[k] * RT + q * 32 + lane] += v;
       } else {
+        acc[q] += v;
+      }
+    };
+    if (RPL == 1 && TT < kCols) {
+      // one row per lane: two columns in lock-step
+      for (int s = tt; s < kCols; s += 2 * TT) {
+        const uint32_t col[2] = {(uint32_t)(lane + s) & (kCols - 1), (uint32_t)(lane + s + TT) & (kCols - 1)};
+        uint32_t slot[2];
+        float v[2];
+        walk_columns<REP, TS, STAGED, CACHED, RT, 2>(gbase, gm.slots, gm.depth, col, ra[0], lut_s, slot, v);
+        use(col[0], 0, v[0], slot[0]);
+        use(col[1], 0, v[1], slot[1]);
+      }
+    } else {
+      for (int s = tt; s < kCols; s += TT) {
+        const uint32_t col[1] = {(uint32_t)(lane + s) & (kCols - 1)};
 #pragma unroll
-        for (int q = 0; q < RPL; ++q) acc[q] += v[q];
+        for (int q = 0; q < RPL; ++q) {
+          uint32_t slot[1];
+          float v[1];
+          walk_columns<REP, TS, STAGED, CACHED, RT, 1>(gbase, gm.slots, gm.depth, col, ra[q], lut_s, slot, v);
+          use(col[0], q, v[0], slot[0]);
+        }
       }
     }
     if (STAGED) {
