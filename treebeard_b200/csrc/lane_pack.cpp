@@ -34,7 +34,7 @@ std::string pack_lanes(const Forest &f, LaneForest *out) {
   q.orig_node.resize(N);
   std::atomic<bool> far{false};
   std::atomic<int32_t> deepest{0};
-#pragma omp parallel for schedule(dynamic, 16) num_threads(pack_threads())
+#pragma omp parallel for schedule(dynamic, 16) num_threads(pack_threads()) if (N > 1 << 15)
   for (int64_t k = 0; k < T; ++k) {
     const int64_t a = f.tree_off[order[k]];
     const uint32_t base = q.root[k], end = q.root[k + 1];

@@ -59,10 +59,9 @@ std::string pack_quant(const Forest &f, QuantForest *out, bool lattice) {
   if (!err.empty()) return err;
 
   std::vector<int32_t> depth(T);
-  for (int64_t t = 0; t < T; ++t) {
-    depth[t] = tree_depth(f, t);
-    q.max_depth = std::max(q.max_depth, depth[t]);
-  }
+#pragma omp parallel for schedule(dynamic, 64) num_threads(pack_threads()) if (f.num_nodes() > 1 << 15)
+  for (int64_t t = 0; t < T; ++t) depth[t] = tree_depth(f, t);
+  for (int64_t t = 0; t < T; ++t) q.max_depth = std::max(q.max_depth, depth[t]);
   if (q.max_depth > kQuantMaxDepth)
     return "trees deeper than " + std::to_string(kQuantMaxDepth) + " levels do not fit the key layout's stages";
   // columns in walking order: trees by depth -- within their class for a multiclass forest,
@@ -106,6 +105,8 @@ std::string pack_quant(const Forest &f, QuantForest *out, bool lattice) {
   q.exact_plane.assign(elems, 0.f);
   q.orig_leaf.assign(elems, -1);
 
+  int64_t num_splits = 0, whole_number_splits = 0;
+#pragma omp parallel for schedule(dynamic, 1) reduction(+ : num_splits, whole_number_splits) num_threads(pack_threads()) if (f.num_nodes() > 1 << 15)
   for (int64_t g = 0; g < G; ++g) {
     const QuantGroup &gm = q.groups[g];
     for (int c = 0; c < kQuantCols; ++c) {
@@ -130,14 +131,16 @@ std::string pack_quant(const Forest &f, QuantForest *out, bool lattice) {
         const float thr = f.thr[a + it.node];
         const uint64_t e = gm.elem_off + (uint64_t)quant_plane_slot(it.slot, it.level, gm.depth) * kQuantCols + c;
         q.node_plane[e] = (quant_feature_code((uint32_t)ft) << 16) | quant_threshold_key15(thr, q.lo[ft], q.scale[ft]);
-        ++q.num_splits;
-        if (thr == std::floor(thr) && !(q.scale[ft] < 0.f)) ++q.whole_number_splits;
+        ++num_splits;
+        if (thr == std::floor(thr) && !(q.scale[ft] < 0.f)) ++whole_number_splits;
         q.exact_plane[e] = thr;
         stack.push_back({f.left[a + it.node], 2 * it.slot + 1, it.level + 1});
         stack.push_back({f.right[a + it.node], 2 * it.slot + 2, it.level + 1});
       }
     }
   }
+  q.num_splits = num_splits;
+  q.whole_number_splits = whole_number_splits;
   return "";
 }
 

@@ -58,7 +58,7 @@ std::string pack_rank(const Forest &f, RankForest *out) {
   std::vector<uint16_t> rank(N, 0);
   std::vector<std::vector<float>> distinct(F);
   std::atomic<uint32_t> most{0};
-#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads())
+#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads()) if (N > 1 << 15)
   for (int i = 0; i < F; ++i) {
     std::sort(split.begin() + first[i], split.begin() + first[i + 1]);
     auto &d = distinct[i];
@@ -108,7 +108,7 @@ std::string pack_rank(const Forest &f, RankForest *out) {
   }
   q.lut.assign(lut_size, 0);
   q.thresholds.assign(thr_size, 0.f);
-#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads())
+#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads()) if (N > 1 << 15)
   for (int i = 0; i < F; ++i) {
     RankFeature &rf = q.features[i];
     std::copy(distinct[i].begin(), distinct[i].end(), q.thresholds.begin() + rf.thr_off);
@@ -118,7 +118,7 @@ std::string pack_rank(const Forest &f, RankForest *out) {
   // ---- columns: trees by (class,) depth
   std::vector<int32_t> depth(T);
   int32_t deepest = 0;
-#pragma omp parallel for schedule(dynamic, 64) reduction(max : deepest) num_threads(pack_threads())
+#pragma omp parallel for schedule(dynamic, 64) reduction(max : deepest) num_threads(pack_threads()) if (N > 1 << 15)
   for (int64_t t = 0; t < T; ++t) {
     depth[t] = tree_depth(f, t);
     deepest = std::max(deepest, depth[t]);
@@ -151,7 +151,7 @@ std::string pack_rank(const Forest &f, RankForest *out) {
   q.node_plane.assign(elems, always_left);
   q.leaf_plane.assign(elems, 0.f);
   q.orig_leaf.assign(elems, -1);
-#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads())
+#pragma omp parallel for schedule(dynamic, 1) num_threads(pack_threads()) if (N > 1 << 15)
   for (int64_t g = 0; g < G; ++g) {
     const QuantGroup &gm = q.groups[g];
     struct Item { int32_t node; uint32_t path, level; };

@@ -57,6 +57,72 @@ int fail(int code, const char *fmt, ...) {
 
 } // namespace
 
+// Pinned, mapped host memory is slow to come by (milliseconds for a few MiB), so what a forest gives
+// back is kept for the next one: blocks of up to 32 MiB, 64 MiB of them in all.
+class PinnedPool {
+public:
+  unsigned char *take(size_t bytes, size_t *capacity) { // null: none to be had
+    bytes = (bytes + 65535) / 65536 * 65536;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      size_t best = free_.size();
+      for (size_t i = 0; i < free_.size(); ++i)
+        if (free_[i].second >= bytes && free_[i].second <= 4 * bytes && (best == free_.size() || free_[i].second < free_[best].second)) best = i;
+      if (best < free_.size()) {
+        const auto b = free_[best];
+        free_.erase(free_.begin() + (ptrdiff_t)best);
+        kept_ -= b.second;
+        *capacity = b.second;
+        return b.first;
+      }
+    }
+    unsigned char *mem = nullptr;
+    if (cudaHostAlloc(&mem, bytes, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    *capacity = bytes;
+    return mem;
+  }
+  void give_back(unsigned char *mem, size_t capacity) {
+    if (!mem) return;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      if (capacity <= ((size_t)32 << 20) && kept_ + capacity <= ((size_t)64 << 20)) {
+        free_.emplace_back(mem, capacity);
+        kept_ += capacity;
+        return;
+      }
+    }
+    cudaFreeHost(mem);
+  }
+  // A status word: 64 bytes of a shared page.
+  int32_t *take_status() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (status_.empty()) {
+      unsigned char *page = nullptr;
+      if (cudaHostAlloc(&page, 4096, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+      for (int i = 0; i < 4096; i += 64) status_.push_back(reinterpret_cast<int32_t *>(page + i));
+    }
+    int32_t *word = status_.back();
+    status_.pop_back();
+    *word = 0;
+    return word;
+  }
+  void give_back_status(int32_t *word) {
+    if (!word) return;
+    std::lock_guard<std::mutex> lock(mu_);
+    status_.push_back(word);
+  }
+
+private:
+  std::mutex mu_;
+  std::vector<std::pair<unsigned char *, size_t>> free_;
+  std::vector<int32_t *> status_;
+  size_t kept_ = 0;
+};
+PinnedPool &pinned_pool() { // (never destroyed: forests may outlive static objects)
+  static PinnedPool *pool = new PinnedPool();
+  return *pool;
+}
+
 // Copies pageable batches into staging slots, chunk after chunk, on a few threads that a forest
 // keeps from its first such batch on: one core moves about 20 GB/s, PCIe takes 55, and starting
 // threads for every call costs more than the copy.  The calling thread enqueues GPU work meanwhile
@@ -212,8 +278,9 @@ struct tbk_forest {
   int32_t *d_qset_groups = nullptr, *d_qgroup_class = nullptr; // multiclass key layout
   int32_t qset_count[2] = {0, 0};
   unsigned long long *d_ties = nullptr;
-  // rank keys (narrow rows)
+  // rank keys (narrow rows): pointers into one block
   bool rank = false;
+  unsigned char *d_rank_block = nullptr;
   tb::RankForest rf;
   uint32_t *d_rnode = nullptr;
   float *d_rleaf = nullptr, *d_rthr = nullptr;
@@ -255,6 +322,7 @@ struct tbk_forest {
   size_t pipe_bytes = 0, pipe_rows = 0; // capacity of a slot
   std::unique_ptr<Stager> stager;
   unsigned char *h_small = nullptr, *d_small = nullptr, *d_small_in = nullptr;
+  size_t small_capacity = 0, pin_capacity[kPipeSlots] = {}, res_capacity[kPipeSlots] = {};
   const float *inline_rows = nullptr; // rows of the small host batch being predicted, which may travel with the launch
   cudaStream_t streams[2] = {nullptr, nullptr};
   cudaEvent_t slot_read[kPipeSlots] = {}, slot_done[kPipeSlots] = {}; // a chunk's rows are copied / its results are there
@@ -1320,11 +1388,10 @@ int upload_key_planes(tbk_forest *f, const std::vector<uint32_t> &node, const st
 }
 
 void free_pipeline(tbk_forest *f) {
+  cudaFree(f->d_in[0]); // (one block)
   for (int i = 0; i < tbk_forest::kPipeSlots; ++i) {
-    cudaFree(f->d_in[i]);
-    cudaFree(f->d_res[i]);
-    cudaFreeHost(f->h_pin[i]);
-    cudaFreeHost(f->h_res[i]);
+    pinned_pool().give_back(f->h_pin[i], f->pin_capacity[i]);
+    pinned_pool().give_back(f->h_res[i], f->res_capacity[i]);
     f->d_in[i] = f->d_res[i] = f->h_pin[i] = f->h_res[i] = nullptr;
   }
   f->pipe_bytes = f->pipe_rows = 0;
@@ -1352,22 +1419,26 @@ int predict_host_small(tbk_forest *f, const float *h_rows, int64_t n_rows, int64
   const bool classes = out_kind == TBK_OUT_I8;
   const size_t out_bytes = (size_t)n_rows * (classes ? 1 : 4);
   cudaStream_t stream = f->streams[0];
-  if (!f->h_small) {
-    CUDA_TRY(cudaHostAlloc(&f->h_small, kSmallRows + kSmallResults, cudaHostAllocMapped));
+  const size_t results_at = (bytes + 255) / 256 * 256;
+  if (f->small_capacity < results_at + out_bytes) {
+    pinned_pool().give_back(f->h_small, f->small_capacity);
+    f->small_capacity = 0;
+    f->h_small = pinned_pool().take(results_at + out_bytes, &f->small_capacity);
+    if (!f->h_small) return fail(TBK_ERR_CUDA, "no pinned memory for the batch");
     CUDA_TRY(cudaHostGetDevicePointer(&f->d_small, f->h_small, 0));
-    CUDA_TRY(cudaMalloc(&f->d_small_in, kSmallRows));
   }
-  unsigned char *results = f->h_small + kSmallRows;
+  unsigned char *results = f->h_small + results_at;
   if (classes) std::memset(results, kNoClass, out_bytes);
   else std::fill_n(reinterpret_cast<uint32_t *>(results), n_rows, kNoResult);
   copy_past_caches(f->h_small, reinterpret_cast<const unsigned char *>(h_rows), bytes);
   const unsigned char *rows = f->d_small;
   if (!f->rank || bytes > kSmallDirect) {
+    if (!f->d_small_in) CUDA_TRY(cudaMalloc(&f->d_small_in, kSmallRows));
     CUDA_TRY(cudaMemcpyAsync(f->d_small_in, f->h_small, bytes, cudaMemcpyHostToDevice, stream));
     rows = f->d_small_in;
   }
   f->inline_rows = h_rows;
-  const int rc = run(f, kPredict, reinterpret_cast<const float *>(rows), n_rows, ld, f->d_small + kSmallRows, out_kind, nullptr,
+  const int rc = run(f, kPredict, reinterpret_cast<const float *>(rows), n_rows, ld, f->d_small + results_at, out_kind, nullptr,
                      nullptr, stream, 0);
   f->inline_rows = nullptr;
   bool idle = rc != TBK_OK;
@@ -1453,7 +1524,7 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
     if (!verr.empty()) return fail(TBK_ERR_INVALID, "%s", verr.c_str());
   }
   int max_depth = 0;
-#pragma omp parallel for reduction(max : max_depth) schedule(dynamic, 64) num_threads(tb::pack_threads())
+#pragma omp parallel for reduction(max : max_depth) schedule(dynamic, 64) num_threads(tb::pack_threads()) if (N > 1 << 15)
   for (int64_t t = 0; t < T; ++t) max_depth = std::max(max_depth, (int)tb::tree_depth(host, t));
   // narrow rows: the key tiles of at least four 32-row tiles fit beside the ring, so the batch
   // kernel applies; measured faster than the fp32 walk on single-output forests of up to 8 levels
@@ -1639,8 +1710,8 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
   if (im.smem_limit > f->max_smem_optin)
     return bail(fail(TBK_ERR_UNSUPPORTED, "the packed image was laid out for %d bytes of shared memory per block, this device has %d",
                      im.smem_limit, f->max_smem_optin));
-  CUDA_TRY_F(cudaHostAlloc(&f->h_status, 4, cudaHostAllocMapped));
-  *f->h_status = 0;
+  f->h_status = pinned_pool().take_status();
+  if (!f->h_status) return bail(fail(TBK_ERR_CUDA, "no pinned memory for the status word"));
   CUDA_TRY_F(cudaHostGetDevicePointer(&f->d_status, f->h_status, 0));
   CUDA_TRY_F(cudaEventCreate(&f->ev0));
   CUDA_TRY_F(cudaEventCreate(&f->ev1));
@@ -1713,17 +1784,40 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     f->packed.num_nodes = q.num_nodes;
     f->packed.max_depth = q.max_depth;
     static_assert(sizeof(tb::RankFeature) == sizeof(tb::DevRankFeature) && sizeof(tb::RankFeature) == 32, "rank table layout");
-    CUDA_TRY_F(upload(&f->d_rnode, q.node_plane));
-    CUDA_TRY_F(upload(&f->d_rleaf, q.leaf_plane));
-    CUDA_TRY_F(upload(&f->d_rorig, q.orig_leaf));
-    CUDA_TRY_F(upload(&f->d_rgroups, q.groups));
-    CUDA_TRY_F(upload(&f->d_rtree_index, q.tree_index));
-    CUDA_TRY_F(upload(&f->d_rclass_begin, q.class_begin));
-    CUDA_TRY_F(upload(&f->d_rfeatures, q.features));
-    CUDA_TRY_F(upload(&f->d_rlut, q.lut));
-    CUDA_TRY_F(upload(&f->d_rthr, q.thresholds));
-    CUDA_TRY_F(cudaMalloc(&f->d_ties, 128));
-    CUDA_TRY_F(cudaMemset(f->d_ties, 0, 128));
+    // one block of device memory; what is small goes there in one copy
+    {
+      struct Part { void **dst; const void *src; size_t bytes, at; };
+      std::vector<Part> parts;
+      size_t total = 0;
+      auto part = [&](auto **dst, const auto &v) {
+        parts.push_back({(void **)dst, v.data(), v.size() * sizeof(v[0]), total});
+        total += (v.size() * sizeof(v[0]) + 255) / 256 * 256 + 256; // (empty vectors get an address too)
+      };
+      const std::vector<unsigned long long> zeros(16, 0);
+      part(&f->d_ties, zeros);
+      part(&f->d_rgroups, q.groups);
+      part(&f->d_rtree_index, q.tree_index);
+      part(&f->d_rclass_begin, q.class_begin);
+      part(&f->d_rfeatures, q.features);
+      part(&f->d_rlut, q.lut);
+      part(&f->d_rthr, q.thresholds);
+      const size_t small = total;
+      part(&f->d_rnode, q.node_plane);
+      part(&f->d_rleaf, q.leaf_plane);
+      part(&f->d_rorig, q.orig_leaf);
+      CUDA_TRY_F(cudaMalloc(&f->d_rank_block, total));
+      const bool together = total <= (size_t)1 << 20;
+      std::vector<unsigned char> staging(together ? total : small);
+      for (const Part &pt : parts) {
+        *pt.dst = f->d_rank_block + pt.at;
+        if (pt.at < staging.size()) {
+          if (pt.bytes) std::memcpy(staging.data() + pt.at, pt.src, pt.bytes);
+        } else {
+          CUDA_TRY_F(cudaMemcpy(*pt.dst, pt.src, pt.bytes, cudaMemcpyHostToDevice));
+        }
+      }
+      CUDA_TRY_F(cudaMemcpy(f->d_rank_block, staging.data(), staging.size(), cudaMemcpyHostToDevice));
+    }
     // of the host copy only the sizes and the feature table stay
     f->rf.num_features = q.num_features;
     f->rf.num_classes = q.num_classes;
@@ -1848,8 +1942,8 @@ int tbk_forest_free(tbk_forest *f) {
   cudaFree(f->d_orig_node);
   cudaFree(f->d_orig_off);
   cudaFree(f->d_lut);
-  cudaFreeHost(f->h_status);
-  cudaFreeHost(f->h_small);
+  pinned_pool().give_back_status(f->h_status);
+  pinned_pool().give_back(f->h_small, f->small_capacity);
   cudaFree(f->d_small_in);
   cudaFree(f->d_scratch);
   cudaFree(f->d_qnode);
@@ -1862,10 +1956,9 @@ int tbk_forest_free(tbk_forest *f) {
   cudaFree(f->d_qgroup_class);
   cudaFree(f->d_qlo);
   cudaFree(f->d_qscale);
-  cudaFree(f->d_ties);
-  for (void *d : {(void *)f->d_rnode, (void *)f->d_rleaf, (void *)f->d_rorig, (void *)f->d_rgroups, (void *)f->d_rtree_index,
-                  (void *)f->d_rclass_begin, (void *)f->d_rfeatures, (void *)f->d_rlut, (void *)f->d_rthr, (void *)f->d_lnodes, (void *)f->d_lroot,
-                  (void *)f->d_ltree_index, (void *)f->d_lorig, (void *)f->d_lclass_end})
+  if (!f->rank) cudaFree(f->d_ties);
+  cudaFree(f->d_rank_block);
+  for (void *d : {(void *)f->d_lnodes, (void *)f->d_lroot, (void *)f->d_ltree_index, (void *)f->d_lorig, (void *)f->d_lclass_end})
     cudaFree(d);
   for (auto &w : f->workspace) {
     cudaFree(w.mem);
@@ -1993,21 +2086,24 @@ int tbk_predict_host(tbk_forest *f, const float *h_rows, int64_t n_rows, int64_t
   // Chunks of about a twelfth of the batch, 4 to 32 MiB: small enough that filling and draining
   // the pipeline is a small part of the whole and that a staging slot stays in the cores' caches.
   size_t chunk_bytes = std::min<size_t>((size_t)32 << 20, std::max<size_t>((size_t)4 << 20, (size_t)n_rows * row_bytes / 12));
-  const int64_t chunk = std::max<int64_t>(1024, (int64_t)(chunk_bytes / row_bytes) / 1024 * 1024);
+  const int64_t chunk = std::min<int64_t>(std::max<int64_t>(1024, (int64_t)(chunk_bytes / row_bytes) / 1024 * 1024), (n_rows + 1023) / 1024 * 1024);
   chunk_bytes = (size_t)chunk * row_bytes;
   const bool in_pinned = is_pinned(h_rows), out_pinned = is_pinned(h_out);
   if (f->pipe_bytes < chunk_bytes || f->pipe_rows < (size_t)chunk) {
     free_pipeline(f);
+    const size_t in = (chunk_bytes + 255) / 256 * 256, res = (size_t)chunk * 4;
+    CUDA_TRY(cudaMalloc(&f->d_in[0], tbk_forest::kPipeSlots * (in + res)));
     for (int i = 0; i < tbk_forest::kPipeSlots; ++i) {
-      CUDA_TRY(cudaMalloc(&f->d_in[i], chunk_bytes));
-      CUDA_TRY(cudaMalloc(&f->d_res[i], (size_t)chunk * 4));
+      f->d_in[i] = f->d_in[0] + (size_t)i * in;
+      f->d_res[i] = f->d_in[0] + tbk_forest::kPipeSlots * in + (size_t)i * res;
     }
     f->pipe_bytes = chunk_bytes;
     f->pipe_rows = (size_t)chunk;
   }
-  for (int i = 0; i < tbk_forest::kPipeSlots; ++i) {
-    if (!in_pinned && !f->h_pin[i]) CUDA_TRY(cudaMallocHost(&f->h_pin[i], f->pipe_bytes));
-    if (!out_pinned && !f->h_res[i]) CUDA_TRY(cudaMallocHost(&f->h_res[i], f->pipe_rows * 4));
+  for (int64_t i = 0; i < std::min<int64_t>(tbk_forest::kPipeSlots, (n_rows + chunk - 1) / chunk); ++i) {
+    if (!in_pinned && !f->h_pin[i]) f->h_pin[i] = pinned_pool().take(f->pipe_bytes, &f->pin_capacity[i]);
+    if (!out_pinned && !f->h_res[i]) f->h_res[i] = pinned_pool().take(f->pipe_rows * 4, &f->res_capacity[i]);
+    if ((!in_pinned && !f->h_pin[i]) || (!out_pinned && !f->h_res[i])) return fail(TBK_ERR_CUDA, "no pinned memory for the batch");
   }
   unsigned char *out = static_cast<unsigned char *>(h_out);
   constexpr int NS = tbk_forest::kPipeSlots;
