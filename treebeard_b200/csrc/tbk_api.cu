@@ -308,7 +308,7 @@ struct tbk_forest {
   // lane layout (what is left)
   bool lanes = false;
   uint2 *d_lnodes = nullptr;
-  uint32_t *d_lroot = nullptr, *d_lclass_end = nullptr;
+  uint32_t *d_lroot = nullptr, *d_lclass_end = nullptr, *d_lclass_tree = nullptr;
   int32_t *d_ltree_index = nullptr, *d_lorig = nullptr;
   // one-tree-per-stage layout (deep trees); shares the device buffers of the key layout
   bool deep = false;
@@ -1106,22 +1106,30 @@ struct LanePlan {
 };
 
 // Enough warps for 48 on every SM, where there are that many: row tiles first, then shares of the
-// trees within a block (at least four trees each, or a class), then further chunks of them.
-LanePlan plan_lanes(const tbk_forest *f, int64_t n_rows, bool chunks_allowed) {
+// trees within a block (at least four trees each, or a class), then further chunks of them.  Batches
+// that leave most warps' places empty even so are one chain of loads: fewer trees to a share, and
+// the tiles go to as many SMs as there are (1146 rows, 25 trees of 13 levels: a call took 9.6 us
+// with 9 blocks and 6 trees in turn, 6.0 with 36 blocks and 2 trees).
+LanePlan plan_lanes(const tbk_forest *f, int64_t n_rows, bool leaf_ids) {
   const auto &pk = f->packed;
   const int64_t tiles = (n_rows + 31) / 32, wanted = std::max<int64_t>(1, 48ll * f->num_sms / tiles);
-  const int64_t parts = pk.num_classes > 0 ? pk.num_classes : std::max<int64_t>(1, pk.num_trees / 4);
+  const bool classes = pk.num_classes > 0 && !leaf_ids;
+  const int64_t parts = classes ? pk.num_classes : std::max<int64_t>(1, pk.num_trees / 4);
+  int64_t most = parts;
+  if (!classes)
+    for (int per = 2; per >= 1 && tiles * most < 16ll * f->num_sms; per /= 2) most = std::max<int64_t>(1, pk.num_trees / per);
   LanePlan p;
-  while (p.shares < 16 && p.shares < wanted && 2 * p.shares <= parts) p.shares *= 2;
-  p.tiles = (int)std::min<int64_t>(tiles, 16 / p.shares);
+  while (p.shares < 16 && p.shares < wanted && 2 * p.shares <= most) p.shares *= 2;
+  if (classes && p.shares < wanted) p.shares = (int)std::min<int64_t>({16, wanted, most}); // (a class each, where they fit)
+  p.tiles = (int)std::min<int64_t>(std::max<int64_t>(1, tiles / f->num_sms), 16 / p.shares);
   auto bytes = [&] { return p.tiles * (pk.num_features + 1) * 128 + p.tiles * p.shares * 256; };
   while (p.tiles > 1 && bytes() > 48 * 1024) --p.tiles;
   p.smem = bytes();
   p.grid_x = (tiles + p.tiles - 1) / p.tiles;
-  if (chunks_allowed) {
-    p.chunks = (int)std::min({(wanted + p.shares - 1) / p.shares, std::max<int64_t>(1, parts / p.shares), (int64_t)64});
-    if (f->user.tree_chunks > 0) p.chunks = (int)std::min<int64_t>(f->user.tree_chunks, std::max<int64_t>(1, pk.num_trees / p.shares));
-  }
+  // (chunks of a multiclass forest take a part of every class each)
+  const int64_t chunks = classes ? pk.num_trees / pk.num_classes / 4 : (parts >= 2 * p.shares ? most : parts) / p.shares;
+  p.chunks = (int)std::min({(wanted + p.shares - 1) / p.shares, std::max<int64_t>(1, chunks), (int64_t)64});
+  if (f->user.tree_chunks > 0 && !classes) p.chunks = (int)std::min<int64_t>(f->user.tree_chunks, std::max<int64_t>(1, pk.num_trees / p.shares));
   return p;
 }
 
@@ -1143,7 +1151,8 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   const int W = std::max(1, pk.num_classes);
   const bool classes = pk.num_classes > 0;
   // (a chunk of a host batch is walked in the shape of the whole batch, see run)
-  LanePlan plan = plan_lanes(f, std::max(n_rows, f->host_batch_rows), !classes || mode == kLeafIds);
+  LanePlan plan = plan_lanes(f, std::max(n_rows, f->host_batch_rows), mode == kLeafIds);
+  if (fixed && classes) plan.chunks = (int)std::max<int64_t>(1, std::min<int64_t>(plan.chunks, (int64_t)fixed_floats / (n_rows * W)));
   plan.grid_x = ((n_rows + 31) / 32 + plan.tiles - 1) / plan.tiles;
   f->last_plan = lane_launch_plan(plan);
   const bool second_pass = fixed != nullptr || (mode != kLeafIds && plan.chunks > 1);
@@ -1156,7 +1165,7 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
                   "scratch holds %zu; split the batch or use tbk_predict", (long long)n_rows, plan.chunks, W,
                   (size_t)plan.chunks * n_rows * W, fixed_floats);
   } else if (second_pass) {
-    const size_t need = ((size_t)plan.chunks * n_rows * sizeof(float) + 255) & ~(size_t)255;
+    const size_t need = ((size_t)plan.chunks * n_rows * W * sizeof(float) + 255) & ~(size_t)255;
     int rc = ensure_scratch(f, 2 * need);
     if (rc) return rc;
     partial = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(f->d_scratch) + (size_t)slot * (f->scratch_bytes / 2));
@@ -1170,6 +1179,7 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   p.tree_index = f->d_ltree_index;
   p.orig_node = f->d_lorig;
   p.class_end = f->d_lclass_end;
+  p.class_tree = f->d_lclass_tree;
   p.rows = d_rows;
   p.n_rows = n_rows;
   p.ld = ld;
@@ -1198,7 +1208,7 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   if (second_pass) {
     const int tpb = 256;
     if (mode == kPartial)
-      tb::tb_sum_partials_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(partial, plan.chunks, n_rows, d_partial);
+      tb::tb_sum_partials_kernel<<<(unsigned)((n_rows * W + tpb - 1) / tpb), tpb, 0, stream>>>(partial, plan.chunks, n_rows * W, d_partial);
     else
       tb::tb_finalize_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(
           partial, plan.chunks, n_rows, W, pk.num_classes, (float)pk.initial_value, pk.transform, d_out, out_kind);
@@ -1767,7 +1777,10 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     CUDA_TRY_F(upload(&f->d_ltree_index, q.tree_index));
     CUDA_TRY_F(upload(&f->d_lorig, q.orig_node));
     CUDA_TRY_F(upload(&f->d_lclass_end, q.class_end));
-    f->last_plan = lane_launch_plan(plan_lanes(f, batch_hint > 0 ? batch_hint : 65536, q.num_classes == 0));
+    std::vector<uint32_t> class_tree; // (end of every class's trees)
+    for (uint32_t end : q.class_end) class_tree.push_back((uint32_t)(std::lower_bound(q.root.begin(), q.root.end(), end) - q.root.begin()));
+    CUDA_TRY_F(upload(&f->d_lclass_tree, class_tree));
+    f->last_plan = lane_launch_plan(plan_lanes(f, batch_hint > 0 ? batch_hint : 65536, false));
     *out = f;
     return TBK_OK;
   }
@@ -1958,7 +1971,7 @@ int tbk_forest_free(tbk_forest *f) {
   cudaFree(f->d_qscale);
   if (!f->rank) cudaFree(f->d_ties);
   cudaFree(f->d_rank_block);
-  for (void *d : {(void *)f->d_lnodes, (void *)f->d_lroot, (void *)f->d_ltree_index, (void *)f->d_lorig, (void *)f->d_lclass_end})
+  for (void *d : {(void *)f->d_lnodes, (void *)f->d_lroot, (void *)f->d_ltree_index, (void *)f->d_lorig, (void *)f->d_lclass_end, (void *)f->d_lclass_tree})
     cudaFree(d);
   for (auto &w : f->workspace) {
     cudaFree(w.mem);

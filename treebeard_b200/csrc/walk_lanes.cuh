@@ -8,8 +8,9 @@
 // A warp = 32 rows and one of `shares` ranges of the trees; the row tile (transposed, bank = row) is
 // shared by the warps that split the trees, and their sums meet in shared memory in share order.
 // The kernel is bound by the latency of the nodes' gathers, so blocks are small and many fit an SM:
-// the trees being walked stay in L1.  blockIdx.y splits the trees further for small batches; a second
-// kernel adds those partial sums (walk_kernels.cuh).
+// the trees being walked stay in L1.  blockIdx.y splits the trees further for small batches, those of
+// every class alike (3000 rows, 3 classes of 30 trees: 50.2 us with whole classes to a warp, 22.6 so); a
+// second kernel adds those partial sums (walk_kernels.cuh).
 //
 // Reference counterparts: the scalar walk that stops at a leaf, src/mlir/CodeGenStateMachine.cpp:
 // 149-243; the tie rule of class ids, src/reduction/LowerReduceOps.cpp:148-189.
@@ -23,10 +24,11 @@ struct LaneParams {
   const uint32_t *root;       // [num_trees + 1]
   const int32_t *tree_index;
   const int32_t *orig_node;
-  const uint32_t *class_end;  // multiclass
+  const uint32_t *class_end;  // multiclass: end of every class's nodes, of its trees
+  const uint32_t *class_tree;
   const float *rows;
   long long n_rows, ld;
-  float *partial;             // write_partial: [chunks][n_rows], or [n_rows][classes]
+  float *partial;             // write_partial: [chunks][n_rows], or [chunks][n_rows][classes]
   void *out;
   int32_t *leaf_ids;
   long long num_trees;
@@ -36,10 +38,13 @@ struct LaneParams {
   int32_t vec4_ok;
 };
 
+// all * i / n in 32 bits (n: at most 1024)
+__device__ __forceinline__ uint32_t lane_share(uint32_t all, uint32_t i, uint32_t n) { return all / n * i + all % n * i / n; }
+
 // Where part `i` of `n` of the trees begins; parts of a multiclass forest are whole classes.
-__device__ __forceinline__ uint32_t lane_part(const LaneParams &p, int i, int n) {
-  if (p.num_classes == 0) return p.root[p.num_trees * i / n];
-  const int c = (int)((long long)p.num_classes * i / n);
+template <bool WHOLE_CLASSES> __device__ __forceinline__ uint32_t lane_part(const LaneParams &p, uint32_t i, uint32_t n) {
+  if constexpr (!WHOLE_CLASSES) return p.root[lane_share((uint32_t)p.num_trees, i, n)];
+  const uint32_t c = lane_share((uint32_t)p.num_classes, i, n);
   return c == 0 ? 0u : p.class_end[c - 1];
 }
 
@@ -70,17 +75,36 @@ __global__ void __launch_bounds__(512) tb_walk_lanes_kernel(const LaneParams p) 
   }
   __syncthreads();
 
-  const int part = (int)blockIdx.y * p.shares + share, parts = (int)gridDim.y * p.shares;
-  uint32_t n = lane_part(p, part, parts);
-  const uint32_t end = lane_part(p, part + 1, parts);
+  constexpr bool WHOLE_CLASSES = CLASSES && !LEAF_IDS;
+  const int part = WHOLE_CLASSES ? share : (int)blockIdx.y * p.shares + share;
+  const int parts = WHOLE_CLASSES ? p.shares : (int)gridDim.y * p.shares;
+  uint32_t n = lane_part<WHOLE_CLASSES>(p, part, parts);
+  const uint32_t end = lane_part<WHOLE_CLASSES>(p, part + 1, parts);
   const float *mine = xs + lane;
   float acc = 0.f;
   [[maybe_unused]] float best = -INFINITY;
   [[maybe_unused]] int cls = 0, best_class = 0, last_class = 0;
   [[maybe_unused]] uint32_t class_end = 0, tree = 0;
-  if constexpr (CLASSES) {
-    cls = (int)((long long)p.num_classes * part / parts);
-    last_class = (int)((long long)p.num_classes * (part + 1) / parts);
+  if constexpr (WHOLE_CLASSES) {
+    cls = (int)lane_share(p.num_classes, part, parts);
+    last_class = (int)lane_share(p.num_classes, part + 1, parts);
+    if (gridDim.y > 1) { // this block's part of every class
+      for (; cls < last_class; ++cls) {
+        const uint32_t a = cls > 0 ? p.class_tree[cls - 1] : 0u, trees = p.class_tree[cls] - a;
+        const uint32_t stop = p.root[a + lane_share(trees, blockIdx.y + 1, gridDim.y)];
+        acc = 0.f;
+        for (n = p.root[a + lane_share(trees, blockIdx.y, gridDim.y)]; n < stop;) {
+          const uint2 node = __ldg(p.nodes + n);
+          const uint32_t f = node.y & 0xffffu;
+          const float t = __uint_as_float(node.x), x = mine[f * 32];
+          const bool leaf = f == (uint32_t)F;
+          acc += leaf ? t : 0.f;
+          n += (node.y >> 16) + (x < t || leaf ? 0u : 1u);
+        }
+        if (live) p.partial[((long long)blockIdx.y * p.n_rows + row) * p.num_classes + cls] = acc;
+      }
+      return;
+    }
     class_end = cls < last_class ? p.class_end[cls] : end;
   }
   // the sum of class `cls` is complete (ties go to the higher class)
@@ -104,7 +128,7 @@ __global__ void __launch_bounds__(512) tb_walk_lanes_kernel(const LaneParams p) 
     tree = lo;
   }
   while (n < end) {
-    if constexpr (CLASSES && !LEAF_IDS)
+    if constexpr (WHOLE_CLASSES)
       while (n >= class_end) close();
     const uint2 node = __ldg(p.nodes + n);
     const uint32_t f = node.y & 0xffffu;
@@ -122,7 +146,7 @@ __global__ void __launch_bounds__(512) tb_walk_lanes_kernel(const LaneParams p) 
   }
   if constexpr (LEAF_IDS) return;
   if constexpr (CLASSES) {
-    const bool empty = (int)((long long)p.num_classes * part / parts) == last_class; // (a part without classes wins nothing)
+    const bool empty = (int)lane_share(p.num_classes, part, parts) == last_class; // (a part without classes wins nothing)
     while (cls < last_class) close();
     if (p.write_partial) return;
     sums[(2 * warp) * 32 + lane] = empty ? __int_as_float(0x7fffffff) : best;
