@@ -84,14 +84,15 @@ typedef struct tbk_schedule {
                               async copies, 2 = read nodes from global memory,
                               0 = auto */
   int32_t feature_bits;    /* how rows are staged in shared memory: 32 = fp32 values,
-                              16 = order-preserving 15/16-bit keys with exact fp32 tie
-                              resolution (leaf selection stays bit-exact): single-output
-                              forests of at most 12 levels; multiclass forests of at most
-                              8 levels over narrow rows (walked in one tree chunk),
+                              16 = order-preserving 15/16-bit keys -- a value's rank among
+                              its feature's thresholds, or rounded values with exact fp32
+                              tie resolution (leaf selection is bit-exact either way):
+                              single-output forests of at most 12 levels; multiclass
+                              forests of at most 8 levels over narrow rows,
                               0 = auto: with representation TBK_REP_AUTO keys for these
-                              forests unless most thresholds are whole numbers that cannot
-                              become lattice features (integer-valued features then tie
-                              all the time), fp32 otherwise */
+                              forests (rounded ones only unless most thresholds are whole
+                              numbers that cannot become lattice features: integer-valued
+                              features then tie all the time), fp32 otherwise */
   int32_t reserved[4];
 } tbk_schedule;
 
@@ -196,8 +197,9 @@ TBK_EXPORT int tbk_predict_host(tbk_forest *forest, const float *h_rows, int64_t
  *     streams, or different forests) race on it.  Serialise them.  Nothing in it needs
  *     clearing between calls: every element read by the second pass is written by the walk
  *     of the same call.
- *   - Forests in a 16-bit key layout (wide rows, deep trees) are not covered
- *     (TBK_ERR_UNSUPPORTED). */
+ *   - Forests of rank keys hold their keys in the array too and take large batches in several
+ *     passes, without a limit.  Of the rounded 16-bit key layouts (deep trees, wide rows) only rows
+ *     that an fp32 tile could hold as well are covered, the rest is TBK_ERR_UNSUPPORTED. */
 TBK_EXPORT int tbk_predict_noalloc(tbk_forest *forest, const float *d_rows, int64_t n_rows, int64_t ld,
                                    void *d_out, int32_t out_kind, void *stream);
 

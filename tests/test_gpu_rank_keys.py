@@ -91,3 +91,20 @@ def test_rank_keys_on_several_streams_and_in_a_graph():
     torch.cuda.synchronize()
     assert torch.equal(out, want[0]) and torch.equal(other, want[1])
     df.check_status()
+
+
+@pytest.mark.parametrize("trees,levels,features,classes,rows", [
+    (33, 6, 20, 0, 1), (97, 8, 64, 0, 70001), (140, 8, 300, 0, 9003), (60, 6, 16, 5, 30011), (40, 6, 700, 0, 1005)])
+def test_the_call_that_may_not_allocate(trees, levels, features, classes, rows):
+    f, marg = _forest(trees, levels, features, classes)
+    dX = torch.from_numpy(_rows(f, marg, rows)).cuda()
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows)
+    want, out = df.predict(dX), torch.empty(rows, device="cuda")
+    for _ in range(2):
+        kernels._check(kernels.lib().tbk_predict_noalloc(df._h, dX.data_ptr(), rows, features, out.data_ptr(), kernels.OUT_F32,
+                                                         torch.cuda.current_stream().cuda_stream))
+        df.check_status()
+        if classes:
+            assert (out == want).float().mean() > 0.999   # (other tree chunks: near-ties may fall either way)
+        else:
+            assert_predictions_close(out.cpu().numpy(), want.cpu().numpy())

@@ -417,7 +417,7 @@ int quant_batch_tiles(const tbk_forest *f, int num_features) {
 // time go to the batch kernel (persistent blocks of 22 warps over batches of up to 16 tiles),
 // wide rows to the kernel that holds one tile (persistent blocks of 24 warps over tiles of 32 rows).
 int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out, int32_t out_kind,
-              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot) {
+              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot, float *fixed = nullptr, size_t fixed_floats = 0) {
   const auto &q = f->qf;
   const int64_t G = (int64_t)q.groups.size();
   const int64_t tiles = (n_rows + 31) / 32;
@@ -443,6 +443,7 @@ int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   // on 4 096 rows x 32 groups: 38 us in one chunk, 47 us in two -- unless the caller asks)
   const int64_t max_chunks = !batched ? G : f->user.tree_chunks > 0 ? std::max<int64_t>(1, G / 2) : std::max<int64_t>(1, G / 32);
   chunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(chunks, max_chunks), 65535));
+  if (fixed) chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, (int64_t)fixed_floats / n_rows));
   const int gpc = (int)((G + chunks - 1) / chunks);
   chunks = (G + gpc - 1) / gpc;
   const bool vec4 = q.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0;
@@ -471,6 +472,8 @@ int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   if (need_partials) {
     if (mode == kPartial && chunks == 1) {
       partial_dst = d_partial;
+    } else if (fixed) {
+      partial_dst = fixed;
     } else {
       const size_t need = ((size_t)chunks * n_rows * sizeof(float) + 255) & ~(size_t)255;
       int rc = ensure_scratch(f, 2 * need);
@@ -994,8 +997,9 @@ void plan_rank_tables(tbk_forest *f) {
   }
 }
 
+// fixed: keys and partial sums go to this memory, in as many passes as that takes (tbk_predict_noalloc).
 int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out, int32_t out_kind,
-             float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream) {
+             float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, unsigned char *fixed = nullptr, size_t fixed_bytes = 0) {
   const auto &q = f->rf;
   const int S = rank_stride(q.num_features), W = std::max(1, q.num_classes);
   const int kmode = mode == kLeafIds ? tb::kRankLeafIds : q.num_classes > 0 ? tb::kRankClasses : tb::kRankSums;
@@ -1005,11 +1009,18 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * 64); // (units of at least 80 rows)
     plan = plan_rank(f, pass, mode == kLeafIds);
   }
+  while (fixed && rank_workspace_bytes(f, plan, pass) > fixed_bytes) { // (128 rows always fit)
+    pass = std::max<int64_t>(128, pass / 256 * 128);
+    plan = plan_rank(f, pass, mode == kLeafIds);
+  }
   f->last_plan = rank_launch_plan(plan);
   tbk_forest::Workspace *ws = nullptr;
-  int rc = workspace_acquire(f, stream, rank_workspace_bytes(f, plan, pass), &ws);
+  int rc = TBK_OK;
+  if (fixed) CUDA_TRY(cudaMemsetAsync(fixed, 0, tb::kRankArrivalBytes, stream)); // (others write it too)
+  else rc = workspace_acquire(f, stream, rank_workspace_bytes(f, plan, pass), &ws);
   if (rc) return rc;
-  unsigned char *keys = ws->mem + tb::kRankArrivalBytes;
+  unsigned char *const mem = fixed ? fixed : ws->mem;
+  unsigned char *keys = mem + tb::kRankArrivalBytes;
   // one unit of rows per block: the variant for small batches, with only as many walker warps as
   // the rows -- or ranking them with two values per thread -- can use
   const bool tiled = rank_tiled(q.num_features), small = !tiled && plan.units == 1;
@@ -1030,7 +1041,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   p.class_begin = f->d_rclass_begin;
   p.keys = keys;
   p.scratch = reinterpret_cast<float *>(keys + rank_key_bytes(f, pass));
-  p.arrivals = reinterpret_cast<unsigned int *>(ws->mem);
+  p.arrivals = reinterpret_cast<unsigned int *>(mem);
   p.num_trees = q.num_trees;
   p.num_groups = (int32_t)q.groups.size();
   p.groups_per_chunk = kmode == tb::kRankClasses ? 0 : plan.per_chunk;
@@ -1093,7 +1104,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     CUDA_TRY(cudaEventRecord(f->ev1, stream));
     f->ev_pending = true;
   }
-  if (ws->done) CUDA_TRY(cudaEventRecord(ws->done, stream)); // (uses are marked)
+  if (ws && ws->done) CUDA_TRY(cudaEventRecord(ws->done, stream)); // (uses are marked)
   return TBK_OK;
 }
 
@@ -2266,7 +2277,9 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   if (!f) return fail(TBK_ERR_INVALID, "null forest");
   std::lock_guard<std::mutex> lock(f->mu);
   const auto &pk = f->packed;
-  if (f->rank || f->quant || f->deep) return fail(TBK_ERR_UNSUPPORTED, "tbk_predict_noalloc does not cover the 16-bit key layouts");
+  // (of the rounded keys only rows that an fp32 tile could hold too)
+  const bool wide = f->quant && quant_batch_tiles(f, pk.num_features) == 0 && (int64_t)(pk.num_features + 1) * 128 + 1024 <= f->max_smem_optin;
+  if ((f->quant && !wide) || f->deep) return fail(TBK_ERR_UNSUPPORTED, "tbk_predict_noalloc does not cover the rounded 16-bit key layouts");
   if (n_rows < 0 || ld < pk.num_features) return fail(TBK_ERR_INVALID, "ld (%lld) is smaller than the row size (%d)", (long long)ld, pk.num_features);
   if (n_rows == 0) return TBK_OK;
   if (!d_rows || !d_out) return fail(TBK_ERR_INVALID, "null pointer");
@@ -2277,6 +2290,11 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   float *scratch = nullptr;
   int rc = noalloc_scratch_address(f->device, &scratch);
   if (rc != TBK_OK) return rc;
+  if (f->rank)
+    return run_rank(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, reinterpret_cast<unsigned char *>(scratch),
+                    kNoAllocScratchFloats * sizeof(float));
+  if (f->quant)
+    return run_quant(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, 0, scratch, kNoAllocScratchFloats);
   if (f->lanes)
     return run_lanes(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, 0, scratch, kNoAllocScratchFloats);
 
