@@ -564,8 +564,8 @@ int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
 bool deep_plan(int num_features, int max_depth, int smem_limit, int *row_warps, int *slots) {
   const int64_t slot = 4ll * tb::deep_tree_words((uint32_t)std::max(max_depth, tb::kDeepMinDepth));
   // four slots hold the node planes of the pair being walked and of the next one
-  for (int rw = 30; rw >= 4; rw -= 2) { // (the block has one more warp, the ring producer)
-    const int64_t keys = (int64_t)num_features * 64 * rw;
+  for (int rw = 30; rw >= 2; rw -= 2) { // (the block has one more warp, the ring producer)
+    const int64_t keys = ((int64_t)num_features * 64 + tb::kDeepLeafBytes) * rw;
     const int64_t room = (int64_t)smem_limit - 128 - keys;
     const int64_t s = std::min<int64_t>(tb::kDeepMaxSlots, room / slot);
     if (s >= 4) {
@@ -578,7 +578,7 @@ bool deep_plan(int num_features, int max_depth, int smem_limit, int *row_warps, 
 }
 int deep_smem_bytes(const tbk_forest *f) {
   return 128 + f->deep_slots * 4 * (int)tb::deep_tree_words((uint32_t)std::max(f->df.max_depth, tb::kDeepMinDepth)) +
-         f->df.num_features * 64 * f->deep_row_warps;
+         (f->df.num_features * 64 + tb::kDeepLeafBytes) * f->deep_row_warps;
 }
 
 template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb::DeepParams) {
@@ -598,7 +598,7 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   // full as the others, and small batches still cover the SMs
   int rw = f->deep_row_warps;
   const int64_t row_tiles = (n_rows + 31) / 32, waves = (row_tiles + (int64_t)rw * f->num_sms - 1) / ((int64_t)rw * f->num_sms);
-  rw = std::max(4, (int)((row_tiles + waves * f->num_sms - 1) / (waves * f->num_sms)));
+  rw = std::max(std::min(4, rw), (int)((row_tiles + waves * f->num_sms - 1) / (waves * f->num_sms)));
   const int64_t rows_per_block = 32 * rw;
   const int64_t grid_x = (n_rows + rows_per_block - 1) / rows_per_block;
   int64_t chunks = 1;
@@ -663,6 +663,7 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   p.slot_bytes = plan.stage_bytes;
   p.tree_words = plan.stage_bytes / 4;
   p.key_tile = 128u * (uint32_t)q.num_features;
+  p.leaf_off = (uint32_t)(plan.smem_bytes - tb::kDeepLeafBytes * f->deep_row_warps);
   p.status = f->d_status;
   p.tie_count = f->d_ties;
   p.skip_first_copy = f->expire_next_wait ? 1 : 0;

@@ -8,16 +8,24 @@
 // issues, the next pair's always in flight while a pair is walked; a row warp frees a slot
 // with one arrival on the slot's "empty" mbarrier and the producer refills it when all row
 // warps have arrived, so the row warps never meet at a block barrier and may drift apart by a
-// pair.  Leaf values are read straight from L2 (32 scattered
-// sectors per warp whatever the layout) and consumed one pair later.  Sums stay in the
+// pair.  Leaf values come straight from L2 (32 scattered
+// sectors per warp whatever the layout) and are consumed one pair later.  Sums stay in the
 // owning thread's register: there is no cross-thread reduction.
+//
+// The kernel is bound by latency: shared-memory pipe 57 % and issue 47 % busy while leaf values
+// were loaded into registers, and a warp that stops for anything but its two chains stops the
+// others two pairs later.  So nothing in the loop waits for global memory: leaf values are copied to
+// shared memory asynchronously (as loads, every pair waited some 600 of 2970 clocks for them, however
+// far ahead they were issued), and a tree behind a key tie is put off until the row's other
+// trees are done.  1048576 rows x 2000 trees of 12 levels over 128 features: 17.65 -> 16.0 ms; either
+// change without the other gains nothing.
 //
 // Every two row warps have a key tile of their own (128 bytes per feature: word j = row j of the even
 // warp | row j of the odd warp << 16), so a warp's key load touches 32 distinct banks and the
 // upper half of a node word -- the byte offset of the feature's line -- is one shift-add away from
 // the key's address.  The in-order numbering of deep_pack.h makes a right turn one addition that
 // depends on the level alone.  A key tie is only flagged on the fast path; the flagged (row, tree) is
-// re-walked with exact fp32 comparisons at the tied steps.
+// walked again at the end, with exact fp32 comparisons at the tied steps.
 //
 // Reference counterparts: src/mlir/CodeGenStateMachine.cpp:149-243 (scalar walk),
 // src/mlir/WalkDecisionTreeLoweringPass.cpp:24-53 (fixed-depth walk of padded trees),
@@ -49,6 +57,7 @@ struct DeepParams {
   uint32_t slot_bytes; // of a tree of the forest's depth
   uint32_t tree_words; // the same in words
   uint32_t key_tile;   // bytes of the key tile of two row warps
+  uint32_t leaf_off;   // where the leaf values on their way are in shared memory
   int32_t *status;
   unsigned long long *tie_count;
   int32_t skip_first_copy; // failure drill: the first piece's copy is never issued, so its wait expires
@@ -56,6 +65,8 @@ struct DeepParams {
 };
 
 constexpr int kDeepMaxSlots = 8;
+constexpr uint32_t kDeepNoLeaf = 0xffffffffu;
+constexpr int kDeepLeafBytes = 512; // per row warp: the leaf values of two pairs
 
 // Fast walk of DEPTH levels of two trees in lock-step, in PTX (the step of walk_quant.cuh: keys
 // are 15-bit integers that compare as fp16 numbers, so one half2 comparison of (key, node word)
@@ -141,12 +152,13 @@ __device__ __forceinline__ void deep_walk_any(uint32_t depth, uint32_t base0, ui
 
 // Re-walk of one (row, tree) behind a key tie: the staged keys decide wherever they can,
 // the tied comparisons read the exact fp32 values from global memory.  Returns the leaf position.
-__device__ __noinline__ uint32_t deep_walk_exact(uint32_t base, uint32_t key_lane, bool wide, uint32_t depth,
+// `nodes`: the tree in global memory, or null to read it from the ring at `base`.
+__device__ __noinline__ uint32_t deep_walk_exact(uint32_t base, const uint32_t *nodes, uint32_t key_lane, bool wide, uint32_t depth,
                                                  const float *exact_tree, const float *rowp) {
   uint32_t at = 0;
   for (uint32_t d = 0; d < depth; ++d) {
     const uint32_t x = 1u << (depth - 1 - d), step = x + (x >> 5) + (x >> 10); // (deep_position)
-    const uint32_t node = lds_u32(base + (at + step) * 4u);
+    const uint32_t node = nodes ? __ldg(nodes + at + step) : lds_u32(base + (at + step) * 4u);
     const uint32_t f = wide ? node >> 16 : node >> 23, kt = node & 0x7fffu;
     const uint32_t kx = lds_u16(key_lane + f * 128u);
     bool right = kx < kt;
@@ -155,6 +167,13 @@ __device__ __noinline__ uint32_t deep_walk_exact(uint32_t base, uint32_t key_lan
   }
   return at;
 }
+
+// A word from global to shared memory behind the thread's back, and the wait for all such copies.
+__device__ __forceinline__ void copy_word(uint32_t dst, const float *src, bool read) { // (zero without reading otherwise)
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(read ? 4u : 0u) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void sts_f32(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
 // UD: depth shared by every pair of the forest (0 = mixed, decided per pair at run time).
 // LEAF_IDS: the launch records leaf ids instead of predictions.
@@ -240,7 +259,14 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   // thousands of leaf values per row: a double accumulator keeps the sum within the
   // fp32 rounding of the exact result (one conversion and one add per tree)
   double acc = 0.0;
-  float pend0 = 0.f, pend1 = 0.f; // leaf values of the previous pair, on their way from L2
+  // leaf values of the last pair on their way from L2, two words of this thread for each parity of a pair
+  [[maybe_unused]] const uint32_t leaf_s = smem_u32(smem_raw) + p.leaf_off + (uint32_t)warp * kDeepLeafBytes + (uint32_t)lane * 4u;
+  if constexpr (!LEAF_IDS) {
+    sts_f32(leaf_s + 256u, 0.f);
+    sts_f32(leaf_s + 384u, 0.f);
+  }
+  // trees behind a key tie: up to four numbers (plus one) of 16 bits, walked after all others
+  [[maybe_unused]] unsigned long long tied = 0;
   bool ok = true;
   unsigned ties = 0;
   int slot = 0;          // ring slot of the next piece to consume
@@ -279,27 +305,30 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
         deep_walk<UD, WIDE>(n0, n1, key_lane, &j0, &j1, &t0, &t1);
       else
         deep_walk_any<WIDE>(depth, n0, n1, key_lane, &j0, &j1, &t0, &t1);
-      if (t0) {
-        j0 = deep_walk_exact(n0, key_lane, WIDE, depth, p.exact_plane + gm.elem_off, rowp);
+      // a tied tree waits for the end, where it holds up nobody; beyond four it is walked here
+      auto resolve = [&](bool tie, int c, uint32_t base, uint32_t &at) {
+        if (!tie) return;
         ++ties;
-      }
-      if (t1) {
-        j1 = deep_walk_exact(n1, key_lane, WIDE, depth, p.exact_plane + gm.elem_off + gm.slots, rowp);
-        ++ties;
-      }
+        const uint32_t number = 2u * (uint32_t)k + (uint32_t)c + 1u;
+        if (!LEAF_IDS && tied >> 48 == 0 && number < 65536u) {
+          tied = tied << 16 | number;
+          at = kDeepNoLeaf;
+        } else {
+          at = deep_walk_exact(base, nullptr, key_lane, WIDE, depth, p.exact_plane + gm.elem_off + (c ? gm.slots : 0u), rowp);
+        }
+      };
+      resolve(t0, 0, n0, j0);
+      resolve(t1, 1, n1, j1);
     }
-    // The two leaf values come straight from L2 and are consumed one pair later: a warp's
-    // 32 leaves are scattered over the leaf plane (one sector each), which moves the same
-    // bytes as staging the plane would, without taking ring slots.
+    // a warp's 32 leaves are scattered over the leaf plane (one sector each), which moves the same
+    // bytes as staging the plane would, without taking ring slots
     if (ok) {
       if (!LEAF_IDS) {
-        // (tied to the walk's end by a condition that is never met: scheduled in front of the walk,
-        // the additions would wait for the loads)
-        asm volatile("{\n .reg .pred p;\n setp.eq.u32 p, %2, 0xffffffff;\n @p mov.f32 %0, 0f00000000;\n @p mov.f32 %1, 0f00000000;\n}"
-                     : "+f"(pend0), "+f"(pend1) : "r"(j0 & j1));
-        acc += (double)pend0 + (double)pend1;
-        pend0 = __ldg(p.leaf_plane + gm.elem_off + j0);
-        pend1 = __ldg(p.leaf_plane + gm.elem_off + gm.slots + j1);
+        const uint32_t here = leaf_s + ((uint32_t)k & 1u) * 256u, last = leaf_s + ((uint32_t)(k + 1) & 1u) * 256u;
+        copies_wait();
+        acc += (double)lds_f32(last) + (double)lds_f32(last + 128u);
+        copy_word(here, p.leaf_plane + gm.elem_off + (j0 == kDeepNoLeaf ? 0u : j0), j0 != kDeepNoLeaf);
+        copy_word(here + 128u, p.leaf_plane + gm.elem_off + gm.slots + (j1 == kDeepNoLeaf ? 0u : j1), j1 != kDeepNoLeaf);
       }
       if (LEAF_IDS && live) {
         const int t0 = p.tree_index[(g0 + k) * 2], t1 = p.tree_index[(g0 + k) * 2 + 1];
@@ -317,10 +346,21 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   // every wait above is bounded: a wait that gave up ends the launch with a status word
   const bool failed = __syncthreads_or(!ok) != 0;
   if (failed) {
+    copies_wait();
     if (tid == 0) set_status(p.status, 4);
     return;
   }
-  acc += (double)pend0 + (double)pend1;
+  if constexpr (!LEAF_IDS) {
+    const uint32_t last = leaf_s + ((uint32_t)(g1 - g0 + 1) & 1u) * 256u;
+    copies_wait();
+    acc += (double)lds_f32(last) + (double)lds_f32(last + 128u);
+    for (; tied; tied >>= 16) {
+      const uint32_t number = (uint32_t)(tied & 0xffff) - 1u;
+      const DevQuantGroup gm = p.pairs[g0 + (int)(number >> 1)];
+      const unsigned long long off = gm.elem_off + (number & 1u ? gm.slots : 0u);
+      acc += (double)__ldg(p.leaf_plane + off + deep_walk_exact(0, p.node_plane + off, key_lane, WIDE, gm.depth, p.exact_plane + off, rowp));
+    }
+  }
   if (p.tie_count != nullptr && ties) atomicAdd(p.tie_count, (unsigned long long)ties);
   if (LEAF_IDS || !live) return;
   if (p.write_partial)
