@@ -31,15 +31,15 @@ from treebeard_b200 import synth  # noqa: E402
 
 HBM_FALLBACK_GBS = 6650.0
 
-# DRAM bytes per row (dram__bytes_read.sum + dram__bytes_write.sum) of the walk kernel, from
-# one ncu capture per workload on a reduced batch (see profiles/); traffic grows in
+# DRAM bytes per row (dram__bytes_read.sum + dram__bytes_write.sum) of the walk kernel (c2, c4: of the
+# ranking kernel as well), from one ncu capture per workload on the full or a reduced batch (see profiles/); traffic grows in
 # proportion to the rows, so a launch's traffic is this figure times its rows.  Each figure
 # belongs to the kernel sources it was captured on: it is reported only while the hash of the
 # code of the headers that make up the workload's kernel (kernel_source_hash) still matches.
 KERNEL_SOURCES = {"c3": ("walk_kernels.cuh", "walk_quant.cuh"),
-                  "c2": ("walk_kernels.cuh", "walk_quant.cuh", "walk_quant_batch.cuh"),
-                  "c4": ("walk_kernels.cuh", "walk_quant.cuh", "walk_quant_batch.cuh")}
-NCU_DRAM_BYTES_PER_ROW = {"c3": (8718.9, "9818290bfb5d6a18"), "c2": (131.6, "e10befea55613438"), "c4": (106.9, "e10befea55613438")}
+                  "c2": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh"),
+                  "c4": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh")}
+NCU_DRAM_BYTES_PER_ROW = {"c3": (8718.4, "72392cc6b65e063e"), "c2": (235.0, "2ebf250b07a70edb"), "c4": (146.5, "2ebf250b07a70edb")}
 
 
 def kernel_source_hash(workload):
@@ -65,7 +65,7 @@ def ncu_traffic(workload, n_rows, custom):
     now = kernel_source_hash(workload)
     if captured_on != now:
         return None, f"kernel sources changed since the ncu capture (captured on {captured_on or 'an earlier build'}, now {now})"
-    return per_row * n_rows, "ncu dram bytes per row on a reduced batch x rows (profiles/)"
+    return per_row * n_rows, "ncu dram bytes per row x rows (profiles/)"
 
 
 def bytes_per_row(cfg):
