@@ -245,6 +245,13 @@ struct RankPlan {
   int64_t grid_x = 1;
 };
 
+// How a batch is cut for the deep-tree kernel: blocks of 32 x row_warps rows, the first `whole` of them
+// over all trees and the rest over `chunks` ranges of them.
+struct DeepSplit {
+  int64_t n_rows = -1, whole = 0;
+  int row_warps = 0, chunks = 1;
+};
+
 struct tbk_forest {
   tb::PackedForest packed; // host copy (orig_node kept for lazy upload)
   int device = 0;
@@ -314,6 +321,7 @@ struct tbk_forest {
   bool deep = false;
   tb::DeepForest df;
   int deep_row_warps = 0, deep_slots = 0;
+  DeepSplit deep_split;
   int uniform_depth = 0; // key layouts: depth shared by all groups / pairs, 0 = mixed
   // host pipeline: slots of device buffers and pinned staging that a large batch streams through,
   // and one pinned buffer that the kernels read and write directly for small batches
@@ -589,21 +597,43 @@ template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb:
              : (ids ? tb::tb_walk_deep_kernel<1024, 0, WIDE, true> : tb::tb_walk_deep_kernel<1024, 0, WIDE, false>);
 }
 
-// One prediction with the deep-tree kernel (one block per 32 x row_warps rows).
-int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
-             float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot) {
+// A pair of trees takes a block about the same time whatever its row warps (12 to 20: 1.42 to 1.57 ms
+// a thousand pairs), so what counts is the waves of blocks.  The blocks that fill no whole wave
+// split the trees, into as many ranges as leave the least of their last wave empty.  A block stages its
+// rows for about the time of 12 pairs, the second pass over partial sums takes that of 8.
+// (1048576 rows, 2000 trees, 18 row warps: 12.3 waves of blocks; 8000 rows, 387 trees of 9 levels: 63
+// blocks in three ranges were two waves.)
+DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
+  const int64_t G = (int64_t)f->df.pairs.size(), row_tiles = (n_rows + 31) / 32, SMs = f->num_sms;
+  DeepSplit best;
+  best.n_rows = n_rows;
+  double best_cost = -1.0;
+  for (int rw = std::min(4, f->deep_row_warps); rw <= f->deep_row_warps; ++rw) {
+    const int64_t blocks = (row_tiles + rw - 1) / rw, rest = blocks % SMs;
+    for (int64_t c = 1; c <= std::min<int64_t>(G, std::max<int64_t>(8, (SMs + blocks - 1) / blocks)); ++c) {
+      const int64_t per = (G + c - 1) / c;
+      if ((G + per - 1) / per != c) continue;
+      const double waves = (double)((rest * c + SMs - 1) / SMs);
+      const double cost = (1.0 + 0.005 * rw) * ((double)(blocks / SMs) * (double)(G + 12) + waves * (double)(per + 12) + (c > 1 ? 8.0 : 0.0));
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best.row_warps = rw;
+        best.chunks = (int)c;
+        best.whole = c > 1 ? blocks - rest : 0;
+      }
+      if (rest == 0) break;
+    }
+  }
+  return best;
+}
+
+// One launch of the deep-tree kernel over `n_rows` rows, and the second pass over chunks.
+int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
+                  float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot, int rw, int64_t chunks) {
   const auto &q = f->df;
   const int64_t G = (int64_t)q.pairs.size();
-  // as few row warps per block as do not cost another wave of blocks: the last wave is then as
-  // full as the others, and small batches still cover the SMs
-  int rw = f->deep_row_warps;
-  const int64_t row_tiles = (n_rows + 31) / 32, waves = (row_tiles + (int64_t)rw * f->num_sms - 1) / ((int64_t)rw * f->num_sms);
-  rw = std::max(std::min(4, rw), (int)((row_tiles + waves * f->num_sms - 1) / (waves * f->num_sms)));
   const int64_t rows_per_block = 32 * rw;
   const int64_t grid_x = (n_rows + rows_per_block - 1) / rows_per_block;
-  int64_t chunks = 1;
-  if (f->user.tree_chunks > 0) chunks = f->user.tree_chunks;
-  else if (grid_x < (int64_t)f->num_sms) chunks = ((int64_t)f->num_sms + grid_x - 1) / grid_x;
   chunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(chunks, G), 65535));
   const int gpc = (int)((G + chunks - 1) / chunks);
   chunks = (G + gpc - 1) / gpc;
@@ -675,7 +705,6 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   const bool d12 = f->uniform_depth == 12, ids = mode == kLeafIds, small = plan.threads <= 768;
   const DeepKernel kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
   CUDA_TRY(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
-  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
   kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
   CUDA_TRY(cudaGetLastError());
@@ -691,11 +720,43 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     CUDA_TRY(cudaGetLastError());
     ++f->launches;
   }
+  if (uses_scratch) return scratch_release(f, slot, stream);
+  return TBK_OK;
+}
+
+// One prediction with the deep-tree kernel.
+int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
+             float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot) {
+  DeepSplit &s = f->deep_split;
+  if (s.n_rows != n_rows) {
+    s = split_deep(f, n_rows);
+    if (f->user.tree_chunks > 0) { // (asked for: all rows)
+      s.whole = 0;
+      s.chunks = f->user.tree_chunks;
+    }
+  }
+  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
+  int64_t first = std::min<int64_t>(n_rows, s.whole * s.row_warps * 32);
+  if (first > 0 && first < n_rows && mode != kLeafIds) { // (no allocation inside a capture: in one piece)
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone && 2 * (size_t)s.chunks * (size_t)(n_rows - first) * sizeof(float) + 512 > f->scratch_bytes)
+      first = n_rows;
+  }
+  if (first > 0) {
+    const int rc = run_deep_rows(f, mode, d_rows, first, ld, d_out, d_partial, d_leaf_ids, stream, slot, s.row_warps, 1);
+    if (rc) return rc;
+  }
+  if (first < n_rows) {
+    const int rc = run_deep_rows(f, mode, d_rows + first * ld, n_rows - first, ld, d_out ? static_cast<float *>(d_out) + first : nullptr,
+                                 d_partial ? d_partial + first : nullptr, d_leaf_ids ? d_leaf_ids + first * f->df.num_trees : nullptr,
+                                 stream, slot, s.row_warps, s.chunks);
+    if (rc) return rc;
+  }
   if (f->timing) {
     CUDA_TRY(cudaEventRecord(f->ev1, stream));
     f->ev_pending = true;
   }
-  if (uses_scratch) return scratch_release(f, slot, stream);
   return TBK_OK;
 }
 
