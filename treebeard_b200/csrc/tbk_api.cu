@@ -597,10 +597,11 @@ template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb:
              : (ids ? tb::tb_walk_deep_kernel<1024, 0, WIDE, true> : tb::tb_walk_deep_kernel<1024, 0, WIDE, false>);
 }
 
-// A pair of trees takes a block about the same time whatever its row warps (12 to 20: 1.42 to 1.57 ms
-// a thousand pairs), so what counts is the waves of blocks.  The blocks that fill no whole wave
-// split the trees, into as many ranges as leave the least of their last wave empty.  A block stages its
-// rows for about the time of 12 pairs, the second pass over partial sums takes that of 8.
+// What counts is the waves of blocks and what a pair of trees takes a block: 300 pairs of 12 levels
+// 0.25 ms with 4 row warps, 0.34 with 18, 0.42 with 24, 0.50 with 30 (9 levels: 0.25, 0.31, 0.36, 0.42) -- all
+// latency up to about 18, then the shared-memory pipe as well.  The blocks that fill no whole wave
+// split the trees, into as many ranges as leave the least of their last wave empty.  Staging
+// the rows takes a block the time of 8 pairs and more, the second pass over partial sums that of 8.
 // (1048576 rows, 2000 trees, 18 row warps: 12.3 waves of blocks; 8000 rows, 387 trees of 9 levels: 63
 // blocks in three ranges were two waves.)
 DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
@@ -610,11 +611,12 @@ DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
   double best_cost = -1.0;
   for (int rw = std::min(4, f->deep_row_warps); rw <= f->deep_row_warps; ++rw) {
     const int64_t blocks = (row_tiles + rw - 1) / rw, rest = blocks % SMs;
+    const double pair = rw <= 18 ? 0.7 + 0.0167 * rw : 1.0 + 0.02 * (rw - 18), start = 8.0 + 0.006 * f->df.num_features * rw;
     for (int64_t c = 1; c <= std::min<int64_t>(G, std::max<int64_t>(8, (SMs + blocks - 1) / blocks)); ++c) {
       const int64_t per = (G + c - 1) / c;
       if ((G + per - 1) / per != c) continue;
       const double waves = (double)((rest * c + SMs - 1) / SMs);
-      const double cost = (1.0 + 0.005 * rw) * ((double)(blocks / SMs) * (double)(G + 12) + waves * (double)(per + 12) + (c > 1 ? 8.0 : 0.0));
+      const double cost = pair * ((double)(blocks / SMs) * ((double)G + start) + waves * ((double)per + start)) + (c > 1 ? 8.0 : 0.0);
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
         best.row_warps = rw;
