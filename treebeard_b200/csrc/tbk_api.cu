@@ -58,7 +58,8 @@ int fail(int code, const char *fmt, ...) {
 } // namespace
 
 // Pinned, mapped host memory is slow to come by (milliseconds for a few MiB), so what a forest gives
-// back is kept for the next one: blocks of up to 32 MiB, 64 MiB of them in all.
+// back is kept for the next one: blocks of up to 32 MiB, 64 MiB of them in all, until the process has
+// no forest any more.
 class PinnedPool {
 public:
   unsigned char *take(size_t bytes, size_t *capacity) { // null: none to be had
@@ -99,6 +100,7 @@ public:
     if (status_.empty()) {
       unsigned char *page = nullptr;
       if (cudaHostAlloc(&page, 4096, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+      pages_.push_back(page);
       for (int i = 0; i < 4096; i += 64) status_.push_back(reinterpret_cast<int32_t *>(page + i));
     }
     int32_t *word = status_.back();
@@ -112,9 +114,26 @@ public:
     status_.push_back(word);
   }
 
+  void attach() {
+    std::lock_guard<std::mutex> lock(mu_);
+    ++forests_;
+  }
+  void detach() { // (the last forest has given back what it had)
+    std::lock_guard<std::mutex> lock(mu_);
+    if (--forests_ > 0) return;
+    for (const auto &b : free_) cudaFreeHost(b.first);
+    for (unsigned char *page : pages_) cudaFreeHost(page);
+    free_.clear();
+    pages_.clear();
+    status_.clear();
+    kept_ = 0;
+  }
+
 private:
   std::mutex mu_;
+  int64_t forests_ = 0;
   std::vector<std::pair<unsigned char *, size_t>> free_;
+  std::vector<unsigned char *> pages_;
   std::vector<int32_t *> status_;
   size_t kept_ = 0;
 };
@@ -1769,6 +1788,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
   *out = nullptr;
   const tb::PackedImage &im = img->im;
   auto *f = new tbk_forest();
+  pinned_pool().attach();
   f->user = im.user;
   if (schedule) { // launch-shape requests of the caller; the layout is the image's
     f->user.rows_per_block = schedule->rows_per_block;
@@ -2058,6 +2078,7 @@ int tbk_forest_free(tbk_forest *f) {
   if (f->ev0) cudaEventDestroy(f->ev0);
   if (f->ev1) cudaEventDestroy(f->ev1);
   delete f;
+  pinned_pool().detach();
   return TBK_OK;
 }
 
