@@ -108,3 +108,20 @@ def test_the_call_that_may_not_allocate(trees, levels, features, classes, rows):
             assert (out == want).float().mean() > 0.999   # (other tree chunks: near-ties may fall either way)
         else:
             assert_predictions_close(out.cpu().numpy(), want.cpu().numpy())
+
+
+@pytest.mark.parametrize("features", [490, 491, 506, 507, 511])
+@pytest.mark.parametrize("rows", [300, 20011])
+def test_widest_rank_key_rows_under_the_deepest_trees(features, rows):
+    """One quad of tiles of 491 features and a ring of three 32 KB planes leave room for 8 walker warps,
+    from 507 on for 4."""
+    f, marg = _forest(40, 8, features)
+    X = _rows(f, marg, rows)
+    want, want_ids = oracle.predict(f, X, leaf_ids=True)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows)
+    assert df.info().schedule.feature_bits == 16
+    dX = torch.from_numpy(X).cuda()
+    assert np.array_equal(df.predict_leaf_ids(dX).cpu().numpy(), want_ids)
+    got = df.predict(dX)
+    df.check_status()
+    assert_predictions_close(got.cpu().numpy(), want)

@@ -861,24 +861,40 @@ RankKernel pick_rank_kernel(int stride, bool small, bool whole, int mode) {
   return whole ? pick_rank<128, 16, true>(mode) : pick_rank<128, 16, false>(mode);
 }
 
-// The same for keys in tiles.  A block takes up to `quads` quads of tiles at a time with 12 to 20
-// walker warps; what fits beside a ring of at least three slots bounds them.
+// How many quads of tiles a block of the tiled kernel takes at a time, with how many walker warps.
+// Rows of 491 to 511 features under trees of 8 levels leave three ring slots beside one quad only with
+// 8 walkers, or 4 (507 to 511).
+struct RankTilesShape { int quads, walkers; };
+constexpr RankTilesShape kRankTilesShapes[] = {{1, 16}, {2, 16}, {3, 12}, {4, 16}, {5, 20}, {6, 12}, {1, 8}, {1, 4}};
+int rank_tiles_slots(const RankTilesShape &sh, int num_features, int max_depth, int smem_limit) {
+  const int room = smem_limit - tb::rank_tiles_smem_bytes(32 * rank_stride(num_features), 4 * sh.quads, sh.walkers, 4, 0, 0);
+  return room < 0 ? 0 : std::min(tb::kRTMaxSlots, room / (128 << max_depth));
+}
+constexpr int kRankTilesMinSlots = 3; // one plane more than the group being walked
+
+// Does some launch shape hold rank keys of such rows and trees?
+bool rank_fits(int num_features, int max_depth, int smem_limit) {
+  if (!rank_tiled(num_features)) return tb::rank_walk_smem_bytes(rank_stride(num_features), 2, 256u << max_depth) <= smem_limit;
+  for (const RankTilesShape &sh : kRankTilesShapes)
+    if (rank_tiles_slots(sh, num_features, max_depth, smem_limit) >= kRankTilesMinSlots) return true;
+  return false;
+}
+
+// The same for keys in tiles.
 RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
   const auto &q = f->rf;
   const int G = (int)q.groups.size(), D = q.max_depth;
   const int tile_bytes = 32 * rank_stride(q.num_features);
   const int64_t quads = (n_rows + 127) / 128;
-  struct Shape { int quads, walkers; };
   RankPlan best;
   double best_cost = -1.0;
-  for (const Shape sh : {Shape{1, 16}, Shape{2, 16}, Shape{3, 12}, Shape{4, 16}, Shape{5, 20}, Shape{6, 12}}) {
+  for (const RankTilesShape &sh : kRankTilesShapes) {
     RankPlan p;
     p.quads = sh.quads;
     p.walkers = sh.walkers;
     p.stage_bytes = 128u << D;
-    const int room = f->max_smem_optin - tb::rank_tiles_smem_bytes(tile_bytes, 4 * sh.quads, sh.walkers, 4, 0, 0);
-    p.stages = std::min(tb::kRTMaxSlots, room / (int)p.stage_bytes);
-    if (p.stages < 3) continue;
+    p.stages = rank_tiles_slots(sh, q.num_features, D, f->max_smem_optin);
+    if (p.stages < kRankTilesMinSlots) continue;
     p.smem = tb::rank_tiles_smem_bytes(tile_bytes, 4 * sh.quads, sh.walkers, 4, p.stages, p.stage_bytes);
     // clocks of a group of trees for a batch of b quads (2 D - 0.25 wavefronts per 32 rows and tree)
     auto group = [&](int64_t b) {
@@ -1644,7 +1660,7 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
   // of 1303 features took 3.3 ms)
   // rank keys: whatever the key kernels would take, over at most kRankMaxFeatures features
   const bool want_rank = want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth);
-  if (want_rank && host.num_features <= tb::kRankMaxFeatures) {
+  if (want_rank && host.num_features <= tb::kRankMaxFeatures && rank_fits(host.num_features, max_depth, smem_limit)) {
     if (tb::pack_rank(host, &im.rf).empty()) {
       im.kind = tb::PackedImage::kRank;
       im.user.representation = TBK_REP_REORG;
