@@ -286,6 +286,7 @@ struct tbk_forest {
   int32_t *d_tree_index = nullptr;
   int32_t *d_orig_node = nullptr;
   unsigned long long *d_orig_off = nullptr;
+  bool orig_ready = false;
   int8_t *d_lut = nullptr;
   int32_t *h_status = nullptr, *d_status = nullptr; // status word in mapped host memory, both addresses
   float *d_scratch = nullptr; // tree-chunk partials, two slots
@@ -417,14 +418,23 @@ int scratch_release(tbk_forest *f, int slot, cudaStream_t stream) {
   return TBK_OK;
 }
 
-int ensure_orig(tbk_forest *f) {
-  if (f->d_orig_node) return TBK_OK;
-  const auto &p = f->packed;
-  CUDA_TRY(cudaMalloc(&f->d_orig_node, std::max<size_t>(4, p.orig_node.size() * 4)));
-  CUDA_TRY(cudaMemcpy(f->d_orig_node, p.orig_node.data(), p.orig_node.size() * 4, cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMalloc(&f->d_orig_off, std::max<size_t>(8, p.orig_off.size() * 8)));
-  CUDA_TRY(cudaMemcpy(f->d_orig_off, p.orig_off.data(), p.orig_off.size() * 8, cudaMemcpyHostToDevice));
+// A copy from pageable memory may return before its data has reached the device, and a memset does:
+// both are work of the legacy stream, which non-blocking streams don't wait for.
+int uploads_done() {
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
   return TBK_OK;
+}
+
+int ensure_orig(tbk_forest *f) {
+  if (f->orig_ready) return TBK_OK;
+  const auto &p = f->packed;
+  if (!f->d_orig_node) CUDA_TRY(cudaMalloc(&f->d_orig_node, std::max<size_t>(4, p.orig_node.size() * 4)));
+  CUDA_TRY(cudaMemcpy(f->d_orig_node, p.orig_node.data(), p.orig_node.size() * 4, cudaMemcpyHostToDevice));
+  if (!f->d_orig_off) CUDA_TRY(cudaMalloc(&f->d_orig_off, std::max<size_t>(8, p.orig_off.size() * 8)));
+  CUDA_TRY(cudaMemcpy(f->d_orig_off, p.orig_off.data(), p.orig_off.size() * 8, cudaMemcpyHostToDevice));
+  const int rc = uploads_done();
+  f->orig_ready = rc == TBK_OK;
+  return rc;
 }
 
 enum Mode { kPredict, kPartial, kLeafIds };
@@ -1825,6 +1835,11 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     if (e__ != cudaSuccess)                                                                \
       return bail(fail(TBK_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e__)));    \
   } while (0)
+  auto done = [&]() { // (calls may come on streams that nothing orders behind the uploads)
+    if (const int rc = uploads_done()) return bail(rc);
+    *out = f;
+    return (int)TBK_OK;
+  };
   CUDA_TRY_F(cudaSetDevice(device));
   CUDA_TRY_F(cudaDeviceGetAttribute(&f->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   CUDA_TRY_F(cudaDeviceGetAttribute(&f->num_sms, cudaDevAttrMultiProcessorCount, device));
@@ -1861,8 +1876,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     tb::LaunchPlan &pl = f->last_plan;
     pl.row_warps = f->deep_row_warps; pl.tree_threads = 1; pl.rows_per_lane = 1; pl.chunks = 1; pl.staged = 1; pl.cache_rows = 1;
     pl.stage_bytes = 4u * tb::deep_tree_words((uint32_t)std::max(q.max_depth, tb::kDeepMinDepth)); pl.smem_bytes = deep_smem_bytes(f); pl.threads = 32 * (f->deep_row_warps + 1);
-    *out = f;
-    return TBK_OK;
+    return done();
   }
   auto upload = [](auto **dst, const auto &v) { // (an empty vector gets a few bytes)
     const size_t bytes = v.size() * sizeof(v[0]);
@@ -1892,8 +1906,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     for (uint32_t end : q.class_end) class_tree.push_back((uint32_t)(std::lower_bound(q.root.begin(), q.root.end(), end) - q.root.begin()));
     CUDA_TRY_F(upload(&f->d_lclass_tree, class_tree));
     f->last_plan = lane_launch_plan(plan_lanes(f, batch_hint > 0 ? batch_hint : 65536, false));
-    *out = f;
-    return TBK_OK;
+    return done();
   }
   if (im.kind == tb::PackedImage::kRank) {
     const auto &q = im.rf;
@@ -1968,8 +1981,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
       CUDA_TRY_F(cudaMemset(w.mem, 0, tb::kRankArrivalBytes));
       w.bytes = bytes;
     }
-    *out = f;
-    return TBK_OK;
+    return done();
   }
   if (im.kind == tb::PackedImage::kQuant) {
     f->qf = im.qf;
@@ -2020,8 +2032,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
       pl.smem_bytes = tb::quant_batch_smem_bytes(q.num_features, batch);
       pl.threads = tb::kQBThreads;
     }
-    *out = f;
-    return TBK_OK;
+    return done();
   }
 
   f->packed = im.packed;
@@ -2045,8 +2056,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
   std::string why = tb::select_launch(shape, f->user, batch_hint > 0 ? batch_hint : 65536, f->max_smem_optin,
                                       f->num_sms, false, &f->last_plan);
   if (!why.empty()) return bail(fail(TBK_ERR_UNSUPPORTED, "%s", why.c_str()));
-  *out = f;
-  return TBK_OK;
+  return done();
 }
 
 int tbk_forest_free(tbk_forest *f) {
