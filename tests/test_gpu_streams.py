@@ -1,5 +1,9 @@
 """Forests of every layout and the streams that calls come on: what creation has uploaded is there
-for a stream that nothing orders behind it."""
+for a stream that nothing orders behind it, and calls that may run at the same time have memory of
+their own."""
+import ctypes
+import threading
+
 import numpy as np
 import pytest
 
@@ -55,3 +59,71 @@ def test_a_new_forest_is_ready_for_every_stream(layout):
         else:
             assert_predictions_close(got.cpu().numpy(), want)
         df.close()
+
+
+def _predict_on(df, rows, out, stream_handle):
+    kernels._check(kernels.lib().tbk_predict(df._h, rows.data_ptr(), rows.shape[0], rows.stride(0), out.data_ptr(),
+                                             kernels.OUT_F32, stream_handle))
+
+
+PER_THREAD = 2   # cudaStreamPerThread: one handle, another stream in every thread
+
+
+@pytest.mark.parametrize("layout", ["rank", "rank_tiles"])
+def test_per_thread_streams_do_not_share_call_memory(layout):
+    f, X, options = _case(layout, 24000)
+    dX = torch.from_numpy(X).cuda()
+    parts = [dX[i * 6000:(i + 1) * 6000] for i in range(4)]
+    df = kernels.DeviceForest(f, batch_hint=6000, **options)
+    want = [df.predict(p).clone() for p in parts]
+    outs = [torch.empty_like(w) for w in want]
+    torch.cuda.synchronize()
+    wrong, start = [], threading.Barrier(len(parts))
+
+    def work(i):
+        mine = torch.cuda.ExternalStream(PER_THREAD)
+        for _ in range(200):
+            start.wait()
+            _predict_on(df, parts[i], outs[i], PER_THREAD)
+            mine.synchronize()
+            if not torch.equal(outs[i].cpu(), want[i].cpu()):
+                wrong.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(parts))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    df.check_status()
+
+
+@pytest.mark.parametrize("layout", ["rank", "rank_tiles"])
+@pytest.mark.parametrize("alive", [1, 3, 11])
+def test_streams_that_come_and_go(layout, alive):
+    """Streams are destroyed with a prediction pending and new ones, often under the same handle, take
+    their place; `alive` of them at a time (more than the forest has workspaces for, at eleven)."""
+    f, X, options = _case(layout, 40000)
+    dX = torch.from_numpy(X).cuda()
+    df = kernels.DeviceForest(f, batch_hint=5000, **options)
+    sizes = [5000 + 307 * i for i in range(12)]
+    batches = [dX[1000 * i:1000 * i + n] for i, n in enumerate(sizes)]
+    want = [df.predict(b).clone() for b in batches]
+    torch.cuda.synchronize()
+    rt, handles, outs = torch.cuda.cudart(), [], []
+    for i in range(60):
+        handle = ctypes.c_void_p()
+        assert int(rt.cudaStreamCreate(ctypes.addressof(handle))) == 0
+        out = torch.empty(sizes[i % 12], device="cuda")
+        torch.cuda.current_stream().synchronize()
+        _predict_on(df, batches[i % 12], out, handle.value)
+        outs.append(out)
+        handles.append(handle.value)
+        if len(handles) == alive:
+            assert int(rt.cudaStreamDestroy(handles.pop(0))) == 0
+    for h in handles:
+        assert int(rt.cudaStreamDestroy(h)) == 0
+    torch.cuda.synchronize()
+    df.check_status()
+    for i, out in enumerate(outs):
+        assert torch.equal(out, want[i % 12]), i

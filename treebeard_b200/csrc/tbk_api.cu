@@ -319,14 +319,15 @@ struct tbk_forest {
   struct Workspace {
     unsigned char *mem = nullptr;
     size_t bytes = 0;
-    cudaStream_t stream = nullptr;
+    unsigned long long stream = 0; // id of the stream that uses it
     bool used = false;
+    bool marked = false;        // `done` stands behind the last use
     cudaEvent_t done = nullptr;
   };
   static constexpr int kWorkspaces = 8;
   bool mark_uses = false;
   Workspace workspace[kWorkspaces];
-  int next_victim = 0;
+  unsigned next_victim = 0;
   std::list<Workspace> captured; // of calls that were captured into graphs
   std::vector<const void *> smem_allowed;
   RankPlan rank_plan;          // of the last batch size
@@ -796,8 +797,11 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
 
 // Device memory that a call needs from its first kernel to its last: the keys of the rows and
 // the partial sums of tree chunks.  Calls on one stream are ordered and share one workspace; a call
-// on a further stream gets one of its own, up to four, and after that waits on the device for the
-// previous user of the one that it takes over.
+// on a further stream gets one of its own, up to kWorkspaces, and after that waits on the device for
+// the last user of the one that it takes over.  A stream is known by its id: a handle may stand for
+// another stream in every thread (cudaStreamPerThread), or for a new stream once its first one is
+// destroyed, with work still pending.  From the fourth stream on every use ends with an event, so that
+// there are marked ones to take over by the time that all are taken; fewer streams need none.
 int workspace_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_forest::Workspace **out) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
@@ -815,32 +819,48 @@ int workspace_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_fore
     *out = w;
     return TBK_OK;
   }
+  unsigned long long id = 0;
+  CUDA_TRY(cudaStreamGetId(stream, &id));
   tbk_forest::Workspace *w = nullptr;
-  for (auto &c : f->workspace)
-    if (c.used && c.stream == stream) w = &c;
-  if (!w)
+  int used = 0;
+  for (auto &c : f->workspace) {
+    used += c.used;
+    if (c.used && c.stream == id) w = &c;
+  }
+  if (!w) {
     for (auto &c : f->workspace)
       if (!c.used && (!w || c.bytes > w->bytes)) w = &c;
-  if (!w) {
-    if (!f->mark_uses) {
-      CUDA_TRY(cudaDeviceSynchronize()); // (earlier uses have left no mark)
-      f->mark_uses = true;
-      for (auto &c : f->workspace) CUDA_TRY(cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming));
-    }
-    w = &f->workspace[f->next_victim++ % tbk_forest::kWorkspaces];
-    CUDA_TRY(cudaStreamWaitEvent(stream, w->done, 0));
+    if (w && used + 1 >= tbk_forest::kWorkspaces / 2) f->mark_uses = true;
   }
-  w->stream = stream;
+  for (int i = 0; !w && i < tbk_forest::kWorkspaces; ++i) {
+    tbk_forest::Workspace &c = f->workspace[f->next_victim++ % tbk_forest::kWorkspaces];
+    if (!c.marked) continue;
+    CUDA_TRY(cudaStreamWaitEvent(stream, c.done, 0));
+    w = &c;
+  }
+  if (!w) { // (no use got as far as its mark)
+    CUDA_TRY(cudaDeviceSynchronize());
+    w = &f->workspace[f->next_victim++ % tbk_forest::kWorkspaces];
+  }
+  w->stream = id;
   w->used = true;
+  w->marked = false;
   if (w->bytes < bytes) {
     if (w->mem) CUDA_TRY(cudaFree(w->mem)); // (waits for the work that uses it)
     w->mem = nullptr;
     w->bytes = 0;
     CUDA_TRY(cudaMalloc(&w->mem, bytes));
-    w->bytes = bytes;
     CUDA_TRY(cudaMemsetAsync(w->mem, 0, tb::kRankArrivalBytes, stream));
+    w->bytes = bytes;
   }
   *out = w;
+  return TBK_OK;
+}
+int workspace_release(tbk_forest *f, tbk_forest::Workspace *w, cudaStream_t stream) {
+  if (!f->mark_uses || !w->used) return TBK_OK; // (a captured call's is never taken over)
+  if (!w->done) CUDA_TRY(cudaEventCreateWithFlags(&w->done, cudaEventDisableTiming));
+  CUDA_TRY(cudaEventRecord(w->done, stream));
+  w->marked = true;
   return TBK_OK;
 }
 
@@ -1213,8 +1233,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     CUDA_TRY(cudaEventRecord(f->ev1, stream));
     f->ev_pending = true;
   }
-  if (ws && ws->done) CUDA_TRY(cudaEventRecord(ws->done, stream)); // (uses are marked)
-  return TBK_OK;
+  return ws ? workspace_release(f, ws, stream) : TBK_OK;
 }
 
 // ---------------------------------------------------------------------------
