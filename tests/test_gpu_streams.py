@@ -127,3 +127,47 @@ def test_streams_that_come_and_go(layout, alive):
     df.check_status()
     for i, out in enumerate(outs):
         assert torch.equal(out, want[i % 12]), i
+
+
+def _captured(df, rows, out):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        df.predict(rows, out=out)
+    return graph
+
+
+@pytest.mark.parametrize("layout", ["rank", "rank_tiles"])
+def test_memory_of_captured_calls_lives_as_long_as_their_graphs(layout):
+    f, X, options = _case(layout, 60000)
+    dX = torch.from_numpy(X).cuda()
+    df = kernels.DeviceForest(f, **options)
+    sizes = [60000 - 1000 * i for i in range(24)]
+    want = [df.predict(dX[:n]).clone() for n in sizes]
+    outs = [torch.empty(n, device="cuda") for n in sizes]
+    # two graphs at a time: replayed side by side, each with its own memory
+    side = torch.cuda.Stream()
+    for i in (0, 1):
+        graphs = [_captured(df, dX[:sizes[j]], outs[j]) for j in (i, i + 2)]
+        for _ in range(20):
+            for g, s in zip(graphs, (side, torch.cuda.Stream())):
+                with torch.cuda.stream(s):
+                    g.replay()
+        torch.cuda.synchronize()
+        for j in (i, i + 2):
+            assert torch.equal(outs[j], want[j])
+        del graphs, g
+    # one after another, a new shape each: the memory of those that are gone serves the next
+    free = []
+    for k in range(48):
+        n, out = sizes[k % 24], outs[k % 24]
+        out.zero_()
+        graph = _captured(df, dX[:n], out)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want[k % 24])
+        del graph
+        free.append(torch.cuda.mem_get_info()[0])
+    keys = {"rank": 4, "rank_tiles": 16}[layout] << 20   # the most that one call's keys take, to a power of two
+    assert min(free[8:]) >= free[0] - 8 * keys
+    assert torch.equal(df.predict(dX[:sizes[0]]), want[0])
+    df.check_status()

@@ -328,7 +328,12 @@ struct tbk_forest {
   bool mark_uses = false;
   Workspace workspace[kWorkspaces];
   unsigned next_victim = 0;
-  std::list<Workspace> captured; // of calls that were captured into graphs
+  // memory of calls that were captured, and whether a graph of such a call still exists
+  struct Captured {
+    Workspace memory;
+    std::shared_ptr<std::atomic<bool>> alive;
+  };
+  std::list<Captured> captured;
   std::vector<const void *> smem_allowed;
   RankPlan rank_plan;          // of the last batch size
   int64_t rank_plan_rows = -1;
@@ -795,6 +800,58 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
 // ---------------------------------------------------------------------------
 // Rank keys (rank_pack.h)
 
+// Memory for a call that is being captured.  The graph may be replayed at any time, so the memory is
+// the graph's: a user object of the graph, which everything instantiated from it holds as well,
+// tells when the last of them is gone (and its replays done).  The memory then serves the next capture, or
+// goes back when a call allocates anyway.  Sizes are powers of two, so that captures of many batch shapes
+// find each other's.
+int captured_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_forest::Workspace **out) {
+  size_t size = (size_t)64 << 10;
+  while (size < bytes) size *= 2;
+  tbk_forest::Captured *c = nullptr;
+  for (auto &old : f->captured)
+    if (old.memory.bytes == size && !old.alive->load(std::memory_order_acquire)) c = &old;
+  if (!c) {
+    unsigned char *mem = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaMalloc(&mem, size);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return fail(TBK_ERR_CUDA, "workspace of a captured call: %s", cudaGetErrorString(e));
+    f->captured.emplace_back();
+    c = &f->captured.back();
+    c->memory.mem = mem;
+    c->memory.bytes = size;
+  }
+  c->alive = std::make_shared<std::atomic<bool>>(false);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  CUDA_TRY(cudaStreamGetCaptureInfo_v2(stream, &status, &id, &graph, nullptr, nullptr));
+  if (!graph) return fail(TBK_ERR_CUDA, "workspace of a captured call: the capture has ended");
+  using Alive = std::shared_ptr<std::atomic<bool>>;
+  auto *token = new Alive(c->alive);
+  cudaUserObject_t object = nullptr;
+  cudaError_t e = cudaUserObjectCreate(&object, token, [](void *p) {
+    auto *mine = static_cast<Alive *>(p);
+    (*mine)->store(false, std::memory_order_release);
+    delete mine;
+  }, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    delete token;
+    return fail(TBK_ERR_CUDA, "workspace of a captured call: %s", cudaGetErrorString(e));
+  }
+  c->alive->store(true, std::memory_order_release);
+  e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(object, 1);
+    return fail(TBK_ERR_CUDA, "workspace of a captured call: %s", cudaGetErrorString(e));
+  }
+  CUDA_TRY(cudaMemsetAsync(c->memory.mem, 0, tb::kRankArrivalBytes, stream));
+  *out = &c->memory;
+  return TBK_OK;
+}
+
 // Device memory that a call needs from its first kernel to its last: the keys of the rows and
 // the partial sums of tree chunks.  Calls on one stream are ordered and share one workspace; a call
 // on a further stream gets one of its own, up to kWorkspaces, and after that waits on the device for
@@ -805,20 +862,7 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
 int workspace_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_forest::Workspace **out) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
-  if (capturing != cudaStreamCaptureStatusNone) {
-    // a captured graph may be replayed at any time: its memory is its own for the forest's life
-    f->captured.emplace_back();
-    tbk_forest::Workspace *w = &f->captured.back();
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-    cudaError_t e = cudaMalloc(&w->mem, bytes);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e == cudaSuccess) e = cudaMemsetAsync(w->mem, 0, tb::kRankArrivalBytes, stream);
-    if (e != cudaSuccess) return fail(TBK_ERR_CUDA, "workspace of a captured call: %s", cudaGetErrorString(e));
-    w->bytes = bytes;
-    *out = w;
-    return TBK_OK;
-  }
+  if (capturing != cudaStreamCaptureStatusNone) return captured_acquire(f, stream, bytes, out);
   unsigned long long id = 0;
   CUDA_TRY(cudaStreamGetId(stream, &id));
   tbk_forest::Workspace *w = nullptr;
@@ -846,6 +890,9 @@ int workspace_acquire(tbk_forest *f, cudaStream_t stream, size_t bytes, tbk_fore
   w->used = true;
   w->marked = false;
   if (w->bytes < bytes) {
+    f->captured.remove_if([](const tbk_forest::Captured &c) {
+      return !c.alive->load(std::memory_order_acquire) && cudaFree(c.memory.mem) == cudaSuccess;
+    });
     if (w->mem) CUDA_TRY(cudaFree(w->mem)); // (waits for the work that uses it)
     w->mem = nullptr;
     w->bytes = 0;
@@ -2117,7 +2164,7 @@ int tbk_forest_free(tbk_forest *f) {
     cudaFree(w.mem);
     if (w.done) cudaEventDestroy(w.done);
   }
-  for (auto &w : f->captured) cudaFree(w.mem);
+  for (auto &c : f->captured) cudaFree(c.memory.mem);
   for (int i = 0; i < 2; ++i)
     if (f->scratch_done[i]) cudaEventDestroy(f->scratch_done[i]);
   if (f->ev0) cudaEventDestroy(f->ev0);
