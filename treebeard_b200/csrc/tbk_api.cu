@@ -289,12 +289,6 @@ struct tbk_forest {
   bool orig_ready = false;
   int8_t *d_lut = nullptr;
   int32_t *h_status = nullptr, *d_status = nullptr; // status word in mapped host memory, both addresses
-  float *d_scratch = nullptr; // tree-chunk partials, two slots
-  size_t scratch_bytes = 0;
-  // a slot's last user: a call on another stream waits for it before reusing the slot
-  cudaEvent_t scratch_done[2] = {nullptr, nullptr};
-  cudaStream_t scratch_stream[2] = {nullptr, nullptr};
-  bool scratch_used[2] = {false, false};
   // 16-bit-key layout (wide rows)
   bool quant = false;
   tb::QuantForest qf;
@@ -397,408 +391,6 @@ KernelFn pick_kernel(int rep, int ts, int rpl, bool staged, bool cached) {
   default: return pick3<1, 4>(rpl, staged, cached);
   }
 }
-
-int ensure_scratch(tbk_forest *f, size_t bytes) {
-  if (bytes <= f->scratch_bytes) return TBK_OK;
-  if (f->d_scratch) CUDA_TRY(cudaFree(f->d_scratch));
-  f->d_scratch = nullptr;
-  f->scratch_bytes = 0;
-  CUDA_TRY(cudaMalloc(&f->d_scratch, bytes));
-  f->scratch_bytes = bytes;
-  return TBK_OK;
-}
-
-// The tree-chunk partial sums of a call live in a slot of the forest's scratch buffer from the
-// walk until the second pass has read them.  Calls on one stream are ordered anyway; a call on
-// another stream first waits (on the device) for the slot's previous user.
-int scratch_acquire(tbk_forest *f, int slot, cudaStream_t stream) {
-  if (f->scratch_used[slot] && f->scratch_stream[slot] != stream)
-    CUDA_TRY(cudaStreamWaitEvent(stream, f->scratch_done[slot], 0));
-  return TBK_OK;
-}
-int scratch_release(tbk_forest *f, int slot, cudaStream_t stream) {
-  if (!f->scratch_done[slot]) CUDA_TRY(cudaEventCreateWithFlags(&f->scratch_done[slot], cudaEventDisableTiming));
-  CUDA_TRY(cudaEventRecord(f->scratch_done[slot], stream));
-  f->scratch_stream[slot] = stream;
-  f->scratch_used[slot] = true;
-  return TBK_OK;
-}
-
-// A copy from pageable memory may return before its data has reached the device, and a memset does:
-// both are work of the legacy stream, which non-blocking streams don't wait for.
-int uploads_done() {
-  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
-  return TBK_OK;
-}
-
-int ensure_orig(tbk_forest *f) {
-  if (f->orig_ready) return TBK_OK;
-  const auto &p = f->packed;
-  if (!f->d_orig_node) CUDA_TRY(cudaMalloc(&f->d_orig_node, std::max<size_t>(4, p.orig_node.size() * 4)));
-  CUDA_TRY(cudaMemcpy(f->d_orig_node, p.orig_node.data(), p.orig_node.size() * 4, cudaMemcpyHostToDevice));
-  if (!f->d_orig_off) CUDA_TRY(cudaMalloc(&f->d_orig_off, std::max<size_t>(8, p.orig_off.size() * 8)));
-  CUDA_TRY(cudaMemcpy(f->d_orig_off, p.orig_off.data(), p.orig_off.size() * 8, cudaMemcpyHostToDevice));
-  const int rc = uploads_done();
-  f->orig_ready = rc == TBK_OK;
-  return rc;
-}
-
-enum Mode { kPredict, kPartial, kLeafIds };
-
-int quant_smem_bytes(int num_features) {
-  return tb::kQBarBytes + tb::kQRingBytes + tb::kQLeafTableBytes + tb::quant_key_tile_bytes(num_features);
-}
-
-// Tiles of 32 rows that the narrow-row kernel can stage together (0: the rows are too wide for it).
-int quant_batch_tiles(const tbk_forest *f, int num_features) {
-  const int room = f->max_smem_optin - tb::kQBBarBytes - tb::kQBRingBytes;
-  const int fit = room / tb::quant_batch_tile_bytes(num_features);
-  return fit >= 4 ? std::min(fit, tb::kQBMaxTiles) : 0;
-}
-
-// One prediction with a 15-bit-key kernel: rows whose key tiles fit shared memory several at a
-// time go to the batch kernel (persistent blocks of 22 warps over batches of up to 16 tiles),
-// wide rows to the kernel that holds one tile (persistent blocks of 24 warps over tiles of 32 rows).
-int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out, int32_t out_kind,
-              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot, float *fixed = nullptr, size_t fixed_floats = 0) {
-  const auto &q = f->qf;
-  const int64_t G = (int64_t)q.groups.size();
-  const int64_t tiles = (n_rows + 31) / 32;
-  const int max_batch = quant_batch_tiles(f, q.num_features);
-  const bool batched = max_batch > 0;
-  const bool multi = q.num_classes > 0;
-  if (multi && !batched) return fail(TBK_ERR_UNSUPPORTED, "multiclass forests in the key layout need rows narrow enough for the batch kernel");
-  // batch kernel: as many tiles per batch as still give every SM a batch
-  int R = 1;
-  if (batched) {
-    R = max_batch;
-    while (R > 1 && (tiles + R - 1) / R < (int64_t)f->num_sms) R = (R + 1) / 2;
-  }
-  const int64_t units = batched ? (tiles + R - 1) / R : tiles; // blocks' units of work along x
-  int64_t chunks = 1;
-  if (multi) chunks = 1; // a class must stay within one leaf warp's sequence of groups
-  else if (f->user.tree_chunks > 0) chunks = f->user.tree_chunks;
-  else if (batched) {
-    if (units < (int64_t)f->num_sms) chunks = ((int64_t)f->num_sms + units - 1) / units;
-  } else if (tiles < 2 * (int64_t)f->num_sms) chunks = (2 * (int64_t)f->num_sms + tiles - 1) / tiles;
-  // (batch kernel: a second pass over partial sums costs about ten microseconds, more than the
-  // walk of a small forest: trees are split only into chunks of at least 32 groups -- measured
-  // on 4 096 rows x 32 groups: 38 us in one chunk, 47 us in two -- unless the caller asks)
-  const int64_t max_chunks = !batched ? G : f->user.tree_chunks > 0 ? std::max<int64_t>(1, G / 2) : std::max<int64_t>(1, G / 32);
-  chunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(chunks, max_chunks), 65535));
-  if (fixed) chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, (int64_t)fixed_floats / n_rows));
-  const int gpc = (int)((G + chunks - 1) / chunks);
-  chunks = (G + gpc - 1) / gpc;
-  const bool vec4 = q.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0;
-  // One block per SM (shared memory allows no more).  With more units than blocks a block is
-  // persistent; the one-tile kernel then stages its next tile in tensor memory while it walks
-  // the current one, a path that reads rows with 16-byte loads.
-  const int64_t blocks_x = std::max<int64_t>(1, (int64_t)f->num_sms / chunks);
-  const int64_t grid_x = batched ? std::min(units, blocks_x) : (vec4 && tiles > blocks_x) ? blocks_x : tiles;
-  tb::LaunchPlan plan;
-  plan.row_warps = batched ? R : 1;
-  plan.tree_threads = tb::kQWalkers;
-  plan.rows_per_lane = 1;
-  plan.chunks = (int32_t)chunks;
-  plan.groups_per_chunk = gpc;
-  plan.staged = 1;
-  plan.cache_rows = 1;
-  plan.stage_bytes = tb::kQPiece;
-  plan.smem_bytes = batched ? tb::quant_batch_smem_bytes(q.num_features, R) : quant_smem_bytes(q.num_features);
-  plan.threads = batched ? tb::kQBThreads : tb::kQThreads;
-  plan.grid_x = grid_x;
-  f->last_plan = plan;
-
-  const bool need_partials = mode == kPartial || (mode == kPredict && chunks > 1);
-  float *partial_dst = nullptr;
-  bool uses_scratch = false;
-  if (need_partials) {
-    if (mode == kPartial && chunks == 1) {
-      partial_dst = d_partial;
-    } else if (fixed) {
-      partial_dst = fixed;
-    } else {
-      const size_t need = ((size_t)chunks * n_rows * sizeof(float) + 255) & ~(size_t)255;
-      int rc = ensure_scratch(f, 2 * need);
-      if (rc) return rc;
-      partial_dst = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(f->d_scratch) + (size_t)slot * (f->scratch_bytes / 2));
-      rc = scratch_acquire(f, slot, stream);
-      if (rc) return rc;
-      uses_scratch = true;
-    }
-  }
-  tb::QuantParams p{};
-  p.node_plane = f->d_qnode;
-  p.leaf_plane = f->d_qleaf;
-  p.exact_plane = f->d_qexact;
-  p.groups = f->d_qgroups;
-  p.tree_index = f->d_qtree_index;
-  p.orig_leaf = f->d_qorig;
-  p.lo = f->d_qlo;
-  p.scale = f->d_qscale;
-  p.rows = d_rows;
-  p.n_rows = n_rows;
-  p.ld = ld;
-  p.partial = partial_dst;
-  p.out = d_out;
-  p.write_partial = need_partials ? 1 : 0;
-  p.leaf_ids = mode == kLeafIds ? d_leaf_ids : nullptr;
-  p.num_trees = q.num_trees;
-  p.num_groups = (int32_t)G;
-  p.groups_per_chunk = gpc;
-  p.num_features = q.num_features;
-  p.transform = q.transform;
-  p.initial_value = (float)q.initial_value;
-  p.vec4_ok = vec4 ? 1 : 0;
-  p.tiles_per_batch = R;
-  p.set_groups = f->d_qset_groups;
-  p.set_count[0] = f->qset_count[0];
-  p.set_count[1] = f->qset_count[1];
-  p.group_class = f->d_qgroup_class;
-  p.num_classes = q.num_classes;
-  p.out_kind = out_kind == TBK_OUT_I8 ? 1 : 0;
-  p.status = f->d_status;
-  p.tie_count = f->d_ties;
-  p.skip_first_copy = f->expire_next_wait ? 1 : 0;
-  p.wait_tries = f->expire_next_wait ? 2000u : 0u;
-  f->expire_next_wait = false;
-  // kernels specialised for forests whose groups all have 8 (or 6) levels; generic otherwise
-  using QuantKernel = void (*)(const tb::QuantParams);
-  const bool ids = mode == kLeafIds;
-  const int ud = (f->uniform_depth == 8 || f->uniform_depth == 6) ? f->uniform_depth : 0;
-  const QuantKernel qkernel =
-      multi ? (ud == 8 ? (ids ? tb::tb_walk_quant_batch_kernel<8, true, true> : tb::tb_walk_quant_batch_kernel<8, false, true>)
-                       : (ids ? tb::tb_walk_quant_batch_kernel<0, true, true> : tb::tb_walk_quant_batch_kernel<0, false, true>))
-      : batched
-          ? (ud == 8   ? (ids ? tb::tb_walk_quant_batch_kernel<8, true, false> : tb::tb_walk_quant_batch_kernel<8, false, false>)
-             : ud == 6 ? (ids ? tb::tb_walk_quant_batch_kernel<6, true, false> : tb::tb_walk_quant_batch_kernel<6, false, false>)
-                       : (ids ? tb::tb_walk_quant_batch_kernel<0, true, false> : tb::tb_walk_quant_batch_kernel<0, false, false>))
-      : ud == 8 ? (ids ? tb::tb_walk_quant_kernel<8, true> : tb::tb_walk_quant_kernel<8, false>)
-      : ud == 6 ? (ids ? tb::tb_walk_quant_kernel<6, true> : tb::tb_walk_quant_kernel<6, false>)
-                : (ids ? tb::tb_walk_quant_kernel<0, true> : tb::tb_walk_quant_kernel<0, false>);
-  CUDA_TRY(cudaFuncSetAttribute((const void *)qkernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
-  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
-  dim3 grid((unsigned)grid_x, (unsigned)chunks);
-  qkernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
-  CUDA_TRY(cudaGetLastError());
-  ++f->launches;
-  const int tpb = 256;
-  if (mode == kPredict && chunks > 1) {
-    tb::tb_finalize_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(
-        partial_dst, (int)chunks, n_rows, 1, 0, (float)q.initial_value, q.transform, d_out, TBK_OUT_F32);
-    CUDA_TRY(cudaGetLastError());
-    ++f->launches;
-  } else if (mode == kPartial && chunks > 1) {
-    tb::tb_sum_partials_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(partial_dst, (int)chunks, n_rows, d_partial);
-    CUDA_TRY(cudaGetLastError());
-    ++f->launches;
-  }
-  if (f->timing) {
-    CUDA_TRY(cudaEventRecord(f->ev1, stream));
-    f->ev_pending = true;
-  }
-  if (uses_scratch) return scratch_release(f, slot, stream);
-  return TBK_OK;
-}
-
-// Shared-memory plan of the deep-tree kernel: the most row warps (even -- one block per SM
-// either way, and more rows per tile mean fewer passes over the forest and more walks in
-// flight) whose key tile leaves room for a ring of at least 4 whole-tree pieces.
-bool deep_plan(int num_features, int max_depth, int smem_limit, int *row_warps, int *slots) {
-  const int64_t slot = 4ll * tb::deep_tree_words((uint32_t)std::max(max_depth, tb::kDeepMinDepth));
-  // four slots hold the node planes of the pair being walked and of the next one
-  for (int rw = 30; rw >= 2; rw -= 2) { // (the block has one more warp, the ring producer)
-    const int64_t keys = ((int64_t)num_features * 64 + tb::kDeepLeafBytes) * rw;
-    const int64_t room = (int64_t)smem_limit - 128 - keys;
-    const int64_t s = std::min<int64_t>(tb::kDeepMaxSlots, room / slot);
-    if (s >= 4) {
-      *row_warps = rw;
-      *slots = (int)s;
-      return true;
-    }
-  }
-  return false;
-}
-int deep_smem_bytes(const tbk_forest *f) {
-  return 128 + f->deep_slots * 4 * (int)tb::deep_tree_words((uint32_t)std::max(f->df.max_depth, tb::kDeepMinDepth)) +
-         (f->df.num_features * 64 + tb::kDeepLeafBytes) * f->deep_row_warps;
-}
-
-template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb::DeepParams) {
-  if (small)
-    return d12 ? (ids ? tb::tb_walk_deep_kernel<768, 12, WIDE, true> : tb::tb_walk_deep_kernel<768, 12, WIDE, false>)
-               : (ids ? tb::tb_walk_deep_kernel<768, 0, WIDE, true> : tb::tb_walk_deep_kernel<768, 0, WIDE, false>);
-  return d12 ? (ids ? tb::tb_walk_deep_kernel<1024, 12, WIDE, true> : tb::tb_walk_deep_kernel<1024, 12, WIDE, false>)
-             : (ids ? tb::tb_walk_deep_kernel<1024, 0, WIDE, true> : tb::tb_walk_deep_kernel<1024, 0, WIDE, false>);
-}
-
-// What counts is the waves of blocks and what a pair of trees takes a block: 300 pairs of 12 levels
-// 0.25 ms with 4 row warps, 0.34 with 18, 0.42 with 24, 0.50 with 30 (9 levels: 0.25, 0.31, 0.36, 0.42) -- all
-// latency up to about 18, then the shared-memory pipe as well.  The blocks that fill no whole wave
-// split the trees, into as many ranges as leave the least of their last wave empty.  Staging
-// the rows takes a block the time of 8 pairs and more, the second pass over partial sums that of 8.
-// (1048576 rows, 2000 trees, 18 row warps: 12.3 waves of blocks; 8000 rows, 387 trees of 9 levels: 63
-// blocks in three ranges were two waves.)
-DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
-  const int64_t G = (int64_t)f->df.pairs.size(), row_tiles = (n_rows + 31) / 32, SMs = f->num_sms;
-  DeepSplit best;
-  best.n_rows = n_rows;
-  double best_cost = -1.0;
-  for (int rw = std::min(4, f->deep_row_warps); rw <= f->deep_row_warps; ++rw) {
-    const int64_t blocks = (row_tiles + rw - 1) / rw, rest = blocks % SMs;
-    const double pair = rw <= 18 ? 0.7 + 0.0167 * rw : 1.0 + 0.02 * (rw - 18), start = 8.0 + 0.006 * f->df.num_features * rw;
-    for (int64_t c = 1; c <= std::min<int64_t>(G, std::max<int64_t>(8, (SMs + blocks - 1) / blocks)); ++c) {
-      const int64_t per = (G + c - 1) / c;
-      if ((G + per - 1) / per != c) continue;
-      const double waves = (double)((rest * c + SMs - 1) / SMs);
-      const double cost = pair * ((double)(blocks / SMs) * ((double)G + start) + waves * ((double)per + start)) + (c > 1 ? 8.0 : 0.0);
-      if (best_cost < 0 || cost < best_cost) {
-        best_cost = cost;
-        best.row_warps = rw;
-        best.chunks = (int)c;
-        best.whole = c > 1 ? blocks - rest : 0;
-      }
-      if (rest == 0) break;
-    }
-  }
-  return best;
-}
-
-// One launch of the deep-tree kernel over `n_rows` rows, and the second pass over chunks.
-int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
-                  float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot, int rw, int64_t chunks) {
-  const auto &q = f->df;
-  const int64_t G = (int64_t)q.pairs.size();
-  const int64_t rows_per_block = 32 * rw;
-  const int64_t grid_x = (n_rows + rows_per_block - 1) / rows_per_block;
-  chunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(chunks, G), 65535));
-  const int gpc = (int)((G + chunks - 1) / chunks);
-  chunks = (G + gpc - 1) / gpc;
-  tb::LaunchPlan plan;
-  plan.row_warps = rw;
-  plan.tree_threads = 1;
-  plan.rows_per_lane = 1;
-  plan.chunks = (int32_t)chunks;
-  plan.groups_per_chunk = gpc;
-  plan.staged = 1;
-  plan.cache_rows = 1;
-  plan.stage_bytes = 4u * tb::deep_tree_words((uint32_t)std::max(q.max_depth, tb::kDeepMinDepth));
-  plan.smem_bytes = deep_smem_bytes(f);
-  plan.threads = 32 * (rw + 1); // row warps + the ring producer
-  plan.grid_x = grid_x;
-  f->last_plan = plan;
-
-  const bool need_partials = mode == kPartial || (mode == kPredict && chunks > 1);
-  float *partial_dst = nullptr;
-  bool uses_scratch = false;
-  if (need_partials) {
-    if (mode == kPartial && chunks == 1) {
-      partial_dst = d_partial;
-    } else {
-      const size_t need = ((size_t)chunks * n_rows * sizeof(float) + 255) & ~(size_t)255;
-      int rc = ensure_scratch(f, 2 * need);
-      if (rc) return rc;
-      partial_dst = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(f->d_scratch) + (size_t)slot * (f->scratch_bytes / 2));
-      rc = scratch_acquire(f, slot, stream);
-      if (rc) return rc;
-      uses_scratch = true;
-    }
-  }
-  tb::DeepParams p{};
-  p.node_plane = f->d_qnode;
-  p.leaf_plane = f->d_qleaf;
-  p.exact_plane = f->d_qexact;
-  p.pairs = f->d_qgroups;
-  p.tree_index = f->d_qtree_index;
-  p.orig_leaf = f->d_qorig;
-  p.lo = f->d_qlo;
-  p.scale = f->d_qscale;
-  p.rows = d_rows;
-  p.n_rows = n_rows;
-  p.ld = ld;
-  p.partial = partial_dst;
-  p.out = d_out;
-  p.write_partial = need_partials ? 1 : 0;
-  p.leaf_ids = mode == kLeafIds ? d_leaf_ids : nullptr;
-  p.num_trees = q.num_trees;
-  p.num_pairs = (int32_t)G;
-  p.pairs_per_chunk = gpc;
-  p.num_features = q.num_features;
-  p.transform = q.transform;
-  p.initial_value = (float)q.initial_value;
-  p.ring_slots = f->deep_slots;
-  p.slot_bytes = plan.stage_bytes;
-  p.tree_words = plan.stage_bytes / 4;
-  p.key_tile = 128u * (uint32_t)q.num_features;
-  p.leaf_off = (uint32_t)(plan.smem_bytes - tb::kDeepLeafBytes * f->deep_row_warps);
-  p.status = f->d_status;
-  p.tie_count = f->d_ties;
-  p.skip_first_copy = f->expire_next_wait ? 1 : 0;
-  p.wait_tries = f->expire_next_wait ? 2000u : 0u;
-  f->expire_next_wait = false;
-  // up to 24 warps (row warps + producer) the compiler may use 80 registers per thread, beyond that 64
-  // specialised for forests whose pairs all have 12 levels; generic otherwise
-  using DeepKernel = void (*)(const tb::DeepParams);
-  const bool d12 = f->uniform_depth == 12, ids = mode == kLeafIds, small = plan.threads <= 768;
-  const DeepKernel kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
-  CUDA_TRY(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
-  dim3 grid((unsigned)grid_x, (unsigned)chunks);
-  kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
-  CUDA_TRY(cudaGetLastError());
-  ++f->launches;
-  const int tpb = 256;
-  if (mode == kPredict && chunks > 1) {
-    tb::tb_finalize_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(
-        partial_dst, (int)chunks, n_rows, 1, 0, (float)q.initial_value, q.transform, d_out, TBK_OUT_F32);
-    CUDA_TRY(cudaGetLastError());
-    ++f->launches;
-  } else if (mode == kPartial && chunks > 1) {
-    tb::tb_sum_partials_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(partial_dst, (int)chunks, n_rows, d_partial);
-    CUDA_TRY(cudaGetLastError());
-    ++f->launches;
-  }
-  if (uses_scratch) return scratch_release(f, slot, stream);
-  return TBK_OK;
-}
-
-// One prediction with the deep-tree kernel.
-int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
-             float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot) {
-  DeepSplit &s = f->deep_split;
-  if (s.n_rows != n_rows) {
-    s = split_deep(f, n_rows);
-    if (f->user.tree_chunks > 0) { // (asked for: all rows)
-      s.whole = 0;
-      s.chunks = f->user.tree_chunks;
-    }
-  }
-  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
-  int64_t first = std::min<int64_t>(n_rows, s.whole * s.row_warps * 32);
-  if (first > 0 && first < n_rows && mode != kLeafIds) { // (no allocation inside a capture: in one piece)
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
-    if (capturing != cudaStreamCaptureStatusNone && 2 * (size_t)s.chunks * (size_t)(n_rows - first) * sizeof(float) + 512 > f->scratch_bytes)
-      first = n_rows;
-  }
-  if (first > 0) {
-    const int rc = run_deep_rows(f, mode, d_rows, first, ld, d_out, d_partial, d_leaf_ids, stream, slot, s.row_warps, 1);
-    if (rc) return rc;
-  }
-  if (first < n_rows) {
-    const int rc = run_deep_rows(f, mode, d_rows + first * ld, n_rows - first, ld, d_out ? static_cast<float *>(d_out) + first : nullptr,
-                                 d_partial ? d_partial + first : nullptr, d_leaf_ids ? d_leaf_ids + first * f->df.num_trees : nullptr,
-                                 stream, slot, s.row_warps, s.chunks);
-    if (rc) return rc;
-  }
-  if (f->timing) {
-    CUDA_TRY(cudaEventRecord(f->ev1, stream));
-    f->ev_pending = true;
-  }
-  return TBK_OK;
-}
-
-// ---------------------------------------------------------------------------
-// Rank keys (rank_pack.h)
 
 // Memory for a call that is being captured.  The graph may be replayed at any time, so the memory is
 // the graph's: a user object of the graph, which everything instantiated from it holds as well,
@@ -910,6 +502,371 @@ int workspace_release(tbk_forest *f, tbk_forest::Workspace *w, cudaStream_t stre
   w->marked = true;
   return TBK_OK;
 }
+
+// Memory for a call's tree-chunk partial sums, behind the counters that rank keys use.
+int partials_acquire(tbk_forest *f, cudaStream_t stream, size_t floats, float **partials, tbk_forest::Workspace **out) {
+  const int rc = workspace_acquire(f, stream, tb::kRankArrivalBytes + floats * sizeof(float), out);
+  if (rc == TBK_OK) *partials = reinterpret_cast<float *>((*out)->mem + tb::kRankArrivalBytes);
+  return rc;
+}
+
+// A copy from pageable memory may return before its data has reached the device, and a memset does:
+// both are work of the legacy stream, which non-blocking streams don't wait for.
+int uploads_done() {
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  return TBK_OK;
+}
+
+int ensure_orig(tbk_forest *f) {
+  if (f->orig_ready) return TBK_OK;
+  const auto &p = f->packed;
+  if (!f->d_orig_node) CUDA_TRY(cudaMalloc(&f->d_orig_node, std::max<size_t>(4, p.orig_node.size() * 4)));
+  CUDA_TRY(cudaMemcpy(f->d_orig_node, p.orig_node.data(), p.orig_node.size() * 4, cudaMemcpyHostToDevice));
+  if (!f->d_orig_off) CUDA_TRY(cudaMalloc(&f->d_orig_off, std::max<size_t>(8, p.orig_off.size() * 8)));
+  CUDA_TRY(cudaMemcpy(f->d_orig_off, p.orig_off.data(), p.orig_off.size() * 8, cudaMemcpyHostToDevice));
+  const int rc = uploads_done();
+  f->orig_ready = rc == TBK_OK;
+  return rc;
+}
+
+enum Mode { kPredict, kPartial, kLeafIds };
+
+int quant_smem_bytes(int num_features) {
+  return tb::kQBarBytes + tb::kQRingBytes + tb::kQLeafTableBytes + tb::quant_key_tile_bytes(num_features);
+}
+
+// Tiles of 32 rows that the narrow-row kernel can stage together (0: the rows are too wide for it).
+int quant_batch_tiles(const tbk_forest *f, int num_features) {
+  const int room = f->max_smem_optin - tb::kQBBarBytes - tb::kQBRingBytes;
+  const int fit = room / tb::quant_batch_tile_bytes(num_features);
+  return fit >= 4 ? std::min(fit, tb::kQBMaxTiles) : 0;
+}
+
+// One prediction with a 15-bit-key kernel: rows whose key tiles fit shared memory several at a
+// time go to the batch kernel (persistent blocks of 22 warps over batches of up to 16 tiles),
+// wide rows to the kernel that holds one tile (persistent blocks of 24 warps over tiles of 32 rows).
+int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out, int32_t out_kind,
+              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, float *fixed = nullptr, size_t fixed_floats = 0) {
+  const auto &q = f->qf;
+  const int64_t G = (int64_t)q.groups.size();
+  const int64_t tiles = (n_rows + 31) / 32;
+  const int max_batch = quant_batch_tiles(f, q.num_features);
+  const bool batched = max_batch > 0;
+  const bool multi = q.num_classes > 0;
+  if (multi && !batched) return fail(TBK_ERR_UNSUPPORTED, "multiclass forests in the key layout need rows narrow enough for the batch kernel");
+  // batch kernel: as many tiles per batch as still give every SM a batch
+  int R = 1;
+  if (batched) {
+    R = max_batch;
+    while (R > 1 && (tiles + R - 1) / R < (int64_t)f->num_sms) R = (R + 1) / 2;
+  }
+  const int64_t units = batched ? (tiles + R - 1) / R : tiles; // blocks' units of work along x
+  int64_t chunks = 1;
+  if (multi) chunks = 1; // a class must stay within one leaf warp's sequence of groups
+  else if (f->user.tree_chunks > 0) chunks = f->user.tree_chunks;
+  else if (batched) {
+    if (units < (int64_t)f->num_sms) chunks = ((int64_t)f->num_sms + units - 1) / units;
+  } else if (tiles < 2 * (int64_t)f->num_sms) chunks = (2 * (int64_t)f->num_sms + tiles - 1) / tiles;
+  // (batch kernel: a second pass over partial sums costs about ten microseconds, more than the
+  // walk of a small forest: trees are split only into chunks of at least 32 groups -- measured
+  // on 4 096 rows x 32 groups: 38 us in one chunk, 47 us in two -- unless the caller asks)
+  const int64_t max_chunks = !batched ? G : f->user.tree_chunks > 0 ? std::max<int64_t>(1, G / 2) : std::max<int64_t>(1, G / 32);
+  chunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(chunks, max_chunks), 65535));
+  if (fixed) chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, (int64_t)fixed_floats / n_rows));
+  const int gpc = (int)((G + chunks - 1) / chunks);
+  chunks = (G + gpc - 1) / gpc;
+  const bool vec4 = q.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0;
+  // One block per SM (shared memory allows no more).  With more units than blocks a block is
+  // persistent; the one-tile kernel then stages its next tile in tensor memory while it walks
+  // the current one, a path that reads rows with 16-byte loads.
+  const int64_t blocks_x = std::max<int64_t>(1, (int64_t)f->num_sms / chunks);
+  const int64_t grid_x = batched ? std::min(units, blocks_x) : (vec4 && tiles > blocks_x) ? blocks_x : tiles;
+  tb::LaunchPlan plan;
+  plan.row_warps = batched ? R : 1;
+  plan.tree_threads = tb::kQWalkers;
+  plan.rows_per_lane = 1;
+  plan.chunks = (int32_t)chunks;
+  plan.groups_per_chunk = gpc;
+  plan.staged = 1;
+  plan.cache_rows = 1;
+  plan.stage_bytes = tb::kQPiece;
+  plan.smem_bytes = batched ? tb::quant_batch_smem_bytes(q.num_features, R) : quant_smem_bytes(q.num_features);
+  plan.threads = batched ? tb::kQBThreads : tb::kQThreads;
+  plan.grid_x = grid_x;
+  f->last_plan = plan;
+
+  const bool need_partials = mode == kPartial || (mode == kPredict && chunks > 1);
+  float *partial_dst = nullptr;
+  tbk_forest::Workspace *ws = nullptr;
+  if (need_partials) {
+    if (mode == kPartial && chunks == 1) {
+      partial_dst = d_partial;
+    } else if (fixed) {
+      partial_dst = fixed;
+    } else {
+      const int rc = partials_acquire(f, stream, (size_t)chunks * n_rows, &partial_dst, &ws);
+      if (rc) return rc;
+    }
+  }
+  tb::QuantParams p{};
+  p.node_plane = f->d_qnode;
+  p.leaf_plane = f->d_qleaf;
+  p.exact_plane = f->d_qexact;
+  p.groups = f->d_qgroups;
+  p.tree_index = f->d_qtree_index;
+  p.orig_leaf = f->d_qorig;
+  p.lo = f->d_qlo;
+  p.scale = f->d_qscale;
+  p.rows = d_rows;
+  p.n_rows = n_rows;
+  p.ld = ld;
+  p.partial = partial_dst;
+  p.out = d_out;
+  p.write_partial = need_partials ? 1 : 0;
+  p.leaf_ids = mode == kLeafIds ? d_leaf_ids : nullptr;
+  p.num_trees = q.num_trees;
+  p.num_groups = (int32_t)G;
+  p.groups_per_chunk = gpc;
+  p.num_features = q.num_features;
+  p.transform = q.transform;
+  p.initial_value = (float)q.initial_value;
+  p.vec4_ok = vec4 ? 1 : 0;
+  p.tiles_per_batch = R;
+  p.set_groups = f->d_qset_groups;
+  p.set_count[0] = f->qset_count[0];
+  p.set_count[1] = f->qset_count[1];
+  p.group_class = f->d_qgroup_class;
+  p.num_classes = q.num_classes;
+  p.out_kind = out_kind == TBK_OUT_I8 ? 1 : 0;
+  p.status = f->d_status;
+  p.tie_count = f->d_ties;
+  p.skip_first_copy = f->expire_next_wait ? 1 : 0;
+  p.wait_tries = f->expire_next_wait ? 2000u : 0u;
+  f->expire_next_wait = false;
+  // kernels specialised for forests whose groups all have 8 (or 6) levels; generic otherwise
+  using QuantKernel = void (*)(const tb::QuantParams);
+  const bool ids = mode == kLeafIds;
+  const int ud = (f->uniform_depth == 8 || f->uniform_depth == 6) ? f->uniform_depth : 0;
+  const QuantKernel qkernel =
+      multi ? (ud == 8 ? (ids ? tb::tb_walk_quant_batch_kernel<8, true, true> : tb::tb_walk_quant_batch_kernel<8, false, true>)
+                       : (ids ? tb::tb_walk_quant_batch_kernel<0, true, true> : tb::tb_walk_quant_batch_kernel<0, false, true>))
+      : batched
+          ? (ud == 8   ? (ids ? tb::tb_walk_quant_batch_kernel<8, true, false> : tb::tb_walk_quant_batch_kernel<8, false, false>)
+             : ud == 6 ? (ids ? tb::tb_walk_quant_batch_kernel<6, true, false> : tb::tb_walk_quant_batch_kernel<6, false, false>)
+                       : (ids ? tb::tb_walk_quant_batch_kernel<0, true, false> : tb::tb_walk_quant_batch_kernel<0, false, false>))
+      : ud == 8 ? (ids ? tb::tb_walk_quant_kernel<8, true> : tb::tb_walk_quant_kernel<8, false>)
+      : ud == 6 ? (ids ? tb::tb_walk_quant_kernel<6, true> : tb::tb_walk_quant_kernel<6, false>)
+                : (ids ? tb::tb_walk_quant_kernel<0, true> : tb::tb_walk_quant_kernel<0, false>);
+  CUDA_TRY(cudaFuncSetAttribute((const void *)qkernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
+  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
+  dim3 grid((unsigned)grid_x, (unsigned)chunks);
+  qkernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
+  CUDA_TRY(cudaGetLastError());
+  ++f->launches;
+  const int tpb = 256;
+  if (mode == kPredict && chunks > 1) {
+    tb::tb_finalize_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(
+        partial_dst, (int)chunks, n_rows, 1, 0, (float)q.initial_value, q.transform, d_out, TBK_OUT_F32);
+    CUDA_TRY(cudaGetLastError());
+    ++f->launches;
+  } else if (mode == kPartial && chunks > 1) {
+    tb::tb_sum_partials_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(partial_dst, (int)chunks, n_rows, d_partial);
+    CUDA_TRY(cudaGetLastError());
+    ++f->launches;
+  }
+  if (f->timing) {
+    CUDA_TRY(cudaEventRecord(f->ev1, stream));
+    f->ev_pending = true;
+  }
+  return ws ? workspace_release(f, ws, stream) : TBK_OK;
+}
+
+// Shared-memory plan of the deep-tree kernel: the most row warps (even -- one block per SM
+// either way, and more rows per tile mean fewer passes over the forest and more walks in
+// flight) whose key tile leaves room for a ring of at least 4 whole-tree pieces.
+bool deep_plan(int num_features, int max_depth, int smem_limit, int *row_warps, int *slots) {
+  const int64_t slot = 4ll * tb::deep_tree_words((uint32_t)std::max(max_depth, tb::kDeepMinDepth));
+  // four slots hold the node planes of the pair being walked and of the next one
+  for (int rw = 30; rw >= 2; rw -= 2) { // (the block has one more warp, the ring producer)
+    const int64_t keys = ((int64_t)num_features * 64 + tb::kDeepLeafBytes) * rw;
+    const int64_t room = (int64_t)smem_limit - 128 - keys;
+    const int64_t s = std::min<int64_t>(tb::kDeepMaxSlots, room / slot);
+    if (s >= 4) {
+      *row_warps = rw;
+      *slots = (int)s;
+      return true;
+    }
+  }
+  return false;
+}
+int deep_smem_bytes(const tbk_forest *f) {
+  return 128 + f->deep_slots * 4 * (int)tb::deep_tree_words((uint32_t)std::max(f->df.max_depth, tb::kDeepMinDepth)) +
+         (f->df.num_features * 64 + tb::kDeepLeafBytes) * f->deep_row_warps;
+}
+
+template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb::DeepParams) {
+  if (small)
+    return d12 ? (ids ? tb::tb_walk_deep_kernel<768, 12, WIDE, true> : tb::tb_walk_deep_kernel<768, 12, WIDE, false>)
+               : (ids ? tb::tb_walk_deep_kernel<768, 0, WIDE, true> : tb::tb_walk_deep_kernel<768, 0, WIDE, false>);
+  return d12 ? (ids ? tb::tb_walk_deep_kernel<1024, 12, WIDE, true> : tb::tb_walk_deep_kernel<1024, 12, WIDE, false>)
+             : (ids ? tb::tb_walk_deep_kernel<1024, 0, WIDE, true> : tb::tb_walk_deep_kernel<1024, 0, WIDE, false>);
+}
+
+// What counts is the waves of blocks and what a pair of trees takes a block: 300 pairs of 12 levels
+// 0.25 ms with 4 row warps, 0.34 with 18, 0.42 with 24, 0.50 with 30 (9 levels: 0.25, 0.31, 0.36, 0.42) -- all
+// latency up to about 18, then the shared-memory pipe as well.  The blocks that fill no whole wave
+// split the trees, into as many ranges as leave the least of their last wave empty.  Staging
+// the rows takes a block the time of 8 pairs and more, the second pass over partial sums that of 8.
+// (1048576 rows, 2000 trees, 18 row warps: 12.3 waves of blocks; 8000 rows, 387 trees of 9 levels: 63
+// blocks in three ranges were two waves.)
+DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
+  const int64_t G = (int64_t)f->df.pairs.size(), row_tiles = (n_rows + 31) / 32, SMs = f->num_sms;
+  DeepSplit best;
+  best.n_rows = n_rows;
+  double best_cost = -1.0;
+  for (int rw = std::min(4, f->deep_row_warps); rw <= f->deep_row_warps; ++rw) {
+    const int64_t blocks = (row_tiles + rw - 1) / rw, rest = blocks % SMs;
+    const double pair = rw <= 18 ? 0.7 + 0.0167 * rw : 1.0 + 0.02 * (rw - 18), start = 8.0 + 0.006 * f->df.num_features * rw;
+    for (int64_t c = 1; c <= std::min<int64_t>(G, std::max<int64_t>(8, (SMs + blocks - 1) / blocks)); ++c) {
+      const int64_t per = (G + c - 1) / c;
+      if ((G + per - 1) / per != c) continue;
+      const double waves = (double)((rest * c + SMs - 1) / SMs);
+      const double cost = pair * ((double)(blocks / SMs) * ((double)G + start) + waves * ((double)per + start)) + (c > 1 ? 8.0 : 0.0);
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best.row_warps = rw;
+        best.chunks = (int)c;
+        best.whole = c > 1 ? blocks - rest : 0;
+      }
+      if (rest == 0) break;
+    }
+  }
+  return best;
+}
+
+// One launch of the deep-tree kernel over `n_rows` rows, and the second pass over chunks.
+int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
+                  float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int rw, int64_t chunks) {
+  const auto &q = f->df;
+  const int64_t G = (int64_t)q.pairs.size();
+  const int64_t rows_per_block = 32 * rw;
+  const int64_t grid_x = (n_rows + rows_per_block - 1) / rows_per_block;
+  chunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(chunks, G), 65535));
+  const int gpc = (int)((G + chunks - 1) / chunks);
+  chunks = (G + gpc - 1) / gpc;
+  tb::LaunchPlan plan;
+  plan.row_warps = rw;
+  plan.tree_threads = 1;
+  plan.rows_per_lane = 1;
+  plan.chunks = (int32_t)chunks;
+  plan.groups_per_chunk = gpc;
+  plan.staged = 1;
+  plan.cache_rows = 1;
+  plan.stage_bytes = 4u * tb::deep_tree_words((uint32_t)std::max(q.max_depth, tb::kDeepMinDepth));
+  plan.smem_bytes = deep_smem_bytes(f);
+  plan.threads = 32 * (rw + 1); // row warps + the ring producer
+  plan.grid_x = grid_x;
+  f->last_plan = plan;
+
+  const bool need_partials = mode == kPartial || (mode == kPredict && chunks > 1);
+  float *partial_dst = nullptr;
+  tbk_forest::Workspace *ws = nullptr;
+  if (need_partials) {
+    if (mode == kPartial && chunks == 1) {
+      partial_dst = d_partial;
+    } else {
+      const int rc = partials_acquire(f, stream, (size_t)chunks * n_rows, &partial_dst, &ws);
+      if (rc) return rc;
+    }
+  }
+  tb::DeepParams p{};
+  p.node_plane = f->d_qnode;
+  p.leaf_plane = f->d_qleaf;
+  p.exact_plane = f->d_qexact;
+  p.pairs = f->d_qgroups;
+  p.tree_index = f->d_qtree_index;
+  p.orig_leaf = f->d_qorig;
+  p.lo = f->d_qlo;
+  p.scale = f->d_qscale;
+  p.rows = d_rows;
+  p.n_rows = n_rows;
+  p.ld = ld;
+  p.partial = partial_dst;
+  p.out = d_out;
+  p.write_partial = need_partials ? 1 : 0;
+  p.leaf_ids = mode == kLeafIds ? d_leaf_ids : nullptr;
+  p.num_trees = q.num_trees;
+  p.num_pairs = (int32_t)G;
+  p.pairs_per_chunk = gpc;
+  p.num_features = q.num_features;
+  p.transform = q.transform;
+  p.initial_value = (float)q.initial_value;
+  p.ring_slots = f->deep_slots;
+  p.slot_bytes = plan.stage_bytes;
+  p.tree_words = plan.stage_bytes / 4;
+  p.key_tile = 128u * (uint32_t)q.num_features;
+  p.leaf_off = (uint32_t)(plan.smem_bytes - tb::kDeepLeafBytes * f->deep_row_warps);
+  p.status = f->d_status;
+  p.tie_count = f->d_ties;
+  p.skip_first_copy = f->expire_next_wait ? 1 : 0;
+  p.wait_tries = f->expire_next_wait ? 2000u : 0u;
+  f->expire_next_wait = false;
+  // up to 24 warps (row warps + producer) the compiler may use 80 registers per thread, beyond that 64
+  // specialised for forests whose pairs all have 12 levels; generic otherwise
+  using DeepKernel = void (*)(const tb::DeepParams);
+  const bool d12 = f->uniform_depth == 12, ids = mode == kLeafIds, small = plan.threads <= 768;
+  const DeepKernel kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
+  CUDA_TRY(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
+  dim3 grid((unsigned)grid_x, (unsigned)chunks);
+  kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
+  CUDA_TRY(cudaGetLastError());
+  ++f->launches;
+  const int tpb = 256;
+  if (mode == kPredict && chunks > 1) {
+    tb::tb_finalize_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(
+        partial_dst, (int)chunks, n_rows, 1, 0, (float)q.initial_value, q.transform, d_out, TBK_OUT_F32);
+    CUDA_TRY(cudaGetLastError());
+    ++f->launches;
+  } else if (mode == kPartial && chunks > 1) {
+    tb::tb_sum_partials_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(partial_dst, (int)chunks, n_rows, d_partial);
+    CUDA_TRY(cudaGetLastError());
+    ++f->launches;
+  }
+  return ws ? workspace_release(f, ws, stream) : TBK_OK;
+}
+
+// One prediction with the deep-tree kernel.
+int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
+             float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream) {
+  DeepSplit &s = f->deep_split;
+  if (s.n_rows != n_rows) {
+    s = split_deep(f, n_rows);
+    if (f->user.tree_chunks > 0) { // (asked for: all rows)
+      s.whole = 0;
+      s.chunks = f->user.tree_chunks;
+    }
+  }
+  if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
+  const int64_t first = std::min<int64_t>(n_rows, s.whole * s.row_warps * 32);
+  if (first > 0) {
+    const int rc = run_deep_rows(f, mode, d_rows, first, ld, d_out, d_partial, d_leaf_ids, stream, s.row_warps, 1);
+    if (rc) return rc;
+  }
+  if (first < n_rows) {
+    const int rc = run_deep_rows(f, mode, d_rows + first * ld, n_rows - first, ld, d_out ? static_cast<float *>(d_out) + first : nullptr,
+                                 d_partial ? d_partial + first : nullptr, d_leaf_ids ? d_leaf_ids + first * f->df.num_trees : nullptr,
+                                 stream, s.row_warps, s.chunks);
+    if (rc) return rc;
+  }
+  if (f->timing) {
+    CUDA_TRY(cudaEventRecord(f->ev1, stream));
+    f->ev_pending = true;
+  }
+  return TBK_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Rank keys (rank_pack.h)
 
 // Dynamic shared memory beyond 48 KB has to be asked for once per kernel and device.
 int allow_smem(tbk_forest *f, const void *kernel) {
@@ -1332,7 +1289,7 @@ tb::LaunchPlan lane_launch_plan(const LanePlan &l) {
 
 // fixed: the partial sums go to this memory, whatever the number of chunks (tbk_predict_noalloc).
 int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out, int32_t out_kind,
-              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot, float *fixed = nullptr, size_t fixed_floats = 0) {
+              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, float *fixed = nullptr, size_t fixed_floats = 0) {
   const auto &pk = f->packed;
   const int W = std::max(1, pk.num_classes);
   const bool classes = pk.num_classes > 0;
@@ -1343,7 +1300,7 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   f->last_plan = lane_launch_plan(plan);
   const bool second_pass = fixed != nullptr || (mode != kLeafIds && plan.chunks > 1);
   float *partial = d_partial;
-  bool uses_scratch = false;
+  tbk_forest::Workspace *ws = nullptr;
   if (fixed) {
     partial = fixed;
     if ((size_t)plan.chunks * n_rows * W > fixed_floats)
@@ -1351,13 +1308,8 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
                   "scratch holds %zu; split the batch or use tbk_predict", (long long)n_rows, plan.chunks, W,
                   (size_t)plan.chunks * n_rows * W, fixed_floats);
   } else if (second_pass) {
-    const size_t need = ((size_t)plan.chunks * n_rows * W * sizeof(float) + 255) & ~(size_t)255;
-    int rc = ensure_scratch(f, 2 * need);
+    const int rc = partials_acquire(f, stream, (size_t)plan.chunks * n_rows * W, &partial, &ws);
     if (rc) return rc;
-    partial = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(f->d_scratch) + (size_t)slot * (f->scratch_bytes / 2));
-    rc = scratch_acquire(f, slot, stream);
-    if (rc) return rc;
-    uses_scratch = true;
   }
   tb::LaneParams p{};
   p.nodes = f->d_lnodes;
@@ -1405,13 +1357,12 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
     CUDA_TRY(cudaEventRecord(f->ev1, stream));
     f->ev_pending = true;
   }
-  if (uses_scratch) return scratch_release(f, slot, stream);
-  return TBK_OK;
+  return ws ? workspace_release(f, ws, stream) : TBK_OK;
 }
 
 // One prediction over device-resident rows.
 int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
-        int32_t out_kind, float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int slot = 0) {
+        int32_t out_kind, float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream) {
   const auto &pk = f->packed;
   if (n_rows < 0 || ld < pk.num_features) return fail(TBK_ERR_INVALID, "ld (%lld) is smaller than the row size (%d)", (long long)ld, pk.num_features);
   if (n_rows == 0) return TBK_OK;
@@ -1423,9 +1374,9 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
   }
   CUDA_TRY(cudaSetDevice(f->device));
   if (f->rank) return run_rank(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
-  if (f->lanes) return run_lanes(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream, slot);
-  if (f->quant) return run_quant(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream, slot);
-  if (f->deep) return run_deep(f, mode, d_rows, n_rows, ld, d_out, d_partial, d_leaf_ids, stream, slot);
+  if (f->lanes) return run_lanes(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
+  if (f->quant) return run_quant(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
+  if (f->deep) return run_deep(f, mode, d_rows, n_rows, ld, d_out, d_partial, d_leaf_ids, stream);
 
   tb::ForestShape shape{pk.num_features, pk.num_classes, (int64_t)pk.groups.size(), pk.max_group_bytes,
                         (int32_t)pk.lut.size(), pk.representation, pk.tile_size};
@@ -1442,7 +1393,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
   const int W = std::max(1, pk.num_classes);
   const bool need_partials = mode == kPartial || (mode == kPredict && plan.chunks > 1);
   float *partial_dst = nullptr;
-  bool uses_scratch = false;
+  tbk_forest::Workspace *ws = nullptr;
   if (mode == kLeafIds) {
     int rc = ensure_orig(f);
     if (rc) return rc;
@@ -1450,14 +1401,8 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
     if (mode == kPartial && plan.chunks == 1) {
       partial_dst = d_partial;
     } else {
-      // two slots, so that the two streams of the host pipeline never share partials
-      const size_t need = ((size_t)plan.chunks * n_rows * W * sizeof(float) + 255) & ~(size_t)255;
-      int rc = ensure_scratch(f, 2 * need);
+      const int rc = partials_acquire(f, stream, (size_t)plan.chunks * n_rows * W, &partial_dst, &ws);
       if (rc) return rc;
-      partial_dst = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(f->d_scratch) + (size_t)slot * (f->scratch_bytes / 2));
-      rc = scratch_acquire(f, slot, stream);
-      if (rc) return rc;
-      uses_scratch = true;
     }
   }
 
@@ -1523,8 +1468,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
     CUDA_TRY(cudaEventRecord(f->ev1, stream));
     f->ev_pending = true;
   }
-  if (uses_scratch) return scratch_release(f, slot, stream);
-  return TBK_OK;
+  return ws ? workspace_release(f, ws, stream) : TBK_OK;
 }
 
 // (after a synchronisation with the forest's launches)
@@ -1635,7 +1579,7 @@ int predict_host_small(tbk_forest *f, const float *h_rows, int64_t n_rows, int64
   }
   f->inline_rows = h_rows;
   const int rc = run(f, kPredict, reinterpret_cast<const float *>(rows), n_rows, ld, f->d_small + results_at, out_kind, nullptr,
-                     nullptr, stream, 0);
+                     nullptr, stream);
   f->inline_rows = nullptr;
   bool idle = rc != TBK_OK;
   for (int64_t r = 0; r < n_rows && !idle; ++r)
@@ -2145,7 +2089,6 @@ int tbk_forest_free(tbk_forest *f) {
   pinned_pool().give_back_status(f->h_status);
   pinned_pool().give_back(f->h_small, f->small_capacity);
   cudaFree(f->d_small_in);
-  cudaFree(f->d_scratch);
   cudaFree(f->d_qnode);
   cudaFree(f->d_qleaf);
   cudaFree(f->d_qexact);
@@ -2165,8 +2108,6 @@ int tbk_forest_free(tbk_forest *f) {
     if (w.done) cudaEventDestroy(w.done);
   }
   for (auto &c : f->captured) cudaFree(c.memory.mem);
-  for (int i = 0; i < 2; ++i)
-    if (f->scratch_done[i]) cudaEventDestroy(f->scratch_done[i]);
   if (f->ev0) cudaEventDestroy(f->ev0);
   if (f->ev1) cudaEventDestroy(f->ev1);
   delete f;
@@ -2351,7 +2292,7 @@ int tbk_predict_host(tbk_forest *f, const float *h_rows, int64_t n_rows, int64_t
       rc = fail(TBK_ERR_CUDA, "host-to-device copy: %s", cudaGetErrorString(e));
       break;
     }
-    rc = run(f, kPredict, reinterpret_cast<const float *>(f->d_in[s]), n, ld, f->d_res[s], out_kind, nullptr, nullptr, stream, s & 1);
+    rc = run(f, kPredict, reinterpret_cast<const float *>(f->d_in[s]), n, ld, f->d_res[s], out_kind, nullptr, nullptr, stream);
     if (rc != TBK_OK) break;
     e = cudaMemcpyAsync(out_pinned ? out + (size_t)(c * chunk) * out_elt : f->h_res[s], f->d_res[s], (size_t)n * out_elt, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaEventRecord(f->slot_done[s], stream);
@@ -2471,9 +2412,9 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
     return run_rank(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, reinterpret_cast<unsigned char *>(scratch),
                     kNoAllocScratchFloats * sizeof(float));
   if (f->quant)
-    return run_quant(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, 0, scratch, kNoAllocScratchFloats);
+    return run_quant(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, scratch, kNoAllocScratchFloats);
   if (f->lanes)
-    return run_lanes(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, 0, scratch, kNoAllocScratchFloats);
+    return run_lanes(f, kPredict, d_rows, n_rows, ld, d_out, out_kind, nullptr, nullptr, stream, scratch, kNoAllocScratchFloats);
 
   tb::ForestShape shape{pk.num_features, pk.num_classes, (int64_t)pk.groups.size(), pk.max_group_bytes,
                         (int32_t)pk.lut.size(), pk.representation, pk.tile_size};
