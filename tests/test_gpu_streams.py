@@ -175,3 +175,39 @@ def test_memory_of_captured_calls_lives_as_long_as_their_graphs(layout):
     assert min(free[8:]) >= free[0] - 8 * keys
     assert torch.equal(df.predict(dX[:sizes[0]]), want[0])
     df.check_status()
+
+
+def test_forests_of_one_kernel_and_different_sizes_in_two_threads():
+    """The same kernels, launched by two threads with different amounts of shared memory."""
+    forests = []
+    for layout, rows, features in (("tiles", 64, 28), ("tiles", 64, 90), ("rounded_wide", 64, 700), ("rounded_wide", 64, 1500),
+                                   ("deep", 64, 20), ("deep", 64, 60)):
+        trees, levels, _, _, options = LAYOUTS[layout]
+        marg = synth.Marginal("normal", features)
+        f = synth.generate_forest(features, 16, levels, features, 0.1, 0.1, marg)
+        X = torch.from_numpy(marg.sample_rows(np.random.Generator(np.random.PCG64(1)), rows)).cuda()
+        df = kernels.DeviceForest(f, **dict(dict(representation="auto"), **options))
+        forests.append((df, X, df.predict(X).clone()))
+    torch.cuda.synchronize()
+    wrong, start = [], threading.Barrier(2)
+
+    def work(mine):
+        stream = torch.cuda.Stream()
+        outs = [torch.zeros_like(want) for _, _, want in mine]
+        torch.cuda.synchronize()
+        start.wait()
+        try:
+            for i in range(9000):
+                df, X, _ = mine[i % len(mine)]
+                _predict_on(df, X, outs[i % len(mine)], stream.cuda_stream)
+        except kernels.TbkError as e:
+            wrong.append(str(e))
+        stream.synchronize()
+        wrong.extend("values" for out, (_, _, want) in zip(outs, mine) if not torch.equal(out, want))
+
+    threads = [threading.Thread(target=work, args=(forests[i::2],)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[0]

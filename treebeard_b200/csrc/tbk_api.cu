@@ -392,6 +392,16 @@ KernelFn pick_kernel(int rep, int ts, int rpl, bool staged, bool cached) {
   }
 }
 
+// Dynamic shared memory beyond 48 KB has to be asked for once per kernel and device.  All forests ask for
+// the most there is: what one asked for just before a launch, a smaller one of another thread would take back.
+int allow_smem(tbk_forest *f, const void *kernel) {
+  for (const void *k : f->smem_allowed)
+    if (k == kernel) return TBK_OK;
+  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f->max_smem_optin));
+  f->smem_allowed.push_back(kernel);
+  return TBK_OK;
+}
+
 // Memory for a call that is being captured.  The graph may be replayed at any time, so the memory is
 // the graph's: a user object of the graph, which everything instantiated from it holds as well,
 // tells when the last of them is gone (and its replays done).  The memory then serves the next capture, or
@@ -657,7 +667,7 @@ int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
       : ud == 8 ? (ids ? tb::tb_walk_quant_kernel<8, true> : tb::tb_walk_quant_kernel<8, false>)
       : ud == 6 ? (ids ? tb::tb_walk_quant_kernel<6, true> : tb::tb_walk_quant_kernel<6, false>)
                 : (ids ? tb::tb_walk_quant_kernel<0, true> : tb::tb_walk_quant_kernel<0, false>);
-  CUDA_TRY(cudaFuncSetAttribute((const void *)qkernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
+  if (const int rc = allow_smem(f, (const void *)qkernel)) return rc;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
   qkernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
@@ -816,7 +826,7 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   using DeepKernel = void (*)(const tb::DeepParams);
   const bool d12 = f->uniform_depth == 12, ids = mode == kLeafIds, small = plan.threads <= 768;
   const DeepKernel kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
-  CUDA_TRY(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
+  if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
   kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
   CUDA_TRY(cudaGetLastError());
@@ -867,15 +877,6 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
 
 // ---------------------------------------------------------------------------
 // Rank keys (rank_pack.h)
-
-// Dynamic shared memory beyond 48 KB has to be asked for once per kernel and device.
-int allow_smem(tbk_forest *f, const void *kernel) {
-  for (const void *k : f->smem_allowed)
-    if (k == kernel) return TBK_OK;
-  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f->max_smem_optin));
-  f->smem_allowed.push_back(kernel);
-  return TBK_OK;
-}
 
 // bytes of keys per row
 bool rank_tiled(int num_features) { return num_features > tb::kRankRowFeatures; }
@@ -1445,7 +1446,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
   p.class_regs = plan.class_regs;
 
   KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan.rows_per_lane, plan.staged, plan.cache_rows);
-  CUDA_TRY(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
+  if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
   fn<<<grid, block, plan.smem_bytes, stream>>>(p);
@@ -2462,7 +2463,7 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   p.status = f->d_status;
   p.class_regs = 0; // class sums go through the shared-memory table the plan has sized
   KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan.rows_per_lane, plan.staged, plan.cache_rows);
-  CUDA_TRY(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem_bytes));
+  if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
   fn<<<grid, block, plan.smem_bytes, stream>>>(p);
   CUDA_TRY(cudaGetLastError());
