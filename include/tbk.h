@@ -96,6 +96,11 @@ typedef struct tbk_schedule {
   int32_t reserved[4];
 } tbk_schedule;
 
+/* where and how a packed forest lies on the device (tbk_forest_info.layout): node tiles over fp32
+ * rows; ranks of row values among a feature's thresholds; rounded keys; rounded keys with whole-tree
+ * stages (9 to 12 levels); nodes in global memory, every lane at its own pace */
+enum { TBK_LAYOUT_TILES = 0, TBK_LAYOUT_RANK_KEYS = 1, TBK_LAYOUT_ROUNDED_KEYS = 2, TBK_LAYOUT_DEEP_KEYS = 3, TBK_LAYOUT_LANES = 4 };
+
 typedef struct tbk_forest tbk_forest; /* opaque: packed forest resident on a device */
 
 typedef struct tbk_forest_info {
@@ -104,11 +109,12 @@ typedef struct tbk_forest_info {
   int32_t max_depth;         /* decision levels on the deepest root-to-leaf path */
   int32_t num_features, num_classes, transform;
   int32_t device;
-  tbk_schedule schedule;     /* the schedule the selector settled on */
+  tbk_schedule schedule;     /* of the last launch; before the first one, of the hinted batch */
   int32_t staged;            /* 1 if tree groups are staged through shared memory */
   int32_t smem_bytes;        /* dynamic shared memory per block of the walk kernel */
   int32_t threads_per_block;
-  int32_t reserved[8];
+  int32_t reserved[7];
+  int32_t layout;            /* TBK_LAYOUT_* */
 } tbk_forest_info;
 
 /* Packs the forest in the requested representation and uploads it to `device`.

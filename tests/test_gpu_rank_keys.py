@@ -125,3 +125,24 @@ def test_widest_rank_key_rows_under_the_deepest_trees(features, rows):
     got = df.predict(dX)
     df.check_status()
     assert_predictions_close(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("features,rows,threads,rows_per_block", [
+    (28, 1, 32 * 3, 4), (28, 5, 32 * 5, 12), (28, 80, 32 * 22, 80), (28, 148 * 320, 32 * 22, 320), (90, 300, None, None),
+    (90, 50003, None, None), (511, 2000, 32 * 6, 128)])
+def test_the_launch_that_is_reported_is_the_one_that_ran(features, rows, threads, rows_per_block):
+    """A walker warp per four rows of a unit (one chunk asked for: the units then come from the rows alone)
+    or per share of a quad, and two warps that copy."""
+    f, marg = _forest(64, 8, features)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=70000, tree_chunks=1)
+    df.predict(torch.from_numpy(_rows(f, marg, rows)).cuda())
+    df.check_status()
+    info = df.info()
+    s = info.schedule
+    assert info.layout == kernels.LAYOUT_RANK_KEYS and s.tree_chunks == 1
+    if threads:
+        assert (info.threads_per_block, s.rows_per_block) == (threads, rows_per_block)
+    if features > 64:
+        assert s.rows_per_block % 128 == 0 and info.threads_per_block == 32 * (s.rows_per_block // 128 * s.tree_threads + 2)
+    else:
+        assert s.tree_threads == 1

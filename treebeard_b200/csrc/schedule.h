@@ -27,6 +27,7 @@ struct LaunchPlan {
   int32_t row_warps = 1;     // warps along the row dimension of a block
   int32_t tree_threads = 1;  // warps sharing one row tile (1, 2, 4, 8 or 16)
   int32_t rows_per_lane = 1; // rows a lane walks in lock-step (1 or 2)
+  int32_t rows_per_block = 0; // where that is not 32 x row warps x rows per lane
   int32_t chunks = 1;        // grid.y
   int32_t groups_per_chunk = 1;
   int32_t staged = 0;        // tree groups staged through shared memory

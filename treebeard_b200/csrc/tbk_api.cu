@@ -1013,10 +1013,19 @@ RankPlan plan_rank(tbk_forest *f, int64_t n_rows, bool leaf_ids) { // (a server'
   return f->rank_plan;
 }
 
-tb::LaunchPlan rank_launch_plan(const RankPlan &r) {
+// Walker warps of a launch over `n_rows` rows.  A batch of less than a unit gets only as many as the rows
+// -- or ranking them with two values per thread -- can use.
+int rank_walkers(const tbk_forest *f, const RankPlan &r, int64_t n_rows) {
+  if (r.quads) return r.walkers;
+  if (n_rows >= tb::kRWUnitRows) return tb::kRWWalkers;
+  return (int)std::min<int64_t>(tb::kRWWalkers, std::max((n_rows + 3) / 4, (n_rows * f->rf.num_features + 63) / 64));
+}
+
+tb::LaunchPlan rank_launch_plan(const RankPlan &r, int walkers) {
   tb::LaunchPlan plan;
-  plan.row_warps = r.quads ? 4 * r.quads : std::max(1, tb::kRWUnitRows * r.units / 32);
-  plan.tree_threads = tb::kRWWalkers;
+  plan.row_warps = r.quads ? r.quads : walkers;
+  plan.rows_per_block = r.quads ? 128 * r.quads : 4 * walkers * r.units;
+  plan.tree_threads = walkers / plan.row_warps;
   plan.rows_per_lane = 1;
   plan.chunks = r.chunks;
   plan.groups_per_chunk = r.per_chunk;
@@ -1024,7 +1033,7 @@ tb::LaunchPlan rank_launch_plan(const RankPlan &r) {
   plan.cache_rows = 1;
   plan.stage_bytes = r.stage_bytes;
   plan.smem_bytes = r.smem;
-  plan.threads = tb::kRWThreads;
+  plan.threads = 32 * (walkers + 2);
   plan.grid_x = r.grid_x;
   return plan;
 }
@@ -1147,7 +1156,9 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     pass = std::max<int64_t>(128, pass / 256 * 128);
     plan = plan_rank(f, pass, mode == kLeafIds);
   }
-  f->last_plan = rank_launch_plan(plan);
+  const bool tiled = rank_tiled(q.num_features);
+  const int walkers = rank_walkers(f, plan, n_rows);
+  f->last_plan = rank_launch_plan(plan, walkers);
   tbk_forest::Workspace *ws = nullptr;
   int rc = TBK_OK;
   if (fixed) CUDA_TRY(cudaMemsetAsync(fixed, 0, tb::kRankArrivalBytes, stream)); // (others write it too)
@@ -1155,12 +1166,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   if (rc) return rc;
   unsigned char *const mem = fixed ? fixed : ws->mem;
   unsigned char *keys = mem + tb::kRankArrivalBytes;
-  // one unit of rows per block: the variant for small batches, with only as many walker warps as
-  // the rows -- or ranking them with two values per thread -- can use
-  const bool tiled = rank_tiled(q.num_features), small = !tiled && plan.units == 1;
-  int walkers = tb::kRWWalkers;
-  if (tiled) walkers = plan.walkers;
-  else if (n_rows < tb::kRWUnitRows) walkers = (int)std::min<int64_t>(walkers, std::max((n_rows + 3) / 4, (n_rows * q.num_features + 63) / 64));
+  const bool small = !tiled && plan.units == 1; // one unit of rows per block: the variant for small batches
   const int unit_rows = tiled ? 128 : 4 * walkers;
   const RankKernel kernel = tiled ? (mode == kLeafIds ? tb::tb_walk_rank_tiles_kernel<4, true> : tb::tb_walk_rank_tiles_kernel<4, false>)
                             : pick_rank_kernel(S, small, q.whole_compare != 0, kmode);
@@ -1984,7 +1990,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     plan_rank_tables(f);
     const int64_t rows = std::min(batch_hint > 0 ? batch_hint : 65536, rank_rows_per_pass(f));
     const RankPlan plan = plan_rank(f, rows, false);
-    f->last_plan = rank_launch_plan(plan);
+    f->last_plan = rank_launch_plan(plan, rank_walkers(f, plan, rows));
     if (batch_hint > 0) { // the batches to come are known: their workspace is laid out now
       tbk_forest::Workspace &w = f->workspace[0];
       const size_t bytes = rank_workspace_bytes(f, plan, rows);
@@ -2136,11 +2142,12 @@ int tbk_forest_get_info(const tbk_forest *f, tbk_forest_info *info) {
   const tb::LaunchPlan &pl = f->last_plan;
   info->schedule.representation = p.representation;
   info->schedule.tile_size = p.tile_size;
-  info->schedule.rows_per_block = pl.row_warps * 32 * pl.rows_per_lane;
+  info->schedule.rows_per_block = pl.rows_per_block ? pl.rows_per_block : pl.row_warps * 32 * pl.rows_per_lane;
   info->schedule.rows_per_thread = pl.rows_per_lane;
   info->schedule.tree_threads = pl.tree_threads;
   info->schedule.tree_chunks = pl.chunks;
   info->schedule.cache_trees = pl.staged ? 1 : 2;
+  info->layout = f->rank ? TBK_LAYOUT_RANK_KEYS : f->quant ? TBK_LAYOUT_ROUNDED_KEYS : f->deep ? TBK_LAYOUT_DEEP_KEYS : f->lanes ? TBK_LAYOUT_LANES : TBK_LAYOUT_TILES;
   info->schedule.feature_bits = (f->rank || f->quant || f->deep) ? 16 : 32;
   info->staged = pl.staged;
   info->smem_bytes = pl.smem_bytes;

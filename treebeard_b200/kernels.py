@@ -12,6 +12,7 @@ from . import _lib
 
 REP_AUTO, REP_SPARSE, REP_ARRAY, REP_REORG = -1, 0, 1, 2
 OUT_F32, OUT_I8 = 0, 1
+LAYOUT_TILES, LAYOUT_RANK_KEYS, LAYOUT_ROUNDED_KEYS, LAYOUT_DEEP_KEYS, LAYOUT_LANES = range(5)   # of ForestInfoC
 REP_BY_NAME = {"auto": REP_AUTO, "sparse": REP_SPARSE, "gpu_sparse": REP_SPARSE, "array": REP_ARRAY,
                "gpu_array": REP_ARRAY, "reorg": REP_REORG, "gpu_reorg": REP_REORG}
 
@@ -40,7 +41,7 @@ class ForestInfoC(ctypes.Structure):
                 ("num_classes", ctypes.c_int32), ("transform", ctypes.c_int32),
                 ("device", ctypes.c_int32), ("schedule", ScheduleC),
                 ("staged", ctypes.c_int32), ("smem_bytes", ctypes.c_int32),
-                ("threads_per_block", ctypes.c_int32), ("reserved", ctypes.c_int32 * 8)]
+                ("threads_per_block", ctypes.c_int32), ("reserved", ctypes.c_int32 * 7), ("layout", ctypes.c_int32)]
 
 
 class TbkError(RuntimeError):
