@@ -275,8 +275,8 @@ def test_kernel_timing_api(tmp_path):
 
 @pytest.mark.parametrize("name", ["c1", "c2", "c3"])
 def test_sixteen_bit_key_kernel_is_exact(name):
-    """The wide-row kernel (rows staged as 16-bit keys) must select exactly the oracle's
-    leaves, ties, NaN and infinities included."""
+    """16-bit keys on request -- ranks for narrow rows (c1, c2), rounded keys for wide ones (c3) -- must
+    select exactly the oracle's leaves, ties, NaN and infinities included."""
     from treebeard_b200 import kernels
     forest, X = small_config(name)
     X = X.copy()
@@ -290,7 +290,8 @@ def test_sixteen_bit_key_kernel_is_exact(name):
     want, want_ids = oracle.predict(forest, X, leaf_ids=True)
     df = kernels.DeviceForest(forest, representation="reorg", feature_bits=16, batch_hint=len(X))
     info = df.info()
-    # wide rows: one key tile per block (24 warps); narrow rows: batches of tiles (20 warps)
+    assert info.layout == (kernels.LAYOUT_ROUNDED_KEYS if name == "c3" else kernels.LAYOUT_RANK_KEYS)
+    # wide rows: one key tile per block (24 warps); narrow rows: 20 walker warps and two that copy
     assert info.schedule.feature_bits == 16 and info.threads_per_block == (768 if name == "c3" else 704)
     dX = _dev(X)
     ids = df.predict_leaf_ids(dX).cpu().numpy()
@@ -312,8 +313,8 @@ def test_sixteen_bit_key_kernel_is_exact(name):
 
 
 def test_auto_representation_picks_keys_for_single_output_forests_of_up_to_eight_levels():
-    """"auto": keys for wide rows (one tile per block) and for narrow rows (batches of tiles,
-    multiclass forests included); fp32 tiles on request and for explicit representations."""
+    """"auto": rounded keys for wide rows and rank keys for narrow ones (multiclass forests included);
+    fp32 tiles on request and for explicit representations."""
     from treebeard_b200 import kernels
     wide, Xw = small_config("c3", rows=64)
     narrow, Xn = small_config("c2", rows=64)
@@ -321,6 +322,7 @@ def test_auto_representation_picks_keys_for_single_output_forests_of_up_to_eight
     a = kernels.DeviceForest(wide, representation="auto")
     b = kernels.DeviceForest(narrow, representation="auto")
     assert a.info().schedule.feature_bits == 16 and a.info().threads_per_block == 768
+    assert a.info().layout == kernels.LAYOUT_ROUNDED_KEYS and b.info().layout == kernels.LAYOUT_RANK_KEYS
     assert b.info().schedule.feature_bits == 16 and b.info().threads_per_block == 704
     assert kernels.DeviceForest(narrow, representation="auto", feature_bits=32).info().schedule.feature_bits == 32
     assert kernels.DeviceForest(narrow, representation="sparse").info().schedule.feature_bits == 32
@@ -331,8 +333,8 @@ def test_auto_representation_picks_keys_for_single_output_forests_of_up_to_eight
     assert_predictions_close(m.predict(_dev(Xm)).cpu().numpy(), want_m, multi, sums_m)
     assert_predictions_close(a.predict(_dev(Xw)).cpu().numpy(), oracle.predict(wide, Xw))
     assert_predictions_close(b.predict(_dev(Xn)).cpu().numpy(), oracle.predict(narrow, Xn))
-    # whole-number thresholds (integer-valued features: rows EQUAL thresholds all the time) become
-    # lattice features of the key layout: exact without a single tie on whole-number rows
+    # whole-number thresholds (integer-valued features: rows EQUAL thresholds all the time): a whole-number
+    # row value's rank is in the table, nothing is compared with thresholds
     import copy
     rounded = copy.copy(narrow)
     rounded.thr = np.where(narrow.left >= 0, np.round(narrow.thr * 4), narrow.thr).astype(np.float32)
@@ -347,9 +349,9 @@ def test_auto_representation_picks_keys_for_single_output_forests_of_up_to_eight
 
 @pytest.mark.parametrize("name,rows,chunks", [("c2", 100003, 0), ("c2", 100003, 3), ("c1", 77777, 0), ("c2", 5000, 0)])
 def test_batched_key_kernel_is_exact(name, rows, chunks):
-    """Narrow rows: the key tiles of up to 16 tiles are staged together and the forest streams
-    once per batch.  Full batches, persistent blocks with several batches, a ragged last
-    batch and tile, tree chunks, partial sums and leaf ids; ties, NaN and infinities included."""
+    """Narrow rows, on rank keys: full batches, persistent blocks with several batches, a ragged last
+    batch and unit, tree chunks, partial sums and leaf ids; ties, NaN and infinities included.
+    (Batches of rounded-key tiles: test_gpu_batch_keys.py.)"""
     from treebeard_b200 import kernels
     forest, X = small_config(name, rows=rows)
     X = X.copy()
@@ -364,6 +366,7 @@ def test_batched_key_kernel_is_exact(name, rows, chunks):
     df = kernels.DeviceForest(forest, representation="auto", batch_hint=rows, tree_chunks=chunks)
     info = df.info()
     assert info.schedule.feature_bits == 16 and info.threads_per_block == 704
+    assert info.layout == kernels.LAYOUT_RANK_KEYS
     dX = _dev(X)
     got = df.predict(dX).cpu().numpy()
     df.check_status()
@@ -596,7 +599,7 @@ def test_runner_rejects_buffers_on_different_sides(tmp_path):
 
 
 def test_sixteen_bit_keys_refuse_what_they_do_not_cover():
-    """Multiclass forests need rows narrow enough for the batch kernel."""
+    """Multiclass forests in 16-bit keys need rows narrow enough to be staged several tiles at a time."""
     from treebeard_b200 import kernels, synth
     wide = synth.generate_forest(40, 60, 6, 1800, 0.1, 0.1, synth.Marginal("normal", 1800), num_classes=3)
     with pytest.raises(kernels.TbkError):
@@ -605,8 +608,8 @@ def test_sixteen_bit_keys_refuse_what_they_do_not_cover():
 
 
 def test_batched_key_kernel_multiclass_on_continuous_features():
-    """Three classes over continuous features (ordinary keys, no lattice): an odd number of
-    classes (the two walker sets get two and one), rare ties resolved exactly."""
+    """Three classes over continuous features, on rank keys: class boundaries inside a group of trees,
+    values equal to thresholds."""
     from treebeard_b200 import kernels, synth
     marg = synth.Marginal("normal", 10)
     forest = synth.generate_forest(77, 93, 6, 10, 0.1, 0.1, marg, num_classes=3)
@@ -628,8 +631,8 @@ def test_batched_key_kernel_multiclass_on_continuous_features():
 
 @pytest.mark.parametrize("rows", [100003, 5000, 77])
 def test_batched_key_kernel_multiclass(rows):
-    """Multiclass forests on the batch kernel: classes laid out group by group, one walker set
-    per class, arg-max on the fly with the reference's tie rule; int8 and fp32 class ids."""
+    """26 classes over whole-number features, on rank keys: arg-max on the fly with the reference's tie
+    rule; int8 and fp32 class ids, per-class partial sums."""
     from treebeard_b200 import kernels
     forest, X = small_config("c4", rows=rows)
     X = X.copy()
@@ -645,6 +648,7 @@ def test_batched_key_kernel_multiclass(rows):
     df = kernels.DeviceForest(forest, representation="auto", feature_bits=16, batch_hint=rows)
     info = df.info()
     assert info.schedule.feature_bits == 16 and info.threads_per_block == 704
+    assert info.layout == kernels.LAYOUT_RANK_KEYS
     dX = _dev(X)
     got = df.predict(dX).cpu().numpy()
     df.check_status()
