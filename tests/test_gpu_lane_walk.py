@@ -62,6 +62,27 @@ def test_lane_walk(trees, levels, features, classes, rows):
     assert abs(float(out[0] - df.predict(dX)[0])) < 1e-5
 
 
+@pytest.mark.parametrize("trees,classes,rows", [(1000, 0, 65536), (2000, 0, 65536), (4000, 0, 2048), (60, 0, 65536), (1200, 3, 40000)])
+def test_long_lane_walks_round_their_sums_once(trees, classes, rows):
+    f, X = _case(trees, 14, 16, classes, rows, 0.25)
+    X = np.nan_to_num(X, nan=0.0, posinf=3.0)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows)
+    part = df.predict_partial(torch.from_numpy(X).cuda())[-3000:].double().cpu().numpy()
+    df.check_status()
+    info = df.info()
+    assert info.layout == kernels.LAYOUT_LANES
+    _, ids = oracle.predict(f, X[-3000:], leaf_ids=True)
+    leaves = f.thr[f.tree_off[:-1][None, :] + ids].astype(np.float64)
+    groups = [f.class_id == c for c in range(classes)] if classes else [np.ones(trees, bool)]
+    for c, g in enumerate(groups):
+        exact, got = leaves[:, g].sum(axis=1), part[:, c]
+        # half an ulp for every rounding, of a sum about as large as the result: a share's or a chunk's and
+        # the result's for long chains; one per leaf, of random sign, for chains of up to 64 leaves in fp32
+        chain = g.sum() / (info.schedule.tree_chunks * (1 if classes else info.schedule.tree_threads))
+        roundings = 3 if chain > 64 else 3 + np.sqrt(64)
+        assert np.linalg.norm(got - exact) <= roundings * 2.0 ** -24 * np.linalg.norm(exact)
+
+
 @pytest.mark.parametrize("tile,rows", [(2, 3001), (2, 20000)])
 def test_groups_that_fit_one_stage(tile, rows):
     f, X = _case(70, 8, 20, 0, rows, 0.1)

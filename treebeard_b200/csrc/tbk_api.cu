@@ -337,6 +337,7 @@ struct tbk_forest {
   uint2 *d_lnodes = nullptr;
   uint32_t *d_lroot = nullptr, *d_lclass_end = nullptr, *d_lclass_tree = nullptr;
   int32_t *d_ltree_index = nullptr, *d_lorig = nullptr;
+  int64_t lane_class_trees = 0; // of the largest class
   // one-tree-per-stage layout (deep trees); shares the device buffers of the key layout
   bool deep = false;
   tb::DeepForest df;
@@ -1342,8 +1343,11 @@ int run_lanes(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   p.shares = plan.shares;
   p.vec4_ok = (pk.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0) ? 1 : 0;
   using K = void (*)(const tb::LaneParams);
-  const K k = classes ? (mode == kLeafIds ? tb::tb_walk_lanes_kernel<true, true> : tb::tb_walk_lanes_kernel<true, false>)
-                      : (mode == kLeafIds ? tb::tb_walk_lanes_kernel<false, true> : tb::tb_walk_lanes_kernel<false, false>);
+  const bool longer = (classes ? (f->lane_class_trees + plan.chunks - 1) / plan.chunks
+                               : (pk.num_trees + plan.shares * plan.chunks - 1) / (plan.shares * plan.chunks)) > tb::kLaneShortChain;
+  const K k = mode == kLeafIds ? (classes ? tb::tb_walk_lanes_kernel<true, true, false> : tb::tb_walk_lanes_kernel<false, true, false>)
+              : classes        ? (longer ? tb::tb_walk_lanes_kernel<true, false, true> : tb::tb_walk_lanes_kernel<true, false, false>)
+                               : (longer ? tb::tb_walk_lanes_kernel<false, false, true> : tb::tb_walk_lanes_kernel<false, false, false>);
   int rc = allow_smem(f, (const void *)k);
   if (rc) return rc;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
@@ -1921,6 +1925,8 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     CUDA_TRY_F(upload(&f->d_lclass_end, q.class_end));
     std::vector<uint32_t> class_tree; // (end of every class's trees)
     for (uint32_t end : q.class_end) class_tree.push_back((uint32_t)(std::lower_bound(q.root.begin(), q.root.end(), end) - q.root.begin()));
+    for (size_t c = 0; c < class_tree.size(); ++c)
+      f->lane_class_trees = std::max<int64_t>(f->lane_class_trees, class_tree[c] - (c ? class_tree[c - 1] : 0u));
     CUDA_TRY_F(upload(&f->d_lclass_tree, class_tree));
     f->last_plan = lane_launch_plan(plan_lanes(f, batch_hint > 0 ? batch_hint : 65536, false));
     return done();
