@@ -914,16 +914,16 @@ int rank_stride(int num_features) {
   return rank_tiled(num_features) ? (num_features + 1) / 2 * 4 : num_features <= tb::kRankPairFeatures ? 64 : 128;
 }
 
-using RankKernel = void (*)(const tb::RankWalkParams);
-template <int S, int NR, bool WHOLE> RankKernel pick_rank(int mode) {
-  return mode == tb::kRankLeafIds ? tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankLeafIds>
-         : mode == tb::kRankClasses ? tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankClasses>
-                                    : tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankSums>;
+template <int S, int NR, bool WHOLE, bool INLINE> const void *pick_rank(int mode) {
+  return mode == tb::kRankLeafIds   ? (const void *)tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankLeafIds, INLINE>
+         : mode == tb::kRankClasses ? (const void *)tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankClasses, INLINE>
+                                    : (const void *)tb::tb_walk_rank_kernel<S, NR, WHOLE, tb::kRankSums, INLINE>;
 }
-RankKernel pick_rank_kernel(int stride, bool small, bool whole, int mode) {
-  if (small) return stride == 64 ? pick_rank<64, 4, true>(mode) : pick_rank<128, 4, true>(mode);
-  if (stride == 64) return whole ? pick_rank<64, 16, true>(mode) : pick_rank<64, 16, false>(mode);
-  return whole ? pick_rank<128, 16, true>(mode) : pick_rank<128, 16, false>(mode);
+const void *pick_rank_kernel(int stride, bool small, bool whole, bool inlined, int mode) {
+  if (inlined) return stride == 64 ? pick_rank<64, 4, true, true>(mode) : pick_rank<128, 4, true, true>(mode);
+  if (small) return stride == 64 ? pick_rank<64, 4, true, false>(mode) : pick_rank<128, 4, true, false>(mode);
+  if (stride == 64) return whole ? pick_rank<64, 16, true, false>(mode) : pick_rank<64, 16, false, false>(mode);
+  return whole ? pick_rank<128, 16, true, false>(mode) : pick_rank<128, 16, false, false>(mode);
 }
 
 // How many quads of tiles a block of the tiled kernel takes at a time, with how many walker warps.
@@ -1198,11 +1198,15 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   unsigned char *keys = mem + tb::kRankArrivalBytes;
   const bool small = !tiled && plan.units == 1; // one unit of rows per block: the variant for small batches
   const int unit_rows = tiled ? 128 : 4 * walkers;
-  const RankKernel kernel = tiled ? (mode == kLeafIds ? tb::tb_walk_rank_tiles_kernel<4, true> : tb::tb_walk_rank_tiles_kernel<4, false>)
-                            : pick_rank_kernel(S, small, q.whole_compare != 0, kmode);
-  rc = allow_smem(f, (const void *)kernel);
+  // rows of a small host batch travel with the launch
+  const bool inlined = f->inline_rows && small && n_rows * q.num_features <= tb::kRankInline;
+  const void *const kernel = tiled ? (mode == kLeafIds ? (const void *)tb::tb_walk_rank_tiles_kernel<4, true>
+                                                       : (const void *)tb::tb_walk_rank_tiles_kernel<4, false>)
+                                   : pick_rank_kernel(S, small, q.whole_compare != 0, inlined, kmode);
+  rc = allow_smem(f, kernel);
   if (rc) return rc;
-  tb::RankWalkParams p{};
+  tb::RankWalkInlineParams p;
+  static_cast<tb::RankWalkParams &>(p) = tb::RankWalkParams{};
   p.node_plane = f->d_rnode;
   p.leaf_plane = reinterpret_cast<const uint32_t *>(f->d_rleaf);
   if (mode == kLeafIds) p.leaf_plane = reinterpret_cast<const uint32_t *>(f->d_rorig);
@@ -1235,16 +1239,12 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     // Up to four values per walker thread: the walk ranks its rows itself.  (Every chunk's blocks
     // read the rows again, which host memory is too slow for.)
     const int64_t block_rows = std::min<int64_t>(n, (int64_t)plan.units * unit_rows);
-    const bool inlined = f->inline_rows && batches == 1 && n * q.num_features <= tb::kRankInline;
     const bool fused = !tiled && pass == n_rows && plan.units < tb::kRWBatchUnits && block_rows * q.num_features <= 128 * walkers &&
                        (!f->inline_rows || inlined || plan.chunks == 1);
     if (fused) {
       p.ranking = rank_rows_params(f, d_rows, n, ld, nullptr);
-      if (inlined) {
-        p.inline_values = (uint32_t)(n * q.num_features);
-        for (int64_t r = 0; r < n; ++r)
-          std::memcpy(p.inline_rows + r * q.num_features, f->inline_rows + r * ld, (size_t)q.num_features * 4);
-      }
+      for (int64_t r = 0; inlined && r < n; ++r)
+        std::memcpy(p.inline_rows + r * q.num_features, f->inline_rows + r * ld, (size_t)q.num_features * 4);
     } else {
       rc = launch_rank_rows(f, d_rows + done * ld, n, ld, reinterpret_cast<uint16_t *>(keys), stream);
       if (rc) return rc;
@@ -1267,7 +1267,8 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = fused ? 0 : 1;
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p));
+    void *args[] = {&p}; // (of which a kernel takes its own type's bytes)
+    CUDA_TRY(cudaLaunchKernelExC(&cfg, kernel, args));
     ++f->launches;
   }
   if (f->timing) {
