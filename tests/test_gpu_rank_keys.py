@@ -146,3 +146,21 @@ def test_the_launch_that_is_reported_is_the_one_that_ran(features, rows, threads
         assert s.rows_per_block % 128 == 0 and info.threads_per_block == 32 * (s.rows_per_block // 128 * s.tree_threads + 2)
     else:
         assert s.tree_threads == 1
+
+
+@pytest.mark.parametrize("features,rows", [(28, 1), (28, 9), (28, 10), (64, 4), (3, 79), (3, 80), (3, 81), (3, 85), (2, 128),
+                                           (1, 161), (1, 256), (1, 257), (5, 300), (33, 640)])
+def test_small_host_batches_on_either_side_of_what_travels_with_the_launch(features, rows):
+    """Up to 256 values in the launch parameters, over one block of rows or several; beyond that rows in mapped
+    memory.  A row stride that is wider than the row."""
+    f, marg = _forest(70, 6, features, p=0.0 if features == 1 else 0.2)
+    X = _rows(f, marg, rows)
+    X[np.isnan(X)] = 0.5
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows)
+    wide = np.full((rows, features + 3), 7.5, np.float32)
+    wide[:, :features] = X
+    want = oracle.predict(f, X)
+    for _ in range(2):
+        assert_predictions_close(df.predict_host(X), want)
+        assert_predictions_close(df.predict_host(wide[:, :features]), want)
+    df.check_status()

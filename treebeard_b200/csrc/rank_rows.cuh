@@ -34,21 +34,59 @@ struct RankRowsParams {
   unsigned long long *searched; // statistics: values that were compared with thresholds
 };
 
-// Rank of one value, tables in global memory (see tb_rank_rows, which ranks several in lock-step).
-__device__ __forceinline__ uint32_t rank_value(float x, const DevRankFeature *feature, const uint16_t *lut, const float *thr,
-                                               unsigned &searched) {
-  const uint4 a = __ldg(reinterpret_cast<const uint4 *>(feature)), b = __ldg(reinterpret_cast<const uint4 *>(feature) + 1);
-  const float lo = __uint_as_float(a.x), scale = __uint_as_float(a.y), top = __uint_as_float(a.z);
-  const float y = fmaxf(fminf(__fmul_rn(__fsub_rn(x, lo), scale), top), 0.f);
-  const uint16_t *l = lut + a.w + (uint32_t)y;
-  uint32_t s = __ldg(l), e = __ldg(l + 1);
-  if (b.w && x == floorf(x)) return x < lo ? 0u : e;
-  searched += s < e;
-  for (uint32_t step = s < e ? 1u << (31 - __clz(e - s)) : 0u; step; step >>= 1) {
-    const uint32_t m = s + step;
-    if (m <= e && !(x < __ldg(thr + b.x + m - 1u))) s = m;
+// Ranks up to N values of a block's rows, tables in global memory: number i0, i0 + stride, ... of `count`, counted
+// row by row.  value(row, feature) gives one, use(row, feature, rank) takes its rank.  They go through their
+// look-ups and search steps in lock-step, as in tb_rank_rows: each of these is an L2 round trip that depends
+// on the last one.
+template <int N, typename Value, typename Use>
+__device__ __forceinline__ void rank_values(const RankRowsParams &r, uint32_t i0, uint32_t stride, uint32_t count, unsigned &searched,
+                                            Value value, Use use) {
+  const uint32_t F = (uint32_t)r.num_features, rows = stride / F, rest = stride - rows * F; // (from one value to the next)
+  float x[N];
+  uint32_t row[N], f[N], s[N], e[N], longest = 0;
+  const float *thr[N]; // of the feature, less one
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    if (k == 0) {
+      row[k] = i0 / F;
+      f[k] = i0 - row[k] * F;
+    } else {
+      const bool over = f[k - 1] + rest >= F;
+      row[k] = row[k - 1] + rows + (over ? 1u : 0u);
+      f[k] = f[k - 1] + rest - (over ? F : 0u);
+    }
+    x[k] = 0.f;
+    s[k] = e[k] = 0;
+    thr[k] = r.thr;
+    if (i0 + k * stride < count) {
+      const uint4 *feature = reinterpret_cast<const uint4 *>(r.features + f[k]);
+      const uint4 a = __ldg(feature), b = __ldg(feature + 1);
+      x[k] = value(row[k], f[k]);
+      const float lo = __uint_as_float(a.x), scale = __uint_as_float(a.y), top = __uint_as_float(a.z);
+      const float y = fmaxf(fminf(__fmul_rn(__fsub_rn(x[k], lo), scale), top), 0.f);
+      const uint16_t *l = r.lut + a.w + (uint32_t)y;
+      s[k] = __ldg(l);
+      e[k] = __ldg(l + 1);
+      thr[k] = r.thr + b.x - 1;
+      if (b.w && x[k] == floorf(x[k])) s[k] = e[k] = x[k] < lo ? 0u : e[k];
+    }
   }
-  return s;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    searched += s[k] < e[k];
+    longest = max(longest, e[k] - s[k]);
+  }
+  for (uint32_t step = longest ? 1u << (31 - __clz(longest)) : 0u; step; step >>= 1) {
+    float t[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) t[k] = s[k] + step <= e[k] ? __ldg(thr[k] + s[k] + step) : INFINITY;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (s[k] + step <= e[k] && !(x[k] < t[k])) s[k] += step;
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (i0 + k * stride < count) use(row[k], f[k], s[k]);
 }
 
 // A warp that ranks a piece of a tile reads its 32 x 8 values as 32-byte stretches of rows and turns

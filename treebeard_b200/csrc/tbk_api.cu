@@ -989,7 +989,11 @@ RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
 // slowest block costs in clocks.  A group takes a warp about 2 D - 1 shared-memory wavefronts per
 // row and 20 warps share the pipe; a few hundred clocks go into the hand-off and the chain of
 // dependent loads, and the stage's copy needs its time too (70 bytes a clock).  A block starts up
-// for about 4000 clocks, and combining chunks adds about 1500.
+// for about 4000 clocks, and combining chunks adds about as much (a fence, an arrival, partial sums out and
+// back: 64 trees of 6 levels over 10 features, 3000 rows, 10.3 us in two chunks, 8.2 in one; with 1500 clocks
+// 34 of 252 small shapes were slower than one launch over rounded keys had been, with 4000 27; 3000 to 5500
+// measure within 1 % of each other over all of them, 7500 2 % slower).
+constexpr double kCombineClocks = 4000.0;
 RankPlan make_rank_plan(const tbk_forest *f, int64_t n_rows, bool leaf_ids) {
   const auto &q = f->rf;
   const int G = (int)q.groups.size(), S = rank_stride(q.num_features);
@@ -1024,7 +1028,7 @@ RankPlan make_rank_plan(const tbk_forest *f, int64_t n_rows, bool leaf_ids) {
       const int per = (parts + c - 1) / c, chunks = (parts + per - 1) / per;
       const double groups = multi ? (double)G * per / parts + 1.0 : per;
       const double waves = (double)((x * chunks + f->num_sms - 1) / f->num_sms);
-      const double cost = waves * (4000.0 + groups * group_clocks(u)) + 1500.0;
+      const double cost = waves * (4000.0 + groups * group_clocks(u)) + kCombineClocks;
       if (cost < best) {
         best = cost;
         set(x, c);

@@ -405,14 +405,22 @@ __global__ void __launch_bounds__(kRWThreads, 1)
         const int F = r.num_features;
         const uint32_t values = (uint32_t)(min((long long)unit1 * UR, p.n_rows) - (long long)unit0 * UR) * (uint32_t)F;
         unsigned searched = 0;
-        for (uint32_t i = tid; i < values; i += 32 * NW) {
-          const uint32_t q = i / (uint32_t)F, f = i - q * (uint32_t)F;
-          float x;
-          if constexpr (INLINE) x = p.inline_rows[(uint32_t)(unit0 * UR * F) + i];
-          else x = __ldg(r.rows + ((long long)unit0 * UR + q) * r.ld + f);
-          const uint32_t at = S == 64 ? (q >> 1) * 128u + 4u * f + (q & 1u) * 2u : q * S + 2u * f;
-          sts_u16(smem_u32(keys) + at, rank_value(x, r.features + f, r.lut, r.thr, searched));
-        }
+        // Two at a time: one after another a value's look-ups are a chain of L2 round trips, and four
+        // at a time are more code than a launch that runs it once gains by.  64 trees of 8 levels over 28
+        // features, 300 rows, calls back to back: 12.3, 10.3 and 10.3 us; a single call 15.1, 13.3, 13.4.
+        // 252 shapes of 30 to 400 trees, 10 to 60 features, 100 to 30000 rows: 3315, 3255 and 3256 us in all,
+        // as single calls 4126, 4044 and 4066.
+#pragma unroll 1
+        for (uint32_t i0 = tid; i0 < values; i0 += 64u * NW)
+          rank_values<2>(r, i0, 32u * NW, values, searched,
+                         [&](uint32_t q, uint32_t f) {
+                           if constexpr (INLINE) return p.inline_rows[((uint32_t)(unit0 * UR) + q) * (uint32_t)F + f];
+                           else return __ldg(r.rows + ((long long)unit0 * UR + q) * r.ld + f);
+                         },
+                         [&](uint32_t q, uint32_t f, uint32_t rank) {
+                           const uint32_t at = S == 64 ? (q >> 1) * 128u + 4u * f + (q & 1u) * 2u : q * S + 2u * f;
+                           sts_u16(smem_u32(keys) + at, rank);
+                         });
         if (blockIdx.y == 0) {
           searched = __reduce_add_sync(0xffffffffu, searched);
           if (elected && searched) atomicAdd(r.searched, (unsigned long long)searched);
