@@ -121,7 +121,10 @@ typedef struct tbk_forest_info {
  * Replaces Init_Model / Init_Offsets / Init_Lengths / Init_ClassIds / Init_LUT /
  * Init_Thresholds / Init_FeatureIndices (src/gpu/GPURepresentations.cpp:22-256,
  * src/gpu/ReorgForestRepresentation.cpp:400-487) and the host-side lowering that
- * feeds them (src/utils/TreeTilingUtils.cpp:427-556).  `schedule` may be NULL. */
+ * feeds them (src/utils/TreeTilingUtils.cpp:427-556).  `schedule` may be NULL.
+ * batch_hint: rows of the batches to come (0 = not known).  Batches of any size can be
+ * predicted; the hint settles the launch shape in advance and, for a few trees over rows
+ * of several hundred features, which layout pays. */
 TBK_EXPORT int tbk_forest_create(const tbk_forest_arrays *forest, const tbk_schedule *schedule,
                                  int32_t device, int64_t batch_hint, tbk_forest **out);
 

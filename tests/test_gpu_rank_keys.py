@@ -164,3 +164,25 @@ def test_small_host_batches_on_either_side_of_what_travels_with_the_launch(featu
         assert_predictions_close(df.predict_host(X), want)
         assert_predictions_close(df.predict_host(wide[:, :features]), want)
     df.check_status()
+
+
+@pytest.mark.parametrize("trees,levels,features,hint,tiles", [
+    (30, 8, 400, 3000, True), (30, 8, 400, 300, False), (100, 6, 400, 5999, True), (101, 6, 400, 5999, False), (64, 8, 400, 10000, True),
+    (64, 8, 400, 20000, False), (30, 8, 400, 0, False), (30, 8, 325, 3000, False), (30, 8, 326, 3000, True), (30, 8, 330, 3000, True), (30, 8, 330, 7000, False)])
+def test_few_trees_over_several_hundred_features(trees, levels, features, hint, tiles):
+    """Where ranking a row costs more than it saves the batches that are announced go through fp32 tiles: the
+    same leaves as on rank keys, for whatever batch comes."""
+    f, marg = _forest(trees, levels, features)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=hint)
+    keys = kernels.DeviceForest(f, representation="auto", feature_bits=16, batch_hint=hint)
+    assert df.info().layout == (kernels.LAYOUT_TILES if tiles else kernels.LAYOUT_RANK_KEYS)
+    assert keys.info().layout == kernels.LAYOUT_RANK_KEYS
+    for rows in (1, 700, 3001):
+        X = _rows(f, marg, rows, seed=rows)
+        want, want_ids = oracle.predict(f, X, leaf_ids=True)
+        dX = torch.from_numpy(X).cuda()
+        assert np.array_equal(df.predict_leaf_ids(dX).cpu().numpy(), want_ids)
+        got = df.predict(dX)
+        df.check_status()
+        assert_predictions_close(got.cpu().numpy(), want)
+        assert_predictions_close(keys.predict(dX).cpu().numpy(), want)

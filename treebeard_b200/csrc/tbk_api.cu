@@ -1644,6 +1644,24 @@ int predict_host_small(tbk_forest *f, const float *h_rows, int64_t n_rows, int64
   return check_status(f);
 }
 
+// Packs a forest; batch_hint: rows of the batches to come, 0 if that is not known.
+int create_image(const tbk_forest_arrays *fa, const tbk_schedule *schedule, int32_t smem_limit, int64_t batch_hint, tbk_image **out);
+
+// Few trees over rows of 326 to 511 features: ranking a row costs about as much as walking it through fp32
+// tiles, and takes a launch of its own.  Measured with 4, 6 and 8 levels, 30 to 400 trees over 350, 400, 450 and 500
+// features, 100 to 30000 rows, microseconds on rank keys against fp32 tiles: 30 trees of 8 levels x 400 features
+// 10.3 / 10.3 at 300 rows, 14.4 / 10.3 at 3000, 22.6 / 17.3 at 10000, 41.9 / 41.0 at 30000; 100 trees x 500 features
+// 18.5 / 12.3 at 3000 rows, 30.7 / 30.8 at 10000, 61.7 / 80.2 at 30000; 64 trees x 450 features (no 16-byte loads)
+// 18.5 / 16.4 at 3000 rows, 24.6 / 28.7 at 10000.  Of 324 such shapes 79 were slower than on fp32 tiles by more than
+// 3 %; with this rule 23 are, and 2 slower than on rank keys.  Without a hint, and below 700 rows, ranks.
+bool few_trees(int num_features, int64_t num_trees, int max_depth, int64_t batch_hint) {
+  if (batch_hint < 700) return false;
+  if (num_features % 4 != 0) return batch_hint >= 1500 && batch_hint < 6000 && 8 * num_trees <= num_features;
+  if (batch_hint < 6000) return 4 * num_trees <= num_features;
+  if (batch_hint < 20000) return 6 * num_trees <= num_features;
+  return 100 * num_trees * max_depth <= 65 * (int64_t)num_features;
+}
+
 } // namespace
 
 extern "C" {
@@ -1658,7 +1676,7 @@ int tbk_forest_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule,
   CUDA_TRY(cudaSetDevice(device));
   CUDA_TRY(cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   tbk_image *img = nullptr;
-  int rc = tbk_image_create(fa, schedule, smem_limit, &img);
+  int rc = create_image(fa, schedule, smem_limit, batch_hint, &img);
   if (rc != TBK_OK) return rc;
   rc = tbk_forest_create_from_image(img, schedule, device, batch_hint, out);
   tbk_image_free(img);
@@ -1666,6 +1684,13 @@ int tbk_forest_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule,
 }
 
 int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, int32_t smem_limit, tbk_image **out) {
+  return create_image(fa, schedule, smem_limit, 0, out);
+}
+
+} // extern "C"
+
+namespace {
+int create_image(const tbk_forest_arrays *fa, const tbk_schedule *schedule, int32_t smem_limit, int64_t batch_hint, tbk_image **out) {
   if (!fa || !out) return fail(TBK_ERR_INVALID, "null argument");
   *out = nullptr;
   if (fa->num_trees <= 0 || !fa->tree_off || !fa->left || !fa->right || !fa->feat || !fa->thr)
@@ -1724,7 +1749,10 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
   // (rows too wide for rank keys: the one-tile kernel; on fp32 tiles of 32 rows, one per block, 98431 rows
   // of 1303 features took 3.3 ms)
   // rank keys: whatever the key kernels would take, over at most kRankMaxFeatures features
-  const bool want_rank = want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth);
+  const bool tiles_do = bits == 0 && !batch_fits && fp32_tile_fits && host.num_classes == 0 &&
+                        few_trees(host.num_features, T, max_depth, batch_hint);
+  const bool want_rank =
+      want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth && !tiles_do);
   if (want_rank && host.num_features <= tb::kRankMaxFeatures && rank_fits(host.num_features, max_depth, smem_limit)) {
     if (tb::pack_rank(host, &im.rf).empty()) {
       im.kind = tb::PackedImage::kRank;
@@ -1824,6 +1852,10 @@ int tbk_image_create(const tbk_forest_arrays *fa, const tbk_schedule *schedule, 
   *out = img.release();
   return TBK_OK;
 }
+
+} // namespace
+
+extern "C" {
 
 int tbk_image_free(tbk_image *img) {
   delete img;
