@@ -279,7 +279,6 @@ struct tbk_forest {
   int64_t batch_hint = 0;
   int max_smem_optin = 0;
   int num_sms = 0;
-  int l2_bytes = 0;
   // device buffers
   uint8_t *d_blob = nullptr;
   tb::DevGroupMeta *d_groups = nullptr;
@@ -731,20 +730,6 @@ template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb:
 // the rows takes a block the time of 8 pairs and more, the second pass over partial sums that of 8.
 // (1048576 rows, 2000 trees, 18 row warps: 12.3 waves of blocks; 8000 rows, 387 trees of 9 levels: 63
 // blocks in three ranges were two waves.)
-//
-// A forest that L2 does not hold is walked in ranges of its pairs, one after another for all rows
-// (deep_ranges): with whole-forest launches the blocks of many waves drift apart, and each streams the
-// planes from DRAM for itself.  1048576 rows through trees of 12 levels: 613 ns per tree and wave of
-// blocks up to 4000 trees (135 MB of planes, as much as L2 holds), 623 with 6000, 641 with 8000; 4194304
-// rows and 16000 trees: 551 ms, in four ranges 480, which is what 8 x 2000 trees take.  A range costs its
-// staging of the rows, so there are as many as whole L2s' worth of planes, rounded; a batch of less than
-// two waves has nothing to gain.
-int64_t deep_ranges(const tbk_forest *f, int64_t blocks) {
-  if (blocks < 2 * (int64_t)f->num_sms || f->l2_bytes <= 0) return 1;
-  const auto &last = f->df.pairs.back();
-  const int64_t planes = 8 * (int64_t)(last.elem_off + 2ull * last.slots);
-  return std::max<int64_t>(1, std::min<int64_t>((planes + f->l2_bytes / 2) / f->l2_bytes, (int64_t)f->df.pairs.size()));
-}
 DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
   const int64_t G = (int64_t)f->df.pairs.size(), row_tiles = (n_rows + 31) / 32, SMs = f->num_sms;
   DeepSplit best;
@@ -752,13 +737,12 @@ DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
   double best_cost = -1.0;
   for (int rw = std::min(4, f->deep_row_warps); rw <= f->deep_row_warps; ++rw) {
     const int64_t blocks = (row_tiles + rw - 1) / rw, rest = blocks % SMs;
-    const double stagings = (double)deep_ranges(f, blocks);
     const double pair = rw <= 18 ? 0.7 + 0.0167 * rw : 1.0 + 0.02 * (rw - 18), start = 8.0 + 0.006 * f->df.num_features * rw;
     for (int64_t c = 1; c <= std::min<int64_t>(G, std::max<int64_t>(8, (SMs + blocks - 1) / blocks)); ++c) {
       const int64_t per = (G + c - 1) / c;
       if ((G + per - 1) / per != c) continue;
       const double waves = (double)((rest * c + SMs - 1) / SMs);
-      const double cost = pair * ((double)(blocks / SMs) * ((double)G + stagings * start) + waves * ((double)per + start)) + (c > 1 ? 8.0 : 0.0);
+      const double cost = pair * ((double)(blocks / SMs) * ((double)G + start) + waves * ((double)per + start)) + (c > 1 ? 8.0 : 0.0);
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
         best.row_warps = rw;
@@ -771,8 +755,7 @@ DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
   return best;
 }
 
-// The launches of the deep-tree kernel over `n_rows` rows -- one, or one per range of the pairs -- and the
-// second pass over chunks.
+// One launch of the deep-tree kernel over `n_rows` rows, and the second pass over chunks.
 int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
                   float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int rw, int64_t chunks) {
   const auto &q = f->df;
@@ -780,9 +763,8 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   const int64_t rows_per_block = 32 * rw;
   const int64_t grid_x = (n_rows + rows_per_block - 1) / rows_per_block;
   chunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(chunks, G), 65535));
-  const int64_t ranges = chunks == 1 ? deep_ranges(f, grid_x) : 1, per_range = (G + ranges - 1) / ranges;
-  const int gpc = (int)(ranges > 1 ? per_range : (G + chunks - 1) / chunks);
-  if (ranges == 1) chunks = (G + gpc - 1) / gpc;
+  const int gpc = (int)((G + chunks - 1) / chunks);
+  chunks = (G + gpc - 1) / gpc;
   tb::LaunchPlan plan;
   plan.row_warps = rw;
   plan.tree_threads = 1;
@@ -808,11 +790,6 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
       if (rc) return rc;
     }
   }
-  float *carry = nullptr; // (doubles)
-  if (ranges > 1 && mode != kLeafIds) {
-    const int rc = partials_acquire(f, stream, 2 * (size_t)n_rows, &carry, &ws);
-    if (rc) return rc;
-  }
   tb::DeepParams p{};
   p.node_plane = f->d_qnode;
   p.leaf_plane = f->d_qleaf;
@@ -830,7 +807,7 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   p.write_partial = need_partials ? 1 : 0;
   p.leaf_ids = mode == kLeafIds ? d_leaf_ids : nullptr;
   p.num_trees = q.num_trees;
-  p.carry = reinterpret_cast<double *>(carry);
+  p.num_pairs = (int32_t)G;
   p.pairs_per_chunk = gpc;
   p.num_features = q.num_features;
   p.transform = q.transform;
@@ -842,6 +819,9 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   p.leaf_off = (uint32_t)(plan.smem_bytes - tb::kDeepLeafBytes * f->deep_row_warps);
   p.status = f->d_status;
   p.tie_count = f->d_ties;
+  p.skip_first_copy = f->expire_next_wait ? 1 : 0;
+  p.wait_tries = f->expire_next_wait ? 2000u : 0u;
+  f->expire_next_wait = false;
   // up to 24 warps (row warps + producer) the compiler may use 80 registers per thread, beyond that 64
   // specialised for forests whose pairs all have 12 levels; generic otherwise
   using DeepKernel = void (*)(const tb::DeepParams);
@@ -849,18 +829,9 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   const DeepKernel kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
   if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
-  for (int64_t first = 0; first < G; first += per_range) {
-    p.first_pair = (int32_t)first;
-    p.num_pairs = (int32_t)std::min(G, first + per_range);
-    p.carry_in = carry && first > 0;
-    p.carry_out = carry && first + per_range < G;
-    p.skip_first_copy = f->expire_next_wait ? 1 : 0;
-    p.wait_tries = f->expire_next_wait ? 2000u : 0u;
-    f->expire_next_wait = false;
-    kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
-    CUDA_TRY(cudaGetLastError());
-    ++f->launches;
-  }
+  kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
+  CUDA_TRY(cudaGetLastError());
+  ++f->launches;
   const int tpb = 256;
   if (mode == kPredict && chunks > 1) {
     tb::tb_finalize_kernel<<<(unsigned)((n_rows + tpb - 1) / tpb), tpb, 0, stream>>>(
@@ -1930,7 +1901,6 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
   CUDA_TRY_F(cudaSetDevice(device));
   CUDA_TRY_F(cudaDeviceGetAttribute(&f->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   CUDA_TRY_F(cudaDeviceGetAttribute(&f->num_sms, cudaDevAttrMultiProcessorCount, device));
-  CUDA_TRY_F(cudaDeviceGetAttribute(&f->l2_bytes, cudaDevAttrL2CacheSize, device));
   if (im.smem_limit > f->max_smem_optin)
     return bail(fail(TBK_ERR_UNSUPPORTED, "the packed image was laid out for %d bytes of shared memory per block, this device has %d",
                      im.smem_limit, f->max_smem_optin));

@@ -51,9 +51,7 @@ struct DeepParams {
   int32_t write_partial;
   int32_t *leaf_ids;
   long long num_trees;
-  int32_t first_pair, num_pairs, pairs_per_chunk, num_features, transform; // of the pairs first_pair .. num_pairs - 1
-  double *carry;              // ranges of the pairs: the rows' sums so far, unless this is the only range
-  int32_t carry_in, carry_out;
+  int32_t num_pairs, pairs_per_chunk, num_features, transform;
   float initial_value;
   int32_t ring_slots;  // 4 .. 8
   uint32_t slot_bytes; // of a tree of the forest's depth
@@ -197,7 +195,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   const long long row = ((long long)blockIdx.x * RW + warp) * 32 + lane;
   const bool live = row < p.n_rows;
   const float *rowp = p.rows + (live ? row : 0) * p.ld;
-  const int g0 = p.first_pair + blockIdx.y * p.pairs_per_chunk;
+  const int g0 = blockIdx.y * p.pairs_per_chunk;
   const int g1 = min(p.num_pairs, g0 + p.pairs_per_chunk);
   const int P = 2 * (g1 - g0); // pieces of this block: the node planes of every tree
 
@@ -260,7 +258,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
 
   // thousands of leaf values per row: a double accumulator keeps the sum within the
   // fp32 rounding of the exact result (one conversion and one add per tree)
-  double acc = !LEAF_IDS && p.carry_in && live ? p.carry[row] : 0.0;
+  double acc = 0.0;
   // leaf values of the last pair on their way from L2, two words of this thread for each parity of a pair
   [[maybe_unused]] const uint32_t leaf_s = smem_u32(smem_raw) + p.leaf_off + (uint32_t)warp * kDeepLeafBytes + (uint32_t)lane * 4u;
   if constexpr (!LEAF_IDS) {
@@ -365,9 +363,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   }
   if (p.tie_count != nullptr && ties) atomicAdd(p.tie_count, (unsigned long long)ties);
   if (LEAF_IDS || !live) return;
-  if (p.carry_out)
-    p.carry[row] = acc;
-  else if (p.write_partial)
+  if (p.write_partial)
     p.partial[(long long)blockIdx.y * p.n_rows + row] = (float)acc;
   else
     reinterpret_cast<float *>(p.out)[row] = apply_transform((float)((double)p.initial_value + acc), p.transform);
