@@ -32,3 +32,28 @@ def test_rows_on_thresholds(trees, levels, features, rows, leaf_p, chunks, meet)
     df.check_status()
     assert_predictions_close(got.cpu().numpy(), want)
     assert_predictions_close(df.finalize(part).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("trees,rows", [(8, 500), (24, 500), (60, 300), (400, 100)])
+def test_more_ties_than_a_thread_keeps_at_hand(trees, rows):
+    """Thresholds and row values from one coarse set of numbers that is no lattice: about one comparison in ten
+    ties, from a few trees per row to far more than can be put off."""
+    marg = synth.Marginal("normal", 16)
+    f = synth.generate_forest(4, trees, 11, 16, 0.05, 0.1, marg)
+    rng = np.random.Generator(np.random.PCG64(6))
+    X = marg.sample_rows(rng, rows)
+    split = f.left >= 0
+    f.thr[split] = (np.round(f.thr[split] / 0.37) * 0.37).astype(np.float32)
+    X = (np.round(X / 0.37) * 0.37).astype(np.float32)
+    want, want_ids = oracle.predict(f, X, leaf_ids=True)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows, tree_chunks=1)
+    assert df.info().layout == kernels.LAYOUT_DEEP_KEYS
+    dX = torch.from_numpy(X).cuda()
+    before = df.info().reserved[0]
+    got = df.predict(dX)
+    assert df.info().reserved[0] - before > rows * min(3, trees // 8)
+    part = df.predict_partial(dX)
+    assert np.array_equal(df.predict_leaf_ids(dX).cpu().numpy(), want_ids)
+    df.check_status()
+    assert_predictions_close(got.cpu().numpy(), want)
+    assert_predictions_close(df.finalize(part).cpu().numpy(), want)

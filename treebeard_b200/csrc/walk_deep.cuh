@@ -67,6 +67,11 @@ struct DeepParams {
 constexpr int kDeepMaxSlots = 8;
 constexpr uint32_t kDeepNoLeaf = 0xffffffffu;
 constexpr int kDeepLeafBytes = 512; // per row warp: the leaf values of two pairs
+// Trees behind a key tie that a thread puts off.  On continuous features one comparison in some 24000 ties:
+// 1.0 per row in 2000 trees of 12 levels, 8.2 in 16000.  A tie walked in place holds up its warp, and with it
+// the block two pairs later.  4194304 rows with room for four: 60.0 ms through 2000 trees, 551.5 through
+// 16000; with room for 32: 60.2 and 475.1.
+constexpr int kDeepTied = 32;
 
 // Fast walk of DEPTH levels of two trees in lock-step, in PTX (the step of walk_quant.cuh: keys
 // are 15-bit integers that compare as fp16 numbers, so one half2 comparison of (key, node word)
@@ -265,8 +270,10 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
     sts_f32(leaf_s + 256u, 0.f);
     sts_f32(leaf_s + 384u, 0.f);
   }
-  // trees behind a key tie: up to four numbers (plus one) of 16 bits, walked after all others
-  [[maybe_unused]] unsigned long long tied = 0;
+  // trees behind a key tie, walked after all others: up to four numbers (plus one) of 16 bits, and, in
+  // local memory, the fours before them
+  [[maybe_unused]] unsigned long long tied = 0, more_tied[kDeepTied / 4 - 1];
+  [[maybe_unused]] int num_more = 0;
   bool ok = true;
   unsigned ties = 0;
   int slot = 0;          // ring slot of the next piece to consume
@@ -305,17 +312,21 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
         deep_walk<UD, WIDE>(n0, n1, key_lane, &j0, &j1, &t0, &t1);
       else
         deep_walk_any<WIDE>(depth, n0, n1, key_lane, &j0, &j1, &t0, &t1);
-      // a tied tree waits for the end, where it holds up nobody; beyond four it is walked here
+      // a tied tree waits for the end, where it holds up nobody; beyond kDeepTied it is walked here
       auto resolve = [&](bool tie, int c, uint32_t base, uint32_t &at) {
         if (!tie) return;
         ++ties;
         const uint32_t number = 2u * (uint32_t)k + (uint32_t)c + 1u;
-        if (!LEAF_IDS && tied >> 48 == 0 && number < 65536u) {
-          tied = tied << 16 | number;
-          at = kDeepNoLeaf;
-        } else {
+        if (LEAF_IDS || number > 0xffffu || (tied >> 48 && num_more == kDeepTied / 4 - 1)) {
           at = deep_walk_exact(base, nullptr, key_lane, WIDE, depth, p.exact_plane + gm.elem_off + (c ? gm.slots : 0u), rowp);
+          return;
         }
+        at = kDeepNoLeaf;
+        if (tied >> 48) {
+          more_tied[num_more++] = tied;
+          tied = 0;
+        }
+        tied = tied << 16 | number;
       };
       resolve(t0, 0, n0, j0);
       resolve(t1, 1, n1, j1);
@@ -354,7 +365,8 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
     const uint32_t last = leaf_s + ((uint32_t)(g1 - g0 + 1) & 1u) * 256u;
     copies_wait();
     acc += (double)lds_f32(last) + (double)lds_f32(last + 128u);
-    for (; tied; tied >>= 16) {
+    for (; tied || num_more; tied >>= 16) {
+      if (!tied) tied = more_tied[--num_more];
       const uint32_t number = (uint32_t)(tied & 0xffff) - 1u;
       const DevQuantGroup gm = p.pairs[g0 + (int)(number >> 1)];
       const unsigned long long off = gm.elem_off + (number & 1u ? gm.slots : 0u);
