@@ -1211,10 +1211,10 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     const int64_t n = std::min(pass, n_rows - done);
     const int64_t units = (n + unit_rows - 1) / unit_rows; // (chunks: at most four units to a block)
     const int64_t batches = std::min(units, plan.grid_x);
-    // Up to four values per walker thread: the walk ranks its rows itself.  (Every chunk's blocks
+    // A couple of values per walker thread: the walk ranks its rows itself.  (Every chunk's blocks
     // read the rows again, which host memory is too slow for.)
     const int64_t block_rows = std::min<int64_t>(n, (int64_t)plan.units * unit_rows);
-    const bool fused = !tiled && pass == n_rows && plan.units < tb::kRWBatchUnits && block_rows * q.num_features <= 128 * walkers &&
+    const bool fused = !tiled && pass == n_rows && plan.units < tb::kRWBatchUnits && block_rows * q.num_features <= 32 * tb::kRankInside * walkers &&
                        (!f->inline_rows || inlined || plan.chunks == 1);
     if (fused) {
       p.ranking = rank_rows_params(f, d_rows, n, ld, nullptr);

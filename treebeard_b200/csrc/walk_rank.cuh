@@ -27,7 +27,7 @@
 // result every time.
 //
 // The smallest batches are ranked by the walkers themselves (every tree chunk's blocks rank their
-// rows again): a launch of its own takes longer than a few values per thread.  They also take a
+// rows again): a launch of its own takes longer than two values per thread.  They also take a
 // variant of the kernel (NR = 4) with at most 20 walker warps of four rows each and every loop
 // rolled up: the code of such a launch is executed once.
 //
@@ -49,6 +49,13 @@
 namespace tb {
 
 constexpr int kRankInline = 256; // row values that travel with the launch
+// Row values that a thread of the walk ranks itself: two, in lock-step.  With more of them the ranking kernel is
+// faster, launched ahead of a walk that sets up meanwhile: 64 trees of 8 levels over 28 features, 300 rows, calls
+// back to back, 12.3 us with four values inside one after another, 10.3 in two pairs, 8.3 apart; over 10 features
+// 8.5 inside and 8.2 apart, but 11.7 against 13.1 for a call by itself.  252 shapes of 30 to 400 trees, 10 to
+// 60 features, 100 to 30000 rows, back to back and as single calls: 3228 and 4080 us with all ranked apart, 3214 and
+// 4055 with up to two values inside, 3247 and 4077 with up to four.
+constexpr int kRankInside = 2;
 
 struct RankWalkParams {
   const uint32_t *node_plane;
@@ -405,22 +412,15 @@ __global__ void __launch_bounds__(kRWThreads, 1)
         const int F = r.num_features;
         const uint32_t values = (uint32_t)(min((long long)unit1 * UR, p.n_rows) - (long long)unit0 * UR) * (uint32_t)F;
         unsigned searched = 0;
-        // Two at a time: one after another a value's look-ups are a chain of L2 round trips, and four
-        // at a time are more code than a launch that runs it once gains by.  64 trees of 8 levels over 28
-        // features, 300 rows, calls back to back: 12.3, 10.3 and 10.3 us; a single call 15.1, 13.3, 13.4.
-        // 252 shapes of 30 to 400 trees, 10 to 60 features, 100 to 30000 rows: 3315, 3255 and 3256 us in all,
-        // as single calls 4126, 4044 and 4066.
-#pragma unroll 1
-        for (uint32_t i0 = tid; i0 < values; i0 += 64u * NW)
-          rank_values<2>(r, i0, 32u * NW, values, searched,
-                         [&](uint32_t q, uint32_t f) {
-                           if constexpr (INLINE) return p.inline_rows[((uint32_t)(unit0 * UR) + q) * (uint32_t)F + f];
-                           else return __ldg(r.rows + ((long long)unit0 * UR + q) * r.ld + f);
-                         },
-                         [&](uint32_t q, uint32_t f, uint32_t rank) {
-                           const uint32_t at = S == 64 ? (q >> 1) * 128u + 4u * f + (q & 1u) * 2u : q * S + 2u * f;
-                           sts_u16(smem_u32(keys) + at, rank);
-                         });
+        rank_values<kRankInside>(r, (uint32_t)tid, 32u * NW, values, searched,
+                       [&](uint32_t q, uint32_t f) {
+                         if constexpr (INLINE) return p.inline_rows[((uint32_t)(unit0 * UR) + q) * (uint32_t)F + f];
+                         else return __ldg(r.rows + ((long long)unit0 * UR + q) * r.ld + f);
+                       },
+                       [&](uint32_t q, uint32_t f, uint32_t rank) {
+                         const uint32_t at = S == 64 ? (q >> 1) * 128u + 4u * f + (q & 1u) * 2u : q * S + 2u * f;
+                         sts_u16(smem_u32(keys) + at, rank);
+                       });
         if (blockIdx.y == 0) {
           searched = __reduce_add_sync(0xffffffffu, searched);
           if (elected && searched) atomicAdd(r.searched, (unsigned long long)searched);
