@@ -39,7 +39,7 @@ HBM_FALLBACK_GBS = 6650.0
 KERNEL_SOURCES = {"c3": ("walk_kernels.cuh", "walk_quant.cuh"),
                   "c2": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh"),
                   "c4": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh")}
-NCU_DRAM_BYTES_PER_ROW = {"c3": (8718.4, "72392cc6b65e063e"), "c2": (235.0, "2ebf250b07a70edb"), "c4": (146.5, "2ebf250b07a70edb")}
+NCU_DRAM_BYTES_PER_ROW = {"c3": (8718.4, "72392cc6b65e063e"), "c2": (231.0, "9398fa168153154b"), "c4": (145.1, "9398fa168153154b")}
 
 
 def kernel_source_hash(workload):
@@ -409,6 +409,7 @@ def main():
     clocks = sampler.stop()
     launches = df.launch_count() - launches0
     df.check_status()
+    info = df.info()   # (of the last launch: later calls have other shapes)
 
     total_ms = sum(per_step_ms)
     t = torch.tensor([total_ms], device=dev, dtype=torch.float64)
@@ -478,7 +479,6 @@ def main():
                          f"reference's parallel CPU schedule ({threads} OpenMP threads)",
                "max_abs_diff_vs_gpu": float(np.abs(ref_out - gpu_out).max())}
 
-    info = df.info()
     c5 = None
     if not args.no_c5 and args.workload == "c3" and not args.trees and not args.rows and not tree_sharded:
         del df, X, out
