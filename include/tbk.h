@@ -162,7 +162,13 @@ TBK_EXPORT int tbk_forest_get_info(const tbk_forest *forest, tbk_forest_info *in
  * src/reduction/LowerReduceOps.cpp:148-189).  Rows are row-major with `ld` floats
  * between rows; inputs and outputs are device-resident; stream-ordered.
  * out_kind TBK_OUT_F32: n_rows floats (class id as a float for multiclass);
- * TBK_OUT_I8: n_rows int8 class ids (multiclass only). */
+ * TBK_OUT_I8: n_rows int8 class ids (multiclass only).
+ * Any stream may be used, cudaStreamPerThread included, and calls on different streams may
+ * run at the same time: a call's device memory belongs to its stream (up to eight streams;
+ * a further one waits on the device for the last user of the memory that it takes over).
+ * A call that is captured allocates memory that lives as long as the graph and what is
+ * instantiated from it; replays of one graph must not overlap, as with any captured buffer.
+ * The forest must outlive its graphs' replays. */
 TBK_EXPORT int tbk_predict(tbk_forest *forest, const float *d_rows, int64_t n_rows, int64_t ld,
                            void *d_out, int32_t out_kind, void *stream);
 

@@ -42,7 +42,7 @@ constexpr int kRankCols = 32, kRankMaxDepth = 8;
 constexpr uint32_t kRankHalfMax = 31742, kRankMax = 65534;
 constexpr int kRankPairFeatures = 32; // up to here the keys of two rows lie side by side
 constexpr int kRankRowFeatures = 64;  // up to here the keys of a row have a bank each
-constexpr int kRankMaxFeatures = 511; // up to here four tiles of keys fit beside the ring (walk_rank_tiles.cuh)
+constexpr int kRankMaxFeatures = 511; // up to here four tiles of keys fit beside the ring and four walker warps (walk_rank_tiles.cuh)
 inline uint32_t rank_key_offset(int32_t num_features, uint32_t feature) {
   if (num_features > kRankRowFeatures) return (feature >> 1) * 128 + (feature & 1) * 2;
   return num_features <= kRankPairFeatures ? 4 * feature : 2 * feature;

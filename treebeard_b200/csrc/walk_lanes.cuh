@@ -3,12 +3,13 @@
 // next tree's root -- so a lane spends no step below a leaf and needs no tree counter; a fixed-depth
 // walk takes every row to the depth of the deepest tree of the group (16 steps where trees grown
 // until their leaves are pure need 5).  65536 rows through 200 such trees of up to 16 levels: 207 us at
-// fixed depth from interleaved groups, 83 us here.
+// fixed depth from interleaved groups, 83.5 us here.
 //
 // A warp = 32 rows and one of `shares` ranges of the trees; the row tile (transposed, bank = row) is
 // shared by the warps that split the trees, and their sums meet in shared memory in share order.
-// The kernel is bound by the latency of the nodes' gathers, so blocks are small and many fit an SM:
-// the trees being walked stay in L1.  blockIdx.y splits the trees further for small batches, those of
+// What bounds the kernel is the nodes' gathers: 19 sectors of L1 a load, 93 % of them hits, 18 warps waiting for
+// one per instruction issued, the load pipe 68 % and issue 49 % busy (65536 rows x 200 trees).  So blocks are
+// small and many fit an SM: the trees being walked stay in L1.  blockIdx.y splits the trees further for small batches, those of
 // every class alike (3000 rows, 3 classes of 30 trees: 50.2 us with whole classes to a warp, 22.6 so); a
 // second kernel adds those partial sums (walk_kernels.cuh).
 //
