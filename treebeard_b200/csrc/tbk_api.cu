@@ -369,27 +369,40 @@ namespace {
 
 using KernelFn = void (*)(const tb::WalkParams);
 
-template <int REP, int TS> KernelFn pick3(int rpl, bool staged, bool cached) {
+template <int REP, int TS> KernelFn pick3(int rpl, bool staged, bool cached, bool turn) {
+  if (turn) return staged ? tb::tb_walk_kernel<REP, TS, 1, true, true, true> : tb::tb_walk_kernel<REP, TS, 1, false, true, true>;
   if (!cached) return staged ? tb::tb_walk_kernel<REP, TS, 1, true, false> : tb::tb_walk_kernel<REP, TS, 1, false, false>;
   if (rpl == 2) return staged ? tb::tb_walk_kernel<REP, TS, 2, true, true> : tb::tb_walk_kernel<REP, TS, 2, false, true>;
   return staged ? tb::tb_walk_kernel<REP, TS, 1, true, true> : tb::tb_walk_kernel<REP, TS, 1, false, true>;
 }
 
-KernelFn pick_kernel(int rep, int ts, int rpl, bool staged, bool cached) {
-  if (rep == tb::kReorg) return pick3<2, 1>(rpl, staged, cached);
+// Rows are turned around in shared memory where there are many of them (few tree threads per row) and a block has
+// its SM to itself.  100000 rows of 54 features through 300 trees of 8 levels, row per lane and turned around: sparse tiles of
+// one node 266 and 198 us, of two 448 and 305, of four 698 and 614; array 395 and 232, reorg 365 and 218.  The loads in flight
+// take 64 registers a thread instead of 32 to 48, which costs small blocks their company on the SM: 30000 rows of 7
+// features, 200 trees, tiles of two 60.7 and 63.9 us, and 12000 rows of 40 features under 16 tree threads 26.3 and 33.5.
+bool turn_rows(const tb::LaunchPlan &plan, int num_features) {
+  return plan.cache_rows && plan.rows_per_lane == 1 && plan.tree_threads < 4 && num_features >= 8 &&
+         2 * (plan.smem_bytes + 1024) > 228 * 1024;
+}
+
+KernelFn pick_kernel(int rep, int ts, const tb::LaunchPlan &plan, int num_features) {
+  const int rpl = plan.rows_per_lane;
+  const bool staged = plan.staged, cached = plan.cache_rows, turn = turn_rows(plan, num_features);
+  if (rep == tb::kReorg) return pick3<2, 1>(rpl, staged, cached, turn);
   if (rep == tb::kSparse) {
     switch (ts) {
-    case 1: return pick3<0, 1>(rpl, staged, cached);
-    case 2: return pick3<0, 2>(rpl, staged, cached);
-    case 3: return pick3<0, 3>(rpl, staged, cached);
-    default: return pick3<0, 4>(rpl, staged, cached);
+    case 1: return pick3<0, 1>(rpl, staged, cached, turn);
+    case 2: return pick3<0, 2>(rpl, staged, cached, turn);
+    case 3: return pick3<0, 3>(rpl, staged, cached, turn);
+    default: return pick3<0, 4>(rpl, staged, cached, turn);
     }
   }
   switch (ts) {
-  case 1: return pick3<1, 1>(rpl, staged, cached);
-  case 2: return pick3<1, 2>(rpl, staged, cached);
-  case 3: return pick3<1, 3>(rpl, staged, cached);
-  default: return pick3<1, 4>(rpl, staged, cached);
+  case 1: return pick3<1, 1>(rpl, staged, cached, turn);
+  case 2: return pick3<1, 2>(rpl, staged, cached, turn);
+  case 3: return pick3<1, 3>(rpl, staged, cached, turn);
+  default: return pick3<1, 4>(rpl, staged, cached, turn);
   }
 }
 
@@ -1460,7 +1473,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
     return fail(TBK_ERR_UNSUPPORTED, "launch plan with register class sums needs a single tree chunk");
   p.class_regs = plan.class_regs;
 
-  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan.rows_per_lane, plan.staged, plan.cache_rows);
+  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features);
   if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
@@ -2512,7 +2525,7 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   p.vec4_ok = (pk.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0) ? 1 : 0;
   p.status = f->d_status;
   p.class_regs = 0; // class sums go through the shared-memory table the plan has sized
-  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan.rows_per_lane, plan.staged, plan.cache_rows);
+  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features);
   if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
   fn<<<grid, block, plan.smem_bytes, stream>>>(p);

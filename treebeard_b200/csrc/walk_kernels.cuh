@@ -21,7 +21,7 @@
 //
 // Tree groups are staged into shared memory with cp.async.bulk (the TMA unit's
 // untiled bulk copy) into a ring of two stages, or one, guarded by mbarriers; feature rows are
-// read with 16-byte loads and transposed through shared memory.  The reference's
+// transposed on their way into shared memory (large batches: stage_pieces).  The reference's
 // counterparts are the cooperative row cache (src/gpu/GPURepresentations.cpp:279-399)
 // and tree cache (:630-715).
 #pragma once
@@ -238,9 +238,41 @@ template <typename Load> __device__ __forceinline__ int argmax_last(int C, Load 
   return arg;
 }
 
+// Stages the features of 32 rows: pieces of 8, numbers tt, tt + TT, .. of them; a rest is the window of the last 8, staged
+// before the piece that it overlaps.  A request reads 32-byte stretches of four rows: with a row per lane every 4 bytes cost
+// a 32-byte sector (30 sectors a request, and a chunk of 5 groups of trees spent a quarter of its time on them at 54 features).
+// A piece is turned around in the lines that it will take: the values of rows 4k .. 4k+3 lie in line k, in an order that
+// meets 32 banks both ways.
+// lines: the rows' place in the first line, as a shared-memory address; the next line is NEXT floats on.
+template <int NEXT>
+__device__ __forceinline__ void stage_pieces(const float *src, long long ld, int rows, int F, uint32_t lines, int tt, int TT) {
+  const int lane = threadIdx.x & 31, i = lane & 7, r = lane >> 3, whole = F / 8;
+  src += r * ld + i;
+  const uint32_t to = lines + (uint32_t)r * 32u, from = lines + (uint32_t)(lane >> 2) * (NEXT * 4u) + (uint32_t)(lane & 3) * 32u;
+  int f0 = F % 8 != 0 && tt == (whole - 1) % TT ? F - 8 : 8 * tt;
+  for (int k = tt; k < whole;) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = 4 * q + r < rows ? __ldg(src + f0 + 4 * q * ld) : 0.f;
+    const uint32_t at = (uint32_t)f0 * (NEXT * 4u);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + at + (uint32_t)(q * NEXT * 4) + (uint32_t)((i ^ q) * 4)), "f"(v[q]) : "memory");
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[q]) : "r"(from + at + (uint32_t)((q ^ (lane >> 2)) * 4)) : "memory");
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) asm volatile("st.shared.f32 [%0], %1;" ::"r"(lines + at + (uint32_t)(q * NEXT * 4) + (uint32_t)lane * 4u), "f"(v[q]) : "memory");
+    __syncwarp(); // (the next piece may take some of these lines)
+    if (f0 == 8 * k) k += TT; // (the window leads to the first piece)
+    f0 = 8 * k;
+  }
+}
+
 // --------------------------------------------------------------------------
 
-template <int REP, int TS, int RPL, bool STAGED, bool CACHED>
+// TURN: the rows are turned around in shared memory (stage_pieces) instead of read one per lane.
+template <int REP, int TS, int RPL, bool STAGED, bool CACHED, bool TURN = false>
 __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -272,27 +304,35 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
     fence_barrier_init();
   }
   for (int i = tid; i < p.lut_bytes; i += blockDim.x) lut_s[i] = p.lut[i];
-
-  // ---- stage the row tile: 16-byte loads, transposed store xs[f][row]
+  // ---- stage the row tile, transposed: xs[f][row]
+  static_assert(!TURN || (CACHED && RPL == 1), "one row per lane of a cached tile");
   if (CACHED) {
     float *xs = xs_all + (size_t)rw * xs_floats;
+    if constexpr (TURN) {
+      const long long row0 = row_base < p.n_rows ? row_base : 0;
+      stage_pieces<RT>(p.rows + row0 * p.ld, p.ld, (int)min(p.n_rows - row0, 32ll), F, smem_u32(xs), tt, TT);
+    } else {
+      // a row per lane
 #pragma unroll
-    for (int q = 0; q < RPL; ++q) {
-      const long long row = row_base + q * 32 + lane;
-      const bool live = row < p.n_rows;
-      const float *src = p.rows + (live ? row : 0) * p.ld;
-      float *dst = xs + q * 32 + lane;
-      if (p.vec4_ok) {
-        for (int k = tt; k < F / 4; k += TT) {
-          float4 v = live ? __ldg(reinterpret_cast<const float4 *>(src) + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-          dst[(4 * k + 0) * RT] = v.x; dst[(4 * k + 1) * RT] = v.y;
-          dst[(4 * k + 2) * RT] = v.z; dst[(4 * k + 3) * RT] = v.w;
+      for (int q = 0; q < RPL; ++q) {
+        const long long row = row_base + q * 32 + lane;
+        const bool live = row < p.n_rows;
+        const float *src = p.rows + (live ? row : 0) * p.ld;
+        float *dst = xs + q * 32 + lane;
+        if (p.vec4_ok) {
+          for (int k = tt; k < F / 4; k += TT) {
+            const float4 v = live ? __ldg(reinterpret_cast<const float4 *>(src) + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            dst[(4 * k + 0) * RT] = v.x; dst[(4 * k + 1) * RT] = v.y;
+            dst[(4 * k + 2) * RT] = v.z; dst[(4 * k + 3) * RT] = v.w;
+          }
+        } else {
+          for (int k = tt; k < F; k += TT) dst[k * RT] = live ? __ldg(src + k) : 0.f;
         }
-      } else {
-        for (int k = tt; k < F; k += TT) dst[k * RT] = live ? __ldg(src + k) : 0.f;
       }
-      if (tt == 0) dst[F * RT] = __int_as_float(0xff800000); // sentinel feature: -inf
     }
+    if (tt == 0)
+#pragma unroll
+      for (int q = 0; q < RPL; ++q) xs[F * RT + q * 32 + lane] = __int_as_float(0xff800000); // sentinel feature: -inf
   }
   __syncthreads();
 
