@@ -269,13 +269,13 @@ std::string deserialize_image(const uint8_t *data, uint64_t size, PackedImage *i
     in.vec(&q.thresholds);
     const size_t n = q.node_plane.size(), columns = q.groups.size() * kRankCols;
     if (in.ok && (q.leaf_plane.size() != n || q.orig_leaf.size() != n || q.tree_index.size() != columns ||
-                  q.features.size() != (size_t)q.num_features || q.num_features > kRankMaxFeatures || q.max_depth > kRankMaxDepth ||
+                  q.features.size() != (size_t)q.num_features || q.num_features > kRankMaxByteFeatures || q.max_depth > kRankMaxDepth ||
                   q.num_classes < 0 || q.class_begin.size() != (q.num_classes > 0 ? (size_t)q.num_classes + 1 : 0)))
       in.ok = false;
     for (size_t c = 0; in.ok && c < q.class_begin.size(); ++c)
       if (q.class_begin[c] < (c ? q.class_begin[c - 1] : 0) || (size_t)q.class_begin[c] > columns) in.ok = false;
     for (const RankFeature &rf : q.features)
-      if (in.ok && (rf.buckets < 1 || (uint64_t)rf.lut_off + rf.buckets + 1 > q.lut.size() || (uint64_t)rf.thr_off + rf.n > q.thresholds.size()))
+      if (in.ok && (rf.buckets < 1 || (rank_bytes(q.num_features) && rf.n > kRankByteMax) || (uint64_t)rf.lut_off + rf.buckets + 1 > q.lut.size() || (uint64_t)rf.thr_off + rf.n > q.thresholds.size()))
         in.ok = false;
     for (const QuantGroup &g : q.groups)
       if (in.ok && (g.depth < 1 || g.depth > (uint32_t)q.max_depth || g.slots != (1u << g.depth) ||

@@ -2,6 +2,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstring>
 #include <numeric>
 
 namespace tb {
@@ -13,6 +14,12 @@ uint32_t bucket_of(const RankFeature &f, float x) {
   const float d = x - f.lo;
   const float y = d * f.scale;
   return (uint32_t)std::fmax(std::fmin(y, f.top), 0.f); // (NaN: the last bucket)
+}
+
+uint32_t bits_of(float x) {
+  uint32_t u;
+  std::memcpy(&u, &x, 4);
+  return u;
 }
 
 // The bucket table of one feature whose sorted distinct thresholds are t[0..n).
@@ -27,7 +34,7 @@ void fill_table(RankFeature *f, const float *t, uint16_t *lut) {
 std::string pack_rank(const Forest &f, RankForest *out) {
   const int64_t T = f.num_trees(), N = f.num_nodes();
   const int F = f.num_features;
-  if (F > kRankMaxFeatures) return "more than " + std::to_string(kRankMaxFeatures) + " features";
+  if (F > kRankMaxByteFeatures) return "more than " + std::to_string(kRankMaxByteFeatures) + " features";
   const bool tiles = F > kRankRowFeatures;
   if (tiles && f.num_classes > 0) return "multiclass forests over more than " + std::to_string(kRankRowFeatures) + " features";
   RankForest &q = *out;
@@ -69,7 +76,7 @@ std::string pack_rank(const Forest &f, RankForest *out) {
     uint32_t seen = most.load();
     while (d.size() > seen && !most.compare_exchange_weak(seen, (uint32_t)d.size())) {}
   }
-  const uint32_t limit = tiles ? kRankHalfMax : kRankMax;
+  const uint32_t limit = rank_bytes(F) ? kRankByteMax : tiles ? kRankHalfMax : kRankMax;
   if (most > limit) return "a feature has more than " + std::to_string(limit) + " distinct thresholds";
   q.whole_compare = most > kRankHalfMax;
 
@@ -178,6 +185,81 @@ std::string pack_rank(const Forest &f, RankForest *out) {
     }
   }
   return "";
+}
+
+namespace {
+
+struct SlabFeature { // buckets of a feature (rank_slabs.cuh)
+  float scale = 0.f, bias = 0.f, most = 0.f;
+  SlabFeature(const float *t, uint32_t n, uint32_t buckets) {
+    if (n == 0) return;
+    most = t[n - 1];
+    const float range = most - t[0];
+    scale = range > 0.f && std::isfinite(range) ? ((float)buckets - 0.5f) / range : 0.f;
+    bias = -(t[0] * scale);
+    // (a range that fp32 cannot cut up: one bucket)
+    if (!std::isfinite(scale) || !std::isfinite(bias) || !(std::fma(most, scale, bias) < (float)buckets)) scale = bias = 0.f;
+  }
+  uint32_t bucket(float x) const { // (as the device: never decreasing in x)
+    const float y = std::fma(std::fmin(x, most), scale, bias);
+    return y > 0.f ? (uint32_t)y : 0u;
+  }
+};
+
+} // namespace
+
+bool make_slab_tables(const RankForest &q, uint32_t room, SlabTables *out) {
+  const int F = q.num_features, slabs = (F + 31) / 32;
+  uint32_t most = 1; // thresholds of a feature
+  for (const RankFeature &f : q.features) most = std::max(most, f.n);
+  SlabTables &t = *out;
+  t = SlabTables();
+  for (const uint32_t per : {1u, 2u, 3u, 4u, 6u, 8u}) {
+    const uint32_t buckets = per * most;
+    uint32_t fullest = 1;
+#pragma omp parallel for schedule(dynamic, 8) reduction(max : fullest) num_threads(pack_threads()) if ((int64_t)F * most > 1 << 15)
+    for (int i = 0; i < F; ++i) {
+      const RankFeature &f = q.features[i];
+      const float *thr = q.thresholds.data() + f.thr_off;
+      const SlabFeature b(thr, f.n, buckets);
+      for (uint32_t k = 0, here = 0; k < f.n; ++k) {
+        here = k && b.bucket(thr[k]) == b.bucket(thr[k - 1]) ? here + 1 : 1;
+        fullest = std::max(fullest, here);
+      }
+    }
+    int32_t steps = 1;
+    while ((1u << steps) - 1 < fullest) ++steps;
+    const uint64_t bytes = 512 + 128ull * buckets + 128ull * (most + (1u << steps) - 1);
+    // a step is paid for by every value, the table's copy by every block: about the same for 64 KB
+    if (bytes > room || (t.bytes && steps + (double)bytes / 65536 >= t.steps + (double)t.bytes / 65536)) continue;
+    t.buckets = buckets;
+    t.steps = steps;
+    t.bytes = (uint32_t)bytes;
+  }
+  if (!t.bytes) return false;
+  t.words.assign((size_t)slabs * (t.bytes / 4), 0);
+#pragma omp parallel for schedule(dynamic, 8) num_threads(pack_threads()) if ((int64_t)F * most > 1 << 15)
+  for (int i = 0; i < slabs * 32; ++i) {
+    uint32_t *w = t.words.data() + (size_t)(i / 32) * (t.bytes / 4) + i % 32;
+    uint32_t *const thr_words = w + 128 + 32 * (size_t)t.buckets;
+    const uint32_t n = i < F ? q.features[i].n : 0, lines = t.bytes / 128 - 4 - t.buckets;
+    for (uint32_t k = n; k < lines; ++k) thr_words[32 * (size_t)k] = bits_of(INFINITY);
+    if (n == 0) continue; // (one bucket, no thresholds)
+    const RankFeature &f = q.features[i];
+    const float *thr = q.thresholds.data() + f.thr_off;
+    const SlabFeature b(thr, n, t.buckets);
+    w[0] = bits_of(b.scale);
+    w[32] = bits_of(b.bias);
+    w[64] = bits_of(b.most);
+    w[96] = f.lattice;
+    uint32_t before = 0;
+    for (uint32_t bucket = 0; bucket < t.buckets; ++bucket) {
+      while (before < n && b.bucket(thr[before]) < bucket) ++before;
+      w[128 + 32 * (size_t)bucket] = 128 * before;
+    }
+    for (uint32_t k = 0; k < n; ++k) thr_words[32 * (size_t)k] = bits_of(thr[k]);
+  }
+  return true;
 }
 
 uint32_t rank_of(const RankForest &q, int32_t feature, float x, bool *searched) {

@@ -1,5 +1,5 @@
 // "Rank keys": the packed layout for forests of at most 8 levels over rows that are narrow
-// enough for the rank kernels (walk_rank.cuh).
+// enough for the rank kernels (walk_rank.cuh, walk_rank_tiles.cuh).
 //
 // A threshold is compared with one feature only, so all that a walk needs to know of a row value
 // x is its RANK among the feature's distinct thresholds t_0 < t_1 < ...:
@@ -19,7 +19,8 @@
 // Planes, per group of 32 trees of (padded) depth D, 2^D slots x 32 columns each:
 //   node plane  u32  (key offset << 16) | (j + 1); the offset is the byte offset of the feature's
 //                    key in a row of keys (2 f), in a pair of rows (up to 32 features: 4 f) or in
-//                    a tile of 32 rows (more than 64 features: (f / 2) 128 + (f mod 2) 2)
+//                    a tile of 32 rows (more than 64 features: (f / 2) 128 + (f mod 2) 2; more than 511,
+//                    whose keys are bytes: (f / 4) 128 + f mod 4)
 //   leaf plane  f32  leaf values
 // Slots: node on level d reached by the decisions r_0 .. r_(d-1) (1 = right) is slot
 // 2^d - 1 + sum r_i 2^i, leaf sum r_i 2^i.  With the decision of level i worth 2^i slots on EVERY
@@ -43,11 +44,17 @@ constexpr uint32_t kRankHalfMax = 31742, kRankMax = 65534;
 constexpr int kRankPairFeatures = 32; // up to here the keys of two rows lie side by side
 constexpr int kRankRowFeatures = 64;  // up to here the keys of a row have a bank each
 constexpr int kRankMaxFeatures = 511; // up to here four tiles of keys fit beside the ring and four walker warps (walk_rank_tiles.cuh)
+// Wider rows: keys of one byte, for features of at most kRankByteMax distinct thresholds.
+constexpr int kRankMaxByteFeatures = 2044; // (offsets in a tile have 16 bits)
+constexpr uint32_t kRankByteMax = 255;
+constexpr bool rank_bytes(int32_t num_features) { return num_features > kRankMaxFeatures; }
 inline uint32_t rank_key_offset(int32_t num_features, uint32_t feature) {
+  if (rank_bytes(num_features)) return (feature >> 2) * 128 + (feature & 3);
   if (num_features > kRankRowFeatures) return (feature >> 1) * 128 + (feature & 1) * 2;
   return num_features <= kRankPairFeatures ? 4 * feature : 2 * feature;
 }
 inline uint32_t rank_feature_at(int32_t num_features, uint32_t offset) {
+  if (rank_bytes(num_features)) return (offset >> 7) * 4 + (offset & 3);
   if (num_features > kRankRowFeatures) return (offset >> 7) * 2 + (offset >> 1 & 1);
   return num_features <= kRankPairFeatures ? offset / 4 : offset / 2;
 }
@@ -82,10 +89,23 @@ struct RankForest {
 };
 
 // Empty string on success; fails (so that the caller can take another layout) for trees deeper
-// than 8 levels, more than kRankMaxFeatures features (kRankRowFeatures for multiclass forests),
+// than 8 levels, more than kRankMaxByteFeatures features (kRankRowFeatures for multiclass forests),
 // non-finite thresholds or leaves, or a feature with more than kRankMax distinct thresholds
-// (kRankHalfMax beyond kRankRowFeatures features).
+// (kRankHalfMax beyond kRankRowFeatures features, kRankByteMax beyond kRankMaxFeatures).
 std::string pack_rank(const Forest &f, RankForest *out);
+
+// The rank tables of 32 neighbouring features each, interleaved for rank_slabs.cuh: 128-byte lines whose word i belongs to
+// feature 32 s + i.  Four lines (buckets per unit, bucket of zero, largest threshold, lattice), then a line per bucket (128 times the
+// thresholds before it), then a line per threshold and 2^steps - 1 of infinity.  Bucket of x: fma(min(x, largest threshold),
+// scale, bias), below zero bucket zero; no bucket holds more than 2^steps - 1 thresholds.
+struct SlabTables {
+  uint32_t buckets = 0; // lines of each slab
+  int32_t steps = 0;
+  uint32_t bytes = 0; // per slab
+  std::vector<uint32_t> words;
+};
+// False where a slab takes more than `room` bytes.  One to eight buckets per threshold of the feature that has most.
+bool make_slab_tables(const RankForest &q, uint32_t room, SlabTables *out);
 
 // Rank of a row value; *searched: the value's bucket held thresholds it was compared with.
 uint32_t rank_of(const RankForest &q, int32_t feature, float x, bool *searched);

@@ -30,6 +30,7 @@ struct RankRowsParams {
   int32_t pieces;               // pieces per slab
   int32_t vec4_ok;
   int32_t lattice;              // some feature is a lattice feature
+  int32_t bytes;                // tiles of one-byte keys (tables in global memory only)
   uint32_t turn_off;            // tiles: the warps' buffers, behind the tables
   unsigned long long *searched; // statistics: values that were compared with thresholds
 };
@@ -236,7 +237,8 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
     if constexpr (TILES) {
       unsigned char *tile = reinterpret_cast<unsigned char *>(p.keys) + (size_t)whole * (32 * p.stride) + (it & 31u) * 4u;
       if constexpr (FW == 1) {
-        *reinterpret_cast<uint16_t *>(tile + (f0 >> 1) * 128 + (f0 & 1) * 2) = (uint16_t)s[0];
+        if (p.bytes) tile[(f0 >> 2) * 128 + (f0 & 3)] = (unsigned char)s[0];
+        else *reinterpret_cast<uint16_t *>(tile + (f0 >> 1) * 128 + (f0 & 1) * 2) = (uint16_t)s[0];
       } else {
 #pragma unroll
         for (int k = 0; k < N / 2; ++k)

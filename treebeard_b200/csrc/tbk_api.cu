@@ -13,6 +13,7 @@
 #include "walk_deep.cuh"
 #include "rank_rows.cuh"
 #include "walk_rank.cuh"
+#include "rank_slabs.cuh"
 #include "walk_rank_tiles.cuh"
 #include "walk_lanes.cuh"
 #include "packed_image.h"
@@ -258,6 +259,7 @@ struct tbk_image {
 struct RankPlan {
   int units = tb::kRWBatchUnits; // units of rows in a block's (first) batch
   int quads = 0, walkers = 0;    // tiled keys: quads of tiles per batch, walker warps
+  int tiles = 4;                 // ... tiles of such a "quad": 4, or 2 where four do not fit
   int chunks = 1, per_chunk = 1; // per_chunk: groups, or classes of a multiclass forest
   int stages = 2, smem = 0;
   uint32_t stage_bytes = 0;
@@ -310,6 +312,9 @@ struct tbk_forest {
   tb::DevRankFeature *d_rfeatures = nullptr;
   uint16_t *d_rlut = nullptr;
   int rank_width = 0, rank_pieces = 1, rank_smem = 0; // the ranking kernel's tables (plan_rank_tables)
+  uint32_t *d_rslabs = nullptr;                       // the same interleaved (rank_slabs.cuh), where they fit
+  uint32_t slab_bytes = 0, slab_buckets = 0;
+  int slab_steps = 0;
   struct Workspace {
     unsigned char *mem = nullptr;
     size_t bytes = 0;
@@ -895,6 +900,7 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
 // bytes of keys per row
 bool rank_tiled(int num_features) { return num_features > tb::kRankRowFeatures; }
 int rank_stride(int num_features) {
+  if (tb::rank_bytes(num_features)) return (num_features + 3) / 4 * 4;
   return rank_tiled(num_features) ? (num_features + 1) / 2 * 4 : num_features <= tb::kRankPairFeatures ? 64 : 128;
 }
 
@@ -910,14 +916,21 @@ const void *pick_rank_kernel(int stride, bool small, bool whole, bool inlined, i
   return whole ? pick_rank<128, 16, true, false>(mode) : pick_rank<128, 16, false, false>(mode);
 }
 
+const void *pick_rank_tiles_kernel(int tiles, bool bytes, bool ids) {
+  if (!bytes) return ids ? (const void *)tb::tb_walk_rank_tiles_kernel<4, false, true> : (const void *)tb::tb_walk_rank_tiles_kernel<4, false, false>;
+  if (tiles == 4) return ids ? (const void *)tb::tb_walk_rank_tiles_kernel<4, true, true> : (const void *)tb::tb_walk_rank_tiles_kernel<4, true, false>;
+  return ids ? (const void *)tb::tb_walk_rank_tiles_kernel<2, true, true> : (const void *)tb::tb_walk_rank_tiles_kernel<2, true, false>;
+}
+
 // How many quads of tiles a block of the tiled kernel takes at a time, with how many walker warps.
 // Rows of 491 to 511 features under trees of 8 levels leave three ring slots beside one quad only with
 // 8 walkers, or 4 (507 to 511).
-struct RankTilesShape { int quads, walkers; };
-constexpr RankTilesShape kRankTilesShapes[] = {{1, 16}, {2, 16}, {3, 12}, {4, 16}, {5, 20}, {6, 12}, {1, 8}, {1, 4}};
+// Rows of one-byte keys that are too wide for four tiles go in pairs of tiles.
+struct RankTilesShape { int quads, walkers, tiles; };
+constexpr RankTilesShape kRankTilesShapes[] = {{1, 16, 4}, {2, 16, 4}, {3, 12, 4}, {4, 16, 4}, {5, 20, 4}, {6, 12, 4}, {1, 8, 4}, {1, 4, 4}, {1, 16, 2}};
 int rank_tiles_slots(const RankTilesShape &sh, int num_features, int max_depth, int smem_limit) {
-  const int room = smem_limit - tb::rank_tiles_smem_bytes(32 * rank_stride(num_features), 4 * sh.quads, sh.walkers, 4, 0, 0);
-  return room < 0 ? 0 : std::min(tb::kRTMaxSlots, room / (128 << max_depth));
+  const int room = smem_limit - tb::rank_tiles_smem_bytes(32 * rank_stride(num_features), sh.tiles * sh.quads, sh.walkers, sh.tiles, 0, 0);
+  return room < 0 || (sh.tiles == 2 && !tb::rank_bytes(num_features)) ? 0 : std::min(tb::kRTMaxSlots, room / (128 << max_depth));
 }
 constexpr int kRankTilesMinSlots = 3; // one plane more than the group being walked
 
@@ -934,7 +947,6 @@ RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
   const auto &q = f->rf;
   const int G = (int)q.groups.size(), D = q.max_depth;
   const int tile_bytes = 32 * rank_stride(q.num_features);
-  const int64_t quads = (n_rows + 127) / 128;
   RankPlan best;
   double best_cost = -1.0;
   for (const RankTilesShape &sh : kRankTilesShapes) {
@@ -944,10 +956,12 @@ RankPlan make_rank_tiles_plan(const tbk_forest *f, int64_t n_rows) {
     p.stage_bytes = 128u << D;
     p.stages = rank_tiles_slots(sh, q.num_features, D, f->max_smem_optin);
     if (p.stages < kRankTilesMinSlots) continue;
-    p.smem = tb::rank_tiles_smem_bytes(tile_bytes, 4 * sh.quads, sh.walkers, 4, p.stages, p.stage_bytes);
-    // clocks of a group of trees for a batch of b quads (2 D - 0.25 wavefronts per 32 rows and tree)
+    p.tiles = sh.tiles;
+    p.smem = tb::rank_tiles_smem_bytes(tile_bytes, sh.tiles * sh.quads, sh.walkers, sh.tiles, p.stages, p.stage_bytes);
+    const int64_t quads = (n_rows + 32 * sh.tiles - 1) / (32 * sh.tiles);
+    // clocks of a group of trees for a batch of b quads (2 D - 0.25 wavefronts per 32 rows and tree; in pairs of tiles 2 D + 0.5)
     auto group = [&](int64_t b) {
-      return std::max(1.15 * 4 * 32 * (double)b * (2 * D - 0.25) + 300.0, std::max(2.0 * p.stage_bytes / 70.0, 32.0 / (sh.walkers / sh.quads) * 50.0 * D));
+      return std::max(1.15 * sh.tiles * 32 * (double)b * (2 * D - (sh.tiles == 4 ? 0.25 : -0.5)) + 300.0, std::max(2.0 * p.stage_bytes / (p.stages >= 5 ? 70.0 : p.stages == 4 ? 50.0 : 35.0), 32.0 / (sh.walkers / sh.quads) * (sh.walkers < 8 ? 85.0 : 50.0) * D));
     };
     auto block = [&](int64_t mine) { return (double)(mine / sh.quads) * group(sh.quads) + (mine % sh.quads ? group(mine % sh.quads) : 0.0); };
     const int most = f->user.tree_chunks > 0 ? std::min(G, f->user.tree_chunks) : std::min(G, 64);
@@ -1042,7 +1056,7 @@ int rank_walkers(const tbk_forest *f, const RankPlan &r, int64_t n_rows) {
 tb::LaunchPlan rank_launch_plan(const RankPlan &r, int walkers) {
   tb::LaunchPlan plan;
   plan.row_warps = r.quads ? r.quads : walkers;
-  plan.rows_per_block = r.quads ? 128 * r.quads : 4 * walkers * r.units;
+  plan.rows_per_block = r.quads ? 32 * r.tiles * r.quads : 4 * walkers * r.units;
   plan.tree_threads = walkers / plan.row_warps;
   plan.rows_per_lane = 1;
   plan.chunks = r.chunks;
@@ -1060,7 +1074,8 @@ tb::LaunchPlan rank_launch_plan(const RankPlan &r, int walkers) {
 // chunks has an arrival counter for every row batch.
 int64_t rank_rows_per_pass(const tbk_forest *f) {
   const int64_t by_keys = ((int64_t)96 << 20) / rank_stride(f->rf.num_features);
-  const int64_t round = rank_tiled(f->rf.num_features) ? (int64_t)128 * f->num_sms : (int64_t)tb::kRWBatchRows * f->num_sms;
+  const int64_t round = tb::rank_bytes(f->rf.num_features)   ? (int64_t)64 * f->num_sms
+                        : rank_tiled(f->rf.num_features) ? (int64_t)128 * f->num_sms : (int64_t)tb::kRWBatchRows * f->num_sms;
   return std::max(round, by_keys / round * round);
 }
 
@@ -1088,8 +1103,13 @@ tb::RankRowsParams rank_rows_params(const tbk_forest *f, const float *rows, int6
   p.stride = rank_stride(F);
   p.vec4_ok = F % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
   p.lattice = q.lattice;
+  p.bytes = tb::rank_bytes(F);
   p.searched = f->d_ties;
   return p;
+}
+
+template <bool BYTES> void (*pick_rank_slabs(int steps))(const tb::SlabParams) {
+  return steps == 1 ? tb::tb_rank_slabs<BYTES, 1> : steps == 2 ? tb::tb_rank_slabs<BYTES, 2> : steps == 3 ? tb::tb_rank_slabs<BYTES, 3> : tb::tb_rank_slabs<BYTES, 0>;
 }
 
 // The kernel that ranks `n` rows into `keys`.
@@ -1098,9 +1118,44 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
   tb::RankRowsParams p = rank_rows_params(f, rows, n, ld, keys);
   const bool pair = F <= tb::kRankPairFeatures, tiled = rank_tiled(F);
   const int64_t lines = pair ? (n + 1) / 2 : tiled ? (n + 31) / 32 * 32 : n;
+  if (f->slab_bytes > 0 && n * F > (int64_t)f->num_sms * 2048 && ld * (n + 64) < (int64_t)1 << 30) {
+    tb::SlabParams sp{};
+    sp.rows = rows;
+    sp.n_rows = n;
+    sp.ld_bytes = 4u * (uint32_t)ld;
+    sp.tables = reinterpret_cast<const unsigned char *>(f->d_rslabs);
+    sp.keys = reinterpret_cast<unsigned char *>(keys);
+    sp.table_bytes = f->slab_bytes;
+    sp.buckets = f->slab_buckets;
+    sp.tile_bytes = 32u * (uint32_t)rank_stride(F);
+    sp.num_features = F;
+    sp.steps = f->slab_steps;
+    sp.searched = f->d_ties;
+    sp.status = f->d_status;
+    const int slabs = (F + 31) / 32;
+    // segments of the tiles: the last wave of blocks nearly full, at about 230 clocks a tile and 3000 for a block's start
+    const int64_t tiles = (n + 31) / 32;
+    int64_t segments = 1;
+    double best = -1.0;
+    for (int64_t c = 1; c <= std::max<int64_t>(8, f->num_sms / slabs) && c <= tiles; ++c) {
+      const double cost = (double)((slabs * c + f->num_sms - 1) / f->num_sms) * ((double)(((tiles + c - 1) / c + 15) / 16 * 16) * 230.0 + 3000.0);
+      if (best < 0 || cost < best) {
+        best = cost;
+        segments = c;
+      }
+    }
+    const int smem = tb::slab_smem_bytes(f->slab_bytes);
+    const auto kernel = tb::rank_bytes(F) ? pick_rank_slabs<true>(f->slab_steps) : pick_rank_slabs<false>(f->slab_steps);
+    if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
+    const dim3 grid((unsigned)slabs, (unsigned)segments);
+    kernel<<<grid, 32 * tb::kSlabWarps, smem, stream>>>(sp);
+    CUDA_TRY(cudaGetLastError());
+    ++f->launches;
+    return TBK_OK;
+  }
   // Tables in shared memory pay once every SM has a few thousand values to rank: loading them
   // takes about as long as ranking 2000 values through L2 (a gather there costs a wavefront per lane).
-  if (f->rank_width > 0 && n * F > (int64_t)f->num_sms * 2048) {
+  if (f->rank_width > 0 && !p.bytes && n * F > (int64_t)f->num_sms * 2048) {
     const int w = f->rank_width, slabs = (F + w * f->rank_pieces - 1) / (w * f->rank_pieces);
     p.pieces = f->rank_pieces;
     p.turn_off = (uint32_t)f->rank_smem;
@@ -1185,11 +1240,10 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   unsigned char *const mem = fixed ? fixed : ws->mem;
   unsigned char *keys = mem + tb::kRankArrivalBytes;
   const bool small = !tiled && plan.units == 1; // one unit of rows per block: the variant for small batches
-  const int unit_rows = tiled ? 128 : 4 * walkers;
+  const int unit_rows = tiled ? 32 * plan.tiles : 4 * walkers;
   // rows of a small host batch travel with the launch
   const bool inlined = f->inline_rows && small && n_rows * q.num_features <= tb::kRankInline;
-  const void *const kernel = tiled ? (mode == kLeafIds ? (const void *)tb::tb_walk_rank_tiles_kernel<4, true>
-                                                       : (const void *)tb::tb_walk_rank_tiles_kernel<4, false>)
+  const void *const kernel = tiled ? pick_rank_tiles_kernel(plan.tiles, tb::rank_bytes(q.num_features), mode == kLeafIds)
                                    : pick_rank_kernel(S, small, q.whole_compare != 0, inlined, kmode);
   rc = allow_smem(f, kernel);
   if (rc) return rc;
@@ -1646,6 +1700,13 @@ bool few_trees(int num_features, int64_t num_trees, int max_depth, int64_t batch
   return 100 * num_trees * max_depth <= 65 * (int64_t)num_features;
 }
 
+// Rows of more than 511 features whose features have at most 255 distinct thresholds: one-byte ranks instead of rounded
+// keys, where the batches to come are announced (without a hint the layout stays that of images made ahead of time).  Of
+// 120 shapes (520 to 2000 features, 100 to 1000 trees of 6 and 8 levels, 1024, 8192 and 65536 rows) none is slower; microseconds
+// on rounded keys and on ranks: 300 trees of 6 levels x 520 features 34.9 / 11.8, 55.0 / 19.6, 241.5 / 85.1; 1000 trees of
+// 8 levels x 2000 features 28.5 / 16.6, 81.2 / 53.8, 367.6 / 350.6, 262144 rows 1397 / 1384.
+bool byte_ranks(int64_t batch_hint) { return batch_hint > 0; }
+
 } // namespace
 
 extern "C" {
@@ -1737,7 +1798,8 @@ int create_image(const tbk_forest_arrays *fa, const tbk_schedule *schedule, int3
                         few_trees(host.num_features, T, max_depth, batch_hint);
   const bool want_rank =
       want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth && !tiles_do);
-  if (want_rank && host.num_features <= tb::kRankMaxFeatures && rank_fits(host.num_features, max_depth, smem_limit)) {
+  const bool bytes_do = !tb::rank_bytes(host.num_features) || (bits == 0 && byte_ranks(batch_hint));
+  if (want_rank && bytes_do && host.num_features <= tb::kRankMaxByteFeatures && rank_fits(host.num_features, max_depth, smem_limit)) {
     if (tb::pack_rank(host, &im.rf).empty()) {
       im.kind = tb::PackedImage::kRank;
       im.user.representation = TBK_REP_REORG;
@@ -2011,6 +2073,13 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
       part(&f->d_rfeatures, q.features);
       part(&f->d_rlut, q.lut);
       part(&f->d_rthr, q.thresholds);
+      tb::SlabTables slabs; // (one request for shared memory holds a slab's table and the warps' buffers)
+      if (rank_tiled(q.num_features) && tb::make_slab_tables(q, (uint32_t)(f->max_smem_optin - tb::slab_smem_bytes(0)), &slabs)) {
+        part(&f->d_rslabs, slabs.words);
+        f->slab_bytes = slabs.bytes;
+        f->slab_buckets = slabs.buckets;
+        f->slab_steps = slabs.steps;
+      }
       const size_t small = total;
       part(&f->d_rnode, q.node_plane);
       part(&f->d_rleaf, q.leaf_plane);

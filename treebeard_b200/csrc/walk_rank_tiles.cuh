@@ -10,6 +10,13 @@
 // fills only some blocks).  The widest rows under the deepest trees leave room for 8 or 4 warps.  The nodes of a column's two topmost levels are loaded once for the four tiles; a tree of 8
 // levels costs 15.75 wavefronts per 32 rows.  Sums stay in the lane that owns the row.
 //
+// Rows of more than 511 features have keys of one byte: line m holds in word j the keys of features 4m .. 4m+3 of row j,
+// so that four tiles fit up to about 1000 features under 8 levels (1600 under 6), and pairs of tiles up to 2018.  A pair with
+// rows of 2000 features leaves three ring slots of 32 KB: 18944 rows x 1000 trees of 8 levels take 70 us, 17.4 wavefronts and
+// 68 instructions per 32 rows and tree, pipe 53 % and issue 55 % busy -- every group's 64 KB are asked for only once the group
+// before is walked.  (Walking four groups before looking up their leaf values, with node planes two ahead: 82 us; 8 warps of
+// four columns each instead of 16 of two: 73.)
+//
 // A block has `quads` x `shares` walker warps (T x quads tiles at a time; the shares of a quad split
 // the 32 columns of every group), a warp that streams the groups (node plane and leaf plane take a
 // ring slot each) and a warp that fetches the keys of the next batch of tiles.  Quads of tiles are
@@ -31,7 +38,7 @@ __host__ __device__ constexpr int rank_tiles_smem_bytes(int tile_bytes, int tile
 
 // T tiles through C columns (addresses col[c] in the node plane); kb[t]: this lane's keys in
 // tile t.  off: where the walks end, as offsets into the leaf plane plus the node plane's address.
-template <int D, int T, int C> __device__ __forceinline__ void rank_tiles_walk(uint32_t (&off)[T * C], const uint32_t *col, const uint32_t *kb) {
+template <int D, int T, int C, bool BYTES> __device__ __forceinline__ void rank_tiles_walk(uint32_t (&off)[T * C], const uint32_t *col, const uint32_t *kb) {
   constexpr int W = T * C;
   uint32_t node[W], key[W], root[C];
   [[maybe_unused]] uint32_t left[C], right[C];
@@ -42,16 +49,17 @@ template <int D, int T, int C> __device__ __forceinline__ void rank_tiles_walk(u
       __VA_ARGS__;                                                                                                  \
     }                                                                                                               \
   }
+  auto key_at = [](uint32_t a) { return BYTES ? lds_u8(a) : lds_u16_imm<0>(a); };
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     root[c] = lds_u32_imm<0>(col[c]);
-    if constexpr (T == 4 && D > 1) { // shared by the tiles: both nodes of level 1 are loaded
+    if constexpr (D > 1) { // shared by the tiles: both nodes of level 1 are loaded
       left[c] = lds_u32_imm<128>(col[c]);
       right[c] = lds_u32_imm<256>(col[c]);
     }
   }
-  TBT_ALL(key[q] = lds_u16_imm<0>((root[c] >> 16) + kb[t]))
-  if constexpr (T == 4 && D > 1) {
+  TBT_ALL(key[q] = key_at((root[c] >> 16) + kb[t]))
+  if constexpr (D > 1) {
     TBT_ALL(asm volatile("{\n .reg .pred p, q;\n setp.ge.f16x2 p|q, %2, %3;\n selp.b32 %0, %5, %4, p;\n selp.b32 %1, %7, %6, p;\n}"
                          : "=&r"(off[q]), "=&r"(node[q])
                          : "r"(key[q]), "r"(root[c]), "r"(col[c]), "r"(col[c] + 128u), "r"(left[c]), "r"(right[c])))
@@ -60,28 +68,30 @@ template <int D, int T, int C> __device__ __forceinline__ void rank_tiles_walk(u
   }
 #define TBT_LEVEL(level)                                                                                            \
   if constexpr (D > level) {                                                                                        \
-    if constexpr (level > 1 || T < 4) TBT_ALL(node[q] = lds_u32_imm<128 * ((1 << level) - 1)>(off[q]))              \
-    TBT_ALL(key[q] = lds_u16_imm<0>((node[q] >> 16) + kb[t]))                                                       \
+    if constexpr (level > 1) TBT_ALL(node[q] = lds_u32_imm<128 * ((1 << level) - 1)>(off[q]))              \
+    TBT_ALL(key[q] = key_at((node[q] >> 16) + kb[t]))                                                       \
     TBT_ALL((rank_step<false, (128u << level)>(off[q], key[q], node[q])))                                           \
   }
   TBT_LEVEL(1) TBT_LEVEL(2) TBT_LEVEL(3) TBT_LEVEL(4) TBT_LEVEL(5) TBT_LEVEL(6) TBT_LEVEL(7)
 #undef TBT_LEVEL
 #undef TBT_ALL
 }
-template <int T, int C> __device__ __forceinline__ void rank_tiles_walk_any(uint32_t depth, uint32_t (&off)[T * C], const uint32_t *col, const uint32_t *kb) {
+template <int T, int C, bool BYTES>
+__device__ __forceinline__ void rank_tiles_walk_any(uint32_t depth, uint32_t (&off)[T * C], const uint32_t *col, const uint32_t *kb) {
   switch (depth) {
-  case 1: return rank_tiles_walk<1, T, C>(off, col, kb);
-  case 2: return rank_tiles_walk<2, T, C>(off, col, kb);
-  case 3: return rank_tiles_walk<3, T, C>(off, col, kb);
-  case 4: return rank_tiles_walk<4, T, C>(off, col, kb);
-  case 5: return rank_tiles_walk<5, T, C>(off, col, kb);
-  case 6: return rank_tiles_walk<6, T, C>(off, col, kb);
-  case 7: return rank_tiles_walk<7, T, C>(off, col, kb);
-  default: return rank_tiles_walk<8, T, C>(off, col, kb);
+  case 1: return rank_tiles_walk<1, T, C, BYTES>(off, col, kb);
+  case 2: return rank_tiles_walk<2, T, C, BYTES>(off, col, kb);
+  case 3: return rank_tiles_walk<3, T, C, BYTES>(off, col, kb);
+  case 4: return rank_tiles_walk<4, T, C, BYTES>(off, col, kb);
+  case 5: return rank_tiles_walk<5, T, C, BYTES>(off, col, kb);
+  case 6: return rank_tiles_walk<6, T, C, BYTES>(off, col, kb);
+  case 7: return rank_tiles_walk<7, T, C, BYTES>(off, col, kb);
+  default: return rank_tiles_walk<8, T, C, BYTES>(off, col, kb);
   }
 }
 
-template <int T, bool LEAF_IDS>
+// T: tiles that a warp walks in lock-step (4, or 2 where four do not fit); BYTES: keys of one byte.
+template <int T, bool BYTES, bool LEAF_IDS>
 __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tiles_kernel(const __grid_constant__ RankWalkParams p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   constexpr int C = 2, W = T * C;
@@ -163,6 +173,10 @@ __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tile
     uint32_t kb[T];
 #pragma unroll
     for (int t = 0; t < T; ++t) kb[t] = smem_u32(keys) + (uint32_t)((quad * T + t) * p.tile_bytes) + (uint32_t)lane * 4u;
+    constexpr bool ONCE = T == 2; // (16 walkers share a pair of tiles: a warp walks two columns of a group)
+    [[maybe_unused]] uint32_t first_col[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) first_col[c] = ((uint32_t)(lane + share * C + c) & 31u) * 4u;
     int slot = 0, it = 0;
     uint32_t parity = 0;
     for (; it < my_batches; ++it) {
@@ -190,11 +204,15 @@ __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tile
         bool leaves_here = false;
         if (busy)
 #pragma unroll 1
-          for (int i = 0; i < cols; i += C) {
+          for (int i = 0; i < (ONCE ? C : cols); i += C) {
             uint32_t col[C], off[W];
 #pragma unroll
-            for (int c = 0; c < C; ++c) col[c] = nodes + ((uint32_t)(lane + share * cols + i + c) & 31u) * 4u;
-            rank_tiles_walk_any<T, C>(depth, off, col, kb);
+            for (int c = 0; c < C; ++c) col[c] = nodes + (ONCE ? first_col[c] : ((uint32_t)(lane + share * cols + i + c) & 31u) * 4u);
+            rank_tiles_walk_any<T, C, BYTES>(depth, off, col, kb);
+            if (ONCE || i + C >= cols) { // done with the node plane: its slot takes the next group's while leaf values are looked up
+              __syncwarp();
+              if (elected) mbar_arrive(empty_s + 8u * sn);
+            }
             if (!leaves_here) {
               leaves_here = ok = wait(full_s + 8u * sl, pl);
               if (!ok) break;
@@ -214,16 +232,15 @@ __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tile
               for (int q = 0; q < W; ++q) sum[q % T] += __uint_as_float(v[q]);
             }
           }
-        else
+        else {
           ok = wait(full_s + 8u * sl, pl);
+          if (elected) mbar_arrive(empty_s + 8u * sn);
+        }
         if (!ok) break;
 #pragma unroll
         for (int t = 0; t < T; ++t) acc[t] += sum[t];
         __syncwarp();
-        if (elected) {
-          mbar_arrive(empty_s + 8u * sn);
-          mbar_arrive(empty_s + 8u * sl);
-        }
+        if (elected) mbar_arrive(empty_s + 8u * sl);
       }
       if (!ok) break;
       // ---- the batch's results: the shares of a quad add up
