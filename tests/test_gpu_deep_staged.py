@@ -1,0 +1,50 @@
+"""Deep trees of one depth, whose leaf values are staged beside the nodes: every depth the kernel is made for, odd and
+single trees, a shallower tree padded to the others' depth, ragged rows, the widest and narrowest blocks, ranges of trees."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from tests.helpers import assert_predictions_close
+from treebeard_b200 import kernels, synth
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("levels", [9, 10, 11, 12])
+@pytest.mark.parametrize("trees,features,rows,chunks", [
+    (1, 3, 1, 0), (7, 16, 33, 0), (40, 128, 1000, 1), (41, 60, 5003, 3), (33, 140, 700, 1), (35, 24, 150001, 0)])
+def test_staged_leaves(levels, trees, features, rows, chunks):
+    marg = synth.Marginal("normal", features)
+    f = synth.generate_forest(7, trees, levels, features, 0.03, 0.1, marg)
+    if trees > 34:  # one tree of a single split among many deep ones
+        a, b = f.tree_off[5], f.tree_off[6]
+        keep = [a, a + f.left[a], a + f.right[a]]
+        size = int(b - a)
+        for name in ("left", "right", "feat", "thr"):
+            v = getattr(f, name)
+            setattr(f, name, np.concatenate([v[:a], v[keep], v[b:]]))
+        f.left[a:a + 3], f.right[a:a + 3] = [1, -1, -1], [2, -1, -1]
+        f.tree_off = f.tree_off.copy()
+        f.tree_off[6:] -= size - 3
+    X = marg.sample_rows(np.random.Generator(np.random.PCG64(5)), rows)
+    split = np.nonzero(f.left >= 0)[0]
+    for i in range(min(3 * rows, 600)):
+        g = split[(i * 37) % len(split)]
+        X[(i * 13) % rows, f.feat[g]] = np.nextafter(f.thr[g], np.float32([-np.inf, np.inf, f.thr[g]][i % 3]))
+    if rows > 4:
+        X[3, :], X[4, 0] = np.nan, np.inf
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows, tree_chunks=chunks)
+    assert df.info().layout == kernels.LAYOUT_DEEP_KEYS
+    dX = torch.from_numpy(X).cuda()
+    some = slice(0, 3000)
+    got, part = df.predict(dX), df.predict_partial(dX)
+    df.check_status()
+    want, want_ids = oracle.predict(f, X[some], leaf_ids=True)
+    assert_predictions_close(got.cpu().numpy()[some], want)
+    assert_predictions_close(df.finalize(part).cpu().numpy()[some], want)
+    assert np.array_equal(df.predict_leaf_ids(dX[some]).cpu().numpy(), want_ids)
+    # the same sums from the oracle's leaves, for the rest of a large batch
+    if rows > 3000:
+        tail = oracle.predict(f, X[-500:])
+        assert_predictions_close(got.cpu().numpy()[-500:], tail)

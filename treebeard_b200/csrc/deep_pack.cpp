@@ -37,9 +37,15 @@ std::string pack_deep(const Forest &f, DeepForest *out) {
   q.pairs.resize(P);
   q.tree_index.assign(P * 2, -1);
   uint64_t elems = 0;
+  // A few shallower trees among many of one depth (2000 trees of 12 levels that end early one time in 20: one or two) are
+  // padded to it: kernels for one depth need no table of pairs.
+  int64_t levels = 0;
+  for (int64_t t = 0; t < T; ++t) levels += depth[t];
+  const bool even = levels * 33 >= T * q.max_depth * 32;
   for (int64_t g = 0; g < P; ++g) {
     uint32_t d = kDeepMinDepth;
     for (int c = 0; c < 2 && 2 * g + c < T; ++c) d = std::max<uint32_t>(d, depth[order[2 * g + c]]);
+    if (even) d = std::max<uint32_t>(d, q.max_depth);
     q.pairs[g] = QuantGroup{elems, d, deep_tree_words(d)};
     elems += 2ull * deep_tree_words(d);
   }

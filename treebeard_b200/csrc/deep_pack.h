@@ -31,12 +31,18 @@
 #include <string>
 #include <vector>
 
+#ifdef __CUDACC__
+#define TB_BOTH_SIDES __host__ __device__
+#else
+#define TB_BOTH_SIDES
+#endif
+
 namespace tb {
 
 constexpr int kDeepMaxDepth = 12;
 constexpr int kDeepMinDepth = 2; // pieces of at least 16 bytes
-constexpr uint32_t deep_position(uint32_t number) { return number + (number >> 5) + (number >> 10); }
-constexpr uint32_t deep_tree_words(uint32_t depth) { return (deep_position((1u << depth) - 1) + 1 + 3) / 4 * 4; }
+TB_BOTH_SIDES constexpr uint32_t deep_position(uint32_t number) { return number + (number >> 5) + (number >> 10); }
+TB_BOTH_SIDES constexpr uint32_t deep_tree_words(uint32_t depth) { return (deep_position((1u << depth) - 1) + 1 + 3) / 4 * 4; }
 constexpr int kDeepNarrowFeatures = 511; // feature codes up to here are byte offsets
 inline uint32_t deep_feature_code(int32_t num_features, uint32_t f) { return num_features <= kDeepNarrowFeatures ? 128 * f : f; }
 

@@ -269,6 +269,7 @@ struct RankPlan {
 // How a batch is cut for the deep-tree kernel: blocks of 32 x row_warps rows, the first `whole` of them
 // over all trees and the rest over `chunks` ranges of them.
 struct DeepSplit {
+  bool staged = false;
   int64_t n_rows = -1, whole = 0;
   int row_warps = 0, chunks = 1;
 };
@@ -347,6 +348,8 @@ struct tbk_forest {
   bool deep = false;
   tb::DeepForest df;
   int deep_row_warps = 0, deep_slots = 0;
+  uint32_t *d_qsplit = nullptr; // deep trees of one depth: the planes in the order of the kernel that stages leaves too
+  int deep_staged_warps = 0, deep_staged_slots = 0;
   DeepSplit deep_split;
   int uniform_depth = 0; // key layouts: depth shared by all groups / pairs, 0 = mixed
   // host pipeline: slots of device buffers and pinned staging that a large batch streams through,
@@ -741,6 +744,29 @@ template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb:
              : (ids ? tb::tb_walk_deep_kernel<1024, 0, WIDE, true> : tb::tb_walk_deep_kernel<1024, 0, WIDE, false>);
 }
 
+// Predictions of a forest of one depth (9 to 12 levels) over at most kDeepNarrowFeatures features take leaf values from
+// shared memory (tb_walk_deep_staged_kernel).
+template <int MAX> void (*pick_deep_staged(int depth))(const tb::DeepStagedParams) {
+  return depth == 9    ? tb::tb_walk_deep_staged_kernel<MAX, 9>
+         : depth == 10 ? tb::tb_walk_deep_staged_kernel<MAX, 10>
+         : depth == 11 ? tb::tb_walk_deep_staged_kernel<MAX, 11>
+                       : tb::tb_walk_deep_staged_kernel<MAX, 12>;
+}
+uint32_t deep_half_words(int depth) { return tb::deep_tree_words((uint32_t)depth - 1); }
+int deep_staged_smem(int num_features, int depth, int row_warps, int slots) {
+  return 128 + slots * 8 * (int)deep_half_words(depth) + num_features * 64 * row_warps;
+}
+bool deep_staged_plan(int num_features, int depth, int smem_limit, int *row_warps, int *slots) {
+  for (int rw = 30; rw >= 2; rw -= 2)
+    for (int s = tb::kDeepMaxSlots; s >= tb::kDeepStagedMinSlots; --s)
+      if (deep_staged_smem(num_features, depth, rw, s) <= smem_limit) {
+        *row_warps = rw;
+        *slots = s;
+        return true;
+      }
+  return false;
+}
+
 // What counts is the waves of blocks and what a pair of trees takes a block: 300 pairs of 12 levels
 // 0.25 ms with 4 row warps, 0.34 with 18, 0.42 with 24, 0.50 with 30 (9 levels: 0.25, 0.31, 0.36, 0.42) -- all
 // latency up to about 18, then the shared-memory pipe as well.  The blocks that fill no whole wave
@@ -748,12 +774,14 @@ template <bool WIDE> void (*pick_deep(bool small, bool d12, bool ids))(const tb:
 // the rows takes a block the time of 8 pairs and more, the second pass over partial sums that of 8.
 // (1048576 rows, 2000 trees, 18 row warps: 12.3 waves of blocks; 8000 rows, 387 trees of 9 levels: 63
 // blocks in three ranges were two waves.)
-DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
+DeepSplit split_deep(const tbk_forest *f, int64_t n_rows, bool staged) {
   const int64_t G = (int64_t)f->df.pairs.size(), row_tiles = (n_rows + 31) / 32, SMs = f->num_sms;
   DeepSplit best;
   best.n_rows = n_rows;
+  best.staged = staged;
   double best_cost = -1.0;
-  for (int rw = std::min(4, f->deep_row_warps); rw <= f->deep_row_warps; ++rw) {
+  const int most = staged ? f->deep_staged_warps : f->deep_row_warps;
+  for (int rw = std::min(4, most); rw <= most; ++rw) {
     const int64_t blocks = (row_tiles + rw - 1) / rw, rest = blocks % SMs;
     const double pair = rw <= 18 ? 0.7 + 0.0167 * rw : 1.0 + 0.02 * (rw - 18), start = 8.0 + 0.006 * f->df.num_features * rw;
     for (int64_t c = 1; c <= std::min<int64_t>(G, std::max<int64_t>(8, (SMs + blocks - 1) / blocks)); ++c) {
@@ -775,7 +803,7 @@ DeepSplit split_deep(const tbk_forest *f, int64_t n_rows) {
 
 // One launch of the deep-tree kernel over `n_rows` rows, and the second pass over chunks.
 int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
-                  float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, int rw, int64_t chunks) {
+                  float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, bool staged, int rw, int64_t chunks) {
   const auto &q = f->df;
   const int64_t G = (int64_t)q.pairs.size();
   const int64_t rows_per_block = 32 * rw;
@@ -792,7 +820,7 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   plan.staged = 1;
   plan.cache_rows = 1;
   plan.stage_bytes = 4u * tb::deep_tree_words((uint32_t)std::max(q.max_depth, tb::kDeepMinDepth));
-  plan.smem_bytes = deep_smem_bytes(f);
+  plan.smem_bytes = staged ? deep_staged_smem(q.num_features, f->uniform_depth, (rw + 1) / 2 * 2, f->deep_staged_slots) : deep_smem_bytes(f);
   plan.threads = 32 * (rw + 1); // row warps + the ring producer
   plan.grid_x = grid_x;
   f->last_plan = plan;
@@ -808,7 +836,7 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
       if (rc) return rc;
     }
   }
-  tb::DeepParams p{};
+  tb::DeepStagedParams p{};
   p.node_plane = f->d_qnode;
   p.leaf_plane = f->d_qleaf;
   p.exact_plane = f->d_qexact;
@@ -830,7 +858,7 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   p.num_features = q.num_features;
   p.transform = q.transform;
   p.initial_value = (float)q.initial_value;
-  p.ring_slots = f->deep_slots;
+  p.ring_slots = staged ? f->deep_staged_slots : f->deep_slots;
   p.slot_bytes = plan.stage_bytes;
   p.tree_words = plan.stage_bytes / 4;
   p.key_tile = 128u * (uint32_t)q.num_features;
@@ -841,13 +869,19 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   p.wait_tries = f->expire_next_wait ? 2000u : 0u;
   f->expire_next_wait = false;
   // up to 24 warps (row warps + producer) the compiler may use 80 registers per thread, beyond that 64
-  // specialised for forests whose pairs all have 12 levels; generic otherwise
-  using DeepKernel = void (*)(const tb::DeepParams);
+  // (specialised for forests whose pairs all have 12 levels; generic otherwise)
   const bool d12 = f->uniform_depth == 12, ids = mode == kLeafIds, small = plan.threads <= 768;
-  const DeepKernel kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
-  if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
-  kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
+  if (staged) {
+    p.split = f->d_qsplit;
+    const auto kernel = small ? pick_deep_staged<768>(f->uniform_depth) : pick_deep_staged<1024>(f->uniform_depth);
+    if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
+    kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
+  } else {
+    const auto kernel = q.num_features > tb::kDeepNarrowFeatures ? pick_deep<true>(small, d12, ids) : pick_deep<false>(small, d12, ids);
+    if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
+    kernel<<<grid, plan.threads, plan.smem_bytes, stream>>>(p);
+  }
   CUDA_TRY(cudaGetLastError());
   ++f->launches;
   const int tpb = 256;
@@ -868,8 +902,9 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
 int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream) {
   DeepSplit &s = f->deep_split;
-  if (s.n_rows != n_rows) {
-    s = split_deep(f, n_rows);
+  const bool staged = f->d_qsplit && mode != kLeafIds;
+  if (s.n_rows != n_rows || s.staged != staged) {
+    s = split_deep(f, n_rows, staged);
     if (f->user.tree_chunks > 0) { // (asked for: all rows)
       s.whole = 0;
       s.chunks = f->user.tree_chunks;
@@ -878,13 +913,13 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   const int64_t first = std::min<int64_t>(n_rows, s.whole * s.row_warps * 32);
   if (first > 0) {
-    const int rc = run_deep_rows(f, mode, d_rows, first, ld, d_out, d_partial, d_leaf_ids, stream, s.row_warps, 1);
+    const int rc = run_deep_rows(f, mode, d_rows, first, ld, d_out, d_partial, d_leaf_ids, stream, staged, s.row_warps, 1);
     if (rc) return rc;
   }
   if (first < n_rows) {
     const int rc = run_deep_rows(f, mode, d_rows + first * ld, n_rows - first, ld, d_out ? static_cast<float *>(d_out) + first : nullptr,
                                  d_partial ? d_partial + first : nullptr, d_leaf_ids ? d_leaf_ids + first * f->df.num_trees : nullptr,
-                                 stream, s.row_warps, s.chunks);
+                                 stream, staged, s.row_warps, s.chunks);
     if (rc) return rc;
   }
   if (f->timing) {
@@ -2002,6 +2037,18 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     int urc = upload_key_planes(f, q.node_plane, q.leaf_plane, q.exact_plane, q.orig_leaf, q.pairs, q.tree_index,
                                 q.lo, q.scale, q.num_features, false);
     if (urc != TBK_OK) return bail(urc);
+    // (where it costs no row warps: 150000 rows of 200 features, 600 trees of 12 levels, 10 of them instead of 12: 946 -> 1117 us)
+    if (f->uniform_depth >= 9 && q.num_features <= tb::kDeepNarrowFeatures &&
+        deep_staged_plan(q.num_features, f->uniform_depth, f->max_smem_optin, &f->deep_staged_warps, &f->deep_staged_slots) &&
+        f->deep_staged_warps >= f->deep_row_warps) {
+      const uint32_t half = deep_half_words(f->uniform_depth);
+      const long long trees = 2ll * (long long)q.pairs.size(), threads = trees << (f->uniform_depth - 1);
+      CUDA_TRY_F(cudaMalloc(&f->d_qsplit, (size_t)trees * 4 * half * 4));
+      tb::tb_deep_split<<<(unsigned)((threads + 255) / 256), 256>>>(f->d_qnode, f->d_qleaf, f->d_qsplit, trees, (uint32_t)f->uniform_depth,
+                                                                    q.pairs[0].slots, half);
+      CUDA_TRY_F(cudaGetLastError());
+      ++f->launches;
+    }
     std::vector<uint32_t>().swap(q.node_plane);
     std::vector<float>().swap(q.leaf_plane);
     std::vector<float>().swap(q.exact_plane);
@@ -2224,6 +2271,7 @@ int tbk_forest_free(tbk_forest *f) {
   cudaFree(f->d_qnode);
   cudaFree(f->d_qleaf);
   cudaFree(f->d_qexact);
+  cudaFree(f->d_qsplit);
   cudaFree(f->d_qorig);
   cudaFree(f->d_qgroups);
   cudaFree(f->d_qtree_index);

@@ -12,9 +12,10 @@
 // sectors per warp whatever the layout), by asynchronous copies, and are consumed one pair later.  Sums stay in the
 // owning thread's register: there is no cross-thread reduction.
 //
-// The kernel is bound by latency and, since nothing else waits any more, the shared-memory pipe: 73 % busy, issue
-// 51 %, 47.7 wavefronts per walk of 32 rows through 12 levels (24 loads, the rest bank conflicts of nodes; 85248
-// rows, one wave of 18 row warps, x 1000 trees).  A warp that stops for anything but its two chains stops
+// The kernel is bound by latency and, since nothing else waits any more, the shared-memory pipe: 71 % busy, issue
+// 50 %, 53.3 wavefronts per walk of 32 rows through 12 levels (24 loads, 4 of bank conflicts of nodes, 23 of leaf
+// values; 85248 rows, one wave of 18 row warps, x 400 trees).  (Where all pairs have one depth and features are few
+// enough, tb_walk_deep_staged_kernel has the leaf values cheaper.)  A warp that stops for anything but its two chains stops
 // the others two pairs later, so nothing in the loop waits for global memory: leaf values are copied to
 // shared memory asynchronously (as loads, every pair waited some 600 of 2970 clocks for them, however
 // far ahead they were issued), and a tree behind a key tie is put off until the row's other
@@ -181,6 +182,32 @@ __device__ __forceinline__ void copy_word(uint32_t dst, const float *src, bool r
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void sts_f32(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
+// Stages the thread's row as keys; each thread reads back only the keys it wrote, so no barrier is needed.
+__device__ __forceinline__ void deep_stage_row(const DeepParams &p, int F, const float *rowp, bool live, uint32_t key_lane) {
+  constexpr uint32_t ks = 128;
+  const bool vec = (F % 4 == 0) && (p.ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.rows) & 15) == 0);
+  if (vec) {
+    for (int f = 0; f < F; f += 4) {
+      const float4 x = live ? __ldg(reinterpret_cast<const float4 *>(rowp + f)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 lo = __ldg(reinterpret_cast<const float4 *>(p.lo + f));
+      const float4 sc = __ldg(reinterpret_cast<const float4 *>(p.scale + f));
+      sts_u16(key_lane + (uint32_t)f * ks, quant_key15_lattice_dev(x.x, lo.x, sc.x));
+      sts_u16(key_lane + (uint32_t)(f + 1) * ks, quant_key15_lattice_dev(x.y, lo.y, sc.y));
+      sts_u16(key_lane + (uint32_t)(f + 2) * ks, quant_key15_lattice_dev(x.z, lo.z, sc.z));
+      sts_u16(key_lane + (uint32_t)(f + 3) * ks, quant_key15_lattice_dev(x.w, lo.w, sc.w));
+    }
+  } else {
+    for (int f = 0; f < F; ++f)
+      sts_u16(key_lane + (uint32_t)f * ks, quant_key15_lattice_dev(live ? __ldg(rowp + f) : 0.f, __ldg(p.lo + f), __ldg(p.scale + f)));
+  }
+}
+
+// The value of one tree of a pair, walked again.
+__device__ __forceinline__ float deep_exact_value(const DeepParams &p, uint32_t depth, int pair, uint32_t c, uint32_t key_lane, const float *rowp) {
+  const unsigned long long off = (2ull * (unsigned long long)pair + c) * p.tree_words;
+  return __ldg(p.leaf_plane + off + deep_walk_exact(0, p.node_plane + off, key_lane, false, depth, p.exact_plane + off, rowp));
+}
+
 // UD: depth shared by every pair of the forest (0 = mixed, decided per pair at run time).
 // LEAF_IDS: the launch records leaf ids instead of predictions.
 // WIDE: more features than the byte offset of a 128-byte line in 16 bits reaches.
@@ -195,7 +222,6 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   unsigned char *ring = smem_raw + 128;
   const uint32_t ring_s = smem_u32(ring);
   const uint32_t keys_s = ring_s + (uint32_t)S * p.slot_bytes;
-  constexpr uint32_t ks = 128;
   const uint32_t key_lane = keys_s + (uint32_t)(warp >> 1) * p.key_tile + (uint32_t)lane * 4u + (uint32_t)(warp & 1) * 2u;
 
   const long long row = ((long long)blockIdx.x * RW + warp) * 32 + lane;
@@ -242,24 +268,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
     return;
   }
 
-  // ---- stage this thread's row as keys
-  {
-    const bool vec = (F % 4 == 0) && (p.ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.rows) & 15) == 0);
-    if (vec) {
-      for (int f = 0; f < F; f += 4) {
-        const float4 x = live ? __ldg(reinterpret_cast<const float4 *>(rowp + f)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 lo = __ldg(reinterpret_cast<const float4 *>(p.lo + f));
-        const float4 sc = __ldg(reinterpret_cast<const float4 *>(p.scale + f));
-        sts_u16(key_lane + (uint32_t)f * ks, quant_key15_lattice_dev(x.x, lo.x, sc.x));
-        sts_u16(key_lane + (uint32_t)(f + 1) * ks, quant_key15_lattice_dev(x.y, lo.y, sc.y));
-        sts_u16(key_lane + (uint32_t)(f + 2) * ks, quant_key15_lattice_dev(x.z, lo.z, sc.z));
-        sts_u16(key_lane + (uint32_t)(f + 3) * ks, quant_key15_lattice_dev(x.w, lo.w, sc.w));
-      }
-    } else {
-      for (int f = 0; f < F; ++f)
-        sts_u16(key_lane + (uint32_t)f * ks, quant_key15_lattice_dev(live ? __ldg(rowp + f) : 0.f, __ldg(p.lo + f), __ldg(p.scale + f)));
-    }
-  }
+  deep_stage_row(p, F, rowp, live, key_lane);
   // (each thread reads back only the keys it wrote: no barrier is needed for the tile)
 
   // thousands of leaf values per row: a double accumulator keeps the sum within the
@@ -376,6 +385,174 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
   }
   if (p.tie_count != nullptr && ties) atomicAdd(p.tie_count, (unsigned long long)ties);
   if (LEAF_IDS || !live) return;
+  if (p.write_partial)
+    p.partial[(long long)blockIdx.y * p.n_rows + row] = (float)acc;
+  else
+    reinterpret_cast<float *>(p.out)[row] = apply_transform((float)((double)p.initial_value + acc), p.transform);
+}
+
+// ---------------------------------------------------------------------------
+// Forests whose pairs all have UD levels, predictions: the leaf planes go through the ring too.  Gathered from L2 a leaf
+// value costs 23 wavefronts of the shared-memory pipe per 32 rows (32 sectors that arrive one by one), nearly as many as
+// the walk itself; from shared memory it is one load of 3.4.  So that a pair's planes fit the ring, the bottom level is a
+// plane of its own, needed only at the end, and so are the left and the right leaves (tb_deep_split):
+//   A  the UD - 1 upper levels, an in-order tree whose leaf positions are those of
+//   B  the nodes of the bottom level and
+//   L  two half planes, the leaves to the left and to the right of these nodes.
+// A pair takes four ring slots of two planes each: A of both trees, B of both, L of the first, L of the second; five slots
+// keep the copy of every piece about a pair ahead of its use.
+// 85248 rows x 400 trees of 12 levels over 128 features: 53.3 -> 35.2 wavefronts per 32 rows and tree, pipe 71 -> 49 % busy,
+// 282 -> 268 us; 1048576 rows x 2000 trees 15.15 -> 14.55 ms; 100000 rows x 500 trees of 10 levels over 30 features, 30 row
+// warps, 387 -> 296 us.  Bound: the chain of a walk, about 100 clocks a level, times too few of them: two trees of 18 row warps
+// are what fits.  (Leaf values as plain loads, consumed a pair later: 15.9 ms, but 304 us at 30 features.)
+struct DeepStagedParams : DeepParams {
+  const uint32_t *split; // per pair: A0 A1 B0 B1 L0 (left, right) L1 (left, right)
+};
+constexpr int kDeepStagedMinSlots = 5;
+
+// Re-orders a forest's planes; a thread handles a position of the planes of a tree.
+__global__ void tb_deep_split(const uint32_t *node_plane, const float *leaf_plane, uint32_t *split, long long trees, uint32_t depth,
+                              uint32_t tree_words, uint32_t half_words) {
+  const uint32_t half = 1u << (depth - 1);
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long tree = i >> (depth - 1);
+  const uint32_t k = (uint32_t)i & (half - 1);
+  if (tree >= trees) return;
+  const uint32_t *node = node_plane + tree * tree_words;
+  const float *leaf = leaf_plane + tree * tree_words;
+  uint32_t *pair = split + (tree >> 1) * 8ll * half_words;
+  const uint32_t c = (uint32_t)tree & 1u, at = deep_position(k);
+  pair[c * half_words + at] = node[deep_position(2 * k)];
+  pair[(2 + c) * half_words + at] = node[deep_position(2 * k + 1)];
+  pair[(4 + 2 * c) * half_words + at] = __float_as_uint(leaf[deep_position(2 * k)]);
+  pair[(5 + 2 * c) * half_words + at] = __float_as_uint(leaf[deep_position(2 * k + 1)]);
+}
+
+template <int MAX_THREADS, int UD> __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_staged_kernel(const DeepStagedParams p) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int RW = (blockDim.x >> 5) - 1; // row warps; the last warp is the ring producer
+  const int F = p.num_features, S = p.ring_slots;
+  constexpr uint32_t H = deep_tree_words(UD - 1) * 4u, SLOT = 2u * H; // bytes of a plane and of a ring slot
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw); // [S], then empty[S]
+  unsigned char *ring = smem_raw + 128;
+  const uint32_t ring_s = smem_u32(ring), full_s = smem_u32(full), empty_s = full_s + 8u * (uint32_t)S;
+  const uint32_t key_lane = ring_s + (uint32_t)S * SLOT + (uint32_t)(warp >> 1) * p.key_tile + (uint32_t)lane * 4u + (uint32_t)(warp & 1) * 2u;
+  const long long row = ((long long)blockIdx.x * RW + warp) * 32 + lane;
+  const bool live = row < p.n_rows;
+  const float *rowp = p.rows + (live ? row : 0) * p.ld;
+  const int g0 = blockIdx.y * p.pairs_per_chunk, pairs = min(p.num_pairs - g0, p.pairs_per_chunk);
+  if (tid == 0) {
+    for (int i = 0; i < S; ++i) mbar_init(&full[i], 1);
+    for (int i = 0; i < S; ++i) mbar_init(&full[S + i], RW);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  const uint32_t tries = p.wait_tries ? p.wait_tries : kQWaitTries;
+  bool ok = true;
+  int slot = 0;
+  if (warp == RW) {
+    // ---- the producer: piece q goes to slot q mod S once every row warp has released the one that was there
+    uint32_t round = 0;
+    int issued = 0;
+    for (int piece = 0; piece < 4 * pairs && ok; ++piece) {
+      if (round > 0) ok = mbar_wait_all_lanes(empty_s + 8u * (uint32_t)slot, (round - 1u) & 1u, tries);
+      if (ok && !(p.skip_first_copy && piece == 0)) {
+        if (lane == 0) {
+          mbar_expect_tx(&full[slot], SLOT);
+          bulk_g2s(ring + (size_t)slot * SLOT, p.split + ((size_t)g0 * 4 + (size_t)piece) * (SLOT / 4), SLOT, &full[slot]);
+        }
+      }
+      issued += ok;
+      if (++slot == S) {
+        slot = 0;
+        ++round;
+      }
+    }
+    if (__syncthreads_or(!ok)) {
+      if (lane == 0) set_status(p.status, 4);
+      for (int q = max(0, issued - S); q < issued; ++q) // no copy may land after the block is gone
+        mbar_wait_all_lanes(full_s + 8u * (uint32_t)(q % S), (uint32_t)(q / S) & 1u, tries);
+    }
+    return;
+  }
+  deep_stage_row(p, F, rowp, live, key_lane);
+
+  double acc = 0.0; // (as in tb_walk_deep_kernel)
+  unsigned long long tied = 0, more_tied[kDeepTied / 4 - 1];
+  int num_more = 0;
+  unsigned ties = 0;
+  uint32_t parity = 0;
+  // takes the next piece: its shared-memory address once it is there
+  auto take = [&](uint32_t *empty) {
+    const uint32_t s = (uint32_t)slot;
+    ok = __all_sync(0xffffffffu, mbar_wait_all_lanes(full_s + 8u * s, parity, tries)) != 0; // (the warp agrees)
+    *empty = empty_s + 8u * s;
+    if (++slot == S) {
+      slot = 0;
+      parity ^= 1u;
+    }
+    return ring_s + s * SLOT;
+  };
+  auto release = [&](uint32_t empty) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty);
+  };
+  for (int k = 0; k < pairs; ++k) {
+    uint32_t e, e1, j0, j1;
+    bool t0, t1;
+    uint32_t at = take(&e);
+    if (!ok) break;
+    deep_walk<UD - 1, false>(at, at + H, key_lane, &j0, &j1, &t0, &t1);
+    release(e);
+    at = take(&e);
+    if (!ok) break;
+    const uint32_t n0 = lds_u32(at + 4u * j0), n1 = lds_u32(at + H + 4u * j1);
+    const uint32_t k0 = lds_u16((n0 >> 16) + key_lane), k1 = lds_u16((n1 >> 16) + key_lane);
+    const bool r0 = k0 < (n0 & 0x7fffu), r1 = k1 < (n1 & 0x7fffu);
+    t0 |= k0 == (n0 & 0x7fffu);
+    t1 |= k1 == (n1 & 0x7fffu);
+    release(e);
+    at = take(&e);
+    if (!ok) break;
+    float v0 = lds_f32(at + 4u * j0 + (r0 ? H : 0u));
+    at = take(&e1);
+    if (!ok) break;
+    float v1 = lds_f32(at + 4u * j1 + (r1 ? H : 0u));
+    release(e);
+    if (lane == 0) mbar_arrive(e1);
+    // a tree behind a key tie waits for the end, where it holds up nobody; beyond kDeepTied it is walked here
+    auto resolve = [&](bool tie, uint32_t c, float &v) {
+      if (!tie) return;
+      ++ties;
+      const uint32_t number = 2u * (uint32_t)k + c + 1u;
+      if (number > 0xffffu || (tied >> 48 && num_more == kDeepTied / 4 - 1)) {
+        v = deep_exact_value(p, UD, g0 + k, c, key_lane, rowp);
+        return;
+      }
+      v = 0.f;
+      if (tied >> 48) {
+        more_tied[num_more++] = tied;
+        tied = 0;
+      }
+      tied = tied << 16 | number;
+    };
+    resolve(t0, 0, v0);
+    resolve(t1, 1, v1);
+    acc += (double)v0 + (double)v1;
+  }
+  // every wait above is bounded: a wait that gave up ends the launch with a status word
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0) set_status(p.status, 4);
+    return;
+  }
+  for (; tied || num_more; tied >>= 16) {
+    if (!tied) tied = more_tied[--num_more];
+    const uint32_t number = (uint32_t)(tied & 0xffff) - 1u;
+    acc += (double)deep_exact_value(p, UD, g0 + (int)(number >> 1), number & 1u, key_lane, rowp);
+  }
+  if (p.tie_count != nullptr && ties) atomicAdd(p.tie_count, (unsigned long long)ties);
+  if (!live) return;
   if (p.write_partial)
     p.partial[(long long)blockIdx.y * p.n_rows + row] = (float)acc;
   else
