@@ -402,8 +402,8 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
 // A pair takes four ring slots of two planes each: A of both trees, B of both, L of the first, L of the second; five slots
 // keep the copy of every piece about a pair ahead of its use.
 // 85248 rows x 400 trees of 12 levels over 128 features: 53.3 -> 35.2 wavefronts per 32 rows and tree, pipe 71 -> 49 % busy,
-// 282 -> 268 us; 1048576 rows x 2000 trees 15.15 -> 14.55 ms; 100000 rows x 500 trees of 10 levels over 30 features, 30 row
-// warps, 387 -> 296 us.  Bound: the chain of a walk, about 100 clocks a level, times too few of them: two trees of 18 row warps
+// 282 -> 268 us; 1048576 rows x 2000 trees 15.15 -> 14.30 ms; 100000 rows x 500 trees of 10 levels over 30 features, 30 row
+// warps, 387 -> 282 us.  (Both L of a pair are looked for at once: 14.55 ms and 296 us one after the other; with B 14.62 and 269.)  Bound: the chain of a walk, about 100 clocks a level, times too few of them: two trees of 18 row warps
 // are what fits.  (Leaf values as plain loads, consumed a pair later: 15.9 ms, but 304 us at 30 features.)
 struct DeepStagedParams : DeepParams {
   const uint32_t *split; // per pair: A0 A1 B0 B1 L0 (left, right) L1 (left, right)
@@ -483,44 +483,56 @@ template <int MAX_THREADS, int UD> __global__ void __launch_bounds__(MAX_THREADS
   int num_more = 0;
   unsigned ties = 0;
   uint32_t parity = 0;
-  // takes the next piece: its shared-memory address once it is there
-  auto take = [&](uint32_t *empty) {
+  // the next piece's slot
+  auto next_slot = [&](uint32_t *phase) {
     const uint32_t s = (uint32_t)slot;
-    ok = __all_sync(0xffffffffu, mbar_wait_all_lanes(full_s + 8u * s, parity, tries)) != 0; // (the warp agrees)
-    *empty = empty_s + 8u * s;
+    *phase = parity;
     if (++slot == S) {
       slot = 0;
       parity ^= 1u;
     }
-    return ring_s + s * SLOT;
+    return s;
   };
-  auto release = [&](uint32_t empty) {
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty);
+  auto arrived = [&](uint32_t s, uint32_t phase) { // (the warp agrees)
+    return __all_sync(0xffffffffu, mbar_wait_all_lanes(full_s + 8u * s, phase, tries)) != 0;
   };
   for (int k = 0; k < pairs; ++k) {
-    uint32_t e, e1, j0, j1;
+    uint32_t j0, j1, pa, pb, p0, p1;
     bool t0, t1;
-    uint32_t at = take(&e);
+    const uint32_t sa = next_slot(&pa), sb = next_slot(&pb), s0 = next_slot(&p0), s1 = next_slot(&p1);
+    ok = arrived(sa, pa);
     if (!ok) break;
-    deep_walk<UD - 1, false>(at, at + H, key_lane, &j0, &j1, &t0, &t1);
-    release(e);
-    at = take(&e);
+    deep_walk<UD - 1, false>(ring_s + sa * SLOT, ring_s + sa * SLOT + H, key_lane, &j0, &j1, &t0, &t1);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty_s + 8u * sa);
+    ok = arrived(sb, pb);
     if (!ok) break;
-    const uint32_t n0 = lds_u32(at + 4u * j0), n1 = lds_u32(at + H + 4u * j1);
+    const uint32_t n0 = lds_u32(ring_s + sb * SLOT + 4u * j0), n1 = lds_u32(ring_s + sb * SLOT + H + 4u * j1);
     const uint32_t k0 = lds_u16((n0 >> 16) + key_lane), k1 = lds_u16((n1 >> 16) + key_lane);
     const bool r0 = k0 < (n0 & 0x7fffu), r1 = k1 < (n1 & 0x7fffu);
     t0 |= k0 == (n0 & 0x7fffu);
     t1 |= k1 == (n1 & 0x7fffu);
-    release(e);
-    at = take(&e);
-    if (!ok) break;
-    float v0 = lds_f32(at + 4u * j0 + (r0 ? H : 0u));
-    at = take(&e1);
-    if (!ok) break;
-    float v1 = lds_f32(at + 4u * j1 + (r1 ? H : 0u));
-    release(e);
-    if (lane == 0) mbar_arrive(e1);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty_s + 8u * sb);
+    // both L: one look at two barriers, which as a rule are complete
+    uint32_t here;
+    asm volatile("{\n .reg .pred p, q;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 " mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n and.pred p, p, q;\n"
+                 " vote.sync.all.pred p, p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(here)
+                 : "r"(full_s + 8u * s0), "r"(p0), "r"(full_s + 8u * s1), "r"(p1)
+                 : "memory");
+    if (!here) {
+      ok = arrived(s0, p0) && arrived(s1, p1);
+      if (!ok) break;
+    }
+    float v0 = lds_f32(ring_s + s0 * SLOT + 4u * j0 + (r0 ? H : 0u));
+    float v1 = lds_f32(ring_s + s1 * SLOT + 4u * j1 + (r1 ? H : 0u));
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(empty_s + 8u * s0);
+      mbar_arrive(empty_s + 8u * s1);
+    }
     // a tree behind a key tie waits for the end, where it holds up nobody; beyond kDeepTied it is walked here
     auto resolve = [&](bool tie, uint32_t c, float &v) {
       if (!tie) return;
