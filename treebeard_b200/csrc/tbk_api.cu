@@ -385,7 +385,8 @@ template <int REP, int TS> KernelFn pick3(int rpl, bool staged, bool cached, boo
 }
 
 // Rows are turned around in shared memory where there are many of them (few tree threads per row) and a block has
-// its SM to itself.  100000 rows of 54 features through 300 trees of 8 levels, row per lane and turned around: sparse tiles of
+// its SM to itself.  100000 rows of 54 features through 300 trees of 8 levels, two columns in
+// lock-step, row per lane and turned around: sparse tiles of
 // one node 266 and 198 us, of two 448 and 305, of four 698 and 614; array 395 and 232, reorg 365 and 218.  The loads in flight
 // take 64 registers a thread instead of 32 to 48, which costs small blocks their company on the SM: 30000 rows of 7
 // features, 200 trees, tiles of two 60.7 and 63.9 us, and 12000 rows of 40 features under 16 tree threads 26.3 and 33.5.

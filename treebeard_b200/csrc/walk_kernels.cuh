@@ -423,7 +423,21 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
         acc[q] += v;
       }
     };
-    if (RPL == 1 && TT < kCols) {
+    if (TURN && TS <= 2) {
+      // Large batches, fewer than four tree threads: four columns in lock-step, twice the
+      // loads in flight that two have.  100000 rows of 54 features, 300 trees of 8 levels: sparse tiles of one node 198 -> 167 us, of two 305 ->
+      // 265, array 232 -> 208, reorg 218 -> 201 (eight columns: 177 and 207 for one node and reorg; tiles of three lose, 463 -> 487).
+      // Bound: issue, 69 % busy with two columns at 231 instructions per 32 rows and tree (tiles of two), shared-memory pipe 64 %.
+      for (int s = tt; s < kCols; s += 4 * TT) {
+        uint32_t col[4], slot[4];
+        float v[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) col[c] = (uint32_t)(lane + s + c * TT) & (kCols - 1);
+        walk_columns<REP, TS, STAGED, CACHED, RT, 4>(gbase, gm.slots, gm.depth, col, ra[0], lut_s, slot, v);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) use(col[c], 0, v[c], slot[c]);
+      }
+    } else if (RPL == 1 && TT < kCols) {
       // one row per lane: two columns in lock-step
       for (int s = tt; s < kCols; s += 2 * TT) {
         const uint32_t col[2] = {(uint32_t)(lane + s) & (kCols - 1), (uint32_t)(lane + s + TT) & (kCols - 1)};
