@@ -99,3 +99,22 @@ def test_more_thresholds_than_a_byte_holds_keep_rounded_keys():
     assert df.info().layout == kernels.LAYOUT_ROUNDED_KEYS
     X = _rows(f, 500, 600)
     assert np.array_equal(df.predict_leaf_ids(torch.from_numpy(X).cuda()).cpu().numpy(), oracle.predict(f, X, leaf_ids=True)[1])
+
+
+def test_one_byte_keys_without_allocation():
+    """tbk_predict_noalloc takes the widths that it took on rounded keys: rows that an fp32 tile could hold."""
+    from treebeard_b200 import kernels
+    f = _forest(200, 6, 700)
+    X = _rows(f, 9001, 700)
+    rows = torch.from_numpy(X).cuda()
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=len(X))
+    out = torch.empty(len(X), device="cuda")
+    kernels._check(kernels.lib().tbk_predict_noalloc(df._h, rows.data_ptr(), len(X), 700, out.data_ptr(), kernels.OUT_F32, None))
+    torch.cuda.synchronize()
+    df.check_status()
+    assert_predictions_close(out.cpu().numpy(), oracle.predict(f, X))
+    f = _forest(100, 6, 2000)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=100)
+    rows = torch.zeros((100, 2000), device="cuda")
+    with pytest.raises(kernels.TbkError, match="16-bit key"):
+        kernels._check(kernels.lib().tbk_predict_noalloc(df._h, rows.data_ptr(), 100, 2000, out.data_ptr(), kernels.OUT_F32, None))

@@ -1739,9 +1739,13 @@ bool few_trees(int num_features, int64_t num_trees, int max_depth, int64_t batch
 // Rows of more than 511 features whose features have at most 255 distinct thresholds: one-byte ranks instead of rounded
 // keys, where the batches to come are announced (without a hint the layout stays that of images made ahead of time).  Of
 // 120 shapes (520 to 2000 features, 100 to 1000 trees of 6 and 8 levels, 1024, 8192 and 65536 rows) none is slower; microseconds
-// on rounded keys and on ranks: 300 trees of 6 levels x 520 features 34.9 / 11.8, 55.0 / 19.6, 241.5 / 85.1; 1000 trees of
-// 8 levels x 2000 features 28.5 / 16.6, 81.2 / 53.8, 367.6 / 350.6, 262144 rows 1397 / 1384.
-bool byte_ranks(int64_t batch_hint) { return batch_hint > 0; }
+// on rounded keys and on ranks: 300 trees of 6 levels x 520 features 34.9 / 11.8, 55.0 / 19.6, 241.5 / 85.1; 600 trees of
+// 8 levels x 1600 features 40.5 / 14.8, 66.3 / 42.7, 282 / 263; 1000 trees of 8 levels x 2000 features 28.5 / 16.6, 81.2 / 53.8,
+// 367.6 / 350.6, and 1397 / 1384 at 262144 rows.  For the last kind, the widest rows through most trees in large batches, the
+// gain does not pay for a preparation that takes 18 ms longer (52 instead of 33 ms: rank tables, memory for the keys of a pass).
+bool byte_ranks(int num_features, int64_t num_trees, int64_t batch_hint) {
+  return batch_hint > 0 && !(num_features >= 1500 && num_trees >= 800 && batch_hint >= 32768);
+}
 
 } // namespace
 
@@ -1834,7 +1838,7 @@ int create_image(const tbk_forest_arrays *fa, const tbk_schedule *schedule, int3
                         few_trees(host.num_features, T, max_depth, batch_hint);
   const bool want_rank =
       want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth && !tiles_do);
-  const bool bytes_do = !tb::rank_bytes(host.num_features) || (bits == 0 && byte_ranks(batch_hint));
+  const bool bytes_do = !tb::rank_bytes(host.num_features) || (bits == 0 && byte_ranks(host.num_features, T, batch_hint));
   if (want_rank && bytes_do && host.num_features <= tb::kRankMaxByteFeatures && rank_fits(host.num_features, max_depth, smem_limit)) {
     if (tb::pack_rank(host, &im.rf).empty()) {
       im.kind = tb::PackedImage::kRank;
@@ -2577,9 +2581,11 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   if (!f) return fail(TBK_ERR_INVALID, "null forest");
   std::lock_guard<std::mutex> lock(f->mu);
   const auto &pk = f->packed;
-  // (of the rounded keys only rows that an fp32 tile could hold too)
-  const bool wide = f->quant && quant_batch_tiles(f, pk.num_features) == 0 && (int64_t)(pk.num_features + 1) * 128 + 1024 <= f->max_smem_optin;
-  if ((f->quant && !wide) || f->deep) return fail(TBK_ERR_UNSUPPORTED, "tbk_predict_noalloc does not cover the rounded 16-bit key layouts");
+  // (of rounded keys and of one-byte ranks only rows that an fp32 tile could hold too)
+  const bool tile_fits = (int64_t)(pk.num_features + 1) * 128 + 1024 <= f->max_smem_optin;
+  const bool wide = f->quant && quant_batch_tiles(f, pk.num_features) == 0 && tile_fits;
+  if ((f->quant && !wide) || f->deep || (f->rank && tb::rank_bytes(pk.num_features) && !tile_fits))
+    return fail(TBK_ERR_UNSUPPORTED, "tbk_predict_noalloc does not cover the rounded 16-bit key layouts");
   if (n_rows < 0 || ld < pk.num_features) return fail(TBK_ERR_INVALID, "ld (%lld) is smaller than the row size (%d)", (long long)ld, pk.num_features);
   if (n_rows == 0) return TBK_OK;
   if (!d_rows || !d_out) return fail(TBK_ERR_INVALID, "null pointer");

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tile
 #pragma unroll
             for (int c = 0; c < C; ++c) col[c] = nodes + (ONCE ? first_col[c] : ((uint32_t)(lane + share * cols + i + c) & 31u) * 4u);
             rank_tiles_walk_any<T, C, BYTES>(depth, off, col, kb);
-            if (ONCE || i + C >= cols) { // done with the node plane: its slot takes the next group's while leaf values are looked up
+            if (ONCE) { // done with the node plane: its slot takes the next group's while leaf values are looked up
               __syncwarp();
               if (elected) mbar_arrive(empty_s + 8u * sn);
             }
@@ -234,13 +234,16 @@ __global__ void __launch_bounds__(32 * (kRTMaxWalkers + 2), 1) tb_walk_rank_tile
           }
         else {
           ok = wait(full_s + 8u * sl, pl);
-          if (elected) mbar_arrive(empty_s + 8u * sn);
+          if (ONCE && elected) mbar_arrive(empty_s + 8u * sn);
         }
         if (!ok) break;
 #pragma unroll
         for (int t = 0; t < T; ++t) acc[t] += sum[t];
         __syncwarp();
-        if (elected) mbar_arrive(empty_s + 8u * sl);
+        if (elected) {
+          if (!ONCE) mbar_arrive(empty_s + 8u * sn);
+          mbar_arrive(empty_s + 8u * sl);
+        }
       }
       if (!ok) break;
       // ---- the batch's results: the shares of a quad add up
