@@ -215,6 +215,7 @@ bool make_slab_tables(const RankForest &q, uint32_t room, SlabTables *out) {
   SlabTables &t = *out;
   t = SlabTables();
   for (const uint32_t per : {1u, 2u, 3u, 4u, 6u, 8u}) {
+    if (512 + 128ull * (per + 1) * most > room) break;
     const uint32_t buckets = per * most;
     uint32_t fullest = 1;
 #pragma omp parallel for schedule(dynamic, 8) reduction(max : fullest) num_threads(pack_threads()) if ((int64_t)F * most > 1 << 15)
@@ -222,8 +223,10 @@ bool make_slab_tables(const RankForest &q, uint32_t room, SlabTables *out) {
       const RankFeature &f = q.features[i];
       const float *thr = q.thresholds.data() + f.thr_off;
       const SlabFeature b(thr, f.n, buckets);
-      for (uint32_t k = 0, here = 0; k < f.n; ++k) {
-        here = k && b.bucket(thr[k]) == b.bucket(thr[k - 1]) ? here + 1 : 1;
+      for (uint32_t k = 0, here = 0, last = buckets; k < f.n; ++k) {
+        const uint32_t bucket = b.bucket(thr[k]);
+        here = bucket == last ? here + 1 : 1;
+        last = bucket;
         fullest = std::max(fullest, here);
       }
     }
@@ -253,8 +256,10 @@ bool make_slab_tables(const RankForest &q, uint32_t room, SlabTables *out) {
     w[64] = bits_of(b.most);
     w[96] = f.lattice;
     uint32_t before = 0;
+    uint32_t first = b.bucket(thr[0]); // of the threshold number `before`
     for (uint32_t bucket = 0; bucket < t.buckets; ++bucket) {
-      while (before < n && b.bucket(thr[before]) < bucket) ++before;
+      while (before < n && first < bucket)
+        if (++before < n) first = b.bucket(thr[before]);
       w[128 + 32 * (size_t)bucket] = 128 * before;
     }
     for (uint32_t k = 0; k < n; ++k) thr_words[32 * (size_t)k] = bits_of(thr[k]);

@@ -1148,13 +1148,16 @@ template <bool BYTES> void (*pick_rank_slabs(int steps))(const tb::SlabParams) {
   return steps == 1 ? tb::tb_rank_slabs<BYTES, 1> : steps == 2 ? tb::tb_rank_slabs<BYTES, 2> : steps == 3 ? tb::tb_rank_slabs<BYTES, 3> : tb::tb_rank_slabs<BYTES, 0>;
 }
 
+// Tables in shared memory pay from here on (see launch_rank_rows).
+bool slab_batch(const tbk_forest *f, int64_t n, int num_features) { return n * num_features > (int64_t)f->num_sms * 2048; }
+
 // The kernel that ranks `n` rows into `keys`.
 int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, uint16_t *keys, cudaStream_t stream) {
   const int F = f->rf.num_features;
   tb::RankRowsParams p = rank_rows_params(f, rows, n, ld, keys);
   const bool pair = F <= tb::kRankPairFeatures, tiled = rank_tiled(F);
   const int64_t lines = pair ? (n + 1) / 2 : tiled ? (n + 31) / 32 * 32 : n;
-  if (f->slab_bytes > 0 && n * F > (int64_t)f->num_sms * 2048 && ld * (n + 64) < (int64_t)1 << 30) {
+  if (f->slab_bytes > 0 && slab_batch(f, n, F) && ld * (n + 64) < (int64_t)1 << 30) {
     tb::SlabParams sp{};
     sp.rows = rows;
     sp.n_rows = n;
@@ -1738,7 +1741,7 @@ bool few_trees(int num_features, int64_t num_trees, int max_depth, int64_t batch
 
 // Rows of more than 511 features whose features have at most 255 distinct thresholds: one-byte ranks instead of rounded
 // keys, where the batches to come are announced (without a hint the layout stays that of images made ahead of time).  Of
-// 120 shapes (520 to 2000 features, 100 to 1000 trees of 6 and 8 levels, 1024, 8192 and 65536 rows) none is slower; microseconds
+// 120 shapes (520 to 2000 features, 100 to 1000 trees of 6 and 8 levels, 1024, 8192 and 65536 rows) none is slower by more than 3 %; microseconds
 // on rounded keys and on ranks: 300 trees of 6 levels x 520 features 34.9 / 11.8, 55.0 / 19.6, 241.5 / 85.1; 600 trees of
 // 8 levels x 1600 features 40.5 / 14.8, 66.3 / 42.7, 282 / 263; 1000 trees of 8 levels x 2000 features 28.5 / 16.6, 81.2 / 53.8,
 // 367.6 / 350.6, and 1397 / 1384 at 262144 rows.  For the last kind, the widest rows through most trees in large batches, the
@@ -2048,11 +2051,15 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
         f->deep_staged_warps >= f->deep_row_warps) {
       const uint32_t half = deep_half_words(f->uniform_depth);
       const long long trees = 2ll * (long long)q.pairs.size(), threads = trees << (f->uniform_depth - 1);
-      CUDA_TRY_F(cudaMalloc(&f->d_qsplit, (size_t)trees * 4 * half * 4));
-      tb::tb_deep_split<<<(unsigned)((threads + 255) / 256), 256>>>(f->d_qnode, f->d_qleaf, f->d_qsplit, trees, (uint32_t)f->uniform_depth,
-                                                                    q.pairs[0].slots, half);
-      CUDA_TRY_F(cudaGetLastError());
-      ++f->launches;
+      if (cudaMalloc(&f->d_qsplit, (size_t)trees * 4 * half * 4) != cudaSuccess) {
+        cudaGetLastError(); // (no room for the planes a second time: leaf values are gathered)
+        f->d_qsplit = nullptr;
+      } else {
+        tb::tb_deep_split<<<(unsigned)((threads + 255) / 256), 256>>>(f->d_qnode, f->d_qleaf, f->d_qsplit, trees, (uint32_t)f->uniform_depth,
+                                                                      q.pairs[0].slots, half);
+        CUDA_TRY_F(cudaGetLastError());
+        ++f->launches;
+      }
     }
     std::vector<uint32_t>().swap(q.node_plane);
     std::vector<float>().swap(q.leaf_plane);
@@ -2125,8 +2132,10 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
       part(&f->d_rfeatures, q.features);
       part(&f->d_rlut, q.lut);
       part(&f->d_rthr, q.thresholds);
-      tb::SlabTables slabs; // (one request for shared memory holds a slab's table and the warps' buffers)
-      if (rank_tiled(q.num_features) && tb::make_slab_tables(q, (uint32_t)(f->max_smem_optin - tb::slab_smem_bytes(0)), &slabs)) {
+      // (one request for shared memory holds a slab's table and the warps' buffers; narrower rows whose batches are announced as too small for slabs need none)
+      tb::SlabTables slabs;
+      const bool large = batch_hint <= 0 || tb::rank_bytes(q.num_features) || slab_batch(f, batch_hint, q.num_features);
+      if (rank_tiled(q.num_features) && large && tb::make_slab_tables(q, (uint32_t)(f->max_smem_optin - tb::slab_smem_bytes(0)), &slabs)) {
         part(&f->d_rslabs, slabs.words);
         f->slab_bytes = slabs.bytes;
         f->slab_buckets = slabs.buckets;
