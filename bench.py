@@ -39,7 +39,7 @@ HBM_FALLBACK_GBS = 6650.0
 KERNEL_SOURCES = {"c3": ("walk_kernels.cuh", "walk_quant.cuh"),
                   "c2": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh"),
                   "c4": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh")}
-NCU_DRAM_BYTES_PER_ROW = {"c3": (8718.4, "72392cc6b65e063e"), "c2": (231.0, "9398fa168153154b"), "c4": (145.1, "9398fa168153154b")}
+NCU_DRAM_BYTES_PER_ROW = {"c3": (8686.3, "271f001d05daf2aa"), "c2": (231.6, "37628a43f4e8c957"), "c4": (145.0, "37628a43f4e8c957")}
 
 
 def kernel_source_hash(workload):
