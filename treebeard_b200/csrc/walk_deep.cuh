@@ -254,17 +254,22 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
     // ---- the producer: piece q goes to slot q mod S, once every row warp has released
     // the piece that was there
     bool ok = true;
-    int slot = 0;
+    int slot = 0, issued = 0;
     uint32_t round = 0;
     for (int piece = 0; piece < P && ok; ++piece) {
       if (round > 0) ok = mbar_wait_all_lanes(empty_s + 8u * (uint32_t)slot, (round - 1u) & 1u, tries);
       if (ok && lane == 0 && !(p.skip_first_copy && piece == 0)) issue(piece, slot);
+      issued += ok;
       if (++slot == S) {
         slot = 0;
         ++round;
       }
     }
-    if (__syncthreads_or(!ok) && lane == 0) set_status(p.status, 4);
+    if (__syncthreads_or(!ok)) {
+      if (lane == 0) set_status(p.status, 4);
+      for (int q = max(0, issued - S); q < issued; ++q) // no copy may land after the block is gone
+        mbar_wait_all_lanes(full_s + 8u * (uint32_t)(q % S), (uint32_t)(q / S) & 1u, tries);
+    }
     return;
   }
 

@@ -402,7 +402,13 @@ __global__ void __launch_bounds__(1024, 1) tb_walk_kernel(const WalkParams p) {
       const uint32_t parity = (p.stages == 2 ? (g - g0) >> 1 : g - g0) & 1;
       const bool ok = mbar_wait_bounded(&mbar[s], parity, p.wait_limit ? p.wait_limit : kWaitLimit);
       if (__syncthreads_or(!ok)) {
-        if (tid == 0) set_status(p.status, 4);
+        if (tid == 0) {
+          set_status(p.status, 4);
+          const uint32_t limit = p.wait_limit ? p.wait_limit : kWaitLimit;
+          // no copy may land after the block is gone: this group's, and the next one's where there are two stages
+          const uint32_t next = p.stages == 2 && g + 1 < g1 ? s ^ 1 : s, phase = next != (uint32_t)s && s ? parity ^ 1 : parity;
+          for (uint32_t it = 0; it < limit && !(mbar_test(&mbar[s], parity) && mbar_test(&mbar[next], phase)); ++it) __nanosleep(64);
+        }
         return;
       }
       gbase = stage0 + (size_t)s * p.stage_bytes;

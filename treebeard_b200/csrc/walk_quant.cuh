@@ -475,6 +475,7 @@ __global__ void __launch_bounds__(kQThreads, 1) tb_walk_quant_kernel(const Quant
   };
 
   bool ok = true;
+  uint32_t issued = 0; // pieces that this producer warp has asked for
   unsigned tie_count = 0;
   const uint64_t keep = l2_policy_keep(), stream = l2_policy_stream();
   const uint32_t wait_tries = p.wait_tries ? p.wait_tries : kQWaitTries;
@@ -615,6 +616,7 @@ __global__ void __launch_bounds__(kQThreads, 1) tb_walk_quant_kernel(const Quant
     for (int it = 0; it < my_tiles && ok; ++it) {
       for (int piece = 0; piece < P && ok; ++piece) {
         if (round > 0) ok = mbar_wait_all_lanes(empty_s + 8u * (uint32_t)slot, (round - 1u) & 1u);
+        issued += ok;
         if (ok && lane == 0 && !(p.skip_first_copy && it == 0 && piece == 0)) issue(piece, slot);
         if (++slot == 3) {
           slot = 0;
@@ -877,6 +879,8 @@ __global__ void __launch_bounds__(kQThreads, 1) tb_walk_quant_kernel(const Quant
   }
   if (failed) {
     if (tid == 0) set_status(p.status, 4);
+    if (producer) // no copy may land after the block is gone
+      for (uint32_t s = 0; s < min(3u, issued); ++s) mbar_wait_all_lanes(full_s + 8u * s, ((issued - 1u - s) / 3u) & 1u);
     return;
   }
   if (p.tie_count != nullptr && tie_count) atomicAdd(p.tie_count, (unsigned long long)tie_count);
