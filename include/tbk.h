@@ -230,7 +230,8 @@ TBK_EXPORT int64_t tbk_last_kernel_time_us(tbk_forest *forest);
 TBK_EXPORT int tbk_check_status(tbk_forest *forest);
 
 /* Failure drill, for tests of the error path: in the next tbk_predict* launch on this forest the
- * bulk copy of the first tree stage is never issued and the stage waits give up after a few
+ * first bulk copy -- of the first tree stage, or, where the rows are ranked from tables in shared
+ * memory that are copied so, of these -- is never issued and the waits of that kernel give up after a few
  * thousand polls, so the launch ends by itself with the status word set -- nothing faults or
  * hangs, the results of that launch are undefined, tbk_check_status() then returns
  * TBK_ERR_DEVICE_WAIT and the forest stays usable.  (The reference has no counterpart: its

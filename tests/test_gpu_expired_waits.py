@@ -22,6 +22,8 @@ CASES = {
     "rank keys, leaf ids": (100, 6, 40, 0, 500, True, dict(representation="auto"), "RANK_KEYS"),
     "rank keys in tiles": (100, 6, 90, 0, 500, False, dict(representation="auto"), "RANK_KEYS"),
     "rank keys in tiles, leaf ids": (100, 6, 90, 0, 500, True, dict(representation="auto"), "RANK_KEYS"),
+    "ranking in slabs": (100, 6, 90, 0, 4000, False, dict(representation="auto"), "RANK_KEYS"),
+    "ranking in slabs, several passes, one-byte keys": (60, 6, 2000, 0, 48000, False, dict(representation="auto"), "RANK_KEYS"),
     "one-byte rank keys, pairs of tiles": (100, 8, 2000, 0, 70, False, dict(representation="auto"), "RANK_KEYS"),
     "deep trees, leaf values staged": (40, 11, 60, 0, 3000, False, dict(representation="auto"), "DEEP_KEYS"),
     "deep trees, leaf ids": (40, 11, 60, 0, 3000, True, dict(representation="auto"), "DEEP_KEYS"),
@@ -57,4 +59,5 @@ def test_a_wait_that_runs_out_ends_the_launch(name):
     with pytest.raises(kernels.TbkError) as err:
         df.check_status()
     assert err.value.status == 4
+    assert ("ranking kernel" if "slabs" in name else "walk kernel") in str(err.value)
     right()

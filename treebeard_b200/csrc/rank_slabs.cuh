@@ -21,6 +21,7 @@
 namespace tb {
 
 constexpr int kSlabWarps = 16, kSlabHeadBytes = 512; // per feature: scale, bias, largest threshold, lattice
+constexpr int32_t kStatusRanking = 5; // status of a wait that gave up here (walks: 4)
 constexpr int kSlabTurnBytes = 32 * 17 * 4;          // per warp: 32 rows x 32 ranks, rows 17 words apart (bytes: 9)
 constexpr int slab_smem_bytes(uint32_t table_bytes) { return 128 + kSlabWarps * kSlabTurnBytes + (int)table_bytes; }
 
@@ -34,7 +35,8 @@ struct SlabParams {
   int32_t num_features, steps;
   unsigned long long *searched; // statistics: values of features other than lattice features
   int32_t *status;
-  uint32_t wait_tries;
+  int32_t skip_copy;   // failure drill: the tables are never copied, so the wait for them expires
+  uint32_t wait_tries; // polls before the wait gives up (0 = kQWaitTries)
 };
 
 // BYTES: keys of one byte (rank_pack.h).  STEPS: search steps of a bucket (0: p.steps of them).
@@ -60,7 +62,7 @@ template <bool BYTES, int STEPS> __global__ void __launch_bounds__(32 * kSlabWar
   const int end = (int)((long long)tiles * (blockIdx.y + 1) / gridDim.y);
   if (threadIdx.x == 0) mbar_expect_tx(bar, p.table_bytes);
   __syncthreads();
-  if (warp == 0 && lane < 8) { // (copies of one thread queue up)
+  if (warp == 0 && lane < 8 && !p.skip_copy) { // (copies of one thread queue up)
     const uint32_t piece = (p.table_bytes / 128u + 7u) / 8u * 128u, at = min(piece * (uint32_t)lane, p.table_bytes);
     const uint32_t bytes = min(piece, p.table_bytes - at);
     if (bytes) bulk_g2s(table + at, p.tables + (size_t)slab * p.table_bytes + at, bytes, bar);
@@ -87,7 +89,7 @@ template <bool BYTES, int STEPS> __global__ void __launch_bounds__(32 * kSlabWar
   const bool ok = mbar_wait_all_lanes(smem_u32(bar), 0, tries);
   if (__syncthreads_or(!ok)) { // (no copy may land after the block is gone)
     mbar_wait_all_lanes(smem_u32(bar), 0, tries);
-    if (threadIdx.x == 0) set_status(p.status, 4);
+    if (threadIdx.x == 0) set_status(p.status, kStatusRanking);
     return;
   }
   const float scale = lds_f32(mine), bias = lds_f32(mine + 128u), most = lds_f32(mine + 256u);

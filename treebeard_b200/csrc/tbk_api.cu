@@ -1171,6 +1171,9 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
     sp.steps = f->slab_steps;
     sp.searched = f->d_ties;
     sp.status = f->d_status;
+    sp.skip_copy = f->expire_next_wait ? 1 : 0;
+    sp.wait_tries = f->expire_next_wait ? 2000u : 0u;
+    f->expire_next_wait = false;
     const int slabs = (F + 31) / 32;
     // segments of the tiles: the last wave of blocks nearly full, at about 230 clocks a tile and 3000 for a block's start
     const int64_t tiles = (n + 31) / 32;
@@ -1599,7 +1602,8 @@ int check_status(tbk_forest *f) {
   const int32_t st = *word;
   if (st != 0) {
     *word = 0;
-    return fail(TBK_ERR_DEVICE_WAIT, "a bounded wait on a bulk copy expired inside the walk kernel (status %d)", st);
+    return fail(TBK_ERR_DEVICE_WAIT, "a bounded wait on a bulk copy expired inside the %s kernel (status %d)",
+                st == tb::kStatusRanking ? "ranking" : "walk", st);
   }
   return TBK_OK;
 }
