@@ -113,7 +113,10 @@ typedef struct tbk_forest_info {
   int32_t staged;            /* 1 if tree groups are staged through shared memory */
   int32_t smem_bytes;        /* dynamic shared memory per block of the walk kernel */
   int32_t threads_per_block;
-  int32_t reserved[7];
+  int32_t reserved[7];       /* keys: [0] + 2^31 * [1] counts, over all calls, rounded keys' comparisons that tied
+                                and were decided on exact values; rank keys' row values that were ranked by
+                                comparing them with thresholds (those of features that splits use, except whole
+                                numbers on features whose thresholds are whole numbers close together) */
   int32_t layout;            /* TBK_LAYOUT_* */
 } tbk_forest_info;
 

@@ -271,8 +271,9 @@ uint32_t rank_of(const RankForest &q, int32_t feature, float x, bool *searched) 
   const RankFeature &f = q.features[feature];
   const uint32_t b = bucket_of(f, x);
   uint32_t s = q.lut[f.lut_off + b], e = q.lut[f.lut_off + b + 1];
-  if (f.lattice && x == std::floor(x)) s = e = x < f.lo ? 0 : e;
-  *searched = s < e;
+  const bool looked_up = f.lattice && x == std::floor(x);
+  if (looked_up) s = e = x < f.lo ? 0 : e;
+  *searched = f.n > 0 && !looked_up;
   while (s < e) {
     const uint32_t m = (s + e) >> 1;
     if (x < q.thresholds[f.thr_off + m]) e = m;

@@ -107,7 +107,8 @@ struct SlabTables {
 // False where a slab takes more than `room` bytes.  One to eight buckets per threshold of the feature that has most.
 bool make_slab_tables(const RankForest &q, uint32_t room, SlabTables *out);
 
-// Rank of a row value; *searched: the value's bucket held thresholds it was compared with.
+// Rank of a row value; *searched: the look-up table alone doesn't give it (a feature with thresholds, and not a whole number
+// on a lattice feature).
 uint32_t rank_of(const RankForest &q, int32_t feature, float x, bool *searched);
 
 // Host interpreter of the packed planes (layout verification only).

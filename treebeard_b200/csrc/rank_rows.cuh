@@ -32,15 +32,24 @@ struct RankRowsParams {
   int32_t lattice;              // some feature is a lattice feature
   int32_t bytes;                // tiles of one-byte keys (tables in global memory only)
   uint32_t turn_off;            // tiles: the warps' buffers, behind the tables
-  unsigned long long *searched; // statistics: values that were compared with thresholds
+  unsigned long long *searched; // statistics: values whose rank the feature's look-up table alone doesn't give (rank_of)
+  int32_t used;                 // features with thresholds
 };
+
+// The statistics of a launch or block that ranks `rows` rows: the values of features with thresholds, less those (of this
+// thread) that the look-up table gave.  The warp is complete.
+__device__ __forceinline__ void count_searched(unsigned long long *searched, long long rows, int used, unsigned looked_up, bool whole_rows) {
+  looked_up = __reduce_add_sync(0xffffffffu, looked_up);
+  const long long n = (whole_rows ? rows * used : 0ll) - (long long)looked_up;
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(searched, (unsigned long long)n);
+}
 
 // Ranks up to N values of a block's rows, tables in global memory: number i0, i0 + stride, ... of `count`, counted
 // row by row.  value(row, feature) gives one, use(row, feature, rank) takes its rank.  They go through their
 // look-ups and search steps in lock-step, as in tb_rank_rows: each of these is an L2 round trip that depends
 // on the last one.
 template <int N, typename Value, typename Use>
-__device__ __forceinline__ void rank_values(const RankRowsParams &r, uint32_t i0, uint32_t stride, uint32_t count, unsigned &searched,
+__device__ __forceinline__ void rank_values(const RankRowsParams &r, uint32_t i0, uint32_t stride, uint32_t count, unsigned &looked_up,
                                             Value value, Use use) {
   const uint32_t F = (uint32_t)r.num_features, rows = stride / F, rest = stride - rows * F; // (from one value to the next)
   float x[N];
@@ -69,14 +78,14 @@ __device__ __forceinline__ void rank_values(const RankRowsParams &r, uint32_t i0
       s[k] = __ldg(l);
       e[k] = __ldg(l + 1);
       thr[k] = r.thr + b.x - 1;
-      if (b.w && x[k] == floorf(x[k])) s[k] = e[k] = x[k] < lo ? 0u : e[k];
+      if (b.w && x[k] == floorf(x[k])) {
+        s[k] = e[k] = x[k] < lo ? 0u : e[k];
+        ++looked_up;
+      }
     }
   }
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    searched += s[k] < e[k];
-    longest = max(longest, e[k] - s[k]);
-  }
+  for (int k = 0; k < N; ++k) longest = max(longest, e[k] - s[k]);
   for (uint32_t step = longest ? 1u << (31 - __clz(longest)) : 0u; step; step >>= 1) {
     float t[N];
 #pragma unroll
@@ -134,7 +143,8 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
   const uint32_t n_rows = (uint32_t)p.n_rows;     // (the host bounds a batch by the bytes of its keys)
   // lines: rows, or pairs of rows, or all rows of the tiles; a warp takes one piece of a tile's rows
   const uint32_t items = (TILES ? (n_rows + 31) & ~31u : (n_rows + RPT - 1) / RPT) * (uint32_t)pieces;
-  unsigned searched = 0;
+  constexpr float kNowhere = 0.5f; // in the places of features and rows that there are not: no whole number
+  unsigned looked_up = 0;
   for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < items; it += gridDim.x * blockDim.x) {
     const uint32_t unit = TILES ? it >> 5 : it, whole = pieces == 1 ? unit : unit / (uint32_t)pieces;
     const uint32_t line = TILES ? whole * 32u + (it & 31u) : whole;
@@ -150,7 +160,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const uint32_t r = 4u * k + (lane >> 3), row = min(whole * 32u + r, n_rows - 1);
-        turn[r * 9 + i] = in ? __ldg(p.rows + (long long)row * p.ld + f0 + i) : 0.f;
+        turn[r * 9 + i] = in ? __ldg(p.rows + (long long)row * p.ld + f0 + i) : kNowhere;
       }
       __syncwarp();
 #pragma unroll
@@ -162,7 +172,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
       if (FW >= 4 && p.vec4_ok) {
 #pragma unroll
         for (int i = 0; i + 3 < FW; i += 4) {
-          const float4 v = f0 + i < F ? __ldg(reinterpret_cast<const float4 *>(src + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 v = f0 + i < F ? __ldg(reinterpret_cast<const float4 *>(src + i)) : make_float4(kNowhere, kNowhere, kNowhere, kNowhere);
           x[r * FW + i] = v.x;
           x[r * FW + i + 1] = v.y;
           x[r * FW + i + 2] = v.z;
@@ -170,8 +180,12 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
         }
       } else {
 #pragma unroll
-        for (int i = 0; i < FW; ++i) x[r * FW + i] = f0 + i < F ? __ldg(src + i) : 0.f;
+        for (int i = 0; i < FW; ++i) x[r * FW + i] = f0 + i < F ? __ldg(src + i) : kNowhere;
       }
+    }
+    if (line * RPT + RPT > n_rows) { // the second row of the last pair, or rows that fill up a tile
+#pragma unroll
+      for (int k = (int)(PAIR) * FW; k < N; ++k) x[k] = kNowhere;
     }
     uint32_t s[N], e[N], first[FW]; // byte offsets of thresholds
     uint32_t longest = 0;
@@ -201,9 +215,9 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
         if (p.lattice && b.w && x[k] == floorf(x[k])) { // a bucket's threshold is at or below its whole number
           s[k] = x[k] < lo ? 0u : e[k];
           e[k] = s[k];
+          ++looked_up;
         }
         longest = max(longest, e[k] - s[k]);
-        searched += s[k] < e[k];
         s[k] = first[i] + 4u * s[k];
         e[k] = first[i] + 4u * e[k];
       }
@@ -249,8 +263,7 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256, 1) tb_rank_rows(const RankR
     else if constexpr (N == 2) *reinterpret_cast<uint32_t *>(dst) = w[0];
     else *reinterpret_cast<uint16_t *>(dst) = (uint16_t)w[0];
   }
-  searched = __reduce_add_sync(0xffffffffu, searched);
-  if ((threadIdx.x & 31) == 0 && searched) atomicAdd(p.searched, (unsigned long long)searched);
+  count_searched(p.searched, p.n_rows, p.used, looked_up, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 32);
 }
 
 } // namespace tb

@@ -312,6 +312,7 @@ struct tbk_forest {
   tb::DevQuantGroup *d_rgroups = nullptr;
   tb::DevRankFeature *d_rfeatures = nullptr;
   uint16_t *d_rlut = nullptr;
+  int rank_used = 0;                                     // features with thresholds
   int rank_width = 0, rank_pieces = 1, rank_smem = 0; // the ranking kernel's tables (plan_rank_tables)
   uint32_t *d_rslabs = nullptr;                       // the same interleaved (rank_slabs.cuh), where they fit
   uint32_t slab_bytes = 0, slab_buckets = 0;
@@ -1141,11 +1142,15 @@ tb::RankRowsParams rank_rows_params(const tbk_forest *f, const float *rows, int6
   p.lattice = q.lattice;
   p.bytes = tb::rank_bytes(F);
   p.searched = f->d_ties;
+  p.used = f->rank_used;
   return p;
 }
 
-template <bool BYTES> void (*pick_rank_slabs(int steps))(const tb::SlabParams) {
-  return steps == 1 ? tb::tb_rank_slabs<BYTES, 1> : steps == 2 ? tb::tb_rank_slabs<BYTES, 2> : steps == 3 ? tb::tb_rank_slabs<BYTES, 3> : tb::tb_rank_slabs<BYTES, 0>;
+template <bool BYTES, bool LATTICE> void (*pick_rank_slabs(int steps))(const tb::SlabParams) {
+  return steps == 1   ? tb::tb_rank_slabs<BYTES, 1, LATTICE>
+         : steps == 2 ? tb::tb_rank_slabs<BYTES, 2, LATTICE>
+         : steps == 3 ? tb::tb_rank_slabs<BYTES, 3, LATTICE>
+                      : tb::tb_rank_slabs<BYTES, 0, LATTICE>;
 }
 
 // Tables in shared memory pay from here on (see launch_rank_rows).
@@ -1170,6 +1175,7 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
     sp.num_features = F;
     sp.steps = f->slab_steps;
     sp.searched = f->d_ties;
+    sp.used = f->rank_used;
     sp.status = f->d_status;
     sp.skip_copy = f->expire_next_wait ? 1 : 0;
     sp.wait_tries = f->expire_next_wait ? 2000u : 0u;
@@ -1187,7 +1193,8 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
       }
     }
     const int smem = tb::slab_smem_bytes(f->slab_bytes);
-    const auto kernel = tb::rank_bytes(F) ? pick_rank_slabs<true>(f->slab_steps) : pick_rank_slabs<false>(f->slab_steps);
+    const auto kernel = tb::rank_bytes(F) ? (f->rf.lattice ? pick_rank_slabs<true, true>(f->slab_steps) : pick_rank_slabs<true, false>(f->slab_steps))
+                                          : (f->rf.lattice ? pick_rank_slabs<false, true>(f->slab_steps) : pick_rank_slabs<false, false>(f->slab_steps));
     if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
     const dim3 grid((unsigned)slabs, (unsigned)segments);
     kernel<<<grid, 32 * tb::kSlabWarps, smem, stream>>>(sp);
@@ -2177,6 +2184,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
     for (const auto &g : q.groups)
       if ((int)g.depth != f->uniform_depth) f->uniform_depth = 0;
     f->rf.features = q.features;
+    for (const auto &rf : q.features) f->rank_used += rf.n > 0;
     plan_rank_tables(f);
     const int64_t rows = std::min(batch_hint > 0 ? batch_hint : 65536, rank_rows_per_pass(f));
     const RankPlan plan = plan_rank(f, rows, false);
@@ -2344,8 +2352,7 @@ int tbk_forest_get_info(const tbk_forest *f, tbk_forest_info *info) {
   info->smem_bytes = pl.smem_bytes;
   info->threads_per_block = pl.threads;
   if (f->d_ties) {
-    // key ties resolved on exact values so far -- with rank keys, row values that had to be compared
-    // with thresholds (statistics; synchronises with the device)
+    // (statistics; synchronises with the device)
     unsigned long long ties = 0;
     if (cudaMemcpy(&ties, f->d_ties, 8, cudaMemcpyDeviceToHost) == cudaSuccess) {
       info->reserved[0] = (int32_t)(ties & 0x7fffffff);

@@ -411,8 +411,8 @@ __global__ void __launch_bounds__(kRWThreads, 1)
         const RankRowsParams &r = p.ranking;
         const int F = r.num_features;
         const uint32_t values = (uint32_t)(min((long long)unit1 * UR, p.n_rows) - (long long)unit0 * UR) * (uint32_t)F;
-        unsigned searched = 0;
-        rank_values<kRankInside>(r, (uint32_t)tid, 32u * NW, values, searched,
+        unsigned looked_up = 0;
+        rank_values<kRankInside>(r, (uint32_t)tid, 32u * NW, values, looked_up,
                        [&](uint32_t q, uint32_t f) {
                          if constexpr (INLINE) return p.inline_rows[((uint32_t)(unit0 * UR) + q) * (uint32_t)F + f];
                          else return __ldg(r.rows + ((long long)unit0 * UR + q) * r.ld + f);
@@ -421,10 +421,7 @@ __global__ void __launch_bounds__(kRWThreads, 1)
                          const uint32_t at = S == 64 ? (q >> 1) * 128u + 4u * f + (q & 1u) * 2u : q * S + 2u * f;
                          sts_u16(smem_u32(keys) + at, rank);
                        });
-        if (blockIdx.y == 0) {
-          searched = __reduce_add_sync(0xffffffffu, searched);
-          if (elected && searched) atomicAdd(r.searched, (unsigned long long)searched);
-        }
+        if (blockIdx.y == 0) count_searched(r.searched, values / (uint32_t)F, r.used, looked_up, warp == 0);
         asm volatile("bar.sync 1, %0;" ::"r"(32 * NW) : "memory");
       } else {
         ok = wait(keys_full_s + 8u * ((uint32_t)it & 1u), (uint32_t)(it >> 1) & 1u);
