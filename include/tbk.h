@@ -101,6 +101,10 @@ typedef struct tbk_schedule {
  * stages (9 to 12 levels); nodes in global memory, every lane at its own pace */
 enum { TBK_LAYOUT_TILES = 0, TBK_LAYOUT_RANK_KEYS = 1, TBK_LAYOUT_ROUNDED_KEYS = 2, TBK_LAYOUT_DEEP_KEYS = 3, TBK_LAYOUT_LANES = 4 };
 
+/* which variants of the kernels the last call ran (tbk_forest_info.reserved[2]): fp32 rows turned around in shared
+ * memory; rows ranked with a feature per lane; leaf values of deep trees staged beside the nodes */
+enum { TBK_RAN_ROWS_TURNED = 1, TBK_RAN_SLABS = 2, TBK_RAN_STAGED_LEAVES = 4 };
+
 typedef struct tbk_forest tbk_forest; /* opaque: packed forest resident on a device */
 
 typedef struct tbk_forest_info {
@@ -116,7 +120,8 @@ typedef struct tbk_forest_info {
   int32_t reserved[7];       /* keys: [0] + 2^31 * [1] counts, over all calls, rounded keys' comparisons that tied
                                 and were decided on exact values; rank keys' row values that were ranked by
                                 comparing them with thresholds (those of features that splits use, except whole
-                                numbers on features whose thresholds are whole numbers close together) */
+                                numbers on features whose thresholds are whole numbers close together).
+                                [2]: TBK_RAN_* of the last call */
   int32_t layout;            /* TBK_LAYOUT_* */
 } tbk_forest_info;
 

@@ -38,7 +38,10 @@ def test_staged_leaves(levels, trees, features, rows, chunks):
     assert df.info().layout == kernels.LAYOUT_DEEP_KEYS
     dX = torch.from_numpy(X).cuda()
     some = slice(0, 3000)
-    got, part = df.predict(dX), df.predict_partial(dX)
+    got = df.predict(dX)
+    assert df.info().reserved[2] & kernels.RAN_STAGED_LEAVES
+    part = df.predict_partial(dX)
+    assert df.info().reserved[2] & kernels.RAN_STAGED_LEAVES
     df.check_status()
     want, want_ids = oracle.predict(f, X[some], leaf_ids=True)
     assert_predictions_close(got.cpu().numpy()[some], want)

@@ -39,6 +39,7 @@ def _check(f, X, rows=None, **options):
     want, want_ids = oracle.predict(f, X, leaf_ids=True)
     ids = df.predict_leaf_ids(rows).cpu().numpy()
     df.check_status()
+    assert bool(df.info().reserved[2] & kernels.RAN_SLABS) == (n * f.num_features > 148 * 2048 and f.num_features > 64)
     assert np.array_equal(ids, want_ids)
     got = df.predict(rows).cpu().numpy()
     part = df.finalize(df.predict_partial(rows)).cpu().numpy()

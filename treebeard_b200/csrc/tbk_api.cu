@@ -279,6 +279,7 @@ struct tbk_forest {
   int device = 0;
   tbk_schedule user{};     // what the caller asked for (zeros = auto)
   tb::LaunchPlan last_plan{};
+  int32_t last_ran = 0;    // TBK_RAN_*
   int64_t batch_hint = 0;
   int max_smem_optin = 0;
   int num_sms = 0;
@@ -396,9 +397,10 @@ bool turn_rows(const tb::LaunchPlan &plan, int num_features) {
          2 * (plan.smem_bytes + 1024) > 228 * 1024;
 }
 
-KernelFn pick_kernel(int rep, int ts, const tb::LaunchPlan &plan, int num_features) {
+KernelFn pick_kernel(int rep, int ts, const tb::LaunchPlan &plan, int num_features, int32_t *ran) {
   const int rpl = plan.rows_per_lane;
   const bool staged = plan.staged, cached = plan.cache_rows, turn = turn_rows(plan, num_features);
+  if (turn) *ran |= TBK_RAN_ROWS_TURNED;
   if (rep == tb::kReorg) return pick3<2, 1>(rpl, staged, cached, turn);
   if (rep == tb::kSparse) {
     switch (ts) {
@@ -875,6 +877,7 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
   const bool d12 = f->uniform_depth == 12, ids = mode == kLeafIds, small = plan.threads <= 768;
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
   if (staged) {
+    f->last_ran |= TBK_RAN_STAGED_LEAVES;
     p.split = f->d_qsplit;
     const auto kernel = small ? pick_deep_staged<768>(f->uniform_depth) : pick_deep_staged<1024>(f->uniform_depth);
     if (const int rc = allow_smem(f, (const void *)kernel)) return rc;
@@ -1163,6 +1166,7 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
   const bool pair = F <= tb::kRankPairFeatures, tiled = rank_tiled(F);
   const int64_t lines = pair ? (n + 1) / 2 : tiled ? (n + 31) / 32 * 32 : n;
   if (f->slab_bytes > 0 && slab_batch(f, n, F) && ld * (n + 64) < (int64_t)1 << 30) {
+    f->last_ran |= TBK_RAN_SLABS;
     tb::SlabParams sp{};
     sp.rows = rows;
     sp.n_rows = n;
@@ -1505,6 +1509,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
     if (out_kind != TBK_OUT_F32 && out_kind != TBK_OUT_I8) return fail(TBK_ERR_INVALID, "unknown output kind %d", out_kind);
   }
   CUDA_TRY(cudaSetDevice(f->device));
+  f->last_ran = 0;
   if (f->rank) return run_rank(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
   if (f->lanes) return run_lanes(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
   if (f->quant) return run_quant(f, mode, d_rows, n_rows, ld, d_out, out_kind, d_partial, d_leaf_ids, stream);
@@ -1576,7 +1581,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
     return fail(TBK_ERR_UNSUPPORTED, "launch plan with register class sums needs a single tree chunk");
   p.class_regs = plan.class_regs;
 
-  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features);
+  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features, &f->last_ran);
   if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
@@ -2351,6 +2356,7 @@ int tbk_forest_get_info(const tbk_forest *f, tbk_forest_info *info) {
   info->staged = pl.staged;
   info->smem_bytes = pl.smem_bytes;
   info->threads_per_block = pl.threads;
+  info->reserved[2] = f->last_ran;
   if (f->d_ties) {
     // (statistics; synchronises with the device)
     unsigned long long ties = 0;
@@ -2614,6 +2620,7 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   CUDA_TRY(cudaSetDevice(f->device));
   float *scratch = nullptr;
+  f->last_ran = 0;
   int rc = noalloc_scratch_address(f->device, &scratch);
   if (rc != TBK_OK) return rc;
   if (f->rank)
@@ -2669,7 +2676,7 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   p.vec4_ok = (pk.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0) ? 1 : 0;
   p.status = f->d_status;
   p.class_regs = 0; // class sums go through the shared-memory table the plan has sized
-  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features);
+  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features, &f->last_ran);
   if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
   fn<<<grid, block, plan.smem_bytes, stream>>>(p);

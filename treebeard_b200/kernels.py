@@ -13,6 +13,7 @@ from . import _lib
 REP_AUTO, REP_SPARSE, REP_ARRAY, REP_REORG = -1, 0, 1, 2
 OUT_F32, OUT_I8 = 0, 1
 LAYOUT_TILES, LAYOUT_RANK_KEYS, LAYOUT_ROUNDED_KEYS, LAYOUT_DEEP_KEYS, LAYOUT_LANES = range(5)   # of ForestInfoC
+RAN_ROWS_TURNED, RAN_SLABS, RAN_STAGED_LEAVES = 1, 2, 4   # of ForestInfoC.reserved[2]
 REP_BY_NAME = {"auto": REP_AUTO, "sparse": REP_SPARSE, "gpu_sparse": REP_SPARSE, "array": REP_ARRAY,
                "gpu_array": REP_ARRAY, "reorg": REP_REORG, "gpu_reorg": REP_REORG}
 
