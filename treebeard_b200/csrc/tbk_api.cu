@@ -8,7 +8,9 @@
 #include "lane_pack.h"
 #include "schedule.h"
 #include "walk_kernels.cuh"
+#include "second_pass.cuh"
 #include "walk_quant.cuh"
+#include "quant_keys.cuh"
 #include "walk_quant_batch.cuh"
 #include "walk_deep.cuh"
 #include "rank_rows.cuh"
@@ -377,15 +379,6 @@ struct tbk_forest {
 
 namespace {
 
-using KernelFn = void (*)(const tb::WalkParams);
-
-template <int REP, int TS> KernelFn pick3(int rpl, bool staged, bool cached, bool turn) {
-  if (turn) return staged ? tb::tb_walk_kernel<REP, TS, 1, true, true, true> : tb::tb_walk_kernel<REP, TS, 1, false, true, true>;
-  if (!cached) return staged ? tb::tb_walk_kernel<REP, TS, 1, true, false> : tb::tb_walk_kernel<REP, TS, 1, false, false>;
-  if (rpl == 2) return staged ? tb::tb_walk_kernel<REP, TS, 2, true, true> : tb::tb_walk_kernel<REP, TS, 2, false, true>;
-  return staged ? tb::tb_walk_kernel<REP, TS, 1, true, true> : tb::tb_walk_kernel<REP, TS, 1, false, true>;
-}
-
 // Rows are turned around in shared memory where there are many of them (few tree threads per row) and a block has
 // its SM to itself.  100000 rows of 54 features through 300 trees of 8 levels, two columns in
 // lock-step, row per lane and turned around: sparse tiles of
@@ -397,25 +390,10 @@ bool turn_rows(const tb::LaunchPlan &plan, int num_features) {
          2 * (plan.smem_bytes + 1024) > 228 * 1024;
 }
 
-KernelFn pick_kernel(int rep, int ts, const tb::LaunchPlan &plan, int num_features, int32_t *ran) {
-  const int rpl = plan.rows_per_lane;
-  const bool staged = plan.staged, cached = plan.cache_rows, turn = turn_rows(plan, num_features);
+tb::WalkKernel pick_kernel(int rep, int ts, const tb::LaunchPlan &plan, int num_features, int32_t *ran) {
+  const bool turn = turn_rows(plan, num_features);
   if (turn) *ran |= TBK_RAN_ROWS_TURNED;
-  if (rep == tb::kReorg) return pick3<2, 1>(rpl, staged, cached, turn);
-  if (rep == tb::kSparse) {
-    switch (ts) {
-    case 1: return pick3<0, 1>(rpl, staged, cached, turn);
-    case 2: return pick3<0, 2>(rpl, staged, cached, turn);
-    case 3: return pick3<0, 3>(rpl, staged, cached, turn);
-    default: return pick3<0, 4>(rpl, staged, cached, turn);
-    }
-  }
-  switch (ts) {
-  case 1: return pick3<1, 1>(rpl, staged, cached, turn);
-  case 2: return pick3<1, 2>(rpl, staged, cached, turn);
-  case 3: return pick3<1, 3>(rpl, staged, cached, turn);
-  default: return pick3<1, 4>(rpl, staged, cached, turn);
-  }
+  return tb::walk_kernel(rep, ts, plan.rows_per_lane, plan.staged, plan.cache_rows, turn);
 }
 
 // Dynamic shared memory beyond 48 KB has to be asked for once per kernel and device.  All forests ask for
@@ -680,19 +658,9 @@ int run_quant(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int
   p.wait_tries = f->expire_next_wait ? 2000u : 0u;
   f->expire_next_wait = false;
   // kernels specialised for forests whose groups all have 8 (or 6) levels; generic otherwise
-  using QuantKernel = void (*)(const tb::QuantParams);
   const bool ids = mode == kLeafIds;
   const int ud = (f->uniform_depth == 8 || f->uniform_depth == 6) ? f->uniform_depth : 0;
-  const QuantKernel qkernel =
-      multi ? (ud == 8 ? (ids ? tb::tb_walk_quant_batch_kernel<8, true, true> : tb::tb_walk_quant_batch_kernel<8, false, true>)
-                       : (ids ? tb::tb_walk_quant_batch_kernel<0, true, true> : tb::tb_walk_quant_batch_kernel<0, false, true>))
-      : batched
-          ? (ud == 8   ? (ids ? tb::tb_walk_quant_batch_kernel<8, true, false> : tb::tb_walk_quant_batch_kernel<8, false, false>)
-             : ud == 6 ? (ids ? tb::tb_walk_quant_batch_kernel<6, true, false> : tb::tb_walk_quant_batch_kernel<6, false, false>)
-                       : (ids ? tb::tb_walk_quant_batch_kernel<0, true, false> : tb::tb_walk_quant_batch_kernel<0, false, false>))
-      : ud == 8 ? (ids ? tb::tb_walk_quant_kernel<8, true> : tb::tb_walk_quant_kernel<8, false>)
-      : ud == 6 ? (ids ? tb::tb_walk_quant_kernel<6, true> : tb::tb_walk_quant_kernel<6, false>)
-                : (ids ? tb::tb_walk_quant_kernel<0, true> : tb::tb_walk_quant_kernel<0, false>);
+  const tb::QuantKernel qkernel = batched ? tb::batch_quant_kernel(ud, ids, multi) : tb::wide_quant_kernel(ud, ids);
   if (const int rc = allow_smem(f, (const void *)qkernel)) return rc;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)grid_x, (unsigned)chunks);
@@ -1581,7 +1549,7 @@ int run(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t l
     return fail(TBK_ERR_UNSUPPORTED, "launch plan with register class sums needs a single tree chunk");
   p.class_regs = plan.class_regs;
 
-  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features, &f->last_ran);
+  const tb::WalkKernel fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features, &f->last_ran);
   if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
@@ -2676,7 +2644,7 @@ extern "C" int tbk_predict_noalloc(tbk_forest *f, const float *d_rows, int64_t n
   p.vec4_ok = (pk.num_features % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(d_rows) & 15) == 0) ? 1 : 0;
   p.status = f->d_status;
   p.class_regs = 0; // class sums go through the shared-memory table the plan has sized
-  KernelFn fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features, &f->last_ran);
+  const tb::WalkKernel fn = pick_kernel(pk.representation, pk.tile_size, plan, pk.num_features, &f->last_ran);
   if (const int rc = allow_smem(f, (const void *)fn)) return rc;
   dim3 grid((unsigned)plan.grid_x, (unsigned)plan.chunks), block((unsigned)plan.threads);
   fn<<<grid, block, plan.smem_bytes, stream>>>(p);

@@ -160,7 +160,7 @@ __device__ __forceinline__ void deep_walk_any(uint32_t depth, uint32_t base0, ui
 // Re-walk of one (row, tree) behind a key tie: the staged keys decide wherever they can,
 // the tied comparisons read the exact fp32 values from global memory.  Returns the leaf position.
 // `nodes`: the tree in global memory, or null to read it from the ring at `base`.
-__device__ __noinline__ uint32_t deep_walk_exact(uint32_t base, const uint32_t *nodes, uint32_t key_lane, bool wide, uint32_t depth,
+static __device__ __noinline__ uint32_t deep_walk_exact(uint32_t base, const uint32_t *nodes, uint32_t key_lane, bool wide, uint32_t depth,
                                                  const float *exact_tree, const float *rowp) {
   uint32_t at = 0;
   for (uint32_t d = 0; d < depth; ++d) {

@@ -256,7 +256,7 @@ __device__ __forceinline__ void quant_upper4_any(uint32_t depth, uint32_t (&A)[4
 // comparisons read the exact fp32 values from global memory.
 // Upper levels 0 .. depth-2 of the column at address `up` of the upper-level piece; returns
 // the number of the bottom-level node reached (0 .. 2^(depth-1) - 1).
-__device__ __noinline__ uint32_t quant_upper_exact(uint32_t up, uint32_t keys_lane, const float *exact_plane,
+static __device__ __noinline__ uint32_t quant_upper_exact(uint32_t up, uint32_t keys_lane, const float *exact_plane,
                                                    size_t plane_row, uint32_t depth, uint32_t col,
                                                    const float *rowp) {
   uint32_t s = 0; // level-order number of the node
@@ -275,7 +275,7 @@ __device__ __noinline__ uint32_t quant_upper_exact(uint32_t up, uint32_t keys_la
 }
 // The bottom level: node j of the column at address `bot` of the bottom-level piece;
 // returns the leaf number.
-__device__ __noinline__ uint32_t quant_bottom_exact(uint32_t bot, uint32_t j, uint32_t keys_lane,
+static __device__ __noinline__ uint32_t quant_bottom_exact(uint32_t bot, uint32_t j, uint32_t keys_lane,
                                                     const float *exact_plane, size_t plane_row, uint32_t depth,
                                                     uint32_t col, const float *rowp) {
   const uint32_t node = lds_u32(bot + j * 128u);
@@ -288,25 +288,6 @@ __device__ __noinline__ uint32_t quant_bottom_exact(uint32_t bot, uint32_t j, ui
     right = !(__ldg(rowp + f) < __ldg(exact_plane + (plane_row + (1u << (depth - 1)) + j) * 32u + col));
   }
   return 2u * j + (right ? 1u : 0u);
-}
-
-// Fills the key field of every split node from its exact threshold (run once at upload,
-// so that thresholds and row values are quantised by the very same device arithmetic).
-// wide = 1: the 15-bit keys and feature codes of the wide-row layout (quant_pack.h);
-// 0: the same keys with the deep-tree layout's codes, `code_unit` per feature (deep_pack.h).
-// Pass-through nodes keep their key 0.
-__global__ void tb_quant_fill_keys(uint32_t *node_plane, const float *exact_plane, const float *lo,
-                                   const float *scale, unsigned long long n, int num_features, int wide, uint32_t code_unit) {
-  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t node = node_plane[i];
-  if (wide) {
-    const uint32_t code = node >> 16, f = (code >> 6) * 2u + (code & 1u);
-    if (f < (uint32_t)num_features) node_plane[i] = (code << 16) | quant_threshold_key15_dev(exact_plane[i], lo[f], scale[f]);
-  } else {
-    const uint32_t code = node >> 16, f = code / code_unit;
-    if (node & 0xffffu) node_plane[i] = (code << 16) | quant_threshold_key15_dev(exact_plane[i], lo[f], scale[f]);
-  }
 }
 
 constexpr int kQPiece = 16384;  // one ring slot: half a plane of a group of 8 levels
@@ -475,7 +456,6 @@ __global__ void __launch_bounds__(kQThreads, 1) tb_walk_quant_kernel(const Quant
   };
 
   bool ok = true;
-  uint32_t issued = 0; // pieces that this producer warp has asked for
   unsigned tie_count = 0;
   const uint64_t keep = l2_policy_keep(), stream = l2_policy_stream();
   const uint32_t wait_tries = p.wait_tries ? p.wait_tries : kQWaitTries;
@@ -616,7 +596,6 @@ __global__ void __launch_bounds__(kQThreads, 1) tb_walk_quant_kernel(const Quant
     for (int it = 0; it < my_tiles && ok; ++it) {
       for (int piece = 0; piece < P && ok; ++piece) {
         if (round > 0) ok = mbar_wait_all_lanes(empty_s + 8u * (uint32_t)slot, (round - 1u) & 1u);
-        issued += ok;
         if (ok && lane == 0 && !(p.skip_first_copy && it == 0 && piece == 0)) issue(piece, slot);
         if (++slot == 3) {
           slot = 0;
@@ -878,12 +857,14 @@ __global__ void __launch_bounds__(kQThreads, 1) tb_walk_quant_kernel(const Quant
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kQTmemCols) : "memory");
   }
   if (failed) {
-    if (tid == 0) set_status(p.status, 4);
-    if (producer) // no copy may land after the block is gone
-      for (uint32_t s = 0; s < min(3u, issued); ++s) mbar_wait_all_lanes(full_s + 8u * s, ((issued - 1u - s) / 3u) & 1u);
+    give_up(p.status, 6);
     return;
   }
   if (p.tie_count != nullptr && tie_count) atomicAdd(p.tie_count, (unsigned long long)tie_count);
 }
+
+using QuantKernel = void (*)(const QuantParams);
+// The kernel for forests whose groups all have `depth` levels, 8 or 6; otherwise 0.  (walk_quant.cu)
+QuantKernel wide_quant_kernel(int depth, bool leaf_ids);
 
 } // namespace tb

@@ -154,7 +154,6 @@ __global__ void __launch_bounds__(kQBMaxThreads, 1) tb_walk_quant_batch_kernel(c
   };
 
   bool ok = true;
-  uint32_t issued = 0; // pieces that this producer warp has asked for
   unsigned tie_count = 0;
   const uint64_t keep = l2_policy_keep();
   const uint32_t wait_tries = p.wait_tries ? p.wait_tries : kQWaitTries;
@@ -168,7 +167,6 @@ __global__ void __launch_bounds__(kQBMaxThreads, 1) tb_walk_quant_batch_kernel(c
     for (int it = 0; it < my_batches && ok; ++it) {
       for (int piece = 0; piece < P && ok; ++piece) {
         if (round > 0) ok = wait(empty_s + 8u * (uint32_t)slot, (round - 1u) & 1u);
-        issued += ok;
         if (ok && lane == 0 && !(p.skip_first_copy && it == 0 && piece == 0)) {
           const uint2 gm = group_of(group_index(piece >> 1));
           const uint32_t hs = 1u << (gm.y - 1); // slots per piece
@@ -461,13 +459,13 @@ __global__ void __launch_bounds__(kQBMaxThreads, 1) tb_walk_quant_batch_kernel(c
   // every wait above is bounded: a wait that gave up ends the launch with a status word
   const bool failed = __syncthreads_or(!ok) != 0;
   if (failed) {
-    if (tid == 0) set_status(p.status, 4);
-    if (producer) // no copy may land after the block is gone
-      for (uint32_t s = 0; s < min((uint32_t)kQBSlots, issued); ++s)
-        wait(full_s + 8u * s, ((issued - 1u - s) / (uint32_t)kQBSlots) & 1u);
+    give_up(p.status, 2 * kQBSlots);
     return;
   }
   if (p.tie_count != nullptr && tie_count) atomicAdd(p.tie_count, (unsigned long long)tie_count);
 }
+
+// depth: 8, 6 or 0, as for wide_quant_kernel; multi: multiclass forests.  (walk_quant_batch.cu)
+QuantKernel batch_quant_kernel(int depth, bool leaf_ids, bool multi);
 
 } // namespace tb
