@@ -119,3 +119,18 @@ def test_one_byte_keys_without_allocation():
     rows = torch.zeros((100, 2000), device="cuda")
     with pytest.raises(kernels.TbkError, match="16-bit key"):
         kernels._check(kernels.lib().tbk_predict_noalloc(df._h, rows.data_ptr(), 100, 2000, out.data_ptr(), kernels.OUT_F32, None))
+
+
+@pytest.mark.parametrize("features,stride", [(130, 480000), (600, 1 << 20)])
+def test_slabs_take_rows_of_a_wide_table(features, stride):
+    """A column range of a table so wide that the rows lie further apart than 32 bits of bytes reach."""
+    from treebeard_b200 import kernels
+    f = _forest(60, 6, features)
+    n = 148 * 2048 // features + 45
+    assert 4 * stride * n > 1 << 31
+    X = _rows(f, n, features)
+    table = torch.empty(7 + n * stride, device="cuda")
+    rows = table[7:].view(n, stride)[:, :features]
+    rows.copy_(torch.from_numpy(X))
+    df = _check(f, X, rows)
+    assert df.info().reserved[2] & kernels.RAN_SLABS

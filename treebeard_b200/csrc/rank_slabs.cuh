@@ -28,7 +28,7 @@ constexpr int slab_smem_bytes(uint32_t table_bytes) { return 128 + kSlabWarps * 
 struct SlabParams {
   const float *rows;
   long long n_rows;
-  uint32_t ld_bytes;
+  uint32_t ld_bytes; // (32 rows within 32 bits; where a tile starts is a matter of 64)
   const unsigned char *tables; // a table per slab
   unsigned char *keys;         // tiles of tile_bytes
   uint32_t table_bytes, buckets, tile_bytes;
@@ -75,10 +75,11 @@ template <bool BYTES, int STEPS, bool LATTICE> __global__ void __launch_bounds__
   auto fetch = [&](int t, auto first) {
     constexpr int c = decltype(first)::value;
     const int rows = t < end ? n_rows - t * 32 : 0;
-    uint32_t at = (uint32_t)(t * 32 + c) * p.ld_bytes; // (the host sees to it that 32 bits do)
+    const char *tile_at = column + (long long)t * (32ll * p.ld_bytes);
+    uint32_t at = c * p.ld_bytes;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %2, %3;\n @p ld.global.nc.f32 %0, [%1];\n}" : "+f"(x[c + k]) : "l"(column + at), "r"(rows), "r"(c + k));
+      asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %2, %3;\n @p ld.global.nc.f32 %0, [%1];\n}" : "+f"(x[c + k]) : "l"(tile_at + at), "r"(rows), "r"(c + k));
       at += p.ld_bytes;
     }
   };

@@ -1133,7 +1133,7 @@ int launch_rank_rows(tbk_forest *f, const float *rows, int64_t n, int64_t ld, ui
   tb::RankRowsParams p = rank_rows_params(f, rows, n, ld, keys);
   const bool pair = F <= tb::kRankPairFeatures, tiled = rank_tiled(F);
   const int64_t lines = pair ? (n + 1) / 2 : tiled ? (n + 31) / 32 * 32 : n;
-  if (f->slab_bytes > 0 && slab_batch(f, n, F) && ld * (n + 64) < (int64_t)1 << 30) {
+  if (f->slab_bytes > 0 && slab_batch(f, n, F) && ld < (int64_t)1 << 25) {
     f->last_ran |= TBK_RAN_SLABS;
     tb::SlabParams sp{};
     sp.rows = rows;
