@@ -1251,6 +1251,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
     plan = plan_rank(f, pass, mode == kLeafIds);
   }
   const bool tiled = rank_tiled(q.num_features);
+  if (tiled && plan.quads == 0) return fail(TBK_ERR_UNSUPPORTED, "no launch shape holds rank keys of %d features under trees of %d levels", q.num_features, q.max_depth);
   const int walkers = rank_walkers(f, plan, n_rows);
   f->last_plan = rank_launch_plan(plan, walkers);
   tbk_forest::Workspace *ws = nullptr;
@@ -1953,6 +1954,11 @@ int tbk_image_deserialize(const void *buffer, uint64_t size, tbk_image **out) {
   std::unique_ptr<tbk_image> img(new tbk_image());
   const std::string err = tb::deserialize_image(static_cast<const uint8_t *>(buffer), size, &img->im);
   if (!err.empty()) return fail(TBK_ERR_IO, "%s", err.c_str());
+  // (not every width below kRankMaxByteFeatures has a launch shape under every depth; an image made here has one)
+  const tb::RankForest &q = img->im.rf;
+  if (img->im.kind == tb::PackedImage::kRank && !rank_fits(q.num_features, q.max_depth, img->im.smem_limit))
+    return fail(TBK_ERR_UNSUPPORTED, "packed image: no launch shape holds rank keys of %d features under trees of %d levels in %d bytes "
+                                     "of shared memory", q.num_features, q.max_depth, img->im.smem_limit);
   *out = img.release();
   return TBK_OK;
 }
