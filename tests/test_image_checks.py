@@ -73,3 +73,41 @@ def test_rank_images_without_a_launch_shape(features, levels, fits):
     else:
         with pytest.raises(kernels.TbkError):
             kernels.PackedImage.from_bytes(data)
+
+
+def _deep_image(pairs, levels):
+    """An image whose table of pairs is `pairs` (elements, levels each; None: as packed) and whose forest has `levels` levels."""
+    body = _image(5, 9, 30)
+    at, n = FOREST + 8, struct.unpack_from("<Q", body, FOREST)[0]
+    table = [struct.unpack_from("<QII", body, at + 16 * i) for i in range(n)]
+    assert [t[1] for t in table] == [9] * n == [9] * 3
+    for i, elements in enumerate(pairs or []):
+        struct.pack_into("<Q", body, at + 16 * i, elements * 2 * table[0][2])
+    struct.pack_into("<i", body, FOREST - 4, levels)
+    return _signed(body)
+
+
+@pytest.mark.parametrize("pairs,levels,whole", [(None, 9, True), ([0, 1, 2], 9, True), ([0, 0, 0], 9, False), ([1, 0, 2], 9, False),
+                                                ([0, 1, 1], 9, False), (None, 12, False), (None, 8, False), (None, -1, False)])
+def test_deep_images_whose_pairs_do_not_lie_one_behind_the_other(pairs, levels, whole):
+    """The re-ordering of a forest's planes and the kernels for one depth count on it."""
+    data = _deep_image(pairs, levels)
+    if whole:
+        assert kernels.PackedImage.from_bytes(data).to_bytes() == data
+    else:
+        with pytest.raises(kernels.TbkError):
+            kernels.PackedImage.from_bytes(data)
+
+
+def test_deep_images_without_all_their_planes():
+    """Two of three pairs' planes, their sizes alike."""
+    body = _image(5, 9, 30)
+    at = FOREST + 8 + 16 * 3
+    for _ in range(4):                                          # nodes, leaves, exact thresholds, original leaves
+        n = struct.unpack_from("<Q", body, at)[0]
+        keep = n // 3 * 2
+        struct.pack_into("<Q", body, at, keep)
+        del body[at + 8 + 4 * keep:at + 8 + 4 * n]
+        at += 8 + 4 * keep
+    with pytest.raises(kernels.TbkError):
+        kernels.PackedImage.from_bytes(_signed(body))

@@ -1,6 +1,7 @@
 #include "packed_image.h"
 #include "checksum.h"
 
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 
@@ -318,8 +319,15 @@ std::string deserialize_image(const uint8_t *data, uint64_t size, PackedImage *i
                   q.tree_index.size() != q.pairs.size() * 2 || q.lo.size() != (size_t)q.num_features + 1 ||
                   q.scale.size() != q.lo.size()))
       in.ok = false;
-    for (const QuantGroup &g : q.pairs)
-      if (in.ok && (g.depth > (uint32_t)kDeepMaxDepth || g.slots != deep_tree_words(g.depth) || g.elem_off + 2ull * g.slots > n)) in.ok = false;
+    // (kernels for one depth find a tree by its number: pairs lie one behind the other, the deepest as deep as the forest)
+    uint64_t end = 0;
+    uint32_t deepest = 0;
+    for (const QuantGroup &g : q.pairs) {
+      if (in.ok && (g.depth < (uint32_t)kDeepMinDepth || g.depth > (uint32_t)kDeepMaxDepth || g.slots != deep_tree_words(g.depth) || g.elem_off != end)) in.ok = false;
+      end += 2ull * g.slots;
+      deepest = std::max(deepest, g.depth);
+    }
+    if (in.ok && (end != n || q.max_depth < 0 || deepest != (uint32_t)std::max(q.max_depth, kDeepMinDepth))) in.ok = false;
   } else {
     return "packed image: unknown layout kind";
   }
