@@ -11,6 +11,10 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
+def _staged(df):
+    return bool(df.info().reserved[2] & kernels.RAN_STAGED_LEAVES)
+
+
 @pytest.mark.parametrize("levels", [9, 10, 11, 12])
 @pytest.mark.parametrize("trees,features,rows,chunks", [
     (1, 3, 1, 0), (7, 16, 33, 0), (40, 128, 1000, 1), (41, 60, 5003, 3), (33, 140, 700, 1), (35, 24, 150001, 0)])
@@ -39,9 +43,9 @@ def test_staged_leaves(levels, trees, features, rows, chunks):
     dX = torch.from_numpy(X).cuda()
     some = slice(0, 3000)
     got = df.predict(dX)
-    assert df.info().reserved[2] & kernels.RAN_STAGED_LEAVES
+    assert _staged(df)
     part = df.predict_partial(dX)
-    assert df.info().reserved[2] & kernels.RAN_STAGED_LEAVES
+    assert _staged(df)
     df.check_status()
     want, want_ids = oracle.predict(f, X[some], leaf_ids=True)
     assert_predictions_close(got.cpu().numpy()[some], want)
@@ -51,3 +55,61 @@ def test_staged_leaves(levels, trees, features, rows, chunks):
     if rows > 3000:
         tail = oracle.predict(f, X[-500:])
         assert_predictions_close(got.cpu().numpy()[-500:], tail)
+
+
+@pytest.mark.parametrize("trees,features,rows,chunks", [(7, 90, 33, 0), (40, 200, 5003, 3), (41, 90, 20011, 1), (40, 83, 1000, 0)])
+def test_gathered_leaves(trees, features, rows, chunks):
+    """12 levels over widths at which a ring with leaf values would cost row warps: leaf values are gathered, by the kernel
+    for 12 levels over narrow rows."""
+    marg = synth.Marginal("normal", features)
+    f = synth.generate_forest(8, trees, 12, features, 0.02, 0.1, marg)
+    X = marg.sample_rows(np.random.Generator(np.random.PCG64(6)), rows)
+    split = np.nonzero(f.left >= 0)[0]
+    for i in range(min(3 * rows, 600)):
+        g = split[(i * 37) % len(split)]
+        X[(i * 13) % rows, f.feat[g]] = np.nextafter(f.thr[g], np.float32([-np.inf, np.inf, f.thr[g]][i % 3]))
+    X[3, :], X[4, 0] = np.nan, np.inf
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=rows, tree_chunks=chunks)
+    assert df.info().layout == kernels.LAYOUT_DEEP_KEYS
+    dX = torch.from_numpy(X).cuda()
+    got, part, ids = df.predict(dX), df.predict_partial(dX), df.predict_leaf_ids(dX)
+    assert not _staged(df)
+    df.predict(dX)
+    assert not _staged(df)
+    df.check_status()
+    some = np.r_[0:min(rows, 3000), max(0, rows - 500):rows]
+    want, want_ids = oracle.predict(f, X[some], leaf_ids=True)
+    assert_predictions_close(got.cpu().numpy()[some], want)
+    assert_predictions_close(df.finalize(part).cpu().numpy()[some], want)
+    assert np.array_equal(ids.cpu().numpy()[some], want_ids)
+
+
+@pytest.mark.parametrize("trees,features,rows,staged", [
+    (80, 24, 90001, True), (80, 92, 60001, True), (60, 128, 40001, True), (66, 128, 80001, False), (80, 96, 80033, False),
+    (80, 160, 50001, False), (300, 128, 2001, True), (1501, 128, 50001, False), (1501, 128, 100001, True)])
+def test_twelve_levels(trees, features, rows, staged):
+    """Leaf values of 12 levels are gathered where rows are wide and blocks walk many pairs, unless many trees meet a large
+    batch; the last block has warps without rows."""
+    marg = synth.Marginal("normal", features)
+    f = synth.generate_forest(9, trees, 12, features, 0.02 if trees < 1000 else 0.12, 0.1, marg)
+    X = np.tile(marg.sample_rows(np.random.Generator(np.random.PCG64(7)), 5003), (rows // 5003 + 1, 1))[:rows]
+    split = np.nonzero(f.left >= 0)[0]
+    some = np.r_[0:300, rows - 300:rows]
+    for i, r in enumerate(np.repeat(some, 3)):
+        g = split[(i * 37) % len(split)]
+        X[r, f.feat[g]] = np.nextafter(f.thr[g], np.float32([-np.inf, np.inf, f.thr[g]][i % 3]))
+    X[3, :], X[4, 0] = np.nan, np.inf
+    df = kernels.DeviceForest(f, representation="auto")
+    assert df.info().layout == kernels.LAYOUT_DEEP_KEYS
+    dX = torch.from_numpy(X).cuda()
+    got = df.predict(dX)
+    assert _staged(df) == staged
+    part = df.predict_partial(dX)
+    assert _staged(df) == staged
+    ids = df.predict_leaf_ids(dX[-5000:]) if trees < 1000 else None
+    df.check_status()
+    want, want_ids = oracle.predict(f, X[some], leaf_ids=True)
+    assert_predictions_close(got.cpu().numpy()[some], want)
+    assert_predictions_close(df.finalize(part).cpu().numpy()[some], want)
+    if ids is not None:
+        assert np.array_equal(ids[-300:].cpu().numpy(), want_ids[-300:])

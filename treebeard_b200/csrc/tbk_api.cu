@@ -773,6 +773,20 @@ DeepSplit split_deep(const tbk_forest *f, int64_t n_rows, bool staged) {
   return best;
 }
 
+// Are staged leaves the faster ones?  A pair of trees costs them one more wait, and 12 levels have a gathering kernel of their own,
+// which wins where rows are so wide that few row warps fit (96 features and more; what a pair costs the shared-memory
+// pipe matters less) and blocks walk enough pairs to make up for a later end -- unless a forest of 1500 trees and more
+// is walked in whole waves and its gathers miss L2.  Staged / gathered, 12 levels: 1200 trees x 128 features, batches of 2500 (21 pairs
+// to a block) 1.00, 7000 (55) 1.02, 24000 1.07, 76000 1.09, 170000 rows 1.03; 500 x 160: 4000 (21) 1.00, 17000 (84) 1.04, 64000 1.07;
+// 2000 x 100: 12000 1.10, 33000 1.04, 125000 0.99, 170000 0.98; 2000 x 128: 17000 1.10, 100000 0.99.  500 x 60 and 30: 0.86 to 0.96
+// from 4000 rows on.  9 to 11 levels: 0.90 to 1.00.
+bool deep_staged_pays(const tbk_forest *f, const DeepSplit &s, int64_t n_rows) {
+  const int64_t pairs = (int64_t)f->df.pairs.size(), per_block = s.whole > 0 ? pairs : (pairs + s.chunks - 1) / s.chunks;
+  const bool waves = n_rows > 32ll * s.row_warps * f->num_sms;
+  return f->uniform_depth < 12 || f->df.num_features < 96 || s.row_warps > f->deep_row_warps || per_block < 32 ||
+         (waves && f->df.num_trees >= 1500);
+}
+
 // One launch of the deep-tree kernel over `n_rows` rows, and the second pass over chunks.
 int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
                   float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream, bool staged, int rw, int64_t chunks) {
@@ -875,7 +889,7 @@ int run_deep_rows(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows,
 int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int64_t ld, void *d_out,
              float *d_partial, int32_t *d_leaf_ids, cudaStream_t stream) {
   DeepSplit &s = f->deep_split;
-  const bool staged = f->d_qsplit && mode != kLeafIds;
+  bool staged = f->d_qsplit && mode != kLeafIds;
   if (s.n_rows != n_rows || s.staged != staged) {
     s = split_deep(f, n_rows, staged);
     if (f->user.tree_chunks > 0) { // (asked for: all rows)
@@ -883,6 +897,7 @@ int run_deep(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
       s.chunks = f->user.tree_chunks;
     }
   }
+  staged = staged && deep_staged_pays(f, s, n_rows);
   if (f->timing) CUDA_TRY(cudaEventRecord(f->ev0, stream));
   const int64_t first = std::min<int64_t>(n_rows, s.whole * s.row_warps * 32);
   if (first > 0) {
