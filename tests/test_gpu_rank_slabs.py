@@ -134,3 +134,90 @@ def test_slabs_take_rows_of_a_wide_table(features, stride):
     rows.copy_(torch.from_numpy(X))
     df = _check(f, X, rows)
     assert df.info().reserved[2] & kernels.RAN_SLABS
+
+
+def _crowded(f, seed):
+    """Thresholds of every feature that crowd in one bucket of its table, whatever the number of buckets (up to eight for
+    each threshold), by kind of feature: within a unit around 1, with one far off; within a unit below one far off; over a range
+    that fp32 cannot divide; between two neighbouring numbers; all over the range (not crowded)."""
+    g = np.random.default_rng(seed)
+    split = np.nonzero(f.left >= 0)[0]
+    thr = f.thr.copy()
+    far = {}
+    for k in split:
+        i = int(f.feat[k])
+        kind = i % 5
+        if kind == 0:
+            thr[k] = 1 + g.random(dtype=np.float32)
+        elif kind == 1:
+            thr[k] = 5e6 + np.float32(g.integers(0, 200) / 2)
+        elif kind == 2:
+            thr[k] = np.float32(g.random() * 10)
+        elif kind == 3:
+            thr[k] = np.nextafter(np.float32(1), np.float32(1 + g.integers(0, 2)))
+        far.setdefault(i, k)
+    for i, k in far.items():
+        thr[k] = {0: -1e7, 1: -3e6, 2: -3.2e38, 3: thr[k], 4: thr[k]}[i % 5]
+    far2 = {}
+    for k in split[::-1]:
+        i = int(f.feat[k])
+        if i % 5 == 2 and i not in far2 and far[i] != k:
+            far2[i] = k
+            thr[k] = 3.2e38
+    f.thr = thr
+    return f
+
+
+@pytest.mark.parametrize("features,trees,levels", [(65, 40, 7), (100, 60, 8), (511, 100, 8), (512, 100, 8), (700, 150, 8), (2000, 300, 8)])
+def test_crowded_thresholds(features, trees, levels):
+    """Buckets that take more search steps than the variants with a number of steps of their own have."""
+    f = _crowded(_forest(trees, levels, features), features)
+    split = f.left >= 0
+    crowd = max(len(np.unique(f.thr[split & (f.feat == i)])) for i in range(0, features, 5))
+    assert 8 < crowd - 1 <= 255   # thresholds in one bucket: four search steps and more
+    n = 148 * 2048 // features + 45
+    X = _rows(f, n, features)
+    g = np.random.default_rng(2)
+    at = np.nonzero(split)[0]
+    for i in range(features):     # both sides of the feature's thresholds
+        mine = f.thr[at[f.feat[at] == i]]
+        if len(mine):
+            pick = mine[g.integers(0, len(mine), n - 4)]
+            X[4:, i] = np.nextafter(pick, np.float32([-np.inf, np.inf])[g.integers(0, 2, n - 4)])
+            X[4::3, i] = pick[::3]
+    _check(f, X)
+
+
+@pytest.mark.parametrize("most,ranks", [(255, True), (256, False)])
+@pytest.mark.parametrize("used", [0, 300, 599])
+def test_the_most_thresholds_that_a_byte_holds(most, ranks, used):
+    """One feature with `most` distinct thresholds, each of them several times, and all others with fewer."""
+    from treebeard_b200 import kernels
+    f = _forest(40, 7, 600)
+    split = np.nonzero(f.left >= 0)[0]
+    mine = split[::5]
+    assert len(mine) > 3 * most
+    f.feat = np.where(f.left >= 0, np.where(f.feat == used, (used + 1) % 600, f.feat), f.feat).astype(f.feat.dtype)
+    f.feat[mine] = used
+    f.thr[mine] = (np.arange(len(mine)) % most / 64).astype(np.float32)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=500)
+    assert df.info().layout == (kernels.LAYOUT_RANK_KEYS if ranks else kernels.LAYOUT_ROUNDED_KEYS)
+    X = _rows(f, 500, 600)
+    X[4:, used] = np.random.default_rng(1).integers(-20, 300, 496) / np.float32(64)
+    assert np.array_equal(df.predict_leaf_ids(torch.from_numpy(X).cuda()).cpu().numpy(), oracle.predict(f, X, leaf_ids=True)[1])
+
+
+@pytest.mark.parametrize("features,levels,fits", [(2019, 8, True), (2024, 8, True), (2025, 8, False), (2044, 7, True), (2045, 7, False)])
+def test_widest_one_byte_keys(features, levels, fits):
+    from treebeard_b200 import kernels
+    f = _forest(70, levels, features)
+    for n in (1, 33, 3001):
+        X = _rows(f, n, features)
+        if fits:
+            _check(f, X)
+            _check(f, X, tree_chunks=2)
+        else:
+            df = kernels.DeviceForest(f, representation="auto", batch_hint=n)
+            assert df.info().layout == kernels.LAYOUT_TILES   # (too wide for rounded keys too)
+            ids = df.predict_leaf_ids(torch.from_numpy(X).cuda()).cpu().numpy()
+            assert np.array_equal(ids, oracle.predict(f, X, leaf_ids=True)[1])

@@ -35,6 +35,8 @@
 #include "forest.h"
 #include "quant_pack.h"
 
+#include <memory>
+
 namespace tb {
 
 constexpr int kRankCols = 32, kRankMaxDepth = 8;
@@ -102,7 +104,8 @@ struct SlabTables {
   uint32_t buckets = 0; // lines of each slab
   int32_t steps = 0;
   uint32_t bytes = 0; // per slab
-  std::vector<uint32_t> words;
+  std::unique_ptr<uint32_t[]> words;
+  size_t num_words = 0;
 };
 // False where a slab takes more than `room` bytes.  One to eight buckets per threshold of the feature that has most.
 bool make_slab_tables(const RankForest &q, uint32_t room, SlabTables *out);

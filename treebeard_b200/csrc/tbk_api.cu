@@ -2127,7 +2127,7 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
       size_t total = 0;
       auto part = [&](auto **dst, const auto &v) {
         parts.push_back({(void **)dst, v.data(), v.size() * sizeof(v[0]), total});
-        total += (v.size() * sizeof(v[0]) + 255) / 256 * 256 + 256; // (empty vectors get an address too)
+        total += (parts.back().bytes + 255) / 256 * 256 + 256; // (empty vectors get an address too)
       };
       const std::vector<unsigned long long> zeros(16, 0);
       part(&f->d_ties, zeros);
@@ -2137,16 +2137,17 @@ int tbk_forest_create_from_image(const tbk_image *img, const tbk_schedule *sched
       part(&f->d_rfeatures, q.features);
       part(&f->d_rlut, q.lut);
       part(&f->d_rthr, q.thresholds);
+      const size_t small = total;
       // (one request for shared memory holds a slab's table and the warps' buffers; narrower rows whose batches are announced as too small for slabs need none)
       tb::SlabTables slabs;
       const bool large = batch_hint <= 0 || tb::rank_bytes(q.num_features) || slab_batch(f, batch_hint, q.num_features);
       if (rank_tiled(q.num_features) && large && tb::make_slab_tables(q, (uint32_t)(f->max_smem_optin - tb::slab_smem_bytes(0)), &slabs)) {
-        part(&f->d_rslabs, slabs.words);
+        parts.push_back({(void **)&f->d_rslabs, slabs.words.get(), slabs.num_words * 4, total});
+        total += (parts.back().bytes + 255) / 256 * 256;
         f->slab_bytes = slabs.bytes;
         f->slab_buckets = slabs.buckets;
         f->slab_steps = slabs.steps;
       }
-      const size_t small = total;
       part(&f->d_rnode, q.node_plane);
       part(&f->d_rleaf, q.leaf_plane);
       part(&f->d_rorig, q.orig_leaf);
