@@ -188,6 +188,16 @@ def test_crowded_thresholds(features, trees, levels):
     _check(f, X)
 
 
+@pytest.mark.parametrize("features,hint", [(1500, 32768), (1750, 70000), (2000, 262144)])
+def test_one_byte_keys_whatever_the_announced_batch(features, hint):
+    from treebeard_b200 import kernels
+    f = _forest(800, 3, features)
+    df = kernels.DeviceForest(f, representation="auto", batch_hint=hint)
+    assert df.info().layout == kernels.LAYOUT_RANK_KEYS
+    X = _rows(f, 300, features)
+    assert np.array_equal(df.predict_leaf_ids(torch.from_numpy(X).cuda()).cpu().numpy(), oracle.predict(f, X, leaf_ids=True)[1])
+
+
 @pytest.mark.parametrize("most,ranks", [(255, True), (256, False)])
 @pytest.mark.parametrize("used", [0, 300, 599])
 def test_the_most_thresholds_that_a_byte_holds(most, ranks, used):

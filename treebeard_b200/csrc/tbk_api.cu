@@ -1741,14 +1741,12 @@ bool few_trees(int num_features, int64_t num_trees, int max_depth, int64_t batch
 
 // Rows of more than 511 features whose features have at most 255 distinct thresholds: one-byte ranks instead of rounded
 // keys, where the batches to come are announced (without a hint the layout stays that of images made ahead of time).  Of
-// 120 shapes (520 to 2000 features, 100 to 1000 trees of 6 and 8 levels, 1024, 8192 and 65536 rows) none is slower by more than 3 %; microseconds
-// on rounded keys and on ranks: 300 trees of 6 levels x 520 features 34.9 / 11.8, 55.0 / 19.6, 241.5 / 85.1; 600 trees of
-// 8 levels x 1600 features 40.5 / 14.8, 66.3 / 42.7, 282 / 263; 1000 trees of 8 levels x 2000 features 28.5 / 16.6, 81.2 / 53.8,
-// 367.6 / 350.6, and 1397 / 1384 at 262144 rows.  For the last kind, the widest rows through most trees in large batches, the
-// gain does not pay for a preparation that takes 18 ms longer (52 instead of 33 ms: rank tables, memory for the keys of a pass).
-bool byte_ranks(int num_features, int64_t num_trees, int64_t batch_hint) {
-  return batch_hint > 0 && !(num_features >= 1500 && num_trees >= 800 && batch_hint >= 32768);
-}
+// 170 shapes (520 to 2018 features, 100 to 1500 trees of 6 to 8 levels, 1024 to 262144 rows) none is slower by more than 3 %; microseconds
+// on rounded keys and on ranks: 300 trees of 6 levels x 520 features 34.9 / 11.8, 55.0 / 19.6, 241.5 / 85.1 for 1024, 8192 and 65536
+// rows; 600 trees of 8 levels x 1600 features 40.5 / 14.8, 66.3 / 42.7, 282 / 263; 800 x 1750 394 / 294 and 1000 x 2000 370 / 355 at
+// 65536 rows, 1422 / 1401 at 262144 (1076 / 1085 at 200000).  Preparation takes up to 5 ms longer (rank tables: 1500 features x 1000 trees 11.3 -> 16.6 ms, 2000 x 1000
+// 14.3 -> 15.5, 520 x 100 2.0 -> 2.3), as much as 30 to 300 calls gain.
+bool byte_ranks(int64_t batch_hint) { return batch_hint > 0; }
 
 } // namespace
 
@@ -1841,7 +1839,7 @@ int create_image(const tbk_forest_arrays *fa, const tbk_schedule *schedule, int3
                         few_trees(host.num_features, T, max_depth, batch_hint);
   const bool want_rank =
       want_quant || (bits == 0 && rep == TBK_REP_AUTO && ts == 1 && max_depth <= tb::kRankMaxDepth && !tiles_do);
-  const bool bytes_do = !tb::rank_bytes(host.num_features) || (bits == 0 && byte_ranks(host.num_features, T, batch_hint));
+  const bool bytes_do = !tb::rank_bytes(host.num_features) || (bits == 0 && byte_ranks(batch_hint));
   if (want_rank && bytes_do && host.num_features <= tb::kRankMaxByteFeatures && rank_fits(host.num_features, max_depth, smem_limit)) {
     if (tb::pack_rank(host, &im.rf).empty()) {
       im.kind = tb::PackedImage::kRank;
