@@ -110,6 +110,21 @@ def test_the_call_that_may_not_allocate(trees, levels, features, classes, rows):
             assert_predictions_close(out.cpu().numpy(), want.cpu().numpy())
 
 
+@pytest.mark.parametrize("rows", [1, 1005, 9601])
+def test_the_call_that_may_not_allocate_on_rounded_keys(rows):
+    """Wide rows whose keys are asked for, or whose batches are not announced, stay on rounded keys."""
+    f, marg = _forest(40, 6, 700)
+    dX = torch.from_numpy(_rows(f, marg, rows)).cuda()
+    for options in (dict(batch_hint=rows, feature_bits=16), {}):
+        df = kernels.DeviceForest(f, representation="auto", **options)
+        assert df.info().layout == kernels.LAYOUT_ROUNDED_KEYS
+        want, out = df.predict(dX), torch.empty(rows, device="cuda")
+        kernels._check(kernels.lib().tbk_predict_noalloc(df._h, dX.data_ptr(), rows, 700, out.data_ptr(), kernels.OUT_F32,
+                                                         torch.cuda.current_stream().cuda_stream))
+        df.check_status()
+        assert_predictions_close(out.cpu().numpy(), want.cpu().numpy())
+
+
 @pytest.mark.parametrize("features", [490, 491, 506, 507, 511])
 @pytest.mark.parametrize("rows", [300, 20011])
 def test_widest_rank_key_rows_under_the_deepest_trees(features, rows):

@@ -20,13 +20,17 @@ LAYOUTS = {
     "rank": (200, 8, 28, 0, {}),
     "rank_tiles": (100, 7, 90, 0, {}),
     "rank_classes": (60, 6, 16, 5, {}),
-    "rounded_wide": (48, 8, 700, 0, {}),
+    "rank_bytes": (48, 8, 700, 0, {}),   # (where batches are announced)
+    "rounded_wide": (48, 8, 700, 0, dict(feature_bits=16)),
     "rounded_classes": (48, 6, 100, 3, {}),
     "deep": (24, 11, 40, 0, {}),
     "lanes": (50, 14, 16, 0, {}),
     "tiles": (300, 8, 28, 0, dict(representation="sparse", tree_chunks=3)),
 }
 
+EXPECTED = {"rank": kernels.LAYOUT_RANK_KEYS, "rank_tiles": kernels.LAYOUT_RANK_KEYS, "rank_classes": kernels.LAYOUT_RANK_KEYS,
+            "rank_bytes": kernels.LAYOUT_RANK_KEYS, "rounded_wide": kernels.LAYOUT_ROUNDED_KEYS, "rounded_classes": kernels.LAYOUT_ROUNDED_KEYS,
+            "deep": kernels.LAYOUT_DEEP_KEYS, "lanes": kernels.LAYOUT_LANES, "tiles": kernels.LAYOUT_TILES}
 
 SINGLE = [name for name, shape in LAYOUTS.items() if not shape[3]]
 
@@ -50,6 +54,7 @@ def test_a_new_forest_is_ready_for_every_stream(layout):
     torch.cuda.synchronize()
     for _ in range(5):
         df = kernels.DeviceForest(f, batch_hint=len(X), **options)
+        assert df.info().layout == EXPECTED[layout]
         assert torch.cuda.default_stream().query()
         with torch.cuda.stream(side):
             ids, got = df.predict_leaf_ids(dX), df.predict(dX)
@@ -78,6 +83,7 @@ def test_per_thread_streams_do_not_share_call_memory(layout):
     dX = torch.from_numpy(X).cuda()
     parts = [dX[i * 6000:(i + 1) * 6000] for i in range(4)]
     df = kernels.DeviceForest(f, batch_hint=6000, **options)
+    assert df.info().layout == EXPECTED[layout]
     want = [df.predict(p).clone() for p in parts]
     outs = [torch.empty_like(w) for w in want]
     torch.cuda.synchronize()
@@ -109,6 +115,7 @@ def test_streams_that_come_and_go(layout, alive):
     f, X, options = _case(layout, 40000)
     dX = torch.from_numpy(X).cuda()
     df = kernels.DeviceForest(f, batch_hint=5000, **options)
+    assert df.info().layout == EXPECTED[layout]
     sizes = [5000 + 307 * i for i in range(12)]
     batches = [dX[1000 * i:1000 * i + n] for i, n in enumerate(sizes)]
     want = [df.predict(b).clone() for b in batches]
@@ -143,7 +150,8 @@ def _captured(df, rows, out):
 def test_memory_of_captured_calls_lives_as_long_as_their_graphs(layout):
     f, X, options = _case(layout, 60000)
     dX = torch.from_numpy(X).cuda()
-    df = kernels.DeviceForest(f, **options)
+    df = kernels.DeviceForest(f, batch_hint=60000 if layout == "rank_bytes" else 0, **options)
+    assert df.info().layout == EXPECTED[layout]
     sizes = [60000 - 1000 * i for i in range(24)]
     want = [df.predict(dX[:n]).clone() for n in sizes]
     outs = [torch.empty(n, device="cuda") for n in sizes]
@@ -171,7 +179,7 @@ def test_memory_of_captured_calls_lives_as_long_as_their_graphs(layout):
         assert torch.equal(out, want[k % 24])
         del graph
         free.append(torch.cuda.mem_get_info()[0])
-    keys = {"rank": 4, "rank_tiles": 16}.get(layout, 1) << 20   # the most that one call takes, to a power of two
+    keys = {"rank": 4, "rank_tiles": 16, "rank_bytes": 64}.get(layout, 1) << 20   # the most that one call takes, to a power of two
     assert min(free[8:]) >= free[0] - 8 * keys
     assert torch.equal(df.predict(dX[:sizes[0]]), want[0])
     df.check_status()
@@ -187,6 +195,7 @@ def test_forests_of_one_kernel_and_different_sizes_in_two_threads():
         f = synth.generate_forest(features, 16, levels, features, 0.1, 0.1, marg)
         X = torch.from_numpy(marg.sample_rows(np.random.Generator(np.random.PCG64(1)), rows)).cuda()
         df = kernels.DeviceForest(f, **dict(dict(representation="auto"), **options))
+        assert df.info().layout == EXPECTED[layout]
         forests.append((df, X, df.predict(X).clone()))
     torch.cuda.synchronize()
     wrong, start = [], threading.Barrier(2)
