@@ -109,7 +109,8 @@ typedef struct tbk_forest tbk_forest; /* opaque: packed forest resident on a dev
 
 typedef struct tbk_forest_info {
   int64_t num_trees, num_nodes, num_groups;
-  int64_t packed_bytes;      /* bytes of node tiles resident on the device */
+  int64_t packed_bytes;      /* bytes of nodes and leaf values resident on the device; of deep trees whose leaf
+                                values are staged both orders of them, twice those of other deep trees */
   int32_t max_depth;         /* decision levels on the deepest root-to-leaf path */
   int32_t num_features, num_classes, transform;
   int32_t device;
@@ -131,19 +132,23 @@ typedef struct tbk_forest_info {
  * src/gpu/ReorgForestRepresentation.cpp:400-487) and the host-side lowering that
  * feeds them (src/utils/TreeTilingUtils.cpp:427-556).  `schedule` may be NULL.
  * batch_hint: rows of the batches to come (0 = not known).  Batches of any size can be
- * predicted; the hint settles the launch shape in advance and, for a few trees over rows
- * of several hundred features, which layout pays. */
+ * predicted; the hint settles the launch shape in advance and which layout pays: for a few
+ * trees over 326 to 511 features fp32 tiles from 700 rows on; for rows of 512 to 2044
+ * features with at most 255 distinct thresholds each, one-byte ranks (with a hint of any
+ * size; without one rounded keys).  Leaf selection is the same in every layout. */
 TBK_EXPORT int tbk_forest_create(const tbk_forest_arrays *forest, const tbk_schedule *schedule,
                                  int32_t device, int64_t batch_hint, tbk_forest **out);
 
-/* The two halves of tbk_forest_create.  An image is the packed forest in host memory: the
+/* The two halves of tbk_forest_create without a batch_hint (the layout is settled by the first,
+ * which knows of no batches; the second's hint settles the launch shape only).  An image is the packed forest in host memory: the
  * layout chosen for it and that layout's buffers (what the reference's serializers build with
  * the host-side lowering of src/utils/TreeTilingUtils.cpp:427-556 before Init_* uploads them).
  * tbk_image_create needs no device: smem_limit is the shared memory per block the layout is
  * chosen for (0 = 227 KB, the B200 figure).  An image can be turned into bytes and back, which
  * is what a compiled-model file caches (the reference reloads its serialized buffers the same
  * way: src/utils/TreeTilingUtils.cpp:95-170, src/runtime/runtime.cpp:35-54); stale or damaged
- * bytes are refused with TBK_ERR_IO.  tbk_image_matches tells whether an image was packed for
+ * bytes are refused with TBK_ERR_IO, images that no kernel has a launch shape for with
+ * TBK_ERR_UNSUPPORTED.  tbk_image_matches tells whether an image was packed for
  * the same layout request (representation, tile size, feature bits of `schedule`; shared-memory
  * limit) and may therefore stand in for a fresh pack.  tbk_forest_create_from_image uploads it;
  * of `schedule` it takes the launch-shape fields, the layout is the image's. */

@@ -113,3 +113,13 @@ def test_twelve_levels(trees, features, rows, staged):
     assert_predictions_close(df.finalize(part).cpu().numpy()[some], want)
     if ids is not None:
         assert np.array_equal(ids[-300:].cpu().numpy(), want_ids[-300:])
+
+
+@pytest.mark.parametrize("features,twice", [(30, True), (600, False)])
+def test_resident_bytes_count_both_orders_of_the_planes(features, twice):
+    f = synth.generate_forest(2, 5, 10, features, 0.0, 0.1, synth.Marginal("normal", features))
+    words = lambda levels: ((2 ** levels - 1) + (2 ** levels - 1) // 32 + (2 ** levels - 1) // 1024 + 4) // 4 * 4
+    df = kernels.DeviceForest(f, representation="auto")
+    df.predict(torch.zeros((100, features), device="cuda"))
+    assert _staged(df) == twice
+    assert df.info().packed_bytes == 6 * (8 * words(10) + (16 * words(9) if twice else 0))

@@ -1744,8 +1744,8 @@ bool few_trees(int num_features, int64_t num_trees, int max_depth, int64_t batch
 // 170 shapes (520 to 2018 features, 100 to 1500 trees of 6 to 8 levels, 1024 to 262144 rows) none is slower by more than 3 %; microseconds
 // on rounded keys and on ranks: 300 trees of 6 levels x 520 features 34.9 / 11.8, 55.0 / 19.6, 241.5 / 85.1 for 1024, 8192 and 65536
 // rows; 600 trees of 8 levels x 1600 features 40.5 / 14.8, 66.3 / 42.7, 282 / 263; 800 x 1750 394 / 294 and 1000 x 2000 370 / 355 at
-// 65536 rows, 1422 / 1401 at 262144 (1076 / 1085 at 200000).  Preparation takes up to 5 ms longer (rank tables: 1500 features x 1000 trees 11.3 -> 16.6 ms, 2000 x 1000
-// 14.3 -> 15.5, 520 x 100 2.0 -> 2.3), as much as 30 to 300 calls gain.
+// 65536 rows, 1422 / 1401 at 262144 (1076 / 1085 at 200000).  Preparation takes as long in a warm process (1000 trees of 8 levels x 2000
+// features 13.9 / 13.4 ms, 400 x 1000 9.1 / 8.7, 100 of 6 levels x 520 2.1 / 2.8); a process's first forest up to 20 ms longer (95 MB for keys).
 bool byte_ranks(int64_t batch_hint) { return batch_hint > 0; }
 
 } // namespace
@@ -2322,7 +2322,8 @@ int tbk_forest_get_info(const tbk_forest *f, tbk_forest_info *info) {
   info->num_nodes = p.num_nodes;
   info->num_groups = f->lanes ? p.num_trees : f->rank ? (int64_t)f->rf.groups.size() : f->quant ? (int64_t)f->qf.groups.size() : f->deep ? (int64_t)f->df.pairs.size() : (int64_t)p.groups.size();
   info->packed_bytes = f->lanes ? 8 * p.num_nodes : f->rank ? (int64_t)(8 * (f->rf.groups.back().elem_off + (uint64_t)f->rf.groups.back().slots * tb::kRankCols)) :
-                       f->deep ? (int64_t)(f->df.pairs.empty() ? 0 : 8 * (f->df.pairs.back().elem_off + 2ull * f->df.pairs.back().slots)) :
+                       f->deep ? (int64_t)(f->df.pairs.empty() ? 0 : 8 * (f->df.pairs.back().elem_off + 2ull * f->df.pairs.back().slots)
+                                                                          + (f->d_qsplit ? 32 * f->df.pairs.size() * deep_half_words(f->uniform_depth) : 0)) :
                        f->quant ? (int64_t)(f->qf.groups.empty() ? 0 : 8 * (f->qf.groups.back().elem_off + (uint64_t)f->qf.groups.back().slots * tb::kQuantCols)) :
                        p.groups.empty() ? 0 : (int64_t)(p.groups.back().byte_off +
       (((uint64_t)p.groups.back().slots * tb::kGroupTrees * p.tile_bytes + 15) & ~15ull));
