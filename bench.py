@@ -31,15 +31,15 @@ from treebeard_b200 import synth  # noqa: E402
 
 HBM_FALLBACK_GBS = 6650.0
 
-# DRAM bytes per row (dram__bytes_read.sum + dram__bytes_write.sum) of the walk kernel (c2, c4: of the
-# ranking kernel as well), from one ncu capture per workload on the full or a reduced batch (see profiles/); traffic grows in
+# DRAM bytes per row (dram__bytes_read.sum + dram__bytes_write.sum) of the walk kernel and the
+# ranking kernel, from one ncu capture per workload on the full or a reduced batch (see profiles/); traffic grows in
 # proportion to the rows, so a launch's traffic is this figure times its rows.  Each figure
 # belongs to the kernel sources it was captured on: it is reported only while the hash of the
 # code of the headers that make up the workload's kernel (kernel_source_hash) still matches.
-KERNEL_SOURCES = {"c3": ("walk_kernels.cuh", "walk_quant.cuh"),
+KERNEL_SOURCES = {"c3": ("walk_quant.cuh", "rank_rows.cuh", "rank_slabs.cuh", "walk_rank.cuh", "walk_rank_tiles.cuh"),
                   "c2": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh"),
                   "c4": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh")}
-NCU_DRAM_BYTES_PER_ROW = {"c3": (8686.3, "271f001d05daf2aa"), "c2": (231.6, "37628a43f4e8c957"), "c4": (145.0, "37628a43f4e8c957")}
+NCU_DRAM_BYTES_PER_ROW = {"c3": (11990.0, "627b26d1568a06c1"), "c2": (231.7, "35b0f2b5a71aa533"), "c4": (146.5, "35b0f2b5a71aa533")}
 
 
 def kernel_source_hash(workload):

@@ -34,7 +34,7 @@ struct PackedImage {
   LaneForest lf;       // kLanes
 };
 
-constexpr uint32_t kPackedImageVersion = 10; // changes whenever a packer's output does
+constexpr uint32_t kPackedImageVersion = 10; // changes whenever images packed before would be read wrongly
 
 void serialize_image(const PackedImage &im, std::vector<uint8_t> *out);
 uint64_t serialized_image_size(const PackedImage &im); // without serialising

@@ -1258,7 +1258,7 @@ int run_rank(tbk_forest *f, Mode mode, const float *d_rows, int64_t n_rows, int6
   int64_t pass = std::min(n_rows, rank_rows_per_pass(f));
   RankPlan plan = plan_rank(f, pass, mode == kLeafIds);
   if (plan.chunks > 1) {
-    pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * 64); // (units of at least 80 rows)
+    pass = std::min<int64_t>(pass, (int64_t)tb::kRankArrivals * 64); // (units of at least 64 rows)
     plan = plan_rank(f, pass, mode == kLeafIds);
   }
   while (fixed && rank_workspace_bytes(f, plan, pass) > fixed_bytes) { // (128 rows always fit)

@@ -14,8 +14,8 @@
 //
 // The kernel is bound by latency and, since nothing else waits any more, the shared-memory pipe: 71 % busy, issue
 // 50 %, 53.3 wavefronts per walk of 32 rows through 12 levels (24 loads, 4 of bank conflicts of nodes, 23 of leaf
-// values; 85248 rows, one wave of 18 row warps, x 400 trees).  (Where all pairs have one depth and features are few
-// enough, tb_walk_deep_staged_kernel has the leaf values cheaper.)  A warp that stops for anything but its two chains stops
+// values; 85248 rows, one wave of 18 row warps, x 400 trees).  (Where all pairs have one depth, tb_walk_deep_staged_kernel
+// has the leaf values cheaper.)  A warp that stops for anything but its two chains stops
 // the others two pairs later, so nothing in the loop waits for global memory: leaf values are copied to
 // shared memory asynchronously (as loads, every pair waited some 600 of 2970 clocks for them, however
 // far ahead they were issued), and a tree behind a key tie is put off until the row's other
@@ -413,10 +413,11 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) tb_walk_deep_kernel(const Deep
 //   L  two half planes, the leaves to the left and to the right of these nodes.
 // A pair takes four ring slots of two planes each: A of both trees, B of both, L of the first, L of the second; five slots
 // keep the copy of every piece about a pair ahead of its use.
-// 85248 rows x 400 trees of 12 levels over 128 features: 53.3 -> 35.2 wavefronts per 32 rows and tree, pipe 71 -> 49 % busy,
-// 282 -> 268 us; 1048576 rows x 2000 trees 15.15 -> 14.30 ms; 100000 rows x 500 trees of 10 levels over 30 features, 30 row
-// warps, 387 -> 282 us.  (Both L of a pair are looked for at once: 14.55 ms and 296 us one after the other; with B 14.62 and 269.)  Bound: the chain of a walk, about 100 clocks a level, times too few of them: two trees of 18 row warps
-// are what fits.  (Leaf values as plain loads, consumed a pair later: 15.9 ms, but 304 us at 30 features.)
+// 85248 rows x 400 trees of 12 levels over 128 features: 53.3 -> 35.2 wavefronts per 32 rows and tree, pipe 71 -> 50 % busy,
+// 252 -> 251 us; 1048576 rows x 2000 trees 15.05 -> 14.52 ms; 100000 rows x 500 trees of 10 levels over 30 features
+// 306 -> 285 us.  Where it is not the faster one, and why: deep_staged_pays (tbk_api.cu).  (Both L of a pair are looked for at once: 14.55
+// instead of 14.30 ms one after the other; with B 14.62.)  Bound: the chain of a walk, about 100 clocks a level, times too few of them: two trees of 18 row warps
+// are what fits.  (Leaf values as plain loads, consumed a pair later: 15.9 ms.)
 struct DeepStagedParams : DeepParams {
   const uint32_t *split; // per pair: A0 A1 B0 B1 L0 (left, right) L1 (left, right)
 };

@@ -11,7 +11,7 @@
 // levels costs 15.75 wavefronts per 32 rows.  Sums stay in the lane that owns the row.
 //
 // Rows of more than 511 features have keys of one byte: line m holds in word j the keys of features 4m .. 4m+3 of row j,
-// so that four tiles fit up to about 1000 features under 8 levels (1600 under 6), and pairs of tiles up to 2018.  A pair with
+// so that four tiles fit up to about 1000 features under 8 levels (1600 under 6), and pairs of tiles up to 2024 (2044 under 7 levels and fewer).  A pair with
 // rows of 2000 features leaves three ring slots of 32 KB: 18944 rows x 1000 trees of 8 levels take 70 us, 17.4 wavefronts and
 // 68 instructions per 32 rows and tree, pipe 53 % and issue 55 % busy -- every group's 64 KB are asked for only once the group
 // before is walked.  (Walking four groups before looking up their leaf values, with node planes two ahead: 82 us; 8 warps of
