@@ -39,7 +39,7 @@ HBM_FALLBACK_GBS = 6650.0
 KERNEL_SOURCES = {"c3": ("walk_quant.cuh", "rank_rows.cuh", "rank_slabs.cuh", "walk_rank.cuh", "walk_rank_tiles.cuh"),
                   "c2": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh"),
                   "c4": ("walk_quant.cuh", "rank_rows.cuh", "walk_rank.cuh")}
-NCU_DRAM_BYTES_PER_ROW = {"c3": (11990.0, "627b26d1568a06c1"), "c2": (231.7, "35b0f2b5a71aa533"), "c4": (146.5, "35b0f2b5a71aa533")}
+NCU_DRAM_BYTES_PER_ROW = {"c3": (11982.8, "1abcc30db307f081"), "c2": (233.4, "2999505a50a9b136"), "c4": (145.3, "2999505a50a9b136")}
 
 
 def kernel_source_hash(workload):
